@@ -397,7 +397,27 @@ RCM_HD void log_tab(int j, double& invc, double& lead, double& trail) {
 #endif
 }
 
-RCM_HD double exp(double x) {
+// The multiplications that are not part of an FMA go through Mul::mul (a
+// correctly rounded multiplication), so that a caller can have them done by
+// another unit; the results do not depend on it.
+struct HwMul {
+  static RCM_HD double mul(double a, double b) { return a * b; }
+};
+
+// e as a double, |e| < 2^24
+RCM_HD double small_int(int e) {
+#ifdef __CUDA_ARCH__
+  // through FP32 and the bit pattern: the FP64 conversion holds the FP64 unit
+  const uint32_t u = __float_as_uint(__int2float_rn(e));
+  const uint32_t h = ((u & 0x7fffffffu) >> 3) + 0x38000000u;
+  return e == 0 ? 0.0 : __hiloint2double((int)(h | (u & 0x80000000u)), (int)(u << 29));
+#else
+  return (double)e;
+#endif
+}
+
+template <class Mul>
+RCM_HD double exp_with(double x) {
   const int64_t b = bits(x);
   if ((b & ABS_MASK) > INF_BITS) return x;                 // NaN
   if (b > EXP_HI_BITS) return HUGE_VAL;                    // x > 709.782712893384
@@ -410,7 +430,7 @@ RCM_HD double exp(double x) {
   r = fma_(-kd, LN2_128_LO, r);
   // e^r - 1 = r + r^2 (1/2 + r/6 + r^2/24 + r^3/120); the first omitted
   // term is below 2^-60
-  const double r2 = r * r;
+  const double r2 = Mul::mul(r, r);
   double q = fma_(1.0 / 120.0, r, 1.0 / 24.0);
   q = fma_(q, r, 1.0 / 6.0);
   q = fma_(q, r, 0.5);
@@ -419,12 +439,16 @@ RCM_HD double exp(double x) {
   exp_tab(k & 127, th, tl);
   const double y = th + fma_(th, p, tl);  // 2^(j/128) e^r, in [0.99, 2)
   const int m = k >> 7;
+#ifdef __CUDA_ARCH__
+  if (m >= -1020 && m <= 1022) return from_bits(bits(y) + ((int64_t)m << 52));  // y * 2^m, exactly
+#endif
   if (m >= -1022 && m <= 1023) return y * pow2i(m);
   const int m1 = m / 2;  // subnormal or near-overflow results: two exact factors
   return (y * pow2i(m1)) * pow2i(m - m1);
 }
 
-RCM_HD double log(double x) {
+template <class Mul>
+RCM_HD double log_with(double x) {
   int64_t b = bits(x);
   if ((b & ABS_MASK) > INF_BITS) return x;                                    // NaN
   if (b <= 0)                                                                 // x <= 0 (incl. -0)
@@ -446,12 +470,12 @@ RCM_HD double log(double x) {
   log_tab(j, invc, lh, ll);
   // log x = e ln2 - log(invc) + log1p(r), r = z invc - 1, |r| <= 2^-8
   const double r = fma_(z, invc, -1.0);
-  const double ed = (double)e;
+  const double ed = small_int(e);
   const double t1 = fma_(ed, LN2_HI42, lh);  // exact
   const double lo = fma_(ed, LN2_LO42, ll);
   // log1p(r) - r = r^2 (-1/2 + r/3 - r^2/4 + r^3/5 - r^4/6 + r^5/7); the first
   // omitted term is below 2^-67
-  const double r2 = r * r;
+  const double r2 = Mul::mul(r, r);
   double q = fma_(1.0 / 7.0, r, -1.0 / 6.0);
   q = fma_(q, r, 1.0 / 5.0);
   q = fma_(q, r, -0.25);
@@ -465,15 +489,25 @@ RCM_HD double log(double x) {
 }
 
 // x > 0 (the reference only takes powers of positive quantities)
-RCM_HD double pow(double x, double y) {
+// with L = log(x) given (used for x > 0, x != 1)
+template <class Mul>
+RCM_HD double pow_log(double x, double y, double L) {
   const int64_t bx = bits(x), by = bits(y);
   if (bx == 0x3ff0000000000000LL || (by & ABS_MASK) == 0) return 1.0;  // x == 1 or y == 0
   if ((bx & ABS_MASK) == 0) return (by > 0 && (by & ABS_MASK) <= INF_BITS) ? 0.0 : HUGE_VAL;  // x == 0
-  const double L = log(x);
-  const double t = y * L;
+  const double t = Mul::mul(y, L);
   const double terr = fma_(y, L, -t);
-  const double p = exp(t);
+  const double p = exp_with<Mul>(t);
   return fma_(p, terr, p);
 }
+
+template <class Mul>
+RCM_HD double pow_with(double x, double y) {
+  return pow_log<Mul>(x, y, log_with<Mul>(x));
+}
+
+RCM_HD double exp(double x) { return exp_with<HwMul>(x); }
+RCM_HD double log(double x) { return log_with<HwMul>(x); }
+RCM_HD double pow(double x, double y) { return pow_with<HwMul>(x, y); }
 
 }  // namespace rcm

@@ -23,31 +23,30 @@ __device__ __forceinline__ int next_chunk(unsigned* counter) {
 // Integrated source of cell i (sourceterm.f90:43-51 with omega replaced by
 // the mean rate over the cell's pseudo time step):
 //   src_k = vol * (rho * ((Y_k(step) - Y_k) / step)).
-template <int NSP>
+template <int NSP, class N>
 __device__ __forceinline__ void integrate_cell(const Dev& d, const ThermoDev<NSP>& th, int i, double tol, int maxsub,
                                                int* nsub, unsigned& err) {
   constexpr int V = 3 + NSP;
   const int NE = d.NE;
-  double P[V], P0[V], Y[NSP], Cp, gama, Rcpcv;
+  N P[V], P0[V], Y[NSP], Cp, gama, Rcpcv;
 #pragma unroll
   for (int k = 0; k < V; ++k) { P[k] = d.PA[k * NE + i]; P0[k] = P[k]; }
-  double s = 0.0;
 #pragma unroll
-  for (int k = 0; k < NSP - 1; ++k) { Y[k] = P[4 + k]; s = s + Y[k]; }
-  Y[NSP - 1] = 1.0 - s;
+  for (int k = 0; k < NSP - 1; ++k) Y[k] = P[4 + k];
+  Y[NSP - 1] = last_y<NSP>(Y);
   gas<NSP>(th, Y, P[3], Cp, gama, Rcpcv, err);
-  const double rho = P[0] / (P[3] * Rcpcv);
-  const double dt = d.step[i];
+  const N rho = P[0] / (P[3] * Rcpcv);
+  const N dt = d.step[i];
   nsub[i] = chem_integrate<NSP>(th, P, dt, tol, maxsub, err);
   const double vol = d.vol[i];
 #pragma unroll
-  for (int k = 0; k < NSP - 1; ++k) d.src[k * NE + i] = vol * (rho * ((P[4 + k] - P0[4 + k]) / dt));
+  for (int k = 0; k < NSP - 1; ++k) d.src[k * NE + i] = val(vol * (rho * ((P[4 + k] - P0[4 + k]) / dt)));
 }
 
 // Cells are taken in `order` (longest previous integration first, so the long
 // cells start early and warps hold cells of similar cost), or in cell order
 // when order is null.
-template <int NSP>
+template <int NSP, class N>
 __global__ void __launch_bounds__(CHEM_THREADS) k_chem_source(const Dev d, const ThermoDev<NSP> th, double tol,
                                                               int maxsub, int* __restrict__ nsub,
                                                               const int* __restrict__ order, unsigned* counter) {
@@ -57,7 +56,7 @@ __global__ void __launch_bounds__(CHEM_THREADS) k_chem_source(const Dev d, const
     const int base = next_chunk(counter);
     if (base >= NE) break;
     const int q = base + (threadIdx.x & 31);
-    if (q < NE) integrate_cell<NSP>(d, th, order ? order[q] : q, tol, maxsub, nsub, err);
+    if (q < NE) integrate_cell<NSP, N>(d, th, order ? order[q] : q, tol, maxsub, nsub, err);
   }
   flag(d, err);
 }
@@ -88,7 +87,7 @@ __global__ void k_chem_scatter(const int* __restrict__ nsub, int n, unsigned* cu
 }
 
 // The same for the cells list[0 .. *nlist) (the surrogate's fallbacks).
-template <int NSP>
+template <int NSP, class N>
 __global__ void __launch_bounds__(CHEM_THREADS) k_chem_list(const Dev d, const ThermoDev<NSP> th, double tol,
                                                             int maxsub, int* __restrict__ nsub,
                                                             const int* __restrict__ list,
@@ -99,13 +98,13 @@ __global__ void __launch_bounds__(CHEM_THREADS) k_chem_list(const Dev d, const T
     const int base = next_chunk(counter);
     if (base >= n) break;
     const int q = base + (threadIdx.x & 31);
-    if (q < n) integrate_cell<NSP>(d, th, list[q], tol, maxsub, nsub, err);
+    if (q < n) integrate_cell<NSP, N>(d, th, list[q], tol, maxsub, nsub, err);
   }
   flag(d, err);
 }
 
 // n primitive states in SoA ([k*n + i]) integrated over dt[i].
-template <int NSP>
+template <int NSP, class N>
 __global__ void __launch_bounds__(CHEM_THREADS) k_chem_batch(const ThermoDev<NSP> th, const double* __restrict__ Pin,
                                                              const double* __restrict__ dts, int n,
                                                              double* __restrict__ Pout, int* __restrict__ nsub,
@@ -118,12 +117,12 @@ __global__ void __launch_bounds__(CHEM_THREADS) k_chem_batch(const ThermoDev<NSP
     if (base >= n) break;
     const int i = base + (threadIdx.x & 31);
     if (i < n) {
-      double P[V];
+      N P[V];
 #pragma unroll
       for (int k = 0; k < V; ++k) P[k] = Pin[(size_t)k * n + i];
-      nsub[i] = chem_integrate<NSP>(th, P, dts[i], tol, maxsub, err);
+      nsub[i] = chem_integrate<NSP, N>(th, P, dts[i], tol, maxsub, err);
 #pragma unroll
-      for (int k = 0; k < V; ++k) Pout[(size_t)k * n + i] = P[k];
+      for (int k = 0; k < V; ++k) Pout[(size_t)k * n + i] = val(P[k]);
     }
   }
   if (err) atomicOr(errp, err);
@@ -152,27 +151,28 @@ void chem_source(const Dev& d, const void* th, double tol, int maxsub, int* nsub
     k_chem_scan<<<1, NBUCKET, 0, s>>>(hist);
     k_chem_scatter<<<nb, 256, 0, s>>>(nsub, d.NE, hist, order);
   }
-  const int grid = chem_grid(k_chem_source<NSP>, d.NE);
+  auto k = k_chem_source<NSP, double>;
+  const int grid = chem_grid(k, d.NE);
   cudaMemsetAsync(counter, 0, sizeof(unsigned), s);
-  k_chem_source<NSP><<<grid, CHEM_THREADS, 0, s>>>(d, *static_cast<const ThermoDev<NSP>*>(th), tol, maxsub, nsub,
-                                                   order, counter);
+  k<<<grid, CHEM_THREADS, 0, s>>>(d, *static_cast<const ThermoDev<NSP>*>(th), tol, maxsub, nsub, order, counter);
 }
 
 template <int NSP>
 void chem_list(const Dev& d, const void* th, double tol, int maxsub, int* nsub, const int* list,
                const unsigned* nlist, unsigned* counter, cudaStream_t s) {
-  const int grid = chem_grid(k_chem_list<NSP>, d.NE);
+  auto k = k_chem_list<NSP, double>;
+  const int grid = chem_grid(k, d.NE);
   cudaMemsetAsync(counter, 0, sizeof(unsigned), s);
-  k_chem_list<NSP><<<grid, CHEM_THREADS, 0, s>>>(d, *static_cast<const ThermoDev<NSP>*>(th), tol, maxsub, nsub, list,
-                                                 nlist, counter);
+  k<<<grid, CHEM_THREADS, 0, s>>>(d, *static_cast<const ThermoDev<NSP>*>(th), tol, maxsub, nsub, list, nlist, counter);
 }
 
 template <int NSP>
 void chem_batch(const void* th, const double* P, const double* dt, int n, double* out, int* nsub, double tol,
                 int maxsub, unsigned* counter, unsigned* errp, cudaStream_t s) {
   cudaMemsetAsync(counter, 0, sizeof(unsigned), s);
-  const int grid = chem_grid(k_chem_batch<NSP>, n);
-  k_chem_batch<NSP><<<grid, CHEM_THREADS, 0, s>>>(*static_cast<const ThermoDev<NSP>*>(th), P, dt, n, out, nsub, tol,
+  auto k = k_chem_batch<NSP, double>;
+  const int grid = chem_grid(k, n);
+  k<<<grid, CHEM_THREADS, 0, s>>>(*static_cast<const ThermoDev<NSP>*>(th), P, dt, n, out, nsub, tol,
                                                   maxsub, counter, errp);
 }
 

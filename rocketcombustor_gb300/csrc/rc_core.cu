@@ -40,59 +40,57 @@ namespace rc {
 
 // oxidizer_inlet_bc / fuel_inlet_bc (oxidizer.f90:53-68, fuel.f90:54-69)
 // with the inlet data of row bc of the case table (w = 0 oxidizer, 1 fuel).
-template <int NSP>
-__device__ __forceinline__ void inlet_bc(const ThermoDev<NSP>& th, const double* bc, int w, double pl, double& pr,
-                                         double& ur, double& vr, double& tr, double& rr, double* Yr, double& Cpr,
-                                         double& gamar, double& Rcpcvr, unsigned& err) {
+template <int NSP, class N>
+__device__ __forceinline__ void inlet_bc(const ThermoDev<NSP>& th, const double* bc, int w, N pl, N& pr, N& ur,
+                                         N& vr, N& tr, N& rr, N* Yr, N& Cpr, N& gamar, N& Rcpcvr, unsigned& err) {
 #pragma unroll
   for (int k = 0; k < NSP; ++k) Yr[k] = bc[BC_Y + w * BC_NSPMAX + k];
   tr = bc[BC_T + w];
   gas<NSP>(th, Yr, tr, Cpr, gamar, Rcpcvr, err);
   pr = pl;
   rr = pr / (Rcpcvr * tr);
-  ur = bc[BC_MFLOW + w] / rr;
+  ur = N(bc[BC_MFLOW + w]) / rr;
   vr = 0.0;
 }
 
 // ----------------------------------------------------------- TimeStep ------
-template <int NSP, bool VISC>
+template <int NSP, bool VISC, class N>
 __global__ void __launch_bounds__(128) k_ts_face(const Dev d, const ThermoDev<NSP> th) {
   constexpr int V = 3 + NSP;
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= d.NF) return;
   unsigned err = 0;
   const int NE = d.NE, NL = d.fNL[f], NR = d.fNR[f];
-  double P[V], yy[NSP];
+  N P[V], yy[NSP];
   if (NR >= 0) {
 #pragma unroll
-    for (int k = 0; k < V; ++k) P[k] = 0.5 * (d.PA[k * NE + NL] + d.PA[k * NE + NR]);
+    for (int k = 0; k < V; ++k) P[k] = half_of(N(d.PA[k * NE + NL]) + d.PA[k * NE + NR]);
   } else {
 #pragma unroll
     for (int k = 0; k < V; ++k) P[k] = d.PA[k * NE + NL];
   }
-  double s = 0.0;
 #pragma unroll
-  for (int k = 0; k < NSP - 1; ++k) { yy[k] = P[4 + k]; s = s + yy[k]; }
-  yy[NSP - 1] = 1.0 - s;
-  const double pp = P[0], uu = P[1], vv = P[2], tt = P[3];
-  double Cp, gama, Rcpcv;
+  for (int k = 0; k < NSP - 1; ++k) yy[k] = P[4 + k];
+  yy[NSP - 1] = last_y<NSP>(yy);
+  const N pp = P[0], uu = P[1], vv = P[2], tt = P[3];
+  N Cp, gama, Rcpcv;
   gas<NSP>(th, yy, tt, Cp, gama, Rcpcv, err);
-  const double rr = pp / (Rcpcv * tt);
-  if (rr < 0. || pp < 0. || tt < 0.) err |= ERR_NEG_TIMESTEP;
-  const double unormal = uu * d.fvec[f] + vv * d.fvec[d.NF + f];
-  const double alpa = fabs(unormal) + sqrt(gama * pp / rr) * d.fss[f];
-  d.alpa[f] = alpa;
+  const N rr = pp / (Rcpcv * tt);
+  if (negative(rr) || negative(pp) || negative(tt)) err |= ERR_NEG_TIMESTEP;
+  const N unormal = uu * d.fvec[f] + vv * d.fvec[d.NF + f];
+  const N alpa = n_abs(unormal) + n_sqrt(gama * pp / rr) * d.fss[f];
+  d.alpa[f] = val(alpa);
   if (VISC) {
-    double vmul, akmu;
+    N vmul, akmu;
     transport<NSP>(th, tt, yy, vmul, akmu, err);
-    const double prl = vmul * Cp / akmu;
-    const double alpaVis = 2. * d.fs2[f] * fmax2(4. / 3., gama / prl) * vmul / rr;
-    const double vl = alpaVis / d.vol[NL];
-    d.visL[f] = vl;
-    d.visR[f] = (NR >= 0) ? alpaVis / d.vol[NR] : 0.0;
-    d.alpaF[f] = alpa + vl;
+    const N prl = vmul * Cp / akmu;
+    const N alpaVis = twice_of(N(d.fs2[f])) * fmax2(N(4. / 3.), gama / prl) * vmul / rr;
+    const N vl = alpaVis / N(d.vol[NL]);
+    d.visL[f] = val(vl);
+    d.visR[f] = (NR >= 0) ? val(alpaVis / N(d.vol[NR])) : 0.0;
+    d.alpaF[f] = val(alpa + vl);
   } else {
-    d.alpaF[f] = alpa;
+    d.alpaF[f] = val(alpa);
   }
   flag(d, err);
 }
@@ -101,7 +99,7 @@ __global__ void __launch_bounds__(128) k_ts_face(const Dev d, const ThermoDev<NS
 // step/dd (TimeStep.f90:94-96, Time_LUSGS_steady.f90:46-53), ghost states
 // (update_flow_variables.f90:90-269), gradient (gradient.f90:4-45), Barth
 // limiter (limiter.f90:5-107), cell gas state and source (sourceterm.f90:2-70).
-template <int NSP>
+template <int NSP, class N>
 __global__ void __launch_bounds__(128) k_cell(const Dev d, const ThermoDev<NSP> th, int do_step, int do_recon,
                                               int limit, int comb, int visc) {
   constexpr int V = 3 + NSP;
@@ -113,49 +111,46 @@ __global__ void __launch_bounds__(128) k_cell(const Dev d, const ThermoDev<NSP> 
   const double vol = d.vol[i];
   if (do_step) {
     const unsigned lb = d.cleft[i];
-    double acc = 0.0;
+    N acc = 0.0;
     for (int q = 0; q < nf; ++q) {
       const int f = d.cface[q * NE + i];
       if (visc) acc = acc + d.alpa[f] + (((lb >> q) & 1u) ? d.visL[f] : d.visR[f]);
       else acc = acc + d.alpa[f];
     }
-    const double st = th.cfl * vol / acc;
-    double dsum = 0.0;
-    for (int q = 0; q < nf; ++q) dsum = dsum + 0.5 * d.alpaF[d.cface[q * NE + i]];
-    d.step[i] = st;
-    const double ddv = dsum + vol / st;
-    d.dd[i] = ddv;
-    const Recip rd = recip_of(ddv);
+    const N st = N(th.cfl) * vol / acc;
+    N dsum = 0.0;
+    for (int q = 0; q < nf; ++q) dsum = dsum + half_of(d.alpaF[d.cface[q * NE + i]]);
+    d.step[i] = val(st);
+    const N ddv = dsum + N(vol) / st;
+    d.dd[i] = val(ddv);
+    const Recip rd = recip(ddv);
     d.rcp[4 * NE + i] = rd.h;
     d.rcp[5 * NE + i] = rd.l;
   }
   if (!do_recon) { flag(d, err); return; }
-  double P[V], Y[NSP];
+  N P[V], Y[NSP];
 #pragma unroll
   for (int k = 0; k < V; ++k) P[k] = d.PA[k * NE + i];
-  double s = 0.0;
 #pragma unroll
-  for (int k = 0; k < NSP - 1; ++k) { Y[k] = P[4 + k]; s = s + Y[k]; }
-  Y[NSP - 1] = 1.0 - s;
-  double Cp, gama, Rcpcv, entha[NSP];
+  for (int k = 0; k < NSP - 1; ++k) Y[k] = P[4 + k];
+  Y[NSP - 1] = last_y<NSP>(Y);
+  N Cp, gama, Rcpcv, entha[NSP];
   gas<NSP>(th, Y, P[3], Cp, gama, Rcpcv, err);
-  const double rr = P[0] / (Rcpcv * P[3]);
+  const N rr = P[0] / (Rcpcv * P[3]);
   enthalpy<NSP>(th, P[3], entha, err);
-  double hh = 0.0;
-#pragma unroll
-  for (int k = 0; k < NSP; ++k) hh = hh + Y[k] * entha[k];
-  d.cst[0 * NE + i] = rr;
-  d.cst[1 * NE + i] = gama;
+  const N hh = dot<NSP>(Y, entha);
+  d.cst[0 * NE + i] = val(rr);
+  d.cst[1 * NE + i] = val(gama);
   {
-    const Recip a = recip_of(rr), b = recip_of(gama - 1);
+    const Recip a = recip(rr), b = recip(gama - 1.0);
     d.rcp[0 * NE + i] = a.h; d.rcp[1 * NE + i] = a.l; d.rcp[2 * NE + i] = b.h; d.rcp[3 * NE + i] = b.l;
   }
-  d.cst[2 * NE + i] = rr * (hh + 0.5 * (P[1] * P[1] + P[2] * P[2])) - P[0];
+  d.cst[2 * NE + i] = val(rr * (hh + half_of(P[1] * P[1] + P[2] * P[2])) - P[0]);
 #pragma unroll
-  for (int k = 0; k < NSP; ++k) d.cst[(3 + k) * NE + i] = entha[k];
+  for (int k = 0; k < NSP; ++k) d.cst[(3 + k) * NE + i] = val(entha[k]);
 
   // gradient with running min/max of the stencil
-  double g0[V], g1[V], mn[V], mx[V];
+  N g0[V], g1[V], mn[V], mx[V];
 #pragma unroll
   for (int k = 0; k < V; ++k) { g0[k] = 0.0; g1[k] = 0.0; mn[k] = P[k]; mx[k] = P[k]; }
   const int nn = d.nnei[i];
@@ -164,8 +159,8 @@ __global__ void __launch_bounds__(128) k_cell(const Dev d, const ThermoDev<NSP> 
     const double w = d.wdis[q * NE + i], a0 = d.amls[(2 * q) * NE + i], a1 = d.amls[(2 * q + 1) * NE + i];
 #pragma unroll
     for (int k = 0; k < V; ++k) {
-      const double x = d.PA[k * NE + j];
-      const double c = w * (x - P[k]);
+      const N x = d.PA[k * NE + j];
+      const N c = w * (x - P[k]);
       g0[k] = g0[k] + a0 * c;
       g1[k] = g1[k] + a1 * c;
       mn[k] = fmin2(mn[k], x);
@@ -176,10 +171,10 @@ __global__ void __launch_bounds__(128) k_cell(const Dev d, const ThermoDev<NSP> 
   for (int q = 0; q < ng; ++q) {
     const int gj = d.cgh[q * NE + i];
     const double s1n = d.gsn[gj], s2n = d.gsn[d.NG + gj];
-    const double pl = P[0], ul = P[1], vl = P[2], tl = P[3];
-    const double ac = sqrt(gama * pl / rr);
-    double G[V], Yr[NSP];
-    double pr = pl, ur = ul, vr = vl, tr = tl, vn;
+    const N pl = P[0], ul = P[1], vl = P[2], tl = P[3];
+    const N ac = n_sqrt(gama * pl / rr);
+    N G[V], Yr[NSP];
+    N pr = pl, ur = ul, vr = vl, tr = tl, vn;
 #pragma unroll
     for (int k = 0; k < NSP; ++k) Yr[k] = Y[k];
     switch (d.gtype[gj]) {
@@ -187,19 +182,19 @@ __global__ void __launch_bounds__(128) k_cell(const Dev d, const ThermoDev<NSP> 
       case 2:
       case 6:
         vn = ul * s1n + vl * s2n;
-        ur = ul - 2 * vn * s1n;
-        vr = vl - 2 * vn * s2n;
+        ur = ul - twice_of(vn) * s1n;
+        vr = vl - twice_of(vn) * s2n;
         break;
       case 3:
       case 4: {
-        double rrb, Cpb, gab, Rb;
+        N rrb, Cpb, gab, Rb;
         inlet_bc<NSP>(th, bc_row(d, d.gcase, gj), d.gtype[gj] == 3 ? 0 : 1, pl, pr, ur, vr, tr, rrb, Yr, Cpb, gab,
                       Rb, err);
         break;
       }
       case 5:
         vn = ul * s1n + vl * s2n;
-        if (!(fabs(vn) > ac)) pr = bc_row(d, d.gcase, gj)[BC_POUT];
+        if (!less(ac, n_abs(vn))) pr = bc_row(d, d.gcase, gj)[BC_POUT];
         break;
       default: err |= ERR_BCTYPE;
     }
@@ -207,12 +202,12 @@ __global__ void __launch_bounds__(128) k_cell(const Dev d, const ThermoDev<NSP> 
 #pragma unroll
     for (int k = 0; k < NSP - 1; ++k) G[4 + k] = Yr[k];
 #pragma unroll
-    for (int k = 0; k < V; ++k) d.GPA[k * d.NG + gj] = G[k];
+    for (int k = 0; k < V; ++k) d.GPA[k * d.NG + gj] = val(G[k]);
     const int m = nn + q;
     const double w = d.wdis[m * NE + i], a0 = d.amls[(2 * m) * NE + i], a1 = d.amls[(2 * m + 1) * NE + i];
 #pragma unroll
     for (int k = 0; k < V; ++k) {
-      const double c = w * (G[k] - P[k]);
+      const N c = w * (G[k] - P[k]);
       g0[k] = g0[k] + a0 * c;
       g1[k] = g1[k] + a1 * c;
       mn[k] = fmin2(mn[k], G[k]);
@@ -224,12 +219,12 @@ __global__ void __launch_bounds__(128) k_cell(const Dev d, const ThermoDev<NSP> 
     for (int q = 0; q < nf; ++q) { lv0[q] = d.lvvh[(2 * q) * NE + i]; lv1[q] = d.lvvh[(2 * q + 1) * NE + i]; }
 #pragma unroll
     for (int k = 0; k < V; ++k) {
-      double phi = 1.0;
+      N phi = 1.0;
       for (int q = 0; q < nf; ++q) {
-        const double fv = P[k] + (g0[k] * lv0[q] + g1[k] * lv1[q]);
-        double pf;
-        if (fv > P[k]) pf = fmin2(1.0, (mx[k] - P[k]) / (fv - P[k]));
-        else if (fv < P[k]) pf = fmin2(1.0, (mn[k] - P[k]) / (fv - P[k]));
+        const N fv = P[k] + (g0[k] * lv0[q] + g1[k] * lv1[q]);
+        N pf;
+        const bool up = less(P[k], fv);
+        if (up || less(fv, P[k])) pf = fmin2(N(1.0), ((up ? mx[k] : mn[k]) - P[k]) / (fv - P[k]));
         else pf = 1.0;
         phi = fmin2(phi, pf);
       }
@@ -239,29 +234,29 @@ __global__ void __launch_bounds__(128) k_cell(const Dev d, const ThermoDev<NSP> 
   }
 #pragma unroll
   for (int k = 0; k < V; ++k) {
-    d.grad[(2 * k) * NE + i] = g0[k];
-    d.grad[(2 * k + 1) * NE + i] = g1[k];
+    d.grad[(2 * k) * NE + i] = val(g0[k]);
+    d.grad[(2 * k + 1) * NE + i] = val(g1[k]);
   }
   if (comb) {
-    double prod[NSP];
+    N prod[NSP];
     production<NSP>(th, P[3], rr, Y, prod);
 #pragma unroll
-    for (int k = 0; k < NSP - 1; ++k) d.src[k * NE + i] = vol * prod[k];
+    for (int k = 0; k < NSP - 1; ++k) d.src[k * NE + i] = val(vol * prod[k]);
   }
   flag(d, err);
 }
 
 // ------------------------------------------------------------ face flux ----
-template <int NSP>
-__device__ __forceinline__ void recon(const Dev& d, int c, double v0, double v1, double* u) {
+template <int NSP, class N>
+__device__ __forceinline__ void recon(const Dev& d, int c, double v0, double v1, N* u) {
   constexpr int V = 3 + NSP;
   const int NE = d.NE;
 #pragma unroll
   for (int k = 0; k < V; ++k)
-    u[k] = d.PA[k * NE + c] + (d.grad[(2 * k) * NE + c] * v0 + d.grad[(2 * k + 1) * NE + c] * v1);
+    u[k] = d.PA[k * NE + c] + (N(d.grad[(2 * k) * NE + c]) * v0 + N(d.grad[(2 * k + 1) * NE + c]) * v1);
 }
 
-template <int NSP, bool VISC>
+template <int NSP, bool VISC, class N>
 __global__ void __launch_bounds__(128) k_face_flux(const Dev d, const ThermoDev<NSP> th) {
   constexpr int V = 3 + NSP;
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
@@ -271,22 +266,20 @@ __global__ void __launch_bounds__(128) k_face_flux(const Dev d, const ThermoDev<
   const int NL = d.fNL[f], NR = d.fNR[f];
   const double sav1 = d.fvec[f], sav2 = d.fvec[NF + f], sav = d.fsav[f];
   const double sav1n = d.fsn[f], sav2n = d.fsn[NF + f];
-  double uL[V], uR[V], Yl0[NSP], Yr0[NSP];
+  N uL[V], uR[V], Yl0[NSP], Yr0[NSP];
   recon<NSP>(d, NL, d.fvL[f], d.fvL[NF + f], uL);
-  double s = 0.0;
 #pragma unroll
-  for (int k = 0; k < NSP - 1; ++k) { Yl0[k] = uL[4 + k]; s = s + Yl0[k]; }
-  Yl0[NSP - 1] = 1.0 - s;
-  double Cpl0, gamal0, Rl0;
+  for (int k = 0; k < NSP - 1; ++k) Yl0[k] = uL[4 + k];
+  Yl0[NSP - 1] = last_y<NSP>(Yl0);
+  N Cpl0, gamal0, Rl0;
   gas<NSP>(th, Yl0, uL[3], Cpl0, gamal0, Rl0, err);
-  const double rl0 = uL[0] / (Rl0 * uL[3]);
-  double Cpr0 = 0.0, gamar0 = 0.0, Rr0 = 0.0, rr0 = 0.0;
+  const N rl0 = uL[0] / (Rl0 * uL[3]);
+  N Cpr0 = 0.0, gamar0 = 0.0, Rr0 = 0.0, rr0 = 0.0;
   if (NR >= 0) {
     recon<NSP>(d, NR, d.fvR[f], d.fvR[NF + f], uR);
-    s = 0.0;
 #pragma unroll
-    for (int k = 0; k < NSP - 1; ++k) { Yr0[k] = uR[4 + k]; s = s + Yr0[k]; }
-    Yr0[NSP - 1] = 1.0 - s;
+    for (int k = 0; k < NSP - 1; ++k) Yr0[k] = uR[4 + k];
+    Yr0[NSP - 1] = last_y<NSP>(Yr0);
     gas<NSP>(th, Yr0, uR[3], Cpr0, gamar0, Rr0, err);
     rr0 = uR[0] / (Rr0 * uR[3]);
   } else {
@@ -296,9 +289,9 @@ __global__ void __launch_bounds__(128) k_face_flux(const Dev d, const ThermoDev<
 
   // ---- Lax/Rusanov flux (flux_lax.f90:17-293)
   {
-    double pl = uL[0], ul = uL[1], vl = uL[2], tl = uL[3], rl = rl0, gamal = gamal0, Rcl = Rl0, Cpl = Cpl0;
-    double pr, ur, vr, tr, rr, gamar, Rcr, Cpr, vn;
-    double Yl[NSP], Yr[NSP];
+    N pl = uL[0], ul = uL[1], vl = uL[2], tl = uL[3], rl = rl0, gamal = gamal0, Rcl = Rl0, Cpl = Cpl0;
+    N pr, ur, vr, tr, rr, gamar, Rcr, Cpr, vn;
+    N Yl[NSP], Yr[NSP];
 #pragma unroll
     for (int k = 0; k < NSP; ++k) Yl[k] = Yl0[k];
     if (NR >= 0) {
@@ -316,12 +309,12 @@ __global__ void __launch_bounds__(128) k_face_flux(const Dev d, const ThermoDev<
       if (NR == -1) { ur = -ul; vr = -vl; }
       else if (NR == -2 || NR == -6) {
         vn = ul * sav1n + vl * sav2n;
-        ur = ul - 2 * vn * sav1n;
-        vr = vl - 2 * vn * sav2n;
+        ur = ul - twice_of(vn) * sav1n;
+        vr = vl - twice_of(vn) * sav2n;
       } else if (NR == -5) {
-        const double ac = sqrt(gamal * pl / rl);
+        const N ac = n_sqrt(gamal * pl / rl);
         vn = ul * sav1n + vl * sav2n;
-        if (!(fabs(vn) > ac)) {
+        if (!less(ac, n_abs(vn))) {
           pr = bc_row(d, d.fcase, f)[BC_POUT];
           ur = ul + sav1n * (pl - pr) / (rl * ac);
           vr = vl + sav2n * (pl - pr) / (rl * ac);
@@ -337,38 +330,34 @@ __global__ void __launch_bounds__(128) k_face_flux(const Dev d, const ThermoDev<
       gamar = gamal; Rcr = Rcl; Cpr = Cpl;
     }
     (void)Cpr; (void)Rcr; (void)Cpl;
-    if (rl < 0. || pl < 0. || (NR >= 0 && (rr < 0. || pr < 0.))) err |= ERR_NEG_FACE;
-    double entha[NSP];
+    if (negative(rl) || negative(pl) || (NR >= 0 && (negative(rr) || negative(pr)))) err |= ERR_NEG_FACE;
+    N entha[NSP];
     enthalpy<NSP>(th, tl, entha, err);
-    double hl = 0.0;
-#pragma unroll
-    for (int k = 0; k < NSP; ++k) hl = hl + Yl[k] * entha[k];
+    N hl = dot<NSP>(Yl, entha);
     enthalpy<NSP>(th, tr, entha, err);
-    double hr = 0.0;
-#pragma unroll
-    for (int k = 0; k < NSP; ++k) hr = hr + Yr[k] * entha[k];
-    const double vaml = ul * ul + vl * vl, vamr = ur * ur + vr * vr;
-    hl = hl + 0.5 * vaml;
-    hr = hr + 0.5 * vamr;
-    const double el = hl - pl / rl, er = hr - pr / rr;
-    const double acl = sqrt(gamal * pl / rl), acr = sqrt(gamar * pr / rr);
-    const double ulnormal = (sav1 * ul + sav2 * vl), urnormal = (sav1 * ur + sav2 * vr);
-    const double coex = fmax2(fabs(ulnormal) + acl * sav, fabs(urnormal) + acr * sav);
-    const double rul = rl * ulnormal, rur = rr * urnormal;
-    d.Finv[0 * NF + f] = 0.5 * (rul + rur - coex * (rr - rl));
-    d.Finv[1 * NF + f] = 0.5 * (rul * ul + rur * ur + sav1 * (pl + pr) - coex * (rr * ur - rl * ul));
-    d.Finv[2 * NF + f] = 0.5 * (rul * vl + rur * vr + sav2 * (pl + pr) - coex * (rr * vr - rl * vl));
-    d.Finv[3 * NF + f] = 0.5 * (rul * hl + rur * hr - coex * (rr * er - rl * el));
+    N hr = dot<NSP>(Yr, entha);
+    const N vaml = ul * ul + vl * vl, vamr = ur * ur + vr * vr;
+    hl = hl + half_of(vaml);
+    hr = hr + half_of(vamr);
+    const N el = hl - pl / rl, er = hr - pr / rr;
+    const N acl = n_sqrt(gamal * pl / rl), acr = n_sqrt(gamar * pr / rr);
+    const N ulnormal = (sav1 * ul + sav2 * vl), urnormal = (sav1 * ur + sav2 * vr);
+    const N coex = fmax2(n_abs(ulnormal) + acl * sav, n_abs(urnormal) + acr * sav);
+    const N rul = rl * ulnormal, rur = rr * urnormal;
+    d.Finv[0 * NF + f] = val(half_of(rul + rur - coex * (rr - rl)));
+    d.Finv[1 * NF + f] = val(half_of(rul * ul + rur * ur + sav1 * (pl + pr) - coex * (rr * ur - rl * ul)));
+    d.Finv[2 * NF + f] = val(half_of(rul * vl + rur * vr + sav2 * (pl + pr) - coex * (rr * vr - rl * vl)));
+    d.Finv[3 * NF + f] = val(half_of(rul * hl + rur * hr - coex * (rr * er - rl * el)));
 #pragma unroll
     for (int k = 0; k < NSP - 1; ++k)
-      d.Finv[(4 + k) * NF + f] = 0.5 * (rul * Yl[k] + rur * Yr[k] - coex * (rr * Yr[k] - rl * Yl[k]));
+      d.Finv[(4 + k) * NF + f] = val(half_of(rul * Yl[k] + rur * Yr[k] - coex * (rr * Yr[k] - rl * Yl[k])));
   }
 
   // ---- viscous flux (flux_viscous.f90:25-343)
   if (VISC) {
-    double pl = uL[0], ul = uL[1], vl = uL[2], tl = uL[3], rl = rl0;
-    double pr, ur, vr, tr;
-    double Yl[NSP], Yr[NSP];
+    N pl = uL[0], ul = uL[1], vl = uL[2], tl = uL[3], rl = rl0;
+    N pr, ur, vr, tr;
+    N Yl[NSP], Yr[NSP];
 #pragma unroll
     for (int k = 0; k < NSP; ++k) Yl[k] = Yl0[k];
     if (NR >= 0) {
@@ -376,23 +365,23 @@ __global__ void __launch_bounds__(128) k_face_flux(const Dev d, const ThermoDev<
 #pragma unroll
       for (int k = 0; k < NSP; ++k) Yr[k] = Yr0[k];
     } else if (NR == -3 || NR == -4) {
-      double rr, Cpr, gamar, Rcr;
+      N rr, Cpr, gamar, Rcr;
       inlet_bc<NSP>(th, bc_row(d, d.fcase, f), NR == -3 ? 0 : 1, pl, pr, ur, vr, tr, rr, Yr, Cpr, gamar, Rcr, err);
       pl = pr; ul = ur; vl = vr; tl = tr; rl = rr;
 #pragma unroll
       for (int k = 0; k < NSP; ++k) Yl[k] = Yr[k];
     } else {
       if (NR == -1) { ul = 0.; vl = 0.; }
-      else if (NR == -2 || NR == -6 || NR == -7) removedirection(ul, vl, sav1n, sav2n);
+      else if (NR == -2 || NR == -6 || NR == -7) removedirection(ul, vl, N(sav1n), N(sav2n));
       pr = pl; tr = tl; ur = ul; vr = vl;
       if (NR == -5) {
-        const double ac = sqrt(gamal0 * pl / rl);
-        const double vn = ul * sav1n + vl * sav2n;
-        if (!(fabs(vn) > ac)) {
+        const N ac = n_sqrt(gamal0 * pl / rl);
+        const N vn = ul * sav1n + vl * sav2n;
+        if (!less(ac, n_abs(vn))) {
           pr = bc_row(d, d.fcase, f)[BC_POUT];
           ur = ul + sav1n * (pl - pr) / (rl * ac);
           vr = vl + sav2n * (pl - pr) / (rl * ac);
-          const double rrb = rl + (pr - pl) / (ac * ac);
+          const N rrb = rl + (pr - pl) / (ac * ac);
           tr = pr / (Rl0 * rrb);
           pl = pr; ul = ur; vl = vr; tl = tr;
         }
@@ -403,47 +392,47 @@ __global__ void __launch_bounds__(128) k_face_flux(const Dev d, const ThermoDev<
       for (int k = 0; k < NSP; ++k) Yr[k] = Yl[k];
     }
     (void)rl;
-    const double pp = 0.5 * (pl + pr), uu = 0.5 * (ul + ur), vv = 0.5 * (vl + vr), tem = 0.5 * (tl + tr);
-    double YY[NSP];
+    const N pp = half_of(pl + pr), uu = half_of(ul + ur), vv = half_of(vl + vr), tem = half_of(tl + tr);
+    N YY[NSP];
 #pragma unroll
-    for (int k = 0; k < NSP; ++k) YY[k] = 0.5 * (Yl[k] + Yr[k]);
-    double Cp, gama, Rcpcv;
+    for (int k = 0; k < NSP; ++k) YY[k] = half_of(Yl[k] + Yr[k]);
+    N Cp, gama, Rcpcv;
     gas<NSP>(th, YY, tem, Cp, gama, Rcpcv, err);
-    const double rr = pp / (Rcpcv * tem);
+    const N rr = pp / (Rcpcv * tem);
     // face gradient (flux_viscous.f90:201-224), signed zeros of the dropped
     // g*0.0 basis terms aside
-    double t0[V], t1[V];
+    N t0[V], t1[V];
     {
-      const double dxl = d.rinv[NL], dyl = d.rinv[NE + NL];
+      const N dxl = d.rinv[NL], dyl = d.rinv[NE + NL];
 #pragma unroll
       for (int k = 0; k < V; ++k) {
-        t0[k] = d.grad[(2 * k) * NE + NL] * dxl;
-        t1[k] = d.grad[(2 * k + 1) * NE + NL] * dyl;
+        t0[k] = N(d.grad[(2 * k) * NE + NL]) * dxl;
+        t1[k] = N(d.grad[(2 * k + 1) * NE + NL]) * dyl;
       }
     }
     if (NR >= 0) {
-      const double dxk = d.fdxk[f], y1 = d.fysn[f], y2 = d.fysn[NF + f];
-      const double rkh = d.fdxkr[f], rkl = d.fdxkr[NF + f];
-      const double dxr = d.rinv[NR], dyr = d.rinv[NE + NR];
+      const N dxk = d.fdxk[f], y1 = d.fysn[f], y2 = d.fysn[NF + f];
+      const Recip rk = {d.fdxkr[f], d.fdxkr[NF + f]};
+      const N dxr = d.rinv[NR], dyr = d.rinv[NE + NR];
 #pragma unroll
       for (int k = 0; k < V; ++k) {
-        const double du = uR[k] - uL[k];
-        t0[k] = 0.5 * (t0[k] + d.grad[(2 * k) * NE + NR] * dxr) + div_rn(y1 * du, dxk, rkh, rkl);
-        t1[k] = 0.5 * (t1[k] + d.grad[(2 * k + 1) * NE + NR] * dyr) + div_rn(y2 * du, dxk, rkh, rkl);
+        const N du = uR[k] - uL[k];
+        t0[k] = half_of(t0[k] + N(d.grad[(2 * k) * NE + NR]) * dxr) + div_by(y1 * du, dxk, rk);
+        t1[k] = half_of(t1[k] + N(d.grad[(2 * k + 1) * NE + NR]) * dyr) + div_by(y2 * du, dxk, rk);
       }
     }
-    double dudx = t0[1], dudy = t1[1], dvdx = t0[2], dvdy = t1[2], dtdx = t0[3], dtdy = t1[3];
-    double dYdx[NSP], dYdy[NSP];
+    N dudx = t0[1], dudy = t1[1], dvdx = t0[2], dvdy = t1[2], dtdx = t0[3], dtdy = t1[3];
+    N dYdx[NSP], dYdy[NSP];
 #pragma unroll
     for (int k = 0; k < NSP - 1; ++k) { dYdx[k] = t0[4 + k]; dYdy[k] = t1[4 + k]; }
-    if (NR == -1 || NR == -6) removedirection(dtdx, dtdy, sav1n, sav2n);
+    if (NR == -1 || NR == -6) removedirection(dtdx, dtdy, N(sav1n), N(sav2n));
     if (NR == -2) {
-      const double snx = sav1n, sny = sav2n, stx = -sny, sty = snx;
+      const N snx = sav1n, sny = sav2n, stx = -sny, sty = snx;
       removedirection(dtdx, dtdy, snx, sny);
 #pragma unroll
       for (int k = 0; k < NSP - 1; ++k) removedirection(dYdx[k], dYdy[k], snx, sny);
-      double dutdx = dudx * stx + dvdx * sty, dutdy = dudy * stx + dvdy * sty;
-      double dundx = dudx * snx + dvdx * sny, dundy = dudy * snx + dvdy * sny;
+      N dutdx = dudx * stx + dvdx * sty, dutdy = dudy * stx + dvdy * sty;
+      N dundx = dudx * snx + dvdx * sny, dundy = dudy * snx + dvdy * sny;
       removedirection(dutdx, dutdy, snx, sny);
       removedirection(dundx, dundy, stx, sty);
       dudx = dutdx * stx + dundx * snx;
@@ -452,43 +441,40 @@ __global__ void __launch_bounds__(128) k_face_flux(const Dev d, const ThermoDev<
       dvdy = dutdy * sty + dundy * sny;
     }
     {
-      double sx = 0.0, sy = 0.0;
+      N sx = NSP > 1 ? plus_zero(dYdx[0]) : N(0.0), sy = NSP > 1 ? plus_zero(dYdy[0]) : N(0.0);
 #pragma unroll
-      for (int k = 0; k < NSP - 1; ++k) { sx = sx + dYdx[k]; sy = sy + dYdy[k]; }
+      for (int k = 1; k < NSP - 1; ++k) { sx = sx + dYdx[k]; sy = sy + dYdy[k]; }
       dYdx[NSP - 1] = -sx;
       dYdy[NSP - 1] = -sy;
     }
-    double entha[NSP], Dk[NSP], vmulc, akmu;
+    N entha[NSP], Dk[NSP], vmulc, akmu;
     enthalpy<NSP>(th, tem, entha, err);
     transport<NSP>(th, tem, YY, vmulc, akmu, err);
     diffusion<NSP>(th, pp, tem, YY, Dk);
-    double uicx = 0.0, uicy = 0.0;
+    const N uicx = dot<NSP>(Dk, dYdx), uicy = dot<NSP>(Dk, dYdy);
+    const N vlac = -2. / 3. * vmulc;
+    const N div = dudx + dvdy;
+    const N txx = twice_of(vmulc) * dudx + vlac * div;
+    const N tyy = twice_of(vmulc) * dvdy + vlac * div;
+    const N txy = vmulc * (dudy + dvdx);
+    N vx[NSP], vy[NSP];
 #pragma unroll
-    for (int k = 0; k < NSP; ++k) uicx = uicx + Dk[k] * dYdx[k];
-#pragma unroll
-    for (int k = 0; k < NSP; ++k) uicy = uicy + Dk[k] * dYdy[k];
-    const double vlac = -2. / 3. * vmulc;
-    const double div = dudx + dvdy;
-    const double txx = 2. * vmulc * dudx + vlac * div;
-    const double tyy = 2. * vmulc * dvdy + vlac * div;
-    const double txy = vmulc * (dudy + dvdx);
-    double sx = 0.0, sy = 0.0;
-#pragma unroll
-    for (int k = 0; k < NSP; ++k) sx = sx + (Dk[k] * dYdx[k] - YY[k] * uicx) * entha[k];
-#pragma unroll
-    for (int k = 0; k < NSP; ++k) sy = sy + (Dk[k] * dYdy[k] - YY[k] * uicy) * entha[k];
-    const double qx = -akmu * dtdx - rr * sx;
-    const double qy = -akmu * dtdy - rr * sy;
-    const double btx = uu * txx + vv * txy - qx;
-    const double bty = uu * txy + vv * tyy - qy;
-    d.Fvis[0 * NF + f] = -(sav1 * txx + sav2 * txy);
-    d.Fvis[1 * NF + f] = -(sav1 * txy + sav2 * tyy);
-    d.Fvis[2 * NF + f] = -(sav1 * btx + sav2 * bty);
+    for (int k = 0; k < NSP; ++k) {
+      vx[k] = Dk[k] * dYdx[k] - YY[k] * uicx;
+      vy[k] = Dk[k] * dYdy[k] - YY[k] * uicy;
+    }
+    const N sx = dot<NSP>(vx, entha), sy = dot<NSP>(vy, entha);
+    const N qx = -akmu * dtdx - rr * sx;
+    const N qy = -akmu * dtdy - rr * sy;
+    const N btx = uu * txx + vv * txy - qx;
+    const N bty = uu * txy + vv * tyy - qy;
+    d.Fvis[0 * NF + f] = val(-(sav1 * txx + sav2 * txy));
+    d.Fvis[1 * NF + f] = val(-(sav1 * txy + sav2 * tyy));
+    d.Fvis[2 * NF + f] = val(-(sav1 * btx + sav2 * bty));
 #pragma unroll
     for (int k = 0; k < NSP - 1; ++k) {
-      const double spx = rr * (Dk[k] * dYdx[k] - YY[k] * uicx);
-      const double spy = rr * (Dk[k] * dYdy[k] - YY[k] * uicy);
-      d.Fvis[(3 + k) * NF + f] = -(sav1 * spx + sav2 * spy);
+      const N spx = rr * vx[k], spy = rr * vy[k];
+      d.Fvis[(3 + k) * NF + f] = val(-(sav1 * spx + sav2 * spy));
     }
   }
   flag(d, err);
@@ -1486,13 +1472,13 @@ __global__ void __launch_bounds__(32) k_sweep4(const Dev d, const ThermoDev<NSP>
   sweep_compute<NSP, FWD>(d, th, p, threadIdx.x & 3, wsm);
 }
 
-template <int NSP>
+template <int NSP, class N>
 __global__ void __launch_bounds__(128) k_update(const Dev d, const ThermoDev<NSP> th) {
   pdl_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= d.NE) return;
   unsigned err = 0;
-  update_cell<NSP>(d, th, i, err);
+  update_cell<NSP, N>(d, th, i, err);
   flag(d, err);
 }
 
@@ -1927,6 +1913,9 @@ void fill_thermo(const rc_thermo* t, const rc_config* g, ThermoDev<NSP>& th) {
       th.cl[j][i] = t->low_coef_Cp_species[j + 7 * i];
       th.ch[j][i] = t->high_coef_Cp_species[j + 7 * i];
     }
+  for (int j = 0; j < 7; ++j)
+    for (int i = 0; i < NSP; ++i)
+      if (th.cl[j][i] != 0.0 || th.ch[j][i] != 0.0) th.cols |= 1 << j;
   for (int i = 0; i < NSP; ++i) { th.b1l[i] = t->low_enthalpy_b1[i]; th.b1h[i] = t->high_enthalpy_b1[i]; }
   th.trlo = t->transport_lowest_tem; th.trcrit = t->transport_critical_tem; th.trhi = t->transport_highest_tem;
   for (int a = 0; a < 4; ++a)
@@ -1977,20 +1966,20 @@ const ThermoDev<NSP>& TH(const rc_ctx* c) { return *reinterpret_cast<const Therm
 // --- the pieces of one iteration, enqueued on c->stream
 template <int NSP>
 void q_timestep_face(rc_ctx* c) {
-  if (c->visc) k_ts_face<NSP, true><<<blocks(c->NF, c->d.bs), c->d.bs, 0, c->stream>>>(c->d, TH<NSP>(c));
-  else k_ts_face<NSP, false><<<blocks(c->NF, c->d.bs), c->d.bs, 0, c->stream>>>(c->d, TH<NSP>(c));
+  auto k = c->visc ? k_ts_face<NSP, true, double> : k_ts_face<NSP, false, double>;
+  k<<<blocks(c->NF, c->d.bs), c->d.bs, 0, c->stream>>>(c->d, TH<NSP>(c));
   c->launches++;
 }
 template <int NSP>
 void q_cell(rc_ctx* c, int do_step, int do_recon) {
-  k_cell<NSP><<<blocks(c->NE, c->d.bs), c->d.bs, 0, c->stream>>>(c->d, TH<NSP>(c), do_step, do_recon, c->limit,
-                                                          c->comb && c->chem == RC_CHEM_EXPLICIT, c->visc);
+  k_cell<NSP, double><<<blocks(c->NE, c->d.bs), c->d.bs, 0, c->stream>>>(
+      c->d, TH<NSP>(c), do_step, do_recon, c->limit, c->comb && c->chem == RC_CHEM_EXPLICIT, c->visc);
   c->launches++;
 }
 template <int NSP>
 void q_face_flux(rc_ctx* c) {
-  if (c->visc) k_face_flux<NSP, true><<<blocks(c->NF, c->d.bs), c->d.bs, 0, c->stream>>>(c->d, TH<NSP>(c));
-  else k_face_flux<NSP, false><<<blocks(c->NF, c->d.bs), c->d.bs, 0, c->stream>>>(c->d, TH<NSP>(c));
+  auto k = c->visc ? k_face_flux<NSP, true, double> : k_face_flux<NSP, false, double>;
+  k<<<blocks(c->NF, c->d.bs), c->d.bs, 0, c->stream>>>(c->d, TH<NSP>(c));
   c->launches++;
 }
 template <int NSP>
@@ -2051,7 +2040,7 @@ void q_flow(rc_ctx* c) {
   else if (c->flow_g == 2) q_flow_g<NSP, 2>(c);
   else q_flow_g<NSP, 1>(c);
   c->launches++;
-  launch_pdl(k_update<NSP>, blocks(c->NE, c->d.bs), c->d.bs, c->stream, c->d, TH<NSP>(c));
+  launch_pdl(k_update<NSP, double>, blocks(c->NE, c->d.bs), c->d.bs, c->stream, c->d, TH<NSP>(c));
   c->launches++;
 }
 template <int NSP>
@@ -2086,7 +2075,7 @@ void q_sweeps(rc_ctx* c, int gather) {
                     c->bwd_off[l + 1]);
     c->launches++;
   }
-  launch_pdl(k_update<NSP>, blocks(c->NE, c->d.bs), c->d.bs, c->stream, c->d, TH<NSP>(c));
+  launch_pdl(k_update<NSP, double>, blocks(c->NE, c->d.bs), c->d.bs, c->stream, c->d, TH<NSP>(c));
   c->launches++;
 }
 // Integrated chemical source on the side stream, forked after the cell pass
@@ -2141,7 +2130,7 @@ void q_sweeps32(rc_ctx* c) {
     cudaMemsetAsync(c->lvl_count, 0, sizeof(unsigned) * c->nlevels, c->stream);
     mixed_lusgs_persistent<NSP>(c->d, c->thermo32.data(), c->fwd_off_dev, (int)c->fwd_off.size() - 1, c->bwd_off_dev,
                                 (int)c->bwd_off.size() - 1, c->lvl_count, c->pers_grid, c->stream);
-    k_update<NSP><<<blocks(c->NE, c->d.bs), c->d.bs, 0, c->stream>>>(c->d, TH<NSP>(c));
+    launch_pdl(k_update<NSP, double>, blocks(c->NE, c->d.bs), c->d.bs, c->stream, c->d, TH<NSP>(c));
     c->launches += 2;
     return;
   }
@@ -2153,7 +2142,7 @@ void q_sweeps32(rc_ctx* c) {
     mixed_sweep<NSP>(c->d, c->thermo32.data(), false, c->bwd_off[l], c->bwd_off[l + 1], c->stream);
     c->launches++;
   }
-  launch_pdl(k_update<NSP>, blocks(c->NE, c->d.bs), c->d.bs, c->stream, c->d, TH<NSP>(c));
+  launch_pdl(k_update<NSP, double>, blocks(c->NE, c->d.bs), c->d.bs, c->stream, c->d, TH<NSP>(c));
   c->launches++;
 }
 // The subroutines of one iteration in the current precision mode.

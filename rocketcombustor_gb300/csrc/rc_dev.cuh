@@ -128,8 +128,9 @@ __device__ __forceinline__ void flag(const Dev& d, unsigned e) {
   if (e) atomicOr(d.err, e);
 }
 
-__device__ __forceinline__ void removedirection(double& vx, double& vy, double nx, double ny) {
-  const double vn = vx * nx + vy * ny;  // flux_viscous.f90:352-361
+template <class N>
+__device__ __forceinline__ void removedirection(N& vx, N& vy, N nx, N ny) {
+  const N vn = vx * nx + vy * ny;  // flux_viscous.f90:352-361
   vx = vx - vn * nx;
   vy = vy - vn * ny;
 }
@@ -151,30 +152,30 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
 }
 
 // WA += hWA and update_primitve_variables (update_flow_variables.f90:4-48).
-template <int NSP>
+template <int NSP, class N = double>
 __device__ __forceinline__ void update_cell(const Dev& d, const ThermoDev<NSP>& th, int i, unsigned& err) {
   constexpr int V = 3 + NSP;
   const int NE = d.NE;
-  double W[V];
+  N W[V];
 #pragma unroll
   for (int k = 0; k < V; ++k) {
     W[k] = d.WA[k * NE + i] + d.hWA[k * NE + i];
-    d.WA[k * NE + i] = W[k];
+    d.WA[k * NE + i] = val(W[k]);
   }
-  const double rho = W[0], u = W[1] / rho, v = W[2] / rho;
-  double Y[NSP], s = 0.0;
+  const N rho = W[0], u = W[1] / rho, v = W[2] / rho;
+  N Y[NSP];
 #pragma unroll
-  for (int k = 0; k < NSP - 1; ++k) { Y[k] = W[4 + k] / rho; s = s + Y[k]; }
-  Y[NSP - 1] = 1.0 - s;
-  double Rcpcv;
-  const double t = newton_T<NSP>(th, W[3] / rho - 0.5 * (u * u + v * v), Y, d.PA[3 * NE + i], Rcpcv, err);
-  d.PA[0 * NE + i] = rho * Rcpcv * t;
-  d.PA[1 * NE + i] = u;
-  d.PA[2 * NE + i] = v;
-  d.PA[3 * NE + i] = t;
+  for (int k = 0; k < NSP - 1; ++k) Y[k] = W[4 + k] / rho;
+  Y[NSP - 1] = last_y<NSP>(Y);
+  N Rcpcv;
+  const N t = newton_T<NSP>(th, W[3] / rho - half_of(u * u + v * v), Y, N(d.PA[3 * NE + i]), Rcpcv, err);
+  d.PA[0 * NE + i] = val(rho * Rcpcv * t);
+  d.PA[1 * NE + i] = val(u);
+  d.PA[2 * NE + i] = val(v);
+  d.PA[3 * NE + i] = val(t);
 #pragma unroll
-  for (int k = 0; k < NSP - 1; ++k) d.PA[(4 + k) * NE + i] = Y[k];
-  if (i == 0 && isnan(W[0])) err |= ERR_NAN;
+  for (int k = 0; k < NSP - 1; ++k) d.PA[(4 + k) * NE + i] = val(Y[k]);
+  if (i == 0 && isnan(val(W[0]))) err |= ERR_NAN;
 }
 
 // Level ordering of the persistent LU-SGS kernels.  wait_count: lane 0 of a

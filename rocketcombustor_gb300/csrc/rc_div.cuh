@@ -55,6 +55,19 @@ __device__ __forceinline__ bool nonzero(double x) { return (__double_as_longlong
 // the floating-point order
 __device__ __forceinline__ long long dbits(double x) { return __double_as_longlong(x); }
 
+// a < b (IEEE: false with a NaN, -0 equal to +0) on the integer pipe.  Two
+// non-negative finite numbers compare as their bit patterns; other finite
+// numbers by magnitude with the sign applied; infinities and NaNs take the
+// FP64 compare.
+__device__ __forceinline__ bool less(double a, double b) {
+  const unsigned ah = (unsigned)__double2hiint(a), bh = (unsigned)__double2hiint(b);
+  const long long ia = __double_as_longlong(a), ib = __double_as_longlong(b);
+  if (max(ah, bh) < 0x7ff00000u) return ia < ib;
+  if (max(ah & 0x7fffffffu, bh & 0x7fffffffu) >= 0x7ff00000u) return a < b;
+  const long long m = 0x7fffffffffffffffLL;
+  return (ia < 0 ? -(ia & m) : ia) < (ib < 0 ? -(ib & m) : ib);
+}
+
 // 0.0 + x on the integer pipe: x, except that -0 becomes +0 (every other
 // value, NaN included, is unchanged by adding +0 in round-to-nearest)
 __device__ __forceinline__ double plus_zero(double x) {
@@ -68,6 +81,14 @@ __device__ __forceinline__ double half_of(double x) {
   const unsigned e = (unsigned)(b >> 52) & 0x7ffu;
   if (e - 2u < 0x7fdu) return __longlong_as_double(b - (1LL << 52));
   return 0.5 * x;
+}
+
+// 2 x, as half_of
+__device__ __forceinline__ double twice_of(double x) {
+  const long long b = __double_as_longlong(x);
+  const unsigned e = (unsigned)(b >> 52) & 0x7ffu;
+  if (e - 1u < 0x7fdu) return __longlong_as_double(b + (1LL << 52));
+  return 2.0 * x;
 }
 
 }  // namespace rc

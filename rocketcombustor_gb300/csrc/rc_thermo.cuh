@@ -13,8 +13,7 @@
 #pragma once
 #include <cstdint>
 
-#include "rc_div.cuh"
-#include "rc_math.h"
+#include "rc_num.cuh"
 
 namespace rc {
 
@@ -49,176 +48,247 @@ struct ThermoDev {
   double wdr[NSP][NSP][2];       // of wd
   double dljr[NSP][NSP][2];      // of dlj
   double mw1000r[2][2];          // of mw1000
+  int cols;                      // bit j: column j of cl or ch has a non-zero coefficient
 };
 
-__device__ __forceinline__ double fmin2(double a, double b) { return (b < a) ? b : a; }
-__device__ __forceinline__ double fmax2(double a, double b) { return (b > a) ? b : a; }
+__device__ __forceinline__ double fmin2(double a, double b) { return less(b, a) ? b : a; }
+__device__ __forceinline__ double fmax2(double a, double b) { return less(a, b) ? b : a; }
+// lo <= x && x <= hi (false for a NaN x)
+__device__ __forceinline__ bool in_range(double lo, double x, double hi) {
+  return (__double_as_longlong(x) & 0x7fffffffffffffffLL) <= 0x7ff0000000000000LL && !less(x, lo) && !less(hi, x);
+}
+
+// The polynomial columns to evaluate at temperature t: those that hold a
+// non-zero coefficient.  A column of zeros adds c b = +-0 to sums that start at
+// +0, which changes no bit as long as its basis value b is finite: every
+// column for a temperature outside 2^-100..2^100, whose powers and reciprocals
+// need not be.  What a column costs is its basis value (two divisions for 1/t
+// and 1/t^2, log t / t and three divisions in the enthalpy) and two operations
+// per species; property files of this solver fill one to three of the seven.
+template <int NSP>
+__device__ __forceinline__ int poly_cols(const ThermoDev<NSP>& th, double t) {
+  const unsigned e = (unsigned)__double2hiint(t) >> 20;  // sign and exponent
+  return e - 923u <= 200u ? th.cols : 127;
+}
+// s_i + c_ij b for every species, c the range's coefficients of column j; the
+// first column of `cols` starts the sums (0 + c b)
+template <int NSP, class N>
+__device__ __forceinline__ void poly_add(const ThermoDev<NSP>& th, int cols, int j, bool low, N b, N* s) {
+  if ((cols & ((1 << j) - 1)) == 0) {
+#pragma unroll
+    for (int i = 0; i < NSP; ++i) s[i] = plus_zero((low ? th.cl[j][i] : th.ch[j][i]) * b);
+  } else {
+#pragma unroll
+    for (int i = 0; i < NSP; ++i) s[i] = s[i] + (low ? th.cl[j][i] : th.ch[j][i]) * b;
+  }
+}
+// the same for the column of the constant term, whose basis value is 1
+template <int NSP, class N>
+__device__ __forceinline__ void poly_add1(const ThermoDev<NSP>& th, int cols, int j, bool low, N* s) {
+  if ((cols & ((1 << j) - 1)) == 0) {
+#pragma unroll
+    for (int i = 0; i < NSP; ++i) s[i] = plus_zero(low ? th.cl[j][i] : th.ch[j][i]);
+  } else {
+#pragma unroll
+    for (int i = 0; i < NSP; ++i) s[i] = s[i] + (low ? th.cl[j][i] : th.ch[j][i]);
+  }
+}
+// sum_i a_i b_i from +0 in index order
+template <int NSP, class A, class N>
+__device__ __forceinline__ N dot(const A* a, const N* b) {
+  N s = plus_zero(a[0] * b[0]);
+#pragma unroll
+  for (int i = 1; i < NSP; ++i) s = s + a[i] * b[i];
+  return s;
+}
+// the last species' mass fraction, 1 - sum of the others (from +0, in order)
+template <int NSP, class N>
+__device__ __forceinline__ N last_y(const N* Y) {
+  if (NSP == 1) return 1.0 - 0.0;
+  N s = plus_zero(Y[0]);
+#pragma unroll
+  for (int k = 1; k < NSP - 1; ++k) s = s + Y[k];
+  return 1.0 - s;
+}
 
 // ComputeGasParameter (thermo_property.f90:78-112)
-template <int NSP>
-__device__ __forceinline__ void gas(const ThermoDev<NSP>& th, const double* Y, double tem, double& Cp,
-                                    double& gama, double& Rcpcv, unsigned& err) {
-  const double t2 = tem * tem;
-  const double b[7] = {1.0 / t2, 1.0 / tem, 1.0, tem, t2, tem * t2, t2 * t2};
-  const bool low = (th.tlo <= tem && tem <= th.tcrit);
-  if (!low && !(th.tcrit < tem && tem <= th.thi)) err |= ERR_THERMO_T;
-  double cps[NSP];
+template <int NSP, class N>
+__device__ __forceinline__ void gas(const ThermoDev<NSP>& th, const N* Y, N tem, N& Cp, N& gama, N& Rcpcv,
+                                    unsigned& err) {
+  const N t2 = tem * tem;
+  const double t = val(tem);
+  const bool low = in_range(th.tlo, t, th.tcrit);
+  if (!low && !(less(th.tcrit, t) && !less(th.thi, t))) err |= ERR_THERMO_T;
+  const int cols = poly_cols(th, t);
+  N cps[NSP];
 #pragma unroll
-  for (int i = 0; i < NSP; ++i) {
-    double s = 0.0;
+  for (int i = 0; i < NSP; ++i) cps[i] = 0.0;
+  if (cols & 1) poly_add(th, cols, 0, low, 1.0 / t2, cps);
+  if (cols & 2) poly_add(th, cols, 1, low, 1.0 / tem, cps);
+  if (cols & 4) poly_add1(th, cols, 2, low, cps);
+  if (cols & 8) poly_add(th, cols, 3, low, tem, cps);
+  if (cols & 16) poly_add(th, cols, 4, low, t2, cps);
+  if (cols & 32) poly_add(th, cols, 5, low, tem * t2, cps);
+  if (cols & 64) poly_add(th, cols, 6, low, t2 * t2, cps);
 #pragma unroll
-    for (int j = 0; j < 7; ++j) s = s + (low ? th.cl[j][i] : th.ch[j][i]) * b[j];
-    cps[i] = s * th.R[i];
-  }
-  double c = 0.0, r = 0.0;
-#pragma unroll
-  for (int i = 0; i < NSP; ++i) c = c + cps[i] * Y[i];
-#pragma unroll
-  for (int i = 0; i < NSP; ++i) r = r + th.R[i] * Y[i];
+  for (int i = 0; i < NSP; ++i) cps[i] = cps[i] * th.R[i];
+  const N c = dot<NSP>(cps, Y), r = dot<NSP>(th.R, Y);
   Cp = c;
   Rcpcv = r;
   gama = c / (c - r);
 }
 
+// RN(1/3), RN(1/5) and their second parts: the pairs of rc_div.cuh
+__device__ constexpr double THIRD[2] = {0x1.5555555555555p-2, 0x1.5555555555555p-56};
+__device__ constexpr double FIFTH[2] = {0x1.999999999999ap-3, -0x1.999999999999ap-57};
+
 // compute_enthalpy (thermo_property.f90:114-144)
-template <int NSP>
-__device__ __forceinline__ void enthalpy(const ThermoDev<NSP>& th, double tem, double* entha, unsigned& err) {
-  const double t2 = tem * tem;
-  const double e[7] = {-(1.0 / t2), rcm::log(tem) / tem, 1.0, tem / 2.0, t2 / 3.0, (tem * t2) / 4.0, (t2 * t2) / 5.0};
-  const bool low = (th.tlo <= tem && tem <= th.tcrit);
-  if (!low && !(th.tcrit < tem && tem <= th.thi)) err |= ERR_THERMO_T;
+template <int NSP, class N>
+__device__ __forceinline__ void enthalpy(const ThermoDev<NSP>& th, N tem, N* entha, unsigned& err) {
+  const N t2 = tem * tem;
+  const double t = val(tem);
+  const bool low = in_range(th.tlo, t, th.tcrit);
+  if (!low && !(less(th.tcrit, t) && !less(th.thi, t))) err |= ERR_THERMO_T;
+  const int cols = poly_cols(th, t);
+  N s[NSP];
 #pragma unroll
-  for (int i = 0; i < NSP; ++i) {
-    double s = 0.0;
+  for (int i = 0; i < NSP; ++i) s[i] = 0.0;
+  if (cols & 1) poly_add(th, cols, 0, low, -(1.0 / t2), s);
+  if (cols & 2) poly_add(th, cols, 1, low, n_log(tem) / tem, s);
+  if (cols & 4) poly_add1(th, cols, 2, low, s);
+  if (cols & 8) poly_add(th, cols, 3, low, half_of(tem), s);
+  if (cols & 16) poly_add(th, cols, 4, low, div_fixed(t2, N(3.0), THIRD), s);
+  if (cols & 32) poly_add(th, cols, 5, low, 0.25 * (tem * t2), s);
+  if (cols & 64) poly_add(th, cols, 6, low, div_fixed(t2 * t2, N(5.0), FIFTH), s);
 #pragma unroll
-    for (int j = 0; j < 7; ++j) s = s + (low ? th.cl[j][i] : th.ch[j][i]) * e[j];
-    entha[i] = th.R[i] * (tem * s + (low ? th.b1l[i] : th.b1h[i]));
-  }
+  for (int i = 0; i < NSP; ++i) entha[i] = th.R[i] * (tem * s[i] + (low ? th.b1l[i] : th.b1h[i]));
 }
 
 // Newton_temperature (thermo_property.f90:146-180); returns T, sets Rcpcv.
-template <int NSP>
-__device__ __forceinline__ double newton_T(const ThermoDev<NSP>& th, double et, const double* Y, double t0,
-                                           double& Rcpcv, unsigned& err) {
-  double t = t0, Cp, gama;
-  double entha[NSP];
+template <int NSP, class N>
+__device__ __forceinline__ N newton_T(const ThermoDev<NSP>& th, N et, const N* Y, N t0, N& Rcpcv, unsigned& err) {
+  N t = t0, Cp, gama;
+  N entha[NSP];
   for (int it = 0; it < 200; ++it) {
     enthalpy<NSP>(th, t, entha, err);
     gas<NSP>(th, Y, t, Cp, gama, Rcpcv, err);
-    double h = 0.0;
-#pragma unroll
-    for (int i = 0; i < NSP; ++i) h = h + Y[i] * entha[i];
-    const double ft = h - Rcpcv * t - et;
-    const double dft = Cp - Rcpcv;
-    const double dtt = -ft / dft;
+    const N h = dot<NSP>(Y, entha);
+    const N ft = h - Rcpcv * t - et;
+    const N dft = Cp - Rcpcv;
+    const N dtt = -ft / dft;
     t = t + dtt;
-    t = fmax2(t, th.tlo);
-    t = fmin2(t, th.thi);
-    if (fabs(dtt) < 1.0e-5) break;
+    t = fmax2(t, N(th.tlo));
+    t = fmin2(t, N(th.thi));
+    if (less(n_abs(dtt), N(1.0e-5))) break;
   }
   return t;
 }
 
+// X_k = (Y_k / M_k) / sum_i Y_i / M_i as transport_property.f90 and
+// diffusion_velocity.f90 form it
+template <int NSP, class N>
+__device__ __forceinline__ void mole_fractions(const ThermoDev<NSP>& th, const N* Y, N* X) {
+  N s = plus_zero(div_fixed(Y[0], N(th.mw[0]), th.mwr[0]));
+#pragma unroll
+  for (int i = 1; i < NSP; ++i) s = s + div_fixed(Y[i], N(th.mw[i]), th.mwr[i]);
+  const N ww = 1.0 / s;
+#pragma unroll
+  for (int i = 0; i < NSP; ++i) X[i] = div_fixed(ww * Y[i], N(th.mw[i]), th.mwr[i]);
+}
+
 // compute_transport_property (transport_property.f90:78-125)
-template <int NSP>
-__device__ __forceinline__ void transport(const ThermoDev<NSP>& th, double tem2, const double* yy, double& vmul,
-                                          double& akmu, unsigned& err) {
-  const double tem = fmax2(th.trlo, tem2);
-  double s = 0.0;
-#pragma unroll
-  for (int i = 0; i < NSP; ++i) s = s + div_rn(yy[i], th.mw[i], th.mwr[i]);
-  const double ww = 1.0 / s;
-  double xx[NSP], mul[NSP], Kl[NSP];
-#pragma unroll
-  for (int i = 0; i < NSP; ++i) xx[i] = div_rn(ww * yy[i], th.mw[i], th.mwr[i]);
-  const bool low = (th.trlo <= tem && tem <= th.trcrit);
-  if (!low && !(th.trcrit < tem && tem <= th.trhi)) err |= ERR_TRANSPORT_T;
+template <int NSP, class N>
+__device__ __forceinline__ void transport(const ThermoDev<NSP>& th, N tem2, const N* yy, N& vmul, N& akmu,
+                                          unsigned& err) {
+  const N tem = fmax2(N(th.trlo), tem2);
+  const double t = val(tem);
+  N xx[NSP], mul[NSP], Kl[NSP];
+  mole_fractions<NSP>(th, yy, xx);
+  const bool low = in_range(th.trlo, t, th.trcrit);
+  if (!low && !(less(th.trcrit, t) && !less(th.trhi, t))) err |= ERR_TRANSPORT_T;
   const int rg = low ? 0 : 1;
-  const double lt = rcm::log(tem);
-  const double t2 = tem * tem;
-  const Recip rt = recip_of(tem), rt2 = recip_of(t2);
+  const N lt = n_log(tem);
+  const N t2 = tem * tem;
+  const Recip rt = pair_of(tem), rt2 = pair_of(t2);
 #pragma unroll
   for (int i = 0; i < NSP; ++i) {
-    mul[i] = rcm::exp(th.mu[rg][0][i] * lt + div_rn(th.mu[rg][1][i], tem, rt.h, rt.l) +
-                      div_rn(th.mu[rg][2][i], t2, rt2.h, rt2.l) + th.mu[rg][3][i]);
-    Kl[i] = rcm::exp(th.kk[rg][0][i] * lt + div_rn(th.kk[rg][1][i], tem, rt.h, rt.l) +
-                     div_rn(th.kk[rg][2][i], t2, rt2.h, rt2.l) + th.kk[rg][3][i]);
+    mul[i] = n_exp(th.mu[rg][0][i] * lt + div_by(N(th.mu[rg][1][i]), tem, rt) +
+                   div_by(N(th.mu[rg][2][i]), t2, rt2) + th.mu[rg][3][i]);
+    Kl[i] = n_exp(th.kk[rg][0][i] * lt + div_by(N(th.kk[rg][1][i]), tem, rt) +
+                  div_by(N(th.kk[rg][2][i]), t2, rt2) + th.kk[rg][3][i]);
   }
 #pragma unroll
   for (int i = 0; i < NSP; ++i) { mul[i] = mul[i] * 1.0e-7; Kl[i] = Kl[i] * 1.0e-4; }
-  double v = 0.0;
+  N v = 0.0;
 #pragma unroll
   for (int i = 0; i < NSP; ++i) {
-    double phil = 0.0;
+    N phil = 0.0;
 #pragma unroll
     for (int j = 0; j < NSP; ++j) {
       // sqrt(mul(i)/mul(i)) is exactly 1
-      const double sq = (i == j) ? 1.0 : sqrt(mul[i] / mul[j]);
-      const double q = 1.0 + sq * th.wc[i][j];
-      phil = phil + div_rn(xx[j] * (q * q), th.wd[i][j], th.wdr[i][j]);
+      const N sq = (i == j) ? N(1.0) : n_sqrt(mul[i] / mul[j]);
+      const N q = 1.0 + sq * th.wc[i][j];
+      const N w = div_fixed(xx[j] * (q * q), N(th.wd[i][j]), th.wdr[i][j]);
+      phil = j ? phil + w : plus_zero(w);
     }
     phil = (0.25 * sqrt(2.0)) * phil;
-    v = v + xx[i] * mul[i] / phil;
+    const N w = xx[i] * mul[i] / phil;
+    v = i ? v + w : plus_zero(w);
   }
-  double s1 = 0.0, s2 = 0.0;
+  const N s1 = dot<NSP>(xx, Kl);
+  N s2 = plus_zero(xx[0] / Kl[0]);
 #pragma unroll
-  for (int i = 0; i < NSP; ++i) s1 = s1 + xx[i] * Kl[i];
-#pragma unroll
-  for (int i = 0; i < NSP; ++i) s2 = s2 + xx[i] / Kl[i];
+  for (int i = 1; i < NSP; ++i) s2 = s2 + xx[i] / Kl[i];
   vmul = v;
-  akmu = 0.5 * (s1 + 1.0 / s2);
+  akmu = half_of(s1 + 1.0 / s2);
 }
 
 // compute_diffusion_velocity (diffusion_velocity.f90:55-118).  D_ij is
 // symmetric bit for bit (every pair term is), so each pair is evaluated once;
 // the diagonal D_ii is never used.
-template <int NSP>
-__device__ __forceinline__ void diffusion(const ThermoDev<NSP>& th, double pp, double tem, const double* YY,
-                                          double* Dk) {
-  double s = 0.0;
-#pragma unroll
-  for (int i = 0; i < NSP; ++i) s = s + div_rn(YY[i], th.mw[i], th.mwr[i]);
-  const double ww = 1.0 / s;
-  double XX[NSP];
-#pragma unroll
-  for (int i = 0; i < NSP; ++i) XX[i] = div_rn(ww * YY[i], th.mw[i], th.mwr[i]);
-  const double num = 0.0266 * sqrt(tem * (tem * tem));
-  double D[NSP][NSP];
+template <int NSP, class N>
+__device__ __forceinline__ void diffusion(const ThermoDev<NSP>& th, N pp, N tem, const N* YY, N* Dk) {
+  N XX[NSP];
+  mole_fractions<NSP>(th, YY, XX);
+  const N num = 0.0266 * n_sqrt(tem * (tem * tem));
+  N D[NSP][NSP];
 #pragma unroll
   for (int i = 0; i < NSP; ++i)
 #pragma unroll
     for (int j = i + 1; j < NSP; ++j) {
-      const double tstar = div_rn(tem, th.dlj[i][j], th.dljr[i][j]);
-      const double om = 1.06036 * rcm::pow(tstar, -0.15610) + 0.19300 * rcm::exp(-0.47635 * tstar) +
-                        1.03587 * rcm::exp(-1.52996 * tstar) + 1.76474 * rcm::exp(-3.89411 * tstar);
-      const double d = num / (pp * th.dmw[i][j] * th.dcd[i][j] * om);
+      const N tstar = div_fixed(tem, N(th.dlj[i][j]), th.dljr[i][j]);
+      const N om = 1.06036 * n_pow(tstar, -0.15610) + 0.19300 * n_exp(-0.47635 * tstar) +
+                   1.03587 * n_exp(-1.52996 * tstar) + 1.76474 * n_exp(-3.89411 * tstar);
+      const N d = num / (pp * th.dmw[i][j] * th.dcd[i][j] * om);
       D[i][j] = d;
       D[j][i] = d;
     }
 #pragma unroll
   for (int i = 0; i < NSP; ++i) {
-    double xd = 0.0;
+    N xd = 0.0;
 #pragma unroll
     for (int j = 0; j < NSP; ++j)
-      if (j != i) xd = xd + XX[j] / D[i][j];
+      if (j != i) {
+        const N w = XX[j] / D[i][j];
+        xd = j == (i == 0 ? 1 : 0) ? plus_zero(w) : xd + w;
+      }
     Dk[i] = (1.0 - XX[i]) / (xd + 1.0e-16);
   }
 }
 
 // compute_production_rate (chemical_kinetics.f90:109-165)
-template <int NSP>
-__device__ __forceinline__ void production(const ThermoDev<NSP>& th, double T, double rho, const double* Y2,
-                                           double* prod) {
-  double kf;
-  const double y0 = fmin2(1.0, fmax2(0.0, Y2[0]));
+template <int NSP, class N>
+__device__ __forceinline__ void production(const ThermoDev<NSP>& th, N T, N rho, const N* Y2, N* prod) {
+  N kf;
+  const N y0 = fmin2(N(1.0), fmax2(N(0.0), Y2[0]));
   if (th.model == 0) {
-    const double y1 = fmin2(1.0, fmax2(0.0, Y2[NSP > 1 ? 1 : 0]));
-    kf = th.Af * rcm::exp(-th.E / (th.Rconstant * T));
-    kf = kf * rcm::pow(div_rn(y0 * rho, th.mw1000[0], th.mw1000r[0]), 0.2);
-    kf = kf * rcm::pow(div_rn(y1 * rho, th.mw1000[1], th.mw1000r[1]), 1.3);
+    const N y1 = fmin2(N(1.0), fmax2(N(0.0), Y2[NSP > 1 ? 1 : 0]));
+    kf = th.Af * n_exp(-th.E / (th.Rconstant * T));
+    kf = kf * n_pow(div_fixed(y0 * rho, N(th.mw1000[0]), th.mw1000r[0]), 0.2);
+    kf = kf * n_pow(div_fixed(y1 * rho, N(th.mw1000[1]), th.mw1000r[1]), 1.3);
   } else {
-    kf = (T > 710.0) ? 1e4 : 0.0;
-    kf = kf * div_rn(y0 * rho, th.mw1000[0], th.mw1000r[0]);
+    kf = less(N(710.0), T) ? 1e4 : 0.0;
+    kf = kf * div_fixed(y0 * rho, N(th.mw1000[0]), th.mw1000r[0]);
   }
 #pragma unroll
   for (int k = 0; k < NSP; ++k) prod[k] = th.prodc[k] * kf;
