@@ -54,7 +54,7 @@ __device__ __forceinline__ void inlet_bc(const ThermoDev<NSP>& th, const double*
 }
 
 // ----------------------------------------------------------- TimeStep ------
-template <int NSP, bool VISC, class N>
+template <int NSP, bool VISC, class N, class NT>
 __global__ void __launch_bounds__(128) k_ts_face(const Dev d, const ThermoDev<NSP> th) {
   constexpr int V = 3 + NSP;
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
@@ -81,8 +81,12 @@ __global__ void __launch_bounds__(128) k_ts_face(const Dev d, const ThermoDev<NS
   const N alpa = n_abs(unormal) + n_sqrt(gama * pp / rr) * d.fss[f];
   d.alpa[f] = val(alpa);
   if (VISC) {
-    N vmul, akmu;
-    transport<NSP>(th, tt, yy, vmul, akmu, err);
+    NT yt[NSP], xt[NSP], vt, at;
+#pragma unroll
+    for (int k = 0; k < NSP; ++k) yt[k] = val(yy[k]);
+    mole_fractions<NSP>(th, yt, xt);
+    transport<NSP>(th, NT(val(tt)), xt, vt, at, err);
+    const N vmul = val(vt), akmu = val(at);
     const N prl = vmul * Cp / akmu;
     const N alpaVis = twice_of(N(d.fs2[f])) * fmax2(N(4. / 3.), gama / prl) * vmul / rr;
     const N vl = alpaVis / N(d.vol[NL]);
@@ -256,7 +260,11 @@ __device__ __forceinline__ void recon(const Dev& d, int c, double v0, double v1,
     u[k] = d.PA[k * NE + c] + (N(d.grad[(2 * k) * NE + c]) * v0 + N(d.grad[(2 * k + 1) * NE + c]) * v1);
 }
 
-template <int NSP, bool VISC, class N>
+// Bound by the FP64 unit (about 1,150 FP64 instructions of a warp per 32
+// faces, 77 cycles each) and, with the divisions, square roots and the
+// transport part's multiplications on them (NT), the integer pipes.  2M
+// triangles, 3.0 M faces: 15.5 -> 8.2 ms; 120,000 triangles 988 -> 552 us.
+template <int NSP, bool VISC, class N, class NT>
 __global__ void __launch_bounds__(128) k_face_flux(const Dev d, const ThermoDev<NSP> th) {
   constexpr int V = 3 + NSP;
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
@@ -447,10 +455,17 @@ __global__ void __launch_bounds__(128) k_face_flux(const Dev d, const ThermoDev<
       dYdx[NSP - 1] = -sx;
       dYdy[NSP - 1] = -sy;
     }
-    N entha[NSP], Dk[NSP], vmulc, akmu;
+    N entha[NSP], Dk[NSP];
     enthalpy<NSP>(th, tem, entha, err);
-    transport<NSP>(th, tem, YY, vmulc, akmu, err);
-    diffusion<NSP>(th, pp, tem, YY, Dk);
+    NT yt[NSP], xt[NSP], dt[NSP], vt, at;
+#pragma unroll
+    for (int k = 0; k < NSP; ++k) yt[k] = val(YY[k]);
+    mole_fractions<NSP>(th, yt, xt);
+    transport<NSP>(th, NT(val(tem)), xt, vt, at, err);
+    diffusion<NSP>(th, NT(val(pp)), NT(val(tem)), xt, dt);
+#pragma unroll
+    for (int k = 0; k < NSP; ++k) Dk[k] = val(dt[k]);
+    const N vmulc = val(vt), akmu = val(at);
     const N uicx = dot<NSP>(Dk, dYdx), uicy = dot<NSP>(Dk, dYdy);
     const N vlac = -2. / 3. * vmulc;
     const N div = dudx + dvdy;
@@ -1964,22 +1979,44 @@ template <int NSP>
 const ThermoDev<NSP>& TH(const rc_ctx* c) { return *reinterpret_cast<const ThermoDev<NSP>*>(c->thermo.data()); }
 
 // --- the pieces of one iteration, enqueued on c->stream
+// The number types of the FP64 kernels: divisions, square roots and comparisons
+// on the integer pipes everywhere (Cheap); in the transport and diffusion
+// functions of the face kernels also the multiplications, once the faces give
+// every SM sub-partition a warp (Busy).  Below that a face's time is one warp's
+// chain, where a multiplication on the integer pipes takes 157-216 cycles
+// instead of 55-62.  Measured, time step / face flux in us with Cheap and with
+// Busy: 11,425 faces 43.3 / 104.7 and 45.4 / 117.0; 24,240 faces 57.7 / 143.6
+// and 49.5 / 132.8; 72,460 faces 96.3 / 326.9 and 69.3 / 227.7; 3.0 M faces
+// 3173 / 9408 and 1893 / 8200 (all in double: 5400 / 15500).
+using Cheap = Num<false>;
+using Busy = Num<true>;
+template <class F>
+void with_face_num(const rc_ctx* c, F f) {
+  if (c->NF >= 32 * 4 * c->pers_grid) f((Busy*)nullptr);
+  else f((Cheap*)nullptr);
+}
 template <int NSP>
 void q_timestep_face(rc_ctx* c) {
-  auto k = c->visc ? k_ts_face<NSP, true, double> : k_ts_face<NSP, false, double>;
-  k<<<blocks(c->NF, c->d.bs), c->d.bs, 0, c->stream>>>(c->d, TH<NSP>(c));
+  with_face_num(c, [&](auto* n) {
+    using NT = std::remove_pointer_t<decltype(n)>;
+    auto k = c->visc ? k_ts_face<NSP, true, Cheap, NT> : k_ts_face<NSP, false, Cheap, Cheap>;
+    k<<<blocks(c->NF, c->d.bs), c->d.bs, 0, c->stream>>>(c->d, TH<NSP>(c));
+  });
   c->launches++;
 }
 template <int NSP>
 void q_cell(rc_ctx* c, int do_step, int do_recon) {
-  k_cell<NSP, double><<<blocks(c->NE, c->d.bs), c->d.bs, 0, c->stream>>>(
+  k_cell<NSP, Cheap><<<blocks(c->NE, c->d.bs), c->d.bs, 0, c->stream>>>(
       c->d, TH<NSP>(c), do_step, do_recon, c->limit, c->comb && c->chem == RC_CHEM_EXPLICIT, c->visc);
   c->launches++;
 }
 template <int NSP>
 void q_face_flux(rc_ctx* c) {
-  auto k = c->visc ? k_face_flux<NSP, true, double> : k_face_flux<NSP, false, double>;
-  k<<<blocks(c->NF, c->d.bs), c->d.bs, 0, c->stream>>>(c->d, TH<NSP>(c));
+  with_face_num(c, [&](auto* n) {
+    using NT = std::remove_pointer_t<decltype(n)>;
+    auto k = c->visc ? k_face_flux<NSP, true, Cheap, NT> : k_face_flux<NSP, false, Cheap, Cheap>;
+    k<<<blocks(c->NF, c->d.bs), c->d.bs, 0, c->stream>>>(c->d, TH<NSP>(c));
+  });
   c->launches++;
 }
 template <int NSP>
@@ -2040,7 +2077,7 @@ void q_flow(rc_ctx* c) {
   else if (c->flow_g == 2) q_flow_g<NSP, 2>(c);
   else q_flow_g<NSP, 1>(c);
   c->launches++;
-  launch_pdl(k_update<NSP, double>, blocks(c->NE, c->d.bs), c->d.bs, c->stream, c->d, TH<NSP>(c));
+  launch_pdl(k_update<NSP, Cheap>, blocks(c->NE, c->d.bs), c->d.bs, c->stream, c->d, TH<NSP>(c));
   c->launches++;
 }
 template <int NSP>
@@ -2075,7 +2112,7 @@ void q_sweeps(rc_ctx* c, int gather) {
                     c->bwd_off[l + 1]);
     c->launches++;
   }
-  launch_pdl(k_update<NSP, double>, blocks(c->NE, c->d.bs), c->d.bs, c->stream, c->d, TH<NSP>(c));
+  launch_pdl(k_update<NSP, Cheap>, blocks(c->NE, c->d.bs), c->d.bs, c->stream, c->d, TH<NSP>(c));
   c->launches++;
 }
 // Integrated chemical source on the side stream, forked after the cell pass
@@ -2130,7 +2167,7 @@ void q_sweeps32(rc_ctx* c) {
     cudaMemsetAsync(c->lvl_count, 0, sizeof(unsigned) * c->nlevels, c->stream);
     mixed_lusgs_persistent<NSP>(c->d, c->thermo32.data(), c->fwd_off_dev, (int)c->fwd_off.size() - 1, c->bwd_off_dev,
                                 (int)c->bwd_off.size() - 1, c->lvl_count, c->pers_grid, c->stream);
-    launch_pdl(k_update<NSP, double>, blocks(c->NE, c->d.bs), c->d.bs, c->stream, c->d, TH<NSP>(c));
+    launch_pdl(k_update<NSP, Cheap>, blocks(c->NE, c->d.bs), c->d.bs, c->stream, c->d, TH<NSP>(c));
     c->launches += 2;
     return;
   }
@@ -2142,7 +2179,7 @@ void q_sweeps32(rc_ctx* c) {
     mixed_sweep<NSP>(c->d, c->thermo32.data(), false, c->bwd_off[l], c->bwd_off[l + 1], c->stream);
     c->launches++;
   }
-  launch_pdl(k_update<NSP, double>, blocks(c->NE, c->d.bs), c->d.bs, c->stream, c->d, TH<NSP>(c));
+  launch_pdl(k_update<NSP, Cheap>, blocks(c->NE, c->d.bs), c->d.bs, c->stream, c->d, TH<NSP>(c));
   c->launches++;
 }
 // The subroutines of one iteration in the current precision mode.

@@ -51,8 +51,13 @@ struct ThermoDev {
   int cols;                      // bit j: column j of cl or ch has a non-zero coefficient
 };
 
+// The functions below take double or Num (rc_soft.cuh); the bits are the same.
 __device__ __forceinline__ double fmin2(double a, double b) { return less(b, a) ? b : a; }
 __device__ __forceinline__ double fmax2(double a, double b) { return less(a, b) ? b : a; }
+template <bool M>
+__device__ __forceinline__ Num<M> fmin2(Num<M> a, Num<M> b) { return less(b, a) ? b : a; }
+template <bool M>
+__device__ __forceinline__ Num<M> fmax2(Num<M> a, Num<M> b) { return less(a, b) ? b : a; }
 // lo <= x && x <= hi (false for a NaN x)
 __device__ __forceinline__ bool in_range(double lo, double x, double hi) {
   return (__double_as_longlong(x) & 0x7fffffffffffffffLL) <= 0x7ff0000000000000LL && !less(x, lo) && !less(hi, x);
@@ -196,14 +201,13 @@ __device__ __forceinline__ void mole_fractions(const ThermoDev<NSP>& th, const N
   for (int i = 0; i < NSP; ++i) X[i] = div_fixed(ww * Y[i], N(th.mw[i]), th.mwr[i]);
 }
 
-// compute_transport_property (transport_property.f90:78-125)
+// compute_transport_property (transport_property.f90:78-125); xx: mole_fractions
 template <int NSP, class N>
-__device__ __forceinline__ void transport(const ThermoDev<NSP>& th, N tem2, const N* yy, N& vmul, N& akmu,
+__device__ __forceinline__ void transport(const ThermoDev<NSP>& th, N tem2, const N* xx, N& vmul, N& akmu,
                                           unsigned& err) {
   const N tem = fmax2(N(th.trlo), tem2);
   const double t = val(tem);
-  N xx[NSP], mul[NSP], Kl[NSP];
-  mole_fractions<NSP>(th, yy, xx);
+  N mul[NSP], Kl[NSP];
   const bool low = in_range(th.trlo, t, th.trcrit);
   if (!low && !(less(th.trcrit, t) && !less(th.trhi, t))) err |= ERR_TRANSPORT_T;
   const int rg = low ? 0 : 1;
@@ -243,13 +247,11 @@ __device__ __forceinline__ void transport(const ThermoDev<NSP>& th, N tem2, cons
   akmu = half_of(s1 + 1.0 / s2);
 }
 
-// compute_diffusion_velocity (diffusion_velocity.f90:55-118).  D_ij is
+// compute_diffusion_velocity (diffusion_velocity.f90:55-118); XX: mole_fractions.  D_ij is
 // symmetric bit for bit (every pair term is), so each pair is evaluated once;
 // the diagonal D_ii is never used.
 template <int NSP, class N>
-__device__ __forceinline__ void diffusion(const ThermoDev<NSP>& th, N pp, N tem, const N* YY, N* Dk) {
-  N XX[NSP];
-  mole_fractions<NSP>(th, YY, XX);
+__device__ __forceinline__ void diffusion(const ThermoDev<NSP>& th, N pp, N tem, const N* XX, N* Dk) {
   const N num = 0.0266 * n_sqrt(tem * (tem * tem));
   N D[NSP][NSP];
 #pragma unroll
