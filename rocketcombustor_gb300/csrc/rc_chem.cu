@@ -2,8 +2,8 @@
 // source of the steady iteration and the batch integration of given states.
 //
 // The work per cell is uneven (1 to maxsub substeps, each with rejections), so
-// both kernels are persistent work queues: every warp takes the next 32 items
-// from a counter until none are left.  Results do not depend on which warp
+// the kernels are persistent work queues: every lane takes the next item from
+// a counter when it has finished one.  Results do not depend on which lane
 // takes which item.
 #include <cuda_runtime.h>
 
@@ -13,60 +13,127 @@
 namespace rc {
 
 constexpr int CHEM_THREADS = 128;
+using ChemNum = Num<false>;
 
-__device__ __forceinline__ int next_chunk(unsigned* counter) {
-  int base = 0;
-  if ((threadIdx.x & 31) == 0) base = (int)atomicAdd(counter, 32u);
-  return __shfl_sync(0xffffffffu, base, 0);
+// Runs the items 0 .. n-1 of a queue through the lanes of a warp: a lane that
+// has finished its item takes the next one while the others go on.  Items need
+// 1 to thousands of attempts; a warp that took 32 and waited for the slowest
+// left most lanes idle (an FP64 instruction costs the same with one active lane
+// as with 32).  The lanes refill when REFILL of them are idle or none is busy:
+// starting an item costs about a tenth of an attempt, for the whole warp.
+// 262,144 states at tolerance 0.005 (median 9 substeps, 90th percentile 509):
+// 276 ms with a warp taking 32 states at a time, 128 ms now.  Three blocks per
+// SM (168 registers, a few spills) against two: 133 ms; the bound is the FP64
+// unit and, when few states are left, one attempt's chain (about 60 us).
+//   begin(item, r)  loads item into reactor r; false when it needs no attempt
+//   end(item, r)    stores the finished item
+constexpr int REFILL = 4;
+template <int NSP, class N, class Begin, class End>
+__device__ __forceinline__ void run_queue(const ThermoDev<NSP>& th, int n, unsigned* counter, double tol, int maxsub,
+                                          unsigned& err, Begin begin, End end) {
+  const int lane = threadIdx.x & 31;
+  Reactor<NSP, N> r;
+  int item = -1;        // the lane's item, -1 when idle
+  bool more = true;     // the queue may hold more (warp-uniform)
+  for (;;) {
+    unsigned idle = __ballot_sync(0xffffffffu, item < 0);
+    while (more && (__popc(idle) >= REFILL)) {
+      int base = 0;
+      if (lane == 0) base = (int)atomicAdd(counter, (unsigned)__popc(idle));
+      base = __shfl_sync(0xffffffffu, base, 0);
+      more = base + __popc(idle) < n;
+      if (item < 0) {
+        const int q = base + __popc(idle & ((1u << lane) - 1u));
+        if (q < n) {
+          item = q;
+          if (!begin(q, r)) {
+            end(q, r);
+            item = -1;
+          }
+        }
+      }
+      __syncwarp();
+      idle = __ballot_sync(0xffffffffu, item < 0);
+    }
+    if (idle == 0xffffffffu) break;
+    if (item >= 0 && !r.attempt(th, tol, maxsub, err)) {
+      end(item, r);
+      item = -1;
+    }
+    __syncwarp();
+  }
 }
 
 // Integrated source of cell i (sourceterm.f90:43-51 with omega replaced by
 // the mean rate over the cell's pseudo time step):
-//   src_k = vol * (rho * ((Y_k(step) - Y_k) / step)).
-template <int NSP, class N>
-__device__ __forceinline__ void integrate_cell(const Dev& d, const ThermoDev<NSP>& th, int i, double tol, int maxsub,
-                                               int* nsub, unsigned& err) {
+//   src_k = vol * (rho * ((Y_k(step) - Y_k) / step)), with the reactor's rho = p / (R_mix T).
+template <int NSP, class N, class Cell>
+__device__ __forceinline__ void run_cells(const Dev& d, const ThermoDev<NSP>& th, int n, Cell cell, double tol,
+                                          int maxsub, int* nsub, unsigned* counter) {
   constexpr int V = 3 + NSP;
   const int NE = d.NE;
-  N P[V], P0[V], Y[NSP], Cp, gama, Rcpcv;
+  unsigned err = 0;
+  run_queue<NSP, N>(
+      th, n, counter, tol, maxsub, err,
+      [&](int q, Reactor<NSP, N>& r) {
+        const int i = cell(q);
 #pragma unroll
-  for (int k = 0; k < V; ++k) { P[k] = d.PA[k * NE + i]; P0[k] = P[k]; }
+        for (int k = 0; k < V; ++k) r.P[k] = d.PA[k * NE + i];
+        return r.begin(th, N(d.step[i]), err);
+      },
+      [&](int q, const Reactor<NSP, N>& r) {
+        const int i = cell(q);
+        nsub[i] = r.nacc;
+        const N dt = d.step[i];
+        const double vol = d.vol[i];
 #pragma unroll
-  for (int k = 0; k < NSP - 1; ++k) Y[k] = P[4 + k];
-  Y[NSP - 1] = last_y<NSP>(Y);
-  gas<NSP>(th, Y, P[3], Cp, gama, Rcpcv, err);
-  const N rho = P[0] / (P[3] * Rcpcv);
-  const N dt = d.step[i];
-  nsub[i] = chem_integrate<NSP>(th, P, dt, tol, maxsub, err);
-  const double vol = d.vol[i];
-#pragma unroll
-  for (int k = 0; k < NSP - 1; ++k) d.src[k * NE + i] = val(vol * (rho * ((P[4 + k] - P0[4 + k]) / dt)));
+        for (int k = 0; k < NSP - 1; ++k)
+          d.src[k * NE + i] = val(vol * (r.rho * ((r.P[4 + k] - d.PA[(4 + k) * NE + i]) / dt)));
+      });
+  flag(d, err);
 }
 
 // Cells are taken in `order` (longest previous integration first, so the long
-// cells start early and warps hold cells of similar cost), or in cell order
-// when order is null.
+// cells start early), or in cell order when order is null.
 template <int NSP, class N>
-__global__ void __launch_bounds__(CHEM_THREADS) k_chem_source(const Dev d, const ThermoDev<NSP> th, double tol,
+__global__ void __launch_bounds__(CHEM_THREADS, 3) k_chem_source(const Dev d, const ThermoDev<NSP> th, double tol,
                                                               int maxsub, int* __restrict__ nsub,
                                                               const int* __restrict__ order, unsigned* counter) {
-  const int NE = d.NE;
-  unsigned err = 0;
-  for (;;) {
-    const int base = next_chunk(counter);
-    if (base >= NE) break;
-    const int q = base + (threadIdx.x & 31);
-    if (q < NE) integrate_cell<NSP, N>(d, th, order ? order[q] : q, tol, maxsub, nsub, err);
-  }
-  flag(d, err);
+  run_cells<NSP, N>(d, th, d.NE, [&](int q) { return order ? order[q] : q; }, tol, maxsub, nsub, counter);
 }
 
 // Counting sort of the cells by their previous substep count, descending
 // (bucket 255 - min(nsub, 255)); the order inside a bucket does not matter.
-constexpr int NBUCKET = 256;
-__global__ void k_chem_hist(const int* __restrict__ nsub, int n, unsigned* hist) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) atomicAdd(&hist[NBUCKET - 1 - min(max(nsub[i], 0), NBUCKET - 1)], 1u);
+// Most cells share a few counts (1, or the cap), so the counting is aggregated:
+// the lanes of a warp that hold one bucket add once, in shared memory, and a
+// block adds its non-empty buckets to the global counters (one global atomic
+// per cell on the same address took 0.6 ms per kernel on a million cells).
+constexpr int NBUCKET = 256, SORT_ITEMS = 8;  // items per thread of the NBUCKET-thread sort blocks
+__device__ __forceinline__ int chem_bucket(int n) { return NBUCKET - 1 - min(max(n, 0), NBUCKET - 1); }
+// adds the warp's `in` lanes to cnt[bucket]; each lane's place in the bucket
+__device__ __forceinline__ unsigned bucket_add(unsigned* cnt, int bucket, bool in) {
+  const int lane = threadIdx.x & 31;
+  const unsigned act = __ballot_sync(0xffffffffu, in);
+  unsigned place = 0;
+  if (in) {
+    const unsigned m = __match_any_sync(act, bucket);
+    unsigned base = 0;
+    if (lane == __ffs(m) - 1) base = atomicAdd(&cnt[bucket], (unsigned)__popc(m));
+    place = __shfl_sync(m, base, __ffs(m) - 1) + __popc(m & ((1u << lane) - 1u));
+  }
+  __syncwarp();
+  return place;
+}
+__global__ void __launch_bounds__(NBUCKET) k_chem_hist(const int* __restrict__ nsub, int n, unsigned* hist) {
+  __shared__ unsigned cnt[NBUCKET];
+  cnt[threadIdx.x] = 0;
+  __syncthreads();
+  for (int u = 0; u < SORT_ITEMS; ++u) {
+    const int i = (blockIdx.x * SORT_ITEMS + u) * NBUCKET + threadIdx.x;
+    bucket_add(cnt, i < n ? chem_bucket(nsub[i]) : 0, i < n);
+  }
+  __syncthreads();
+  if (cnt[threadIdx.x]) atomicAdd(&hist[threadIdx.x], cnt[threadIdx.x]);
 }
 __global__ void k_chem_scan(unsigned* hist) {  // one block of NBUCKET threads: exclusive scan in place
   __shared__ unsigned sh[NBUCKET];
@@ -81,50 +148,60 @@ __global__ void k_chem_scan(unsigned* hist) {  // one block of NBUCKET threads: 
   }
   hist[t] = t ? sh[t - 1] : 0u;
 }
-__global__ void k_chem_scatter(const int* __restrict__ nsub, int n, unsigned* cursor, int* __restrict__ order) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) order[atomicAdd(&cursor[NBUCKET - 1 - min(max(nsub[i], 0), NBUCKET - 1)], 1u)] = i;
+__global__ void __launch_bounds__(NBUCKET) k_chem_scatter(const int* __restrict__ nsub, int n, unsigned* cursor,
+                                                          int* __restrict__ order) {
+  __shared__ unsigned cnt[NBUCKET], base[NBUCKET];
+  cnt[threadIdx.x] = 0;
+  __syncthreads();
+  unsigned place[SORT_ITEMS];
+  int bucket[SORT_ITEMS];
+#pragma unroll
+  for (int u = 0; u < SORT_ITEMS; ++u) {
+    const int i = (blockIdx.x * SORT_ITEMS + u) * NBUCKET + threadIdx.x;
+    bucket[u] = i < n ? chem_bucket(nsub[i]) : 0;
+    place[u] = bucket_add(cnt, bucket[u], i < n);
+  }
+  __syncthreads();
+  base[threadIdx.x] = cnt[threadIdx.x] ? atomicAdd(&cursor[threadIdx.x], cnt[threadIdx.x]) : 0u;
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < SORT_ITEMS; ++u) {
+    const int i = (blockIdx.x * SORT_ITEMS + u) * NBUCKET + threadIdx.x;
+    if (i < n) order[base[bucket[u]] + place[u]] = i;
+  }
 }
 
 // The same for the cells list[0 .. *nlist) (the surrogate's fallbacks).
 template <int NSP, class N>
-__global__ void __launch_bounds__(CHEM_THREADS) k_chem_list(const Dev d, const ThermoDev<NSP> th, double tol,
+__global__ void __launch_bounds__(CHEM_THREADS, 3) k_chem_list(const Dev d, const ThermoDev<NSP> th, double tol,
                                                             int maxsub, int* __restrict__ nsub,
                                                             const int* __restrict__ list,
                                                             const unsigned* __restrict__ nlist, unsigned* counter) {
-  const int n = (int)min(*nlist, (unsigned)d.NE);
-  unsigned err = 0;
-  for (;;) {
-    const int base = next_chunk(counter);
-    if (base >= n) break;
-    const int q = base + (threadIdx.x & 31);
-    if (q < n) integrate_cell<NSP, N>(d, th, list[q], tol, maxsub, nsub, err);
-  }
-  flag(d, err);
+  run_cells<NSP, N>(d, th, (int)min(*nlist, (unsigned)d.NE), [&](int q) { return list[q]; }, tol, maxsub, nsub,
+                    counter);
 }
 
 // n primitive states in SoA ([k*n + i]) integrated over dt[i].
 template <int NSP, class N>
-__global__ void __launch_bounds__(CHEM_THREADS) k_chem_batch(const ThermoDev<NSP> th, const double* __restrict__ Pin,
+__global__ void __launch_bounds__(CHEM_THREADS, 3) k_chem_batch(const ThermoDev<NSP> th, const double* __restrict__ Pin,
                                                              const double* __restrict__ dts, int n,
                                                              double* __restrict__ Pout, int* __restrict__ nsub,
                                                              double tol, int maxsub, unsigned* counter,
                                                              unsigned* errp) {
   constexpr int V = 3 + NSP;
   unsigned err = 0;
-  for (;;) {
-    const int base = next_chunk(counter);
-    if (base >= n) break;
-    const int i = base + (threadIdx.x & 31);
-    if (i < n) {
-      N P[V];
+  run_queue<NSP, N>(
+      th, n, counter, tol, maxsub, err,
+      [&](int i, Reactor<NSP, N>& r) {
 #pragma unroll
-      for (int k = 0; k < V; ++k) P[k] = Pin[(size_t)k * n + i];
-      nsub[i] = chem_integrate<NSP, N>(th, P, dts[i], tol, maxsub, err);
+        for (int k = 0; k < V; ++k) r.P[k] = Pin[(size_t)k * n + i];
+        return r.begin(th, N(dts[i]), err);
+      },
+      [&](int i, const Reactor<NSP, N>& r) {
+        nsub[i] = r.nacc;
 #pragma unroll
-      for (int k = 0; k < V; ++k) Pout[(size_t)k * n + i] = val(P[k]);
-    }
-  }
+        for (int k = 0; k < V; ++k) Pout[(size_t)k * n + i] = val(r.P[k]);
+      });
   if (err) atomicOr(errp, err);
 }
 
@@ -145,13 +222,13 @@ template <int NSP>
 void chem_source(const Dev& d, const void* th, double tol, int maxsub, int* nsub, int* order, unsigned* hist,
                  unsigned* counter, cudaStream_t s) {
   if (order) {
-    const int nb = (d.NE + 255) / 256;
+    const int nb = (d.NE + NBUCKET * SORT_ITEMS - 1) / (NBUCKET * SORT_ITEMS);
     cudaMemsetAsync(hist, 0, sizeof(unsigned) * NBUCKET, s);
-    k_chem_hist<<<nb, 256, 0, s>>>(nsub, d.NE, hist);
+    k_chem_hist<<<nb, NBUCKET, 0, s>>>(nsub, d.NE, hist);
     k_chem_scan<<<1, NBUCKET, 0, s>>>(hist);
-    k_chem_scatter<<<nb, 256, 0, s>>>(nsub, d.NE, hist, order);
+    k_chem_scatter<<<nb, NBUCKET, 0, s>>>(nsub, d.NE, hist, order);
   }
-  auto k = k_chem_source<NSP, double>;
+  auto k = k_chem_source<NSP, ChemNum>;
   const int grid = chem_grid(k, d.NE);
   cudaMemsetAsync(counter, 0, sizeof(unsigned), s);
   k<<<grid, CHEM_THREADS, 0, s>>>(d, *static_cast<const ThermoDev<NSP>*>(th), tol, maxsub, nsub, order, counter);
@@ -160,7 +237,7 @@ void chem_source(const Dev& d, const void* th, double tol, int maxsub, int* nsub
 template <int NSP>
 void chem_list(const Dev& d, const void* th, double tol, int maxsub, int* nsub, const int* list,
                const unsigned* nlist, unsigned* counter, cudaStream_t s) {
-  auto k = k_chem_list<NSP, double>;
+  auto k = k_chem_list<NSP, ChemNum>;
   const int grid = chem_grid(k, d.NE);
   cudaMemsetAsync(counter, 0, sizeof(unsigned), s);
   k<<<grid, CHEM_THREADS, 0, s>>>(d, *static_cast<const ThermoDev<NSP>*>(th), tol, maxsub, nsub, list, nlist, counter);
@@ -170,7 +247,7 @@ template <int NSP>
 void chem_batch(const void* th, const double* P, const double* dt, int n, double* out, int* nsub, double tol,
                 int maxsub, unsigned* counter, unsigned* errp, cudaStream_t s) {
   cudaMemsetAsync(counter, 0, sizeof(unsigned), s);
-  auto k = k_chem_batch<NSP, double>;
+  auto k = k_chem_batch<NSP, ChemNum>;
   const int grid = chem_grid(k, n);
   k<<<grid, CHEM_THREADS, 0, s>>>(*static_cast<const ThermoDev<NSP>*>(th), P, dt, n, out, nsub, tol,
                                                   maxsub, counter, errp);

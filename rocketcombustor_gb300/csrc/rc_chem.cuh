@@ -132,37 +132,42 @@ __device__ __forceinline__ void dwdp(const ThermoDev<NSP>& th, const N* pri, N* 
 }
 
 // Gaussian elimination with partial pivoting, in place; b gets the solution.
-// Returns false for a singular matrix.
+// Returns false for a singular matrix.  Columns are a template recursion, so
+// that every index is known and the system stays in registers (a loop over
+// the columns was left rolled, with the matrix in local memory).
+template <int NV, int K, class N>
+__device__ __forceinline__ bool gepp_column(N* A, N* b) {
+  int piv = K;
+  N best = n_abs(A[K * NV + K]);
+#pragma unroll
+  for (int r = K + 1; r < NV; ++r) {
+    const N a = n_abs(A[r * NV + K]);
+    if (less(best, a)) { best = a; piv = r; }
+  }
+  if (!less(N(0.0), best)) return false;
+  if (piv != K) {
+#pragma unroll
+    for (int r = K + 1; r < NV; ++r)
+      if (r == piv) {
+#pragma unroll
+        for (int c = K; c < NV; ++c) { const N t = A[K * NV + c]; A[K * NV + c] = A[r * NV + c]; A[r * NV + c] = t; }
+        const N t = b[K]; b[K] = b[r]; b[r] = t;
+      }
+  }
+  const N dk = A[K * NV + K];
+#pragma unroll
+  for (int r = K + 1; r < NV; ++r) {
+    const N f = A[r * NV + K] / dk;
+#pragma unroll
+    for (int c = K + 1; c < NV; ++c) A[r * NV + c] = A[r * NV + c] - f * A[K * NV + c];
+    b[r] = b[r] - f * b[K];
+  }
+  if constexpr (K + 1 < NV) return gepp_column<NV, K + 1>(A, b);
+  return true;
+}
 template <int NV, class N>
 __device__ __forceinline__ bool gepp_solve(N* A, N* b) {
-#pragma unroll
-  for (int k = 0; k < NV; ++k) {
-    int piv = k;
-    N best = n_abs(A[k * NV + k]);
-#pragma unroll
-    for (int r = k + 1; r < NV; ++r) {
-      const N a = n_abs(A[r * NV + k]);
-      if (less(best, a)) { best = a; piv = r; }
-    }
-    if (!less(N(0.0), best)) return false;
-    if (piv != k) {
-#pragma unroll
-      for (int r = k + 1; r < NV; ++r)
-        if (r == piv) {
-#pragma unroll
-          for (int c = 0; c < NV; ++c) { const N tmp = A[k * NV + c]; A[k * NV + c] = A[r * NV + c]; A[r * NV + c] = tmp; }
-          const N tb = b[k]; b[k] = b[r]; b[r] = tb;
-        }
-    }
-    const N dk = A[k * NV + k];
-#pragma unroll
-    for (int r = k + 1; r < NV; ++r) {
-      const N f = A[r * NV + k] / dk;
-#pragma unroll
-      for (int c = k + 1; c < NV; ++c) A[r * NV + c] = A[r * NV + c] - f * A[k * NV + c];
-      b[r] = b[r] - f * b[k];
-    }
-  }
+  if (!gepp_column<NV, 0>(A, b)) return false;
 #pragma unroll
   for (int k = NV - 1; k >= 0; --k) {
     N s = b[k];
@@ -173,37 +178,42 @@ __device__ __forceinline__ bool gepp_solve(N* A, N* b) {
   return true;
 }
 
-// Integrates primitive state P (in place) over dt; returns the accepted substeps.
+// One reactor on its way: primitive state P, its fixed rho and e, the time
+// left and the next substep.
 template <int NSP, class N>
-__device__ __noinline__ int chem_integrate(const ThermoDev<NSP>& th, N* P, N dt, double tol, int maxsub,
-                                           unsigned& err) {
-  constexpr int V = 3 + NSP, NS1 = NSP - 1;
-  N Y2[NSP], entha[NSP], A[V * V], J[V * V], D[(NS1 > 0 ? NS1 : 1) * V], b[V], prod[NSP], Cp, gama, Rcpcv;
-  N s = 0.0;
+struct Reactor {
+  N P[3 + NSP], rho, e, rem, hs;
+  int nacc, natt;
+
+  // starts at P over dt; false when there is nothing to integrate
+  __device__ __forceinline__ bool begin(const ThermoDev<NSP>& th, N dt, unsigned& err) {
+    N Y[NSP], entha[NSP], Cp, gama, Rcpcv;
 #pragma unroll
-  for (int i = 0; i < NS1; ++i) { Y2[i] = P[4 + i]; s = s + Y2[i]; }
-  Y2[NSP - 1] = 1. - s;
-  gas<NSP>(th, Y2, P[3], Cp, gama, Rcpcv, err);
-  const N rho = P[0] / (Rcpcv * P[3]);
-  enthalpy<NSP>(th, P[3], entha, err);
-  N h = 0.0;
-#pragma unroll
-  for (int i = 0; i < NSP; ++i) h = h + Y2[i] * entha[i];
-  const N e = h - Rcpcv * P[3];
-  N rem = dt, hs = dt;
-  int nacc = 0, natt = 0;
-  while (less(N(0.0), rem)) {
+    for (int i = 0; i < NSP - 1; ++i) Y[i] = P[4 + i];
+    Y[NSP - 1] = last_y<NSP>(Y);
+    gas<NSP>(th, Y, P[3], Cp, gama, Rcpcv, err);
+    rho = P[0] / (Rcpcv * P[3]);
+    enthalpy<NSP>(th, P[3], entha, err);
+    e = dot<NSP>(Y, entha) - Rcpcv * P[3];
+    rem = dt;
+    hs = dt;
+    nacc = 0;
+    natt = 0;
+    return less(N(0.0), rem);
+  }
+
+  // one attempted substep; false when the reactor has reached its end
+  __device__ __forceinline__ bool attempt(const ThermoDev<NSP>& th, double tol, int maxsub, unsigned& err) {
+    constexpr int V = 3 + NSP, NS1 = NSP - 1;
+    N A[V * V], D[(NS1 > 0 ? NS1 : 1) * V], b[V], prod[NSP], Y[NSP], Rcpcv;
     const bool last = nacc + 1 >= maxsub || natt >= 2 * maxsub;
     if (last || less(rem, hs)) hs = rem;
-    con_to_pri_jaco<NSP>(th, P, J, err);
+    con_to_pri_jaco<NSP>(th, P, A, err);
     dwdp<NSP>(th, P, D, err);
-    N yc[NSP], sc = 0.0;
 #pragma unroll
-    for (int i = 0; i < NS1; ++i) { yc[i] = P[4 + i]; sc = sc + yc[i]; }
-    yc[NSP - 1] = 1. - sc;
-    production<NSP>(th, P[3], rho, yc, prod);
-#pragma unroll
-    for (int k = 0; k < V * V; ++k) A[k] = J[k];
+    for (int i = 0; i < NS1; ++i) Y[i] = P[4 + i];
+    Y[NSP - 1] = last_y<NSP>(Y);
+    production<NSP>(th, P[3], rho, Y, prod);
 #pragma unroll
     for (int i = 0; i < NS1; ++i)
 #pragma unroll
@@ -212,23 +222,20 @@ __device__ __noinline__ int chem_integrate(const ThermoDev<NSP>& th, N* P, N dt,
     for (int k = 0; k < 4; ++k) b[k] = 0.0;
 #pragma unroll
     for (int i = 0; i < NS1; ++i) b[4 + i] = hs * prod[i];
-    if (!gepp_solve<V>(A, b)) { err |= ERR_NAN; break; }
+    if (!gepp_solve<V>(A, b)) { err |= ERR_NAN; return false; }
     ++natt;
     N d = n_abs(b[3]) / (N(0.1) * tol * P[3]);
 #pragma unroll
     for (int i = 0; i < NS1; ++i) d = fmax2(d, n_abs(b[4 + i]) / (N(tol) * (n_abs(P[4 + i]) + 1.0e-3)));
     if (less(N(1.0), d) && !last) {
       hs = hs * fmax2(N(0.2), 0.9 / d);
-      continue;
+      return true;
     }
 #pragma unroll
-    for (int i = 0; i < NS1; ++i) P[4 + i] = P[4 + i] + b[4 + i];
-    s = 0.0;
-#pragma unroll
-    for (int i = 0; i < NS1; ++i) { Y2[i] = P[4 + i]; s = s + Y2[i]; }
-    Y2[NSP - 1] = 1. - s;
+    for (int i = 0; i < NS1; ++i) { P[4 + i] = P[4 + i] + b[4 + i]; Y[i] = P[4 + i]; }
+    Y[NSP - 1] = last_y<NSP>(Y);
     const N tg = fmin2(fmax2(P[3] + b[3], N(th.tlo)), N(th.thi));
-    const N t = newton_T<NSP>(th, e, Y2, tg, Rcpcv, err);
+    const N t = newton_T<NSP>(th, e, Y, tg, Rcpcv, err);
     P[3] = t;
     P[0] = rho * Rcpcv * t;
     rem = rem - hs;
@@ -236,8 +243,8 @@ __device__ __noinline__ int chem_integrate(const ThermoDev<NSP>& th, N* P, N dt,
     if (less(N(0.0), d)) hs = hs * fmin2(N(2.0), 0.9 / d);
     else hs = twice_of(hs);
     if (less(rem - hs, 0.01 * hs)) hs = rem;
+    return less(N(0.0), rem);
   }
-  return nacc;
-}
+};
 
 }  // namespace rc
