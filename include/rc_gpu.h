@@ -19,14 +19,19 @@
  * Threading: one host thread per context; each context owns one CUDA stream.
  *
  * LU-SGS schedule: by default both sweeps of an iteration run as one
- * cooperative dataflow kernel (per-SM blocks of cells, each pass waiting only
- * for the passes of other blocks that hold its neighbours; FP64 and mixed
- * forms each have theirs); rc_autotune picks the fastest of the schedules,
- * and the environment variable RC_LUSGS_SCHEDULE, read by rc_init, fixes one:
- * "flow", "levels", "levels8", "levels2w", "levels4w" (one kernel per level,
- * with 4 or 8 lanes per cell or, in the FP64 form, each slot's work over two
- * or four warps) or "persistent" (one cooperative kernel with a grid-wide
- * level counter).  All compute the same recurrences bit for bit.
+ * cooperative dataflow kernel with compact passes (blocks of cells on as many
+ * SMs as shorten the chain of levels, each pass waiting only for the passes of
+ * other blocks that hold its neighbours; FP64 and mixed forms each have
+ * theirs), or as one kernel per level where a level alone fills the GPU or, in
+ * the mixed forms, where there are at most 16 levels; rc_autotune picks the
+ * fastest of the schedules, and the environment variable RC_LUSGS_SCHEDULE,
+ * read by rc_init, fixes one: "flowc", "flowc2" (compact passes of one or two
+ * groups), "flow", "flow2", "flow3" (passes of 1..3 groups of 8 cells with a
+ * lane per slot, one block per SM), "levels", "levels8", "levels2w",
+ * "levels4w" (one kernel per level, with 4 or 8 lanes per cell or, in the FP64
+ * form, each slot's work over two or four warps) or "persistent" (one
+ * cooperative kernel with a grid-wide level counter).  All compute the same
+ * recurrences bit for bit.
  */
 #ifndef RC_GPU_H
 #define RC_GPU_H

@@ -1086,278 +1086,326 @@ __global__ void __launch_bounds__(flow_threads(G), 1) k_lusgs_flow(const Dev d, 
 // In a sweep only the faces to lower (forward) or upper (backward) neighbours
 // carry a term: on a triangulation about 1.5 of a cell's 3 slots.  The
 // per-slot lanes of k_lusgs_flow spend the other lanes' FP64 issue on terms
-// that are zero.  Here a group of four warps takes up to 32 ACTIVE (cell,
-// slot) pairs of up to 16 consecutive cells, one pair per lane, so one
-// group holds about twice the cells of a k_lusgs_flow group on the same
-// FP64 instruction count.  The finishing sums add only the active slots, in
-// slot order: a sum that starts at +0.0 is never -0.0, so leaving out the
-// +0.0 terms of the inactive slots leaves its bits unchanged.
+// that are zero.  Here a group of eight warps takes up to 32 ACTIVE (cell,
+// slot) pairs of up to flowc_cells(V) consecutive cells, one pair per lane.
+// The finishing sums add only the active slots, in slot order: a sum that
+// starts at +0.0 is never -0.0, so leaving out the +0.0 terms of the inactive
+// slots leaves its bits unchanged.
 constexpr int FLOWC_GMAX = 2;
-constexpr int FLOWC_STAGERS = 2, FLOWC_NBUF = 4;
-// compute groups, the coordinator warp, the staging warps
-__host__ __device__ constexpr int flowc_threads(int G) { return 128 * G + 32 + 32 * FLOWC_STAGERS; }
-// What the sweep step of one active pair needs (the neighbour j's gas state
-// and its products, the face), staged before the pass may start: the fields
-// of SweepPre that the step reads, formed with the same expressions.
+constexpr int FLOWC_NBUF = 6;
+__host__ __device__ constexpr int flowc_preps(int G) { return G == 1 ? 5 : 3; }
+// compute groups, the starting warp, the publishing warps, the preparing warps
+__host__ __device__ constexpr int flowc_threads(int G) { return 256 * G + 32 + 32 * FLOWC_PUBS + 32 * flowc_preps(G); }
+// One group's part of a ring slot: what the sweep step of its 32 pairs needs
+// (the neighbour's gas state and its products, the face; a field per row, so
+// that a warp reads a row without bank conflicts), the increments of the
+// neighbours that an earlier pass or another block wrote (nb), and the group's
+// cells.
 template <int NSP>
-struct PairPre {
-  int j;   // the neighbour (-1: no pair in this lane)
-  int cs;  // the pair's cell within its group << 2 | its slot
-  double dx, dy, uu, vv, tt, rr, gama, aF;
-  double rrh, rrl, gmh, gml;
-  double rou, rov, gm1, roepp, unormal;
-  double cs_h[NSP];
-  double ry[NSP > 1 ? NSP - 1 : 1];
+struct FlowcSlot {
+  static constexpr int V = 3 + NSP, NS = NSP > 1 ? NSP - 1 : 1, CAP = flowc_cells(V);
+  double dx[32], dy[32], uu[32], vv[32], tt[32], rr[32], gama[32], aF[32], rou[32], rov[32], gm1[32], roepp[32], un[32];
+  double h[NSP][32], ry[NS][32];
+  double nb[V][32];
+  double rrh[32], rrl[32], gmh[32], gml[32];  // reciprocal pairs of rr and gm1
+  double dd[CAP], ddh[CAP], ddl[CAP];
+  int j[32];         // the neighbour (-1: no pair in this lane)
+  int src[32];       // where its increments are among those of the block's last passes, -1: in nb
+  int cell[CAP];     // the group's cells (-1 past the last)
+  int pairs[CAP];    // a cell's first pair, its number of pairs << 8
 };
-template <int NSP, bool FWD>
-__device__ __forceinline__ PairPre<NSP> pair_load(const Dev& d, int t, int q, int tg) {
-  constexpr int DIR = FWD ? 0 : 1;
-  const int NE = d.NE, NF = d.NF;
-  PairPre<NSP> p;
-  const int j = d.swj[DIR][q * NE + t], fs = d.swf[DIR][q * NE + t], f = fs >= 0 ? fs : ~fs;
-  p.j = j;
-  p.cs = ((t - tg) << 2) | q;
-  p.dx = d.fvec[f];
-  p.dy = d.fvec[NF + f];
-  if (fs < 0) { p.dx = -p.dx; p.dy = -p.dy; }
-  const double pp = d.PA[0 * NE + j];
-  p.uu = d.PA[1 * NE + j]; p.vv = d.PA[2 * NE + j]; p.tt = d.PA[3 * NE + j];
-  p.rr = d.cst[0 * NE + j]; p.gama = d.cst[1 * NE + j];
-  const double roe = d.cst[2 * NE + j];
-  p.rrh = d.rcp[0 * NE + j]; p.rrl = d.rcp[1 * NE + j]; p.gmh = d.rcp[2 * NE + j]; p.gml = d.rcp[3 * NE + j];
-  p.aF = d.alpaF[f];
-#pragma unroll
-  for (int k = 0; k < NSP; ++k) p.cs_h[k] = d.cst[(3 + k) * NE + j];
-#pragma unroll
-  for (int k = 0; k < NSP - 1; ++k) p.ry[k] = p.rr * d.PA[(4 + k) * NE + j];
-  p.rou = p.rr * p.uu;
-  p.rov = p.rr * p.vv;
-  p.gm1 = p.gama - 1;
-  p.roepp = roe + pp;
-  p.unormal = p.uu * p.dx + p.vv * p.dy;
-  return p;
-}
-// one ring slot: G groups of 32 pairs and 16 cells
 template <int NSP, int G>
-__host__ __device__ constexpr int flowc_slot_bytes() {
-  return (int)(32 * G * sizeof(PairPre<NSP>) + flowc_cells(3 + NSP) * G * 32);
-}
-template <int NSP, int G>
-__host__ __device__ constexpr int flowc_dsmem() { return FLOWC_NBUF * flowc_slot_bytes<NSP, G>(); }
-// The cell a finishing lane needs: its index, dd and dd's reciprocal pair,
-// and its active slots (bit q: slot q has a neighbour in this sweep).
-struct FinC {
-  int i, mask;
-  double dd, ddh, ddl;
-};
-template <bool FWD>
-__device__ __forceinline__ FinC finc_load(const Dev& d, int t) {
-  constexpr int DIR = FWD ? 0 : 1;
-  FinC f;
-  const int NE = d.NE;
-  f.i = d.swi[DIR][t];
-  f.dd = d.dd[f.i];
-  f.ddh = d.rcp[4 * NE + f.i];
-  f.ddl = d.rcp[5 * NE + f.i];
-  f.mask = 0;
+__host__ __device__ constexpr int flowc_dsmem() { return FLOWC_NBUF * G * (int)sizeof(FlowcSlot<NSP>); }
+
+// Stages one group of pass k: pairs [e0, e0 + np) of the plan's pair lists,
+// cells at sweep positions [t0, t0 + nc).  All loads are issued before `wait`
+// (the slot becoming free), the stores follow.  The products of the
+// neighbour's constants are formed with the operations of the reference
+// expressions, the multiplications on the integer pipes: the FP64 units belong
+// to the compute warps.
+template <int NSP, bool FWD, class Wait>
+__device__ __forceinline__ bool flowc_stage(const Dev& d, const FlowDev& f, FlowcSlot<NSP>& s, int k, int G, int e0,
+                                            int np, int t0, int nc, Wait wait) {
+  constexpr int DIR = FWD ? 0 : 1, NS = FlowcSlot<NSP>::NS, CAP = FlowcSlot<NSP>::CAP;
+  const int NE = d.NE, NF = d.NF, lane = threadIdx.x & 31;
+  int j = -1, src = -1, cell = -1, pairs = 0;
+  double dx = 0, dy = 0, pp = 0, uu = 0, vv = 0, tt = 0, rr = 0, gama = 0, roe = 0, aF = 0, h[NSP], Y[NS];
+  double rrh = 0, rrl = 0, gmh = 0, gml = 0, dd = 0, ddh = 0, ddl = 0;
+  if (lane < np) {
+    j = f.plj[e0 + lane];
+    src = flowc_src<3 + NSP>(f.psrc[e0 + lane], k, G);
+    const int fs = f.plf[e0 + lane], fc = fs >= 0 ? fs : ~fs;
+    dx = d.fvec[fc];
+    dy = d.fvec[NF + fc];
+    if (fs < 0) { dx = -dx; dy = -dy; }
+    aF = d.alpaF[fc];
+    pp = d.PA[0 * NE + j]; uu = d.PA[1 * NE + j]; vv = d.PA[2 * NE + j]; tt = d.PA[3 * NE + j];
+    rr = d.cst[0 * NE + j]; gama = d.cst[1 * NE + j]; roe = d.cst[2 * NE + j];
+    rrh = d.rcp[0 * NE + j]; rrl = d.rcp[1 * NE + j]; gmh = d.rcp[2 * NE + j]; gml = d.rcp[3 * NE + j];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) f.mask |= (d.swj[DIR][q * NE + t] >= 0 ? 1 : 0) << q;
-  return f;
+    for (int k = 0; k < NSP; ++k) h[k] = d.cst[(3 + k) * NE + j];
+#pragma unroll
+    for (int k = 0; k < NSP - 1; ++k) Y[k] = d.PA[(4 + k) * NE + j];
+  }
+  if (lane < nc) {
+    cell = d.swi[DIR][t0 + lane];
+    const int p0 = f.ppos[DIR][t0 + lane];
+    pairs = (p0 - e0) | (f.ppos[DIR][t0 + lane + 1] - p0) << 8;
+    dd = d.dd[cell];
+    ddh = d.rcp[4 * NE + cell];
+    ddl = d.rcp[5 * NE + cell];
+  }
+  if (!wait()) return false;
+  if (lane < np) {
+    s.dx[lane] = dx; s.dy[lane] = dy; s.uu[lane] = uu; s.vv[lane] = vv; s.tt[lane] = tt;
+    s.rr[lane] = rr; s.gama[lane] = gama; s.aF[lane] = aF;
+    s.rrh[lane] = rrh; s.rrl[lane] = rrl; s.gmh[lane] = gmh; s.gml[lane] = gml;
+    s.rou[lane] = rcs::mul(rr, uu);
+    s.rov[lane] = rcs::mul(rr, vv);
+    s.gm1[lane] = gama - 1;
+    s.roepp[lane] = roe + pp;
+    s.un[lane] = rcs::mul(uu, dx) + rcs::mul(vv, dy);
+#pragma unroll
+    for (int k = 0; k < NSP; ++k) s.h[k][lane] = h[k];
+#pragma unroll
+    for (int k = 0; k < NSP - 1; ++k) s.ry[k][lane] = rcs::mul(rr, Y[k]);
+  }
+  s.j[lane] = j;
+  s.src[lane] = src;
+  if (lane < CAP) { s.cell[lane] = cell; s.pairs[lane] = pairs; s.dd[lane] = dd; s.ddh[lane] = ddh; s.ddl[lane] = ddl; }
+  return true;
 }
-// One group's step (threads 128 g .. 128 g + 127): in the term phases lane l
-// holds the group's l-th active pair (p; p.j < 0 past the last pair) and nbv
-// its neighbour's hWA; in the finishing phase the group's thread x = 32 role
-// + lane finishes variable x % V of local cell x / V (fn: that cell, fn.i < 0
-// past the last cell).  The expressions are sweep4w_compute's, each rounded
-// operation the same in the same order, but the parts of every term that do
-// not wait for du, dv, dp or dun are formed in phase A, where the four warps
-// have room, so that fewer dependent FP64 operations follow (on GB300 a
-// warp's FP64 instruction holds its sub-partition's FP64 unit for 64
-// cycles, so the count per warp on the critical path sets the step's time):
-//   A  warp 0: s = 0 + dY_0 + dY_1 + dY_2, dY_3 = drho - s; s1 = 0 + sum h_k dY_k;
-//      es1 = dE - s1; S_k = -aF dY_k + dY_k un for k = 0, 1
-//      warp 1: dY; s2 = 0 + sum R_k dY_k; Q = (T s2) gamma / (gamma - 1)
-//      warp 2: du = (drho u - u drho) / rho; c0; a1 = drho u * u, a3 = drho v * v;
-//      P1 = -aF drho u + drho u un
-//      warp 3: dY; dv; P2 = -aF drho v + drho v un; A3 = -aF dE; S_2
-//   B  warp 3: dun = du nx + dv ny (barrier B6 to warps 0, 1), then the species
-//      terms half(S_k + ry_k dun)
-//      warp 2: X = ((a1 + du rho u) + a3) + dv rho v, dp = gm1 ((es1 + Q) - X / 2)
-//      (barrier B8 to warps 0, 1)
-//      warp 0: c1p = P1 + rho u dun; warp 1: c2p = P2 + rho v dun, c3p = A3 + dun (rho E + p)
-//   C  warp 0: c1 = half(c1p + dp nx); warp 1: c2 = half(c2p + dp ny);
-//      warp 2: c3 = half(c3p + un (dE + dp))
-// with 0 + x and 0.5 x on the integer pipe (plus_zero, half_of: the same bits).
+
+// a / b through b's reciprocal pair (div_rn), the rare operands out of line:
+// on the chain of a pass an instruction costs about 10 cycles, so the test for
+// them is one comparison
+__device__ __noinline__ double div_other(double a, double b) { return rcs::div(a, b); }
+__device__ __forceinline__ double div_pair(double a, double b, double yh, double yl) {
+  const unsigned ea = ((unsigned)__double2hiint(a) & rcs::EXP_MASK) - rcs::EXP_LO,
+                 eb = ((unsigned)__double2hiint(b) & rcs::EXP_MASK) - rcs::EXP_LO;
+  if (max(ea, eb) > rcs::EXP_SPAN) return div_other(a, b);
+  const double q0 = fma(a, yh, a * yl);
+  return fma(fma(-b, q0, a), yh, q0);
+}
+
+// One group's step on slot s.  In the term phases lane l of each warp holds
+// the group's l-th active pair; in the finishing phase thread x = 32 role +
+// lane of warps 0-3 finishes variable x % V of local cell x / V.  ring: the
+// increments of the block's last passes, res: this pass's place there.  The
+// expressions are sweep_compute's, each rounded operation the same in the same
+// order, split over the warps by when their operands are known:
+//   warp 0: s = 0 + dY_0 + .., dY_last = drho - s; s1 = 0 + sum h_k dY_k;
+//           es1 = dE - s1 (to warp 2)
+//   warp 1: the same dY; s2 = 0 + sum R_k dY_k; Q = (T s2) gamma / (gamma - 1)
+//           (to warp 2)
+//   warp 2: du = (drho u - u drho) / rho; X' = (a1 + du rho u) + a3 with
+//           a1 = drho u * u, a3 = drho v * v; du nx (to warp 3); then
+//           X = X' + dv rho v, dp = gm1 ((es1 + Q) - X / 2) (to warps 4-6)
+//   warp 3: dv; dv rho v (to warp 2); dv ny; then dun = du nx + dv ny (to warps
+//           0, 4-7)
+//   warps 0 (k = 0) and 7 (k = 1 ..): S_k = -aF dY_k + dY_k un, after dun
+//           c_{4+k} = half(S_k + ry_k dun); warp 7 also c0
+//   warp 4: -aF dE + dun (rho E + p), + un (dE + dp): c3
+//   warp 5: P = -aF drho u + drho u un, + rho u dun, + dp nx: c1; warp 6: c2
+// Warps w and w + 4 share an SM sub-partition and its FP64 unit (62-77 cycles
+// per warp instruction whatever the active lanes): each unit gets about the
+// same number of instructions, and the chain from the neighbours' increments
+// to dp and dun holds only what it needs.
 template <int NSP, bool FWD, int G>
-__device__ __forceinline__ void sweepc_compute(const Dev& d, const ThermoDev<NSP>& th, const PairPre<NSP>& p,
-                                               const double* nbv, const FinC& fn) {
-  constexpr int V = 3 + NSP, NS = NSP > 1 ? NSP - 1 : 1;
-  const int NE = d.NE, gi = G > 1 ? (int)(threadIdx.x >> 7) : 0, role = (threadIdx.x >> 5) & 3,
-            lane = threadIdx.x & 31, q = p.cs & 3;
-  const bool act = p.j >= 0;
-  constexpr int CAP = flowc_cells(V);
-  __shared__ double wsc_g[G][CAP * V * 4];
-  // per pair: es1, Q, du, dv, dun, dp, P1, P2, A3, c3p, S_0, S_1
-  __shared__ double xc_g[G][12][32];
-  double* wsm = wsc_g[gi];
-  double(*xc)[32] = xc_g[gi];
-  enum { ES1, XQ, XDU, XDV, XDN, XDP, XP1, XP2, XA3, XC3, XS0, XS1 };
-  const int B5 = 5 + 4 * gi, B6 = B5 + 1, B7 = B5 + 2, B8 = B5 + 3;
-  const int x = role * 32 + lane, fc = x / V, r = x - fc * V;
-  const bool fvalid = fc < CAP && fn.i >= 0;
-  const int fi = fvalid ? fn.i : 0;
-  const double R = fvalid ? __ldcg(d.hWA + r * NE + fi) : 0.0;
-  double* w = wsm + min(p.cs >> 2, CAP - 1) * V * 4;
-  const double aF = p.aF, un = p.unormal;
-  const double drr = nbv[0], dru = nbv[1], drv = nbv[2], dre = nbv[3];
-  // the species increments dY_k (warps 0, 1 and 3)
-  double dry[NSP];
-#pragma unroll
-  for (int k = 0; k < NSP; ++k) dry[k] = 0.0;
-  if (role != 2 && act) {
-    double s = 0.0;
-    if (NSP > 1) {
-      dry[0] = nbv[4];
-      s = plus_zero(dry[0]);
-#pragma unroll
-      for (int k = 1; k < NSP - 1; ++k) { dry[k] = nbv[4 + k]; s = s + dry[k]; }
+__device__ __forceinline__ void flowc_step(const Dev& d, const ThermoDev<NSP>& th, const FlowcSlot<NSP>& s, int gi,
+                                           int role, const double* ring, double* res) {
+  constexpr int V = 3 + NSP, CAP = FlowcSlot<NSP>::CAP;
+  __shared__ double T_g[G][V][32];  // the pairs' terms
+  // per pair: es1, Q, dv rho v, du nx, dun, dp
+  __shared__ double x_g[G][6][32];
+  enum { ES1, XQ, XM2, XDUX, XDN, XDP };
+  double(*T)[32] = T_g[gi];
+  double(*xc)[32] = x_g[gi];
+  // barriers: es1, Q, dv, du nx ready / dun for the momentum and energy terms
+  // / terms done / dp
+  const int lane = threadIdx.x & 31, B5 = 5 + 4 * gi, B6 = B5 + 1, B7 = B5 + 2, B8 = B5 + 3;
+  const bool act = s.j[lane] >= 0;
+  const int src = s.src[lane];
+  // the neighbour's increments: variable v at np[v * ns]
+  const double* np = src >= 0 ? ring + src : &s.nb[0][lane];
+  const int ns = src >= 0 ? 1 : 32;
+  // the finishing lane's own residual (forward) or forward increment
+  int fi = -1, fc = 0, r = 0, pr = 0;
+  double R = 0.0;
+  if (role < 4) {
+    const int x = role * 32 + lane;
+    fc = x / V;
+    r = x - fc * V;
+    if (fc < CAP) {
+      fi = s.cell[fc];
+      pr = s.pairs[fc];
     }
-    dry[NSP - 1] = drr - s;
+    if (fi >= 0) R = __ldcg(d.hWA + (size_t)r * d.NE + fi);
   }
-  // A
-  double S2 = 0.0;  // warp 3: S_{NSP-2}
-  if (act) {
-    if (role == 0) {
-      double s1 = plus_zero(p.cs_h[0] * dry[0]);
-#pragma unroll
-      for (int k = 1; k < NSP; ++k) s1 = s1 + p.cs_h[k] * dry[k];
-      xc[ES1][lane] = dre - s1;
-      if (NSP > 1) xc[XS0][lane] = -aF * dry[0] + dry[0] * un;
-      if (NSP > 2) xc[XS1][lane] = -aF * dry[1] + dry[1] * un;
-    } else if (role == 1) {
-      double s2 = plus_zero(th.R[0] * dry[0]);
-#pragma unroll
-      for (int k = 1; k < NSP; ++k) s2 = s2 + th.R[k] * dry[k];
-      xc[XQ][lane] = div_rn(p.tt * s2 * p.gama, p.gm1, p.gmh, p.gml);
-    } else if (role == 2) {
-      xc[XDU][lane] = div_rn(dru - p.uu * drr, p.rr, p.rrh, p.rrl);
-      w[q] = half_of(-aF * drr + dru * p.dx + drv * p.dy);
-      xc[XP1][lane] = -aF * dru + dru * un;
-    } else {
-      xc[XDV][lane] = div_rn(drv - p.vv * drr, p.rr, p.rrh, p.rrl);
-      xc[XP2][lane] = -aF * drv + drv * un;
-      xc[XA3][lane] = -aF * dre;
-      if (NSP > 3) S2 = -aF * dry[2] + dry[2] * un;
-    }
-  }
-  // the X partials of warp 2, formed while the others finish phase A
-  double a1 = 0.0, a3 = 0.0;
-  if (role == 2 && act) {
-    a1 = dru * p.uu;
-    a3 = drv * p.vv;
-  }
-  bar_named(B5, 128);
-  // B, C
-  if (role == 3) {
-    double dun = 0.0;
+  if (role < 2) {
+    double dY[NSP];
     if (act) {
-      dun = xc[XDU][lane] * p.dx + xc[XDV][lane] * p.dy;
-      xc[XDN][lane] = dun;
-    }
-    bar_arrive(B6, 96);
-    if (act) {
+      const double drr = np[0];
+      double q = 0.0;
+      if (NSP > 1) {
+        dY[0] = np[4 * ns];
+        q = plus_zero(dY[0]);
 #pragma unroll
-      for (int k = 0; k < NSP - 1; ++k) {
-        const double Sk = k == 0 ? xc[XS0][lane] : k == 1 ? xc[XS1][lane] : S2;
-        w[(4 + k) * 4 + q] = half_of(Sk + p.ry[k] * dun);
+        for (int k = 1; k < NSP - 1; ++k) { dY[k] = np[(4 + k) * ns]; q = q + dY[k]; }
       }
+      dY[NSP - 1] = drr - q;
+      if (role == 0) {
+        const double dre = np[3 * ns];
+        double s1 = plus_zero(s.h[0][lane] * dY[0]);
+#pragma unroll
+        for (int k = 1; k < NSP; ++k) s1 = s1 + s.h[k][lane] * dY[k];
+        xc[ES1][lane] = dre - s1;
+      } else {
+        double s2 = plus_zero(th.R[0] * dY[0]);
+#pragma unroll
+        for (int k = 1; k < NSP; ++k) s2 = s2 + th.R[k] * dY[k];
+        xc[XQ][lane] = div_pair(s.tt[lane] * s2 * s.gama[lane], s.gm1[lane], s.gmh[lane], s.gml[lane]);
+      }
+    }
+    bar_arrive(B5, 128);
+    if (NSP > 1 && role == 0) {
+      double S = 0.0;
+      if (act) S = -s.aF[lane] * dY[0] + dY[0] * s.un[lane];
+      bar_named(B6, 192);
+      if (act) T[4][lane] = half_of(S + s.ry[0][lane] * xc[XDN][lane]);
     }
   } else if (role == 2) {
-    double dpp = 0.0;
+    double X = 0.0;
     if (act) {
-      const double duu = xc[XDU][lane], dvv = xc[XDV][lane];
-      const double X = a1 + duu * p.rou + a3 + dvv * p.rov;
-      dpp = p.gm1 * (xc[ES1][lane] + xc[XQ][lane] - half_of(X));
-      xc[XDP][lane] = dpp;
+      const double uu = s.uu[lane], dru = np[ns];
+      const double du = div_pair(dru - uu * np[0], s.rr[lane], s.rrh[lane], s.rrl[lane]);
+      xc[XDUX][lane] = du * s.dx[lane];
+      X = dru * uu + du * s.rou[lane] + np[2 * ns] * s.vv[lane];
     }
-    bar_named(B8, 96);
-    if (act) w[3 * 4 + q] = half_of(xc[XC3][lane] + un * (dre + dpp));
-  } else {
-    bar_named(B6, 96);
-    double cp = 0.0;
+    bar_named(B5, 128);
     if (act) {
-      const double dun = xc[XDN][lane];
-      if (role == 0) {
-        cp = xc[XP1][lane] + p.rou * dun;
-      } else {
-        cp = xc[XP2][lane] + p.rov * dun;
-        xc[XC3][lane] = xc[XA3][lane] + dun * p.roepp;
+      const double e = xc[ES1][lane] + xc[XQ][lane];
+      X = X + xc[XM2][lane];
+      xc[XDP][lane] = s.gm1[lane] * (e - half_of(X));
+    }
+    bar_arrive(B8, 128);
+  } else if (role == 3) {
+    double dvy = 0.0;
+    if (act) {
+      const double dv = div_pair(np[2 * ns] - s.vv[lane] * np[0], s.rr[lane], s.rrh[lane], s.rrl[lane]);
+      xc[XM2][lane] = dv * s.rov[lane];
+      dvy = dv * s.dy[lane];
+    }
+    bar_named(B5, 128);
+    if (act) xc[XDN][lane] = xc[XDUX][lane] + dvy;
+    bar_arrive(B6, NSP > 1 ? 192 : 128);
+  } else if (role == 7) {
+    double S[NSP];
+    if (act) {
+      const double aF = s.aF[lane], un = s.un[lane];
+      T[0][lane] = half_of(-aF * np[0] + np[ns] * s.dx[lane] + np[2 * ns] * s.dy[lane]);
+#pragma unroll
+      for (int k = 1; k < NSP - 1; ++k) {
+        const double dY = np[(4 + k) * ns];
+        S[k] = -aF * dY + dY * un;
       }
     }
-    bar_named(B8, 96);
+    if (NSP > 1) {
+      bar_named(B6, 192);
+      if (act) {
+#pragma unroll
+        for (int k = 1; k < NSP - 1; ++k) T[4 + k][lane] = half_of(S[k] + s.ry[k][lane] * xc[XDN][lane]);
+      }
+    }
+  } else {
+    double c = 0.0, dn = 0.0;
     if (act) {
-      const double dpp = xc[XDP][lane];
-      if (role == 0) w[1 * 4 + q] = half_of(cp + dpp * p.dx);
-      else w[2 * 4 + q] = half_of(cp + dpp * p.dy);
+      dn = np[(role == 4 ? 3 : role - 4) * ns];  // dE, drho u, drho v
+      c = -s.aF[lane] * dn;
+      if (role > 4) c = c + dn * s.un[lane];
+    }
+    bar_named(B6, NSP > 1 ? 192 : 128);
+    if (act) c = c + (role == 5 ? s.rou : role == 6 ? s.rov : s.roepp)[lane] * xc[XDN][lane];
+    bar_named(B8, 128);
+    if (act) {
+      const double dp = xc[XDP][lane];
+      if (role == 4) T[3][lane] = half_of(c + s.un[lane] * (dn + dp));
+      else T[role - 4][lane] = half_of(c + dp * (role == 5 ? s.dx : s.dy)[lane]);
     }
   }
-  (void)NS;
-  bar_named(B7, 128);
-  if (!fvalid) return;
-  const double* wf = wsm + fc * V * 4;
-  double df = 0.0;
-  bool first = true;
+  if (role >= 4) {
+    bar_arrive(B7, 256);
+    return;
+  }
+  const int p0 = pr & 255, n = pr >> 8;
+  const double* Tr = &T[r][p0];
+  bar_named(B7, 256);
+  if (fi < 0) return;
+  double df = n > 0 ? plus_zero(Tr[0]) : 0.0;
 #pragma unroll
-  for (int sl = 0; sl < 4; ++sl)
-    if ((fn.mask >> sl) & 1) {
-      df = first ? plus_zero(wf[r * 4 + sl]) : df + wf[r * 4 + sl];
-      first = false;
-    }
-  d.hWA[r * NE + fi] = FWD ? div_rn(R - df, fn.dd, fn.ddh, fn.ddl) : R - div_rn(df, fn.dd, fn.ddh, fn.ddl);
+  for (int u = 1; u < MAXF; ++u)
+    if (u < n) df = df + Tr[u];
+  const double a = FWD ? R - df : df, qd = div_pair(a, s.dd[fc], s.ddh[fc], s.ddl[fc]), out = FWD ? qd : R - qd;
+  res[fc * V + r] = out;
+  d.hWA[(size_t)r * d.NE + fi] = out;
 }
 // Both LU-SGS sweeps as a dataflow over one cooperative launch with compact
 // passes: block b owns cells [bC, (b+1)C); a pass is a run of consecutive
 // positions of one level owned by the block, split into G groups of at most
-// 16 cells and 32 active pairs, group g on warps 4g .. 4g+3.  The work
-// around a pass is spread over more warps than k_lusgs_flow's single staging
-// warp, whose gathers, polls and publishing took longer than a pass:
-//  - FLOWC_STAGERS staging warps: warp s stages passes s, s + STAGERS, ...
-//    (pair_load / finc_load) into a ring of FLOWC_NBUF shared slots, once
-//    the pass that held the slot before is finished (s_consumed); s_slot[b]
-//    = k + 1 marks pass k staged in slot b;
-//  - the coordinator warp (4G): looks at the flags of the next pass, hands
-//    it to the compute warps (barrier 3) once it is staged, its flags are
-//    set and the current pass is done (barrier 4), and publishes the
-//    finished pass (flag = this launch's epoch), before any blocking wait, so
-//    no block waits while holding a finished pass.
-// With each hand-over the coordinator writes s_go[slot]: 0 after any wait
-// gave up (ERR_SYNC), when the staging may have stopped; all warps of a group
-// read the same s_go and skip the pass together, so the group's barriers
-// stay matched.  Every wait is bounded.  A group without cells in the pass
-// only joins the hand-over.
+// flowc_cells(V) cells and 32 active pairs, group g on warps 8g .. 8g+7
+// (flowc_step).  The sweeps are a chain of passes, so everything that is not
+// on the chain is done beside it, passes ahead:
+//  - the preparing warps: warp s takes passes s, s + S, ... into a ring of
+//    FLOWC_NBUF shared slots (flowc_stage, once the pass that held the slot
+//    before is done), waits for the flags of the passes of other blocks that
+//    the pass depends on, and fetches the increments that it reads from those
+//    and from the block's passes up to k - 1 - FLOWC_BACK (nb); those of the
+//    block's last FLOWC_BACK passes it reads from shared memory, where their
+//    finishing lanes put them.  s_ready[slot] = k + 1 marks pass k prepared;
+//  - the starting warp: arrives on pass k's start barrier (3 or 13, by k's
+//    parity) once the pass is prepared, which the compute warps reach when they
+//    are done with pass k - 1, and marks passes done (s_done) at their end
+//    barriers (4 or 14);
+//  - the publishing warps, alternate passes each: the finished pass's flag =
+//    this launch's epoch (a release, about 1,300 cycles).  A pass is marked
+//    done and published whether or not the next one can start, so no block
+//    waits while holding a finished pass.
+// Barriers of one parity never mix: pass k is started after the starting warp
+// has seen the end of pass k - 2.  s_go[k & 1]: pass k runs; 0 after any wait
+// gave up (ERR_SYNC), when the preparation may have stopped: the compute warps
+// then skip the remaining passes, together.  Every wait on memory is bounded,
+// and the only warps that meet at a barrier are the compute warps (which wait
+// for nothing else) and the starting warp.  A group without cells in the pass
+// only joins these barriers.
+// Bound by latency: a pass is one chain of dependent FP64 operations (55
+// cycles each), about 4,500 cycles with the hand-over, whatever its number of
+// cells.  A whole FP64 iteration, ms, with the launch of a lane per slot and
+// one block per SM (k_lusgs_flow) and with this one: 720 cells (142 levels in
+// the two sweeps) 0.75 -> 0.51, 20,000 gas cells (242) 0.75 -> 0.54, 120,000
+// (602) 3.02 -> 2.32, 2 million 33.1 -> 19.0.
 template <int NSP, int G>
 __global__ void __launch_bounds__(flowc_threads(G), 1) k_lusgs_flowc(const Dev d, const ThermoDev<NSP> th, const FlowDev f) {
-  constexpr int V = 3 + NSP, T34 = 128 * G + 32, SLOT = flowc_slot_bytes<NSP, G>(), CAP = flowc_cells(V);
+  using Slot = FlowcSlot<NSP>;
+  constexpr int V = 3 + NSP, CAP = Slot::CAP, CW = 8 * G, T34 = 32 * CW + 32, S = flowc_preps(G);
   extern __shared__ __align__(16) uint8_t flowc_smem[];
-  auto slot_pre = [&](int s) { return reinterpret_cast<PairPre<NSP>*>(flowc_smem + s * SLOT); };
-  auto slot_fin = [&](int s) {
-    return reinterpret_cast<FinC*>(flowc_smem + s * SLOT + 32 * G * sizeof(PairPre<NSP>));
-  };
+  Slot* const slots = reinterpret_cast<Slot*>(flowc_smem);  // [FLOWC_NBUF][G]
+  __shared__ double s_res[(FLOWC_BACK + 1) * G * CAP * V];
   __shared__ unsigned s_epoch;
-  __shared__ volatile int s_bad, s_consumed;
-  __shared__ volatile int s_slot[FLOWC_NBUF], s_go[FLOWC_NBUF];
+  __shared__ volatile int s_bad, s_done, s_go[2];
+  __shared__ volatile int s_ready[FLOWC_NBUF];
   if (threadIdx.x == 0) {
     s_epoch = ld_acquire(f.ctr) + 1u;
     s_bad = 0;
-    s_consumed = 0;
-    for (int s = 0; s < FLOWC_NBUF; ++s) { s_slot[s] = 0; s_go[s] = 0; }
+    s_done = 0;
+    for (int s = 0; s < FLOWC_NBUF; ++s) s_ready[s] = 0;
   }
   __syncthreads();
   const unsigned epoch = s_epoch;
   const int b = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int f0 = f.boff[0][b], b0 = f.boff[1][b];
   const int nf = f.boff[0][b + 1] - f0, n = nf + (f.boff[1][b + 1] - b0);
-  auto pass_of = [&](int k) { return k < nf ? f.blist[0][f0 + k] : f.blist[1][b0 + k - nf]; };
+  // the block's k-th pass in the tables
+  auto at = [&](int k) { return k < nf ? f0 + k : f.nfwd + b0 + k - nf; };
   auto give_up = [&]() {
     if (lane == 0) {
       s_bad = 1;
@@ -1365,105 +1413,100 @@ __global__ void __launch_bounds__(flowc_threads(G), 1) k_lusgs_flowc(const Dev d
     }
     __syncwarp();
   };
-  if (warp > 4 * G) {
-    // staging warp s: the data of its passes that the sweep does not change
-    const int s = warp - 4 * G - 1;
-    for (int k = s; k < n && !s_bad; k += FLOWC_STAGERS) {
-      for (unsigned spin = 0; s_consumed < k - FLOWC_NBUF + 1 && !s_bad; ++spin)
-        if (spin >= d.spin_limit) give_up();
-      if (s_bad) break;
-      const int pz = pass_of(k), sl = k % FLOWC_NBUF;
-      PairPre<NSP>* pre = slot_pre(sl);
-      FinC* fin = slot_fin(sl);
-      int tg = f.pstart[pz];
-#pragma unroll
-      for (int g = 0; g < G; ++g) {
-        const int nc = f.gcell[pz * G + g], e0 = f.poff[pz * G + g], np = f.poff[pz * G + g + 1] - e0;
-        PairPre<NSP> pl;
-        pl.j = -1;
-        pl.cs = 0;
-        if (lane < np) {
-          const int e = f.plist[e0 + lane];
-          pl = k < nf ? pair_load<NSP, true>(d, e >> 2, e & 3, tg) : pair_load<NSP, false>(d, e >> 2, e & 3, tg);
-        }
-        pre[32 * g + lane] = pl;
-        if (lane < CAP) {
-          FinC fc = {-1, 0, 1.0, 1.0, 0.0};
-          if (lane < nc) fc = k < nf ? finc_load<true>(d, tg + lane) : finc_load<false>(d, tg + lane);
-          fin[CAP * g + lane] = fc;
-        }
-        tg += nc;
-      }
-      __syncwarp();
-      __threadfence_block();
-      if (lane == 0) s_slot[sl] = k + 1;
-      __syncwarp();
-    }
-  } else if (warp == 4 * G) {
-    // the coordinator
-    auto staged = [&](int k) {  // wait (bounded) until pass k is staged
-      for (unsigned spin = 0; s_slot[k % FLOWC_NBUF] != k + 1 && !s_bad; ++spin)
-        if (spin >= d.spin_limit) give_up();
-      __threadfence_block();
-    };
-    auto poll = [&](int k) {
-      if (s_bad) return;
-      const int pz = pass_of(k), d0 = f.doff[pz], nd = f.doff[pz + 1] - d0;
-      bool ok = true;
-      for (int u = lane; u < nd; u += 32) ok = ok && wait_flag(f.pflag + f.deps[d0 + u], epoch, d.err, d.spin_limit);
-      if (__any_sync(0xffffffffu, !ok)) give_up();
-    };
-    auto ready = [&](int k) -> bool {
-      if (s_bad) return true;
-      if (s_slot[k % FLOWC_NBUF] != k + 1) return false;
-      const int pz = pass_of(k), d0 = f.doff[pz], nd = f.doff[pz + 1] - d0;
-      bool ok = true;
-      for (int u = lane; u < nd; u += 32) ok = ok && ld_acquire(f.pflag + f.deps[d0 + u]) >= epoch;
-      return __all_sync(0xffffffffu, ok) != 0;
-    };
-    // hand pass k over: the compute warps run it iff nothing gave up
-    auto hand_over = [&](int k) {
-      if (lane == 0) s_go[k % FLOWC_NBUF] = s_bad ? 0 : 1;
-      __syncwarp();
-      __threadfence_block();
-      bar_arrive(3, T34);
-    };
-    if (n > 0) {
-      staged(0);
-      poll(0);
-      hand_over(0);
-    }
+  // wait until passes 0 .. k are done; false after a give-up
+  auto done = [&](int k) {
+    for (unsigned spin = 0; s_done <= k && !s_bad; ++spin)
+      if (spin >= d.spin_limit) give_up();
+    __threadfence_block();
+    return !s_bad;
+  };
+  if (warp < CW) {
+    const int gi = G > 1 ? warp >> 3 : 0, role = warp & 7;
     for (int k = 0; k < n; ++k) {
-      const bool more = k + 1 < n;
-      const bool go = more && ready(k + 1);
-      if (go) __threadfence_block();
-      bar_named(4, T34);
-      __threadfence_block();
-      if (lane == 0) s_consumed = k + 1;  // pass k's slot is free
-      if (go) hand_over(k + 1);
-      if (lane == 0 && !s_bad) st_release(f.pflag + pass_of(k), epoch);
-      if (more && !go) {
-        poll(k + 1);
-        staged(k + 1);
-        hand_over(k + 1);
+      bar_named(3 + 10 * (k & 1), T34);
+      const Slot& s = slots[(k % FLOWC_NBUF) * G + gi];
+      // the group's first cell exists iff the group has work in this pass
+      if (s_go[k & 1] && s.cell[0] >= 0) {
+        double* res = s_res + ((k % (FLOWC_BACK + 1)) * G + gi) * CAP * V;
+        if (k < nf) flowc_step<NSP, true, G>(d, th, s, gi, role, s_res, res);
+        else flowc_step<NSP, false, G>(d, th, s, gi, role, s_res, res);
       }
+      bar_arrive(4 + 10 * (k & 1), T34);
+    }
+  } else if (warp == CW) {
+    // the starting warp: pass k is started as soon as it is prepared, before
+    // the end of pass k - 1 where that comes later
+    auto start = [&](int k) {
+      if (lane == 0) s_go[k & 1] = s_bad ? 0 : 1;
+      __syncwarp();
+      __threadfence_block();
+      bar_arrive(3 + 10 * (k & 1), T34);
+    };
+    for (int k = 0; k < n; ++k) {
+      const bool early = s_ready[k % FLOWC_NBUF] == k + 1;
+      if (early) start(k);
+      if (k > 0) {
+        bar_named(4 + 10 * ((k - 1) & 1), T34);  // the end of pass k - 1
+        __threadfence_block();
+        if (lane == 0) s_done = k;  // passes 0 .. k - 1
+      }
+      if (!early) {
+        for (unsigned spin = 0; s_ready[k % FLOWC_NBUF] != k + 1 && !s_bad; ++spin)
+          if (spin >= d.spin_limit) give_up();
+        start(k);
+      }
+    }
+    if (n > 0) {
+      bar_named(4 + 10 * ((n - 1) & 1), T34);
+      __threadfence_block();
+      if (lane == 0) s_done = n;
+    }
+  } else if (warp <= CW + FLOWC_PUBS) {
+    for (int k = warp - CW - 1; k < n; k += FLOWC_PUBS) {
+      const int pz = f.prec[at(k)].z;
+      if (!done(k)) break;
+      if (lane == 0) st_release(f.pflag + pz, epoch);
     }
   } else {
-    const int gi = threadIdx.x >> 7, role = (threadIdx.x >> 5) & 3;
-    for (int k = 0; k < n; ++k) {
-      bar_named(3, T34);
-      const int sl = k % FLOWC_NBUF;
-      // the group's first cell exists iff the group has work in this pass
-      if (s_go[sl] && slot_fin(sl)[CAP * gi].i >= 0) {
-        const PairPre<NSP> p = slot_pre(sl)[32 * gi + lane];
-        const FinC fn = slot_fin(sl)[CAP * gi + min((role * 32 + lane) / V, CAP - 1)];
-        double nbv[V];
+    for (int k = warp - CW - 1 - FLOWC_PUBS; k < n && !s_bad; k += S) {
+      auto free = [&]() { return done(k - FLOWC_NBUF); };
+      const int4 rec = f.prec[at(k)];
+      const int2 dep = f.pdep[at(k)];
+      int t = rec.x, e = rec.y, cnt = rec.w;
+      bool ok = true;
 #pragma unroll
-        for (int v = 0; v < V; ++v) nbv[v] = p.j >= 0 ? __ldcg(d.hWA + (size_t)v * d.NE + p.j) : 0.0;
-        if (k < nf) sweepc_compute<NSP, true, G>(d, th, p, nbv, fn);
-        else sweepc_compute<NSP, false, G>(d, th, p, nbv, fn);
+      for (int g = 0; g < G; ++g) {
+        const int nc = cnt & 255, np = (cnt >> 8) & 255;
+        Slot& s = slots[(k % FLOWC_NBUF) * G + g];
+        ok = ok && (k < nf ? flowc_stage<NSP, true>(d, f, s, k, G, e, np, t, nc, free)
+                           : flowc_stage<NSP, false>(d, f, s, k, G, e, np, t, nc, free));
+        t += nc;
+        e += np;
+        cnt >>= 16;
       }
-      bar_arrive(4, T34);
+      if (!ok) break;
+      bool set = true;
+      for (int u = lane; u < dep.y; u += 32)
+        set = set && wait_flag(f.pflag + f.deps[dep.x + u], epoch, d.err, d.spin_limit);
+      if (__any_sync(0xffffffffu, !set)) give_up();
+      __syncwarp();
+      if (!done(k - 1 - FLOWC_BACK)) break;
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        Slot& s = slots[(k % FLOWC_NBUF) * G + g];
+        const int j = s.j[lane];
+        if (j >= 0 && s.src[lane] < 0) {
+          double x[V];
+#pragma unroll
+          for (int v = 0; v < V; ++v) x[v] = __ldcg(d.hWA + (size_t)v * d.NE + j);
+#pragma unroll
+          for (int v = 0; v < V; ++v) s.nb[v][lane] = x[v];
+        }
+      }
+      __syncwarp();
+      __threadfence_block();
+      if (lane == 0) s_ready[k % FLOWC_NBUF] = k + 1;
+      __syncwarp();
     }
   }
   __syncthreads();
@@ -1681,6 +1724,7 @@ struct rc_ctx {
   bool can_flow[FLOW_GMAX] = {};  // the device can co-schedule the k_lusgs_flow grid (per G)
   bool can_flow32 = false;      // ... and the k_lusgs_flow32 grid (mixed forms)
   int flow_grid = 0;            // its blocks (one per SM)
+  int flowc_grid[FLOWC_GMAX] = {};  // blocks of the compact plans
   FlowDev flows[FLOW_GMAX] = {};  // its pass tables for G = 1..3 groups (passes of up to 8 G cells;
                                   // G = 1 is also the mixed forms' k_lusgs_flow32)
   int flow_g = 1;                 // the groups of the FP64 dataflow launch
@@ -1840,6 +1884,9 @@ struct FlowPlan {
   std::vector<int> cellpass[2];
   int groups = 0;
   std::vector<int> gcell, poff, plist;
+  std::vector<short> psrc;   // per pair: (a << 8) | the neighbour's place in the block's pass 1 + a before, a <
+                             // FLOWC_BACK; -1 elsewhere
+  std::vector<int> ppos[2];  // first pair of each sweep position
 };
 // the slot q of cell i has a neighbour in sweep dir (0 forward: a lower one)
 template <class NF>
@@ -1914,7 +1961,87 @@ FlowPlan flow_plan(int NE, int G, const NF& nface, const std::vector<int>& cothe
     }
     fp.doff.push_back((int)fp.deps.size());
   }
+  if (groups > 0) {
+    // what each pair reads from the passes that its block runs just before
+    fp.psrc.assign(fp.plist.size(), -1);
+    for (int dir = 0; dir < 2; ++dir) {
+      fp.ppos[dir].assign((size_t)NE + 1, 0);
+      std::vector<int> place(NE, -1);            // of a cell in its pass
+      std::vector<int> seq(fp.pstart.size(), 0);  // of a pass in its block's list
+      for (int bb = 0; bb < G; ++bb)
+        for (int k = fp.boff[dir][bb]; k < fp.boff[dir][bb + 1]; ++k) {
+          const int pz = fp.blist[dir][k];
+          seq[pz] = k;
+          int t = fp.pstart[pz];
+          for (int g = 0; g < groups; ++g) {
+            int e = fp.poff[(size_t)pz * groups + g];
+            const int e1 = fp.poff[(size_t)pz * groups + g + 1];
+            for (int c = 0; c < fp.gcell[(size_t)pz * groups + g]; ++c, ++t) {
+              const int i = so.cells[dir][t];
+              place[i] = g * cap + c;
+              fp.ppos[dir][t] = e;
+              for (; e < e1 && (fp.plist[e] >> 2) == t; ++e) {
+                const int j = cother[(size_t)(fp.plist[e] & 3) * NE + i];
+                if (j / C != bb) continue;
+                const int a = k - 1 - seq[fp.cellpass[dir][j]];
+                if (a >= 0 && a < FLOWC_BACK) fp.psrc[e] = (short)(a << 8 | place[j]);
+              }
+              fp.ppos[dir][t + 1] = e;
+            }
+          }
+        }
+    }
+  }
   return fp;
+}
+
+// The passes that the compact plan of one group per pass puts one after
+// another over G blocks if every level waits for its slowest block: per level
+// the most passes that one block cuts its cells into, summed over both sweeps.
+template <class NF>
+long flowc_length(int NE, int G, const NF& nface, const std::vector<int>& cother, const SweepOrder& so, int cap) {
+  const int C = (NE + G - 1) / G;
+  long sum = 0;
+  for (int dir = 0; dir < 2; ++dir)
+    for (size_t l = 0; l + 1 < so.off[dir].size(); ++l) {
+      int own = -1, nc = 0, np = 0, passes = 0, most = 0;
+      for (int t = so.off[dir][l]; t < so.off[dir][l + 1]; ++t) {
+        const int i = so.cells[dir][t];
+        int a = 0;
+        for (int q = 0; q < 4; ++q) a += sweep_slot(NE, nface, cother, dir, i, q) ? 1 : 0;
+        if (i / C != own) { own = i / C; nc = 0; np = 0; passes = 1; }
+        else if (nc == cap || np + a > FLOWC_PAIRS) { nc = 0; np = 0; ++passes; }
+        ++nc;
+        np += a;
+        most = std::max(most, passes);
+      }
+      sum += most;
+    }
+  return sum;
+}
+// Blocks of the compact plan of one group per pass: the fewest, in steps of
+// 15 % from one per SM, that lengthen no level's passes.  A pass costs the same
+// for one cell as for a full group, and every block boundary that the sweep
+// crosses costs a publication, a poll and a fetch through L2 (about 3,000
+// cycles), so small meshes run on few SMs: 720 cells 0.74 -> 0.54 ms per FP64
+// iteration, 0.42 -> 0.23 mixed (152 -> 6 blocks); 120,000 cells 2.49 -> 2.33 FP64
+// (36 blocks; 28, with two passes in some levels, 3.18).  In the mixed forms at
+// most about 6.5 cells of a level per block: their blocks also run the Newton
+// update (120,000 cells: 152 blocks 1.10, 64 1.00, 36 1.08 ms).
+template <class NF>
+int flowc_blocks(int NE, int nsm, bool mixed, const NF& nface, const std::vector<int>& cother, const SweepOrder& so,
+                 int cap) {
+  const long length = flowc_length(NE, nsm, nface, cother, so, cap);
+  const double level = (double)NE / std::max<size_t>(1, so.off[0].size() - 1);
+  const int least = mixed ? std::min(nsm, (int)std::ceil(level / 6.5)) : 1;
+  int best = nsm, fails = 0;
+  for (double g = 0.85 * nsm; fails < 2; g *= 0.85) {
+    const int G = std::max((int)g, least);
+    if (flowc_length(NE, G, nface, cother, so, cap) <= length) best = G;
+    else ++fails;
+    if (G == least) break;
+  }
+  return best;
 }
 
 template <int NSP>
@@ -2053,7 +2180,7 @@ void q_flow_g(rc_ctx* c) {
 template <int NSP, int G>
 void q_flowc_g(rc_ctx* c) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)c->flow_grid);
+  cfg.gridDim = dim3((unsigned)c->flowc_grid[G - 1]);
   cfg.blockDim = dim3(flowc_threads(G));
   cfg.dynamicSmemBytes = (size_t)flowc_dsmem<NSP, G>();
   cfg.stream = c->stream;
@@ -2153,7 +2280,7 @@ void q_sweeps32(rc_ctx* c) {
   if (!c->persistent && c->wide == 4 && c->flow_c && c->flow_g <= FLOWC_GMAX && c->can_flowc32[c->flow_g - 1]) {
     // compact passes; the Newton update runs inside the dataflow launch
     mixed_lusgs_flowc<NSP>(c->d, c->thermo32.data(), c->thermo.data(), c->flowc[c->flow_g - 1], c->flow_g,
-                           c->flow_grid, c->stream);
+                           c->flowc_grid[c->flow_g - 1], c->stream);
     c->launches += 1;
     return;
   }
@@ -2719,7 +2846,9 @@ int init_impl(const rc_mesh* m, const rc_thermo* t, const rc_config* g, const Ba
       // G = 1..3 groups of 8 positions, then the compact plans of 1..2 groups
       const int cg = gr > FLOW_GMAX ? gr - FLOW_GMAX : 0;
       const int cap = flowc_cells(c->V);
-      FlowPlan fp = cg ? flow_plan(NE, G, nface, cother, so, cap * cg, cg, cap) : flow_plan(NE, G, nface, cother, so, 8 * gr);
+      const int GB = cg == 1 ? flowc_blocks(NE, G, g->precision != RC_PREC_FP64, nface, cother, so, cap) : G;
+      if (cg) c->flowc_grid[cg - 1] = GB;
+      FlowPlan fp = cg ? flow_plan(NE, GB, nface, cother, so, cap * cg, cg, cap) : flow_plan(NE, G, nface, cother, so, 8 * gr);
       std::vector<int>& pstart = fp.pstart;
       std::vector<int>& pcount = fp.pcount;
       std::vector<int>& doff = fp.doff;
@@ -2729,18 +2858,45 @@ int init_impl(const rc_mesh* m, const rc_thermo* t, const rc_config* g, const Ba
       FlowDev& f = cg ? c->flowc[cg - 1] : c->flows[gr - 1];
       int* ip;
       if (cg) {
-        st |= dev_upload(c, fp.gcell, &ip); f.gcell = ip;
-        st |= dev_upload(c, fp.poff, &ip); f.poff = ip;
-        if (fp.plist.empty()) fp.plist.push_back(0);
-        st |= dev_upload(c, fp.plist, &ip); f.plist = ip;
+        // the pairs and passes as k_lusgs_flowc reads them
+        std::vector<int> plj(fp.plist.size() + 1, -1), plf(fp.plist.size() + 1, 0);
+        std::vector<int4> prec;
+        std::vector<int2> pdep;
+        for (int dir = 0; dir < 2; ++dir) {
+          const std::vector<int>& lst = dir == 0 ? fc : bc;
+          for (int pz : fp.blist[dir]) {
+            int4 r = {pstart[pz], fp.poff[(size_t)pz * cg], pz, 0};
+            for (int g = 0; g < cg; ++g) {
+              const int e0 = fp.poff[(size_t)pz * cg + g], e1 = fp.poff[(size_t)pz * cg + g + 1];
+              r.w |= (fp.gcell[(size_t)pz * cg + g] | (e1 - e0) << 8) << (16 * g);
+              for (int e = e0; e < e1; ++e) {
+                const int i = lst[fp.plist[e] >> 2], q = fp.plist[e] & 3, fa = cface[(size_t)q * NE + i];
+                plj[e] = cother[(size_t)q * NE + i];
+                plf[e] = ((cleft[i] >> q) & 1u) ? fa : ~fa;
+              }
+            }
+            prec.push_back(r);
+            pdep.push_back({doff[pz], doff[pz + 1] - doff[pz]});
+          }
+          st |= dev_upload(c, fp.ppos[dir], &ip); f.ppos[dir] = ip;
+        }
+        f.nfwd = (int)fp.blist[0].size();
+        int4* rp;
+        int2* dp;
+        short* sp;
+        st |= dev_upload(c, prec, &rp); f.prec = rp;
+        st |= dev_upload(c, pdep, &dp); f.pdep = dp;
+        st |= dev_upload(c, plj, &ip); f.plj = ip;
+        st |= dev_upload(c, plf, &ip); f.plf = ip;
+        if (fp.psrc.empty()) fp.psrc.push_back(-1);
+        st |= dev_upload(c, fp.psrc, &sp); f.psrc = sp;
+      } else {
+        st |= dev_upload(c, pstart, &ip); f.pstart = ip;
+        st |= dev_upload(c, pcount, &ip); f.pcount = ip;
+        for (int dir = 0; dir < 2; ++dir) { st |= dev_upload(c, blist[dir], &ip); f.blist[dir] = ip; }
+        st |= dev_upload(c, doff, &ip); f.doff = ip;
       }
-      st |= dev_upload(c, pstart, &ip); f.pstart = ip;
-      st |= dev_upload(c, pcount, &ip); f.pcount = ip;
-      for (int dir = 0; dir < 2; ++dir) {
-        st |= dev_upload(c, boff[dir], &ip); f.boff[dir] = ip;
-        st |= dev_upload(c, blist[dir], &ip); f.blist[dir] = ip;
-      }
-      st |= dev_upload(c, doff, &ip); f.doff = ip;
+      for (int dir = 0; dir < 2; ++dir) { st |= dev_upload(c, boff[dir], &ip); f.boff[dir] = ip; }
       if (deps.empty()) deps.push_back(0);
       st |= dev_upload(c, deps, &ip); f.deps = ip;
       st |= dev_upload(c, std::vector<unsigned>(pstart.size() + 1, 0u), &f.pflag);
@@ -2780,10 +2936,26 @@ int init_impl(const rc_mesh* m, const rc_thermo* t, const rc_config* g, const Ba
     const char* sched = std::getenv("RC_LUSGS_SCHEDULE");
     c->pers_grid = nsm;
     c->can_persistent = coop && nsm > 0 && occ64 >= 1 && occ32 >= 1;
-    // default (no or another value): the dataflow launches (where they cannot
-    // run: the four-warp per-level sweeps for FP64, the per-level sweeps for
-    // the mixed forms)
-    const std::string sc = sched ? sched : "";
+    // Default (no or another value): the compact dataflow launch, with two
+    // groups per pass where an SM's cells of a level fill more than one (18
+    // for four species), and one launch per level where they fill more than
+    // two, or where the mixed forms have few levels: those are throughput, not
+    // chains.  Measured, ms per iteration, compact with one / two groups / per
+    // level: 120,000 cells in 301 levels (2.6 cells per SM and level) FP64 2.33
+    // / 2.55 / 3.57 (four warps), mixed 1.00 / 1.12 / 1.44; 64 cases (32 cells)
+    // FP64 31.0 / 30.6 / 32.4; 120,000 cells in random order (11 levels, 72
+    // cells) FP64 1.50 / 1.41 / 1.33, mixed 0.52 / 0.51 / 0.34; 12,000 cells in 10
+    // levels mixed 0.17 / 0.17 / 0.12, FP64 0.33 / 0.33 / 0.34.  Where the
+    // dataflow launch cannot run: the four-warp per-level sweeps for FP64, the
+    // per-level sweeps for the mixed forms.
+    const double per_sm = (double)NE / (std::max<size_t>(c->fwd_off.size(), 2) - 1) / std::max(nsm, 1);
+    const double group = flowc_cells(c->V);
+    const bool few = g->precision != RC_PREC_FP64 && c->fwd_off.size() - 1 <= 16;
+    std::string sc = sched ? sched : "";
+    bool known = false;
+    for (const char* name : {"persistent", "levels", "levels8", "levels2w", "levels4w", "flow", "flow2", "flow3", "flowc", "flowc2"})
+      known = known || sc == name;
+    if (!known) sc = few || per_sm > 2 * group ? "levels" : per_sm > group ? "flowc2" : "flowc";
     c->persistent = c->can_persistent && sc == "persistent";
     c->wide = sc == "levels" ? 0 : sc == "levels8" ? 1 : sc == "levels2w" ? 2 : sc == "levels4w" ? 3 : 4;
     c->flow_g = sc == "flow3" ? 3 : sc == "flow2" || sc == "flowc2" ? 2 : 1;
@@ -2853,6 +3025,27 @@ int flow_plan_check_width(int ne, int nblocks, const std::vector<int>& nf, const
       }
       if (tot != fp.pcount[pz]) ok = false;
     }
+    // ppos delimits each position's pairs; psrc names the neighbour's place in
+    // one of the block's last FLOWC_BACK passes exactly where one of those
+    // holds the neighbour
+    for (int dir = 0; dir < 2 && ok; ++dir)
+      for (int b = 0; b < nblocks && ok; ++b)
+        for (int k = fp.boff[dir][b]; k < fp.boff[dir][b + 1] && ok; ++k) {
+          const int pz = fp.blist[dir][k];
+          for (int e = fp.poff[pz * groups]; e < fp.poff[(pz + 1) * groups] && ok; ++e) {
+            const int t = fp.plist[e] >> 2, j = co[(size_t)(fp.plist[e] & 3) * ne + so.cells[dir][t]];
+            if (e < fp.ppos[dir][t] || e >= fp.ppos[dir][t + 1]) ok = false;
+            int from = -1;  // how many passes back
+            for (int a = 0; a < FLOWC_BACK && k - 1 - a >= fp.boff[dir][b]; ++a)
+              if (fp.blist[dir][k - 1 - a] == fp.cellpass[dir][j]) from = a;
+            if ((fp.psrc[e] < 0 ? -1 : fp.psrc[e] >> 8) != from) ok = false;
+            if (!ok || from < 0) continue;
+            const int src = fp.blist[dir][k - 1 - from], g = (fp.psrc[e] & 255) / cap, c = (fp.psrc[e] & 255) % cap;
+            int at = fp.pstart[src] + c;
+            for (int u = 0; u < g; ++u) at += fp.gcell[src * groups + u];
+            ok = g < groups && c < fp.gcell[src * groups + g] && so.cells[dir][at] == j;
+          }
+        }
   }
   // every cell in exactly one pass per sweep; a pass is 1..8 positions of one
   // level, all owned by its block

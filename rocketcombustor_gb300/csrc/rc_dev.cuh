@@ -207,31 +207,51 @@ __device__ __forceinline__ void bar_named(int id, int count) {
 __device__ __forceinline__ void bar_arrive(int id, int count) {
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory");
 }
-// Tables of the dataflow LU-SGS (k_lusgs_flow): cells are
-// split into per-SM blocks, a pass is a run of at most 8 consecutive sweep
-// positions of one level whose cells one block owns.
+// Tables of the dataflow LU-SGS: cells are split into per-SM blocks, a pass is
+// a run of consecutive sweep positions of one level whose cells one block owns
+// (k_lusgs_flow: at most 8 per group; k_lusgs_flowc: see below).
 struct FlowDev {
-  const int* pstart;   // first sweep position of pass p
-  const int* pcount;   // its number of cells (1..8)
-  const int* boff[2];  // passes of block b: blist[d][boff[d][b] .. boff[d][b+1]), d = 0 forward, 1 backward
-  const int* blist[2];
-  const int* doff;     // passes that pass p waits for: deps[doff[p] .. doff[p+1])
-  const int* deps;
+  const int* boff[2];  // passes of block b: boff[d][b] .. boff[d][b+1] of the sweep's list, d = 0 forward, 1 backward
+  const int* deps;     // the passes that the passes wait for, a range of it each
   unsigned* pflag;     // per pass: epoch of the launch that finished it
   unsigned* ctr;       // [0] epoch of the last finished launch, [1] finished blocks
-  // compact passes only (k_lusgs_flowc; null otherwise): a pass is split into
-  // G groups of consecutive cells; group g of pass p holds gcell[p*G + g]
-  // cells (0..16) and the active (position, slot) pairs
-  // plist[poff[p*G + g] .. poff[p*G + g + 1]) (0..32), each position << 2 | slot
-  const int* gcell;
-  const int* poff;
-  const int* plist;
+  // k_lusgs_flow (null for compact plans)
+  const int* pstart;   // first sweep position of pass p
+  const int* pcount;   // its number of cells
+  const int* blist[2]; // the sweep's list of passes
+  const int* doff;     // pass p's range of deps: doff[p] .. doff[p+1]
+  // k_lusgs_flowc (null otherwise): a pass is split into G groups of
+  // consecutive cells, a group's active (cell, slot) pairs are consecutive.
+  // Passes in the order the blocks run them (the forward passes of all blocks,
+  // then the backward ones; nfwd forward):
+  int nfwd;
+  const int4* prec;    // first sweep position, first pair, pass number (its flag), cells and pairs of each group (8 bits each)
+  const int2* pdep;    // the pass's range of deps: start, count
+  // per pair: neighbour, signed face (as swf), and where one of the
+  // block's last FLOWC_BACK passes of the sweep holds the neighbour:
+  // (a << 8) | (group * cells per group + cell) for the pass 1 + a before, -1
+  // elsewhere
+  const int* plj;
+  const int* plf;
+  const short* psrc;
+  const int* ppos[2];  // first pair of each sweep position (NE + 1)
 };
 // Compact passes: at most FLOWC_PAIRS active pairs per group (one per lane
 // of a warp) and flowc_cells(V) cells, the cells that 128 finishing lanes
 // hold at V lanes per cell (18 for four species, 32 for one).
 constexpr int FLOWC_PAIRS = 32;
 __host__ __device__ constexpr int flowc_cells(int V) { return 128 / V < 32 ? 128 / V : 32; }
+
+// The compact dataflow launches: passes whose increments stay in shared memory
+// for the block's next ones, publishing warps.
+constexpr int FLOWC_BACK = 3, FLOWC_PUBS = 2;
+// a pair's psrc as the offset of the neighbour's increments in the ring of the
+// last FLOWC_BACK + 1 passes ([pass % (FLOWC_BACK + 1)][G * cells][V]) for pass k
+template <int V>
+__device__ __forceinline__ int flowc_src(int psrc, int k, int G) {
+  if (psrc < 0) return -1;
+  return (((k - 1 - (psrc >> 8)) % (FLOWC_BACK + 1)) * G * flowc_cells(V) + (psrc & 255)) * V;
+}
 
 // Dataflow LU-SGS: pass flags.  wait_flag: the calling thread waits until
 // the flag reaches `epoch` (acquire); bounded like wait_count.  set_flag

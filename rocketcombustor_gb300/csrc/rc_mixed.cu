@@ -892,105 +892,151 @@ __global__ void __launch_bounds__(FLOW32_THREADS, 1) k_lusgs_flow32(const Dev d,
 }
 
 // Both FP32 sweeps as a dataflow on the compact pass tables of k_lusgs_flowc
-// (rc_core.cu): a pass is split into G groups of at most flowc_cells(V)
-// cells and 32 active (cell, slot) pairs.  Group g is two warps (2g, 2g+1):
-// warp 2g forms the FP32 terms of its 32 pairs (terms32, one pair per lane)
-// into the group's [cell][variable][slot] scratch, then both warps finish the
-// group's cells in two rounds, thread x = 64 round + 32 h + lane taking
-// variable x % V of cell x / V:
-// the terms of the active slots added in slot order from +0 (the inactive
-// slots' +0 terms of k_lusgs_flow32 leave such a sum unchanged: with FP32
-// denormals flushed every partial sum is normal or +0), then the FP64
-// division by the diagonal and the FP32 copy.  The work around a pass is
-// k_lusgs_flowc's: two staging warps fill a ring of FLOWC32_NBUF shared
-// slots ahead of the compute warps, and a coordinator warp looks at the next
-// pass's flags, hands it over (barrier 3) once it is staged and the current
-// pass is done (barrier 4), then publishes the finished pass; s_go[slot]
-// (0 after a give-up) keeps both warps of a group on the same path.
+// (rc_core.cu), with its protocol: preparing warps stage the passes, wait for
+// their flags and fetch the increments they read from other blocks and older
+// passes; a starting warp joins the compute warps at the barrier between
+// passes; publishing warps set the finished passes' flags; the increments of
+// the last passes stay in shared memory.  A group is four warps: its first forms
+// the FP32 terms of its 32 pairs (flowc32_terms, one pair per lane), then
+// thread x = 32 role + lane finishes variable x % V of cell x / V: the terms of
+// the active slots added in slot order from +0 (the inactive slots' +0 terms of
+// k_lusgs_flow32 leave such a sum unchanged: with FP32 denormals flushed every
+// partial sum is normal or +0), then the FP64 product with the diagonal's
+// reciprocal and the FP32 copy.
 // FLOWC32_UPD more warps run the FP64 Newton update of each finished
 // backward pass during the sweep, as in k_lusgs_flow32 (the sweeps read only
-// the FP32 copies PA32, cst32 of the state).  The update is FP64 work of
-// about a quarter of a plain FP64 iteration's face flux: two warps per SM
-// (k_lusgs_flow32) fall behind the compact sweep on a large mesh and finish
-// long after its last pass, so there are enough update warps to keep each
-// sub-partition's FP64 unit busy.  Seven keep the block at 12 warps, three
-// per SM sub-partition, so a thread may hold the 149 registers the kernel
-// uses; a fourth warp on a sub-partition caps it at 128 (on the 2,000,000-cell
-// nozzle: 6 update warps 8.77 ms per mixed iteration, 7 warps 7.95, 8 warps
-// 8.38 with 168 bytes of spills, 10 warps 8.99).  Every wait is bounded
-// (ERR_SYNC).
-constexpr int FLOWC32_NBUF = 4, FLOWC32_UPD = 7;
-__host__ __device__ constexpr int flowc32_threads(int G) { return 32 * (2 * G + 3 + FLOWC32_UPD); }
-template <int NSP>
-struct PairPre32 {
-  int j;   // the neighbour (-1: no pair in this lane)
-  int cq;  // the pair's cell within its group << 2 | its slot
-  float dx, dy, pp, uu, vv, tt, rr, gama, roe, aF;
-  float cs[NSP];  // h_k of the neighbour
-  float Yk[NSP > 1 ? NSP - 1 : 1];
-};
-// sweep_load32's reads for one active pair (position t, slot q)
-template <int NSP, bool FWD>
-__device__ __forceinline__ PairPre32<NSP> pair_load32(const Dev& d, int t, int q, int tg) {
-  constexpr int DIR = FWD ? 0 : 1;
-  const int NE = d.NE, NF = d.NF;
-  PairPre32<NSP> p;
-  const int j = d.swj[DIR][q * NE + t], fs = d.swf[DIR][q * NE + t], f = fs >= 0 ? fs : ~fs;
-  p.j = j;
-  p.cq = ((t - tg) << 2) | q;
-  p.dx = d.fvec32[f];
-  p.dy = d.fvec32[NF + f];
-  if (fs < 0) { p.dx = -p.dx; p.dy = -p.dy; }
-  p.pp = d.PA32[0 * NE + j]; p.uu = d.PA32[1 * NE + j]; p.vv = d.PA32[2 * NE + j]; p.tt = d.PA32[3 * NE + j];
-  p.rr = d.cst32[0 * NE + j]; p.gama = d.cst32[1 * NE + j]; p.roe = d.cst32[2 * NE + j];
-  p.aF = d.alpaF32[f];
-#pragma unroll
-  for (int k = 0; k < NSP; ++k) p.cs[k] = d.cst32[(3 + k) * NE + j];
-#pragma unroll
-  for (int k = 0; k < NSP - 1; ++k) p.Yk[k] = d.PA32[(4 + k) * NE + j];
-  return p;
+// the FP32 copies PA32, cst32 of the state), 32 cells at a time.  Every wait is
+// bounded (ERR_SYNC).
+// Bound by the pass's chain and the hops between blocks, about 1.5 us a level
+// together; an iteration with k_lusgs_flow32 and with this launch: 120,000
+// cells 1.28 -> 0.98 ms, 2 million 15.1 -> 6.0 ms.
+constexpr int FLOWC32_NBUF = 8, FLOWC32_UPD = 6;
+__host__ __device__ constexpr int flowc32_preps(int G) { return G == 1 ? 5 : 3; }
+__host__ __device__ constexpr int flowc32_threads(int G) {
+  return 32 * (4 * G + 1 + FLOWC_PUBS + flowc32_preps(G) + FLOWC32_UPD);
 }
-struct FinC32 {
-  int i, mask;
-  double rdd;  // 1 / dd of the cell
+// One group's part of a ring slot (FlowcSlot's fields in FP32).
+template <int NSP>
+struct FlowcSlot32 {
+  static constexpr int V = 3 + NSP, NS = NSP > 1 ? NSP - 1 : 1, CAP = flowc_cells(V);
+  double rdd[CAP];  // 1 / dd of the cells
+  float dx[32], dy[32], uu[32], vv[32], tt[32], rinv[32], gama[32], aF[32], rou[32], rov[32], gm1[32], roepp[32], un[32];
+  float h[NSP][32], ry[NS][32];
+  float nb[V][32];
+  int j[32];       // the neighbour (-1: no pair in this lane)
+  int src[32];     // where its increments are among those of the block's last passes, -1: in nb
+  int cell[CAP];   // the group's cells (-1 past the last)
+  int pairs[CAP];  // a cell's first pair, its number of pairs << 8
 };
-template <bool FWD>
-__device__ __forceinline__ FinC32 finc_load32(const Dev& d, int t) {
-  constexpr int DIR = FWD ? 0 : 1;
-  FinC32 f;
-  const int NE = d.NE;
-  f.i = d.swi[DIR][t];
-  f.rdd = 1.0 / d.dd[f.i];
-  f.mask = 0;
+template <int NSP, int G>
+__host__ __device__ constexpr int flowc32_dsmem() { return FLOWC32_NBUF * G * (int)sizeof(FlowcSlot32<NSP>); }
+// Stages one group of a pass (flowc_stage's FP32 form).
+template <int NSP, bool FWD, class Wait>
+__device__ __forceinline__ bool flowc32_stage(const Dev& d, const FlowDev& f, FlowcSlot32<NSP>& s, int k, int G, int e0,
+                                              int np, int t0, int nc, Wait wait) {
+  constexpr int DIR = FWD ? 0 : 1, NS = FlowcSlot32<NSP>::NS, CAP = FlowcSlot32<NSP>::CAP;
+  const int NE = d.NE, NF = d.NF, lane = threadIdx.x & 31;
+  int j = -1, src = -1, cell = -1, pairs = 0;
+  float dx = 0, dy = 0, pp = 0, uu = 0, vv = 0, tt = 0, rr = 1, gama = 0, roe = 0, aF = 0, h[NSP], Y[NS];
+  double dd = 1.0;
+  if (lane < np) {
+    j = f.plj[e0 + lane];
+    src = flowc_src<3 + NSP>(f.psrc[e0 + lane], k, G);
+    const int fs = f.plf[e0 + lane], fc = fs >= 0 ? fs : ~fs;
+    dx = d.fvec32[fc];
+    dy = d.fvec32[NF + fc];
+    if (fs < 0) { dx = -dx; dy = -dy; }
+    aF = d.alpaF32[fc];
+    pp = d.PA32[0 * NE + j]; uu = d.PA32[1 * NE + j]; vv = d.PA32[2 * NE + j]; tt = d.PA32[3 * NE + j];
+    rr = d.cst32[0 * NE + j]; gama = d.cst32[1 * NE + j]; roe = d.cst32[2 * NE + j];
 #pragma unroll
-  for (int q = 0; q < 4; ++q) f.mask |= (d.swj[DIR][q * NE + t] >= 0 ? 1 : 0) << q;
-  return f;
+    for (int k = 0; k < NSP; ++k) h[k] = d.cst32[(3 + k) * NE + j];
+#pragma unroll
+    for (int k = 0; k < NSP - 1; ++k) Y[k] = d.PA32[(4 + k) * NE + j];
+  }
+  if (lane < nc) {
+    cell = d.swi[DIR][t0 + lane];
+    const int p0 = f.ppos[DIR][t0 + lane];
+    pairs = (p0 - e0) | (f.ppos[DIR][t0 + lane + 1] - p0) << 8;
+    dd = d.dd[cell];
+  }
+  if (!wait()) return false;
+  if (lane < np) {
+    s.dx[lane] = dx; s.dy[lane] = dy; s.uu[lane] = uu; s.vv[lane] = vv; s.tt[lane] = tt;
+    s.gama[lane] = gama; s.aF[lane] = aF;
+    s.rinv[lane] = 1.f / rr;
+    s.rou[lane] = rr * uu;
+    s.rov[lane] = rr * vv;
+    s.gm1[lane] = gama - 1.f;
+    s.roepp[lane] = roe + pp;
+    s.un[lane] = uu * dx + vv * dy;
+#pragma unroll
+    for (int k = 0; k < NSP; ++k) s.h[k][lane] = h[k];
+#pragma unroll
+    for (int k = 0; k < NSP - 1; ++k) s.ry[k][lane] = rr * Y[k];
+  }
+  s.j[lane] = j;
+  s.src[lane] = src;
+  if (lane < CAP) { s.cell[lane] = cell; s.pairs[lane] = pairs; s.rdd[lane] = val(1.0 / Num<false>(dd)); }
+  return true;
+}
+// terms32 of the lane's pair, from the slot's fields (the same expressions).
+template <int NSP>
+__device__ __forceinline__ void flowc32_terms(const ThermoDev32<NSP>& th, const FlowcSlot32<NSP>& s, int lane,
+                                              const float* nb, float* c) {
+  const float dx = s.dx[lane], dy = s.dy[lane], uu = s.uu[lane], vv = s.vv[lane], gama = s.gama[lane];
+  const float rou = s.rou[lane], rov = s.rov[lane], rinv = s.rinv[lane], gm1 = s.gm1[lane], un = s.un[lane];
+  const float drr = nb[0], dru = nb[1], drv = nb[2], dre = nb[3];
+  float dry[NSP], q = 0.f;
+#pragma unroll
+  for (int k = 0; k < NSP - 1; ++k) { dry[k] = nb[4 + k]; q += dry[k]; }
+  dry[NSP - 1] = drr - q;
+  const float duu = (dru - uu * drr) * rinv;
+  const float dvv = (drv - vv * drr) * rinv;
+  float s1 = 0.f, s2 = 0.f;
+#pragma unroll
+  for (int k = 0; k < NSP; ++k) {
+    s1 += s.h[k][lane] * dry[k];
+    s2 += th.R[k] * dry[k];
+  }
+  const float dpp = gm1 * (dre - s1 + s.tt[lane] * s2 * gama / gm1 -
+                           0.5f * (dru * uu + duu * rou + drv * vv + dvv * rov));
+  const float dun = duu * dx + dvv * dy;
+  const float aF = s.aF[lane];
+  c[0] = 0.5f * (-aF * drr + dru * dx + drv * dy);
+  c[1] = 0.5f * (-aF * dru + dru * un + rou * dun + dpp * dx);
+  c[2] = 0.5f * (-aF * drv + drv * un + rov * dun + dpp * dy);
+  c[3] = 0.5f * (-aF * dre + dun * s.roepp[lane] + un * (dre + dpp));
+#pragma unroll
+  for (int k = 0; k < NSP - 1; ++k) c[4 + k] = 0.5f * (-aF * dry[k] + dry[k] * un + s.ry[k][lane] * dun);
 }
 template <int NSP, int G>
 __global__ void __launch_bounds__(flowc32_threads(G), 1) k_lusgs_flowc32(const Dev d, const ThermoDev32<NSP> th,
                                                                         const ThermoDev<NSP> th64, const FlowDev f) {
-  constexpr int V = 3 + NSP, T34 = 64 * G + 32, CW = 2 * G;  // compute warps 0 .. CW-1
-  constexpr int CAP = flowc_cells(V);
-  __shared__ PairPre32<NSP> s_pre[FLOWC32_NBUF][32 * G];
-  __shared__ FinC32 s_fin[FLOWC32_NBUF][CAP * G];
-  __shared__ float wsc[G][CAP * V * 4];
+  using Slot = FlowcSlot32<NSP>;
+  constexpr int V = 3 + NSP, CAP = Slot::CAP, CW = 4 * G, S = flowc32_preps(G);  // compute warps 0 .. CW-1
+  constexpr int T34 = 32 * CW + 32;
+  extern __shared__ __align__(16) uint8_t flowc32_smem[];
+  Slot* const slots = reinterpret_cast<Slot*>(flowc32_smem);  // [FLOWC32_NBUF][G]
+  __shared__ float s_T[G][V][32];                             // the pairs' terms
+  __shared__ float s_res[(FLOWC_BACK + 1) * G * CAP * V];     // increments of the last passes
   __shared__ int s_cells[FLOWC32_UPD][32];
   __shared__ unsigned s_epoch;
-  __shared__ volatile int s_bad, s_consumed, s_done;
-  __shared__ volatile int s_slot[FLOWC32_NBUF], s_go[FLOWC32_NBUF];
+  __shared__ volatile int s_bad, s_done, s_go[2];
+  __shared__ volatile int s_ready[FLOWC32_NBUF];
   if (threadIdx.x == 0) {
     s_epoch = ld_acquire(f.ctr) + 1u;
     s_bad = 0;
-    s_consumed = 0;
     s_done = 0;
-    for (int s = 0; s < FLOWC32_NBUF; ++s) { s_slot[s] = 0; s_go[s] = 0; }
+    for (int s = 0; s < FLOWC32_NBUF; ++s) s_ready[s] = 0;
   }
   __syncthreads();
   const unsigned epoch = s_epoch;
   const int b = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int f0 = f.boff[0][b], b0 = f.boff[1][b];
   const int nf = f.boff[0][b + 1] - f0, n = nf + (f.boff[1][b + 1] - b0);
-  auto pass_of = [&](int k) { return k < nf ? f.blist[0][f0 + k] : f.blist[1][b0 + k - nf]; };
+  // the block's k-th pass in the tables
+  auto at = [&](int k) { return k < nf ? f0 + k : f.nfwd + b0 + k - nf; };
   auto give_up = [&]() {
     if (lane == 0) {
       s_bad = 1;
@@ -998,148 +1044,133 @@ __global__ void __launch_bounds__(flowc32_threads(G), 1) k_lusgs_flowc32(const D
     }
     __syncwarp();
   };
-  if (warp == CW + 1 || warp == CW + 2) {
-    // staging warp s: its passes s, s + 2, ... into the ring
-    const int s = warp - CW - 1;
-    for (int k = s; k < n && !s_bad; k += 2) {
-      for (unsigned spin = 0; s_consumed < k - FLOWC32_NBUF + 1 && !s_bad; ++spin)
-        if (spin >= d.spin_limit) give_up();
-      if (s_bad) break;
-      const int pz = pass_of(k), sl = k % FLOWC32_NBUF;
-      int tg = f.pstart[pz];
-#pragma unroll
-      for (int g = 0; g < G; ++g) {
-        const int nc = f.gcell[pz * G + g], e0 = f.poff[pz * G + g], np = f.poff[pz * G + g + 1] - e0;
-        PairPre32<NSP> pl;
-        pl.j = -1;
-        pl.cq = 0;
-        if (lane < np) {
-          const int e = f.plist[e0 + lane];
-          pl = k < nf ? pair_load32<NSP, true>(d, e >> 2, e & 3, tg) : pair_load32<NSP, false>(d, e >> 2, e & 3, tg);
-        }
-        s_pre[sl][32 * g + lane] = pl;
-        if (lane < CAP) {
-          FinC32 fc = {-1, 0, 0.0};
-          if (lane < nc) fc = k < nf ? finc_load32<true>(d, tg + lane) : finc_load32<false>(d, tg + lane);
-          s_fin[sl][CAP * g + lane] = fc;
-        }
-        tg += nc;
-      }
-      __syncwarp();
-      __threadfence_block();
-      if (lane == 0) s_slot[sl] = k + 1;
-      __syncwarp();
-    }
-  } else if (warp == CW) {
-    // the coordinator
-    auto staged = [&](int k) {
-      for (unsigned spin = 0; s_slot[k % FLOWC32_NBUF] != k + 1 && !s_bad; ++spin)
-        if (spin >= d.spin_limit) give_up();
-      __threadfence_block();
-    };
-    auto poll = [&](int k) {
-      if (s_bad) return;
-      const int pz = pass_of(k), d0 = f.doff[pz], nd = f.doff[pz + 1] - d0;
-      bool ok = true;
-      for (int u = lane; u < nd; u += 32) ok = ok && wait_flag(f.pflag + f.deps[d0 + u], epoch, d.err, d.spin_limit);
-      if (__any_sync(0xffffffffu, !ok)) give_up();
-    };
-    auto ready = [&](int k) -> bool {
-      if (s_bad) return true;
-      if (s_slot[k % FLOWC32_NBUF] != k + 1) return false;
-      const int pz = pass_of(k), d0 = f.doff[pz], nd = f.doff[pz + 1] - d0;
-      bool ok = true;
-      for (int u = lane; u < nd; u += 32) ok = ok && ld_acquire(f.pflag + f.deps[d0 + u]) >= epoch;
-      return __all_sync(0xffffffffu, ok) != 0;
-    };
-    auto hand_over = [&](int k) {
-      if (lane == 0) s_go[k % FLOWC32_NBUF] = s_bad ? 0 : 1;
-      __syncwarp();
-      __threadfence_block();
-      bar_arrive(3, T34);
-    };
-    if (n > 0) {
-      staged(0);
-      poll(0);
-      hand_over(0);
-    }
+  // wait until passes 0 .. k are done; false after a give-up
+  auto done = [&](int k) {
+    for (unsigned spin = 0; s_done <= k && !s_bad; ++spin)
+      if (spin >= d.spin_limit) give_up();
+    __threadfence_block();
+    return !s_bad;
+  };
+  if (warp < CW) {
+    const int gi = G > 1 ? warp >> 2 : 0, role = warp & 3, x = role * 32 + lane, fc = x / V, r = x - fc * V;
+    float(*T)[32] = s_T[gi];
     for (int k = 0; k < n; ++k) {
-      const bool more = k + 1 < n;
-      const bool go = more && ready(k + 1);
-      if (go) __threadfence_block();
-      bar_named(4, T34);
-      __threadfence_block();
-      if (lane == 0) {
-        s_consumed = k + 1;  // pass k's slot is free
-        s_done = k + 1;      // and its increments are final
-      }
-      if (go) hand_over(k + 1);
-      if (lane == 0 && !s_bad) st_release(f.pflag + pass_of(k), epoch);
-      if (more && !go) {
-        poll(k + 1);
-        staged(k + 1);
-        hand_over(k + 1);
-      }
-    }
-  } else if (warp < CW) {
-    const int gi = warp >> 1, h = warp & 1;
-    float* wsm = wsc[gi];
-    for (int k = 0; k < n; ++k) {
-      bar_named(3, T34);
-      const int sl = k % FLOWC32_NBUF;
-      if (s_go[sl] && s_fin[sl][CAP * gi].i >= 0) {
+      bar_named(3 + 10 * (k & 1), T34);
+      const Slot& s = slots[(k % FLOWC32_NBUF) * G + gi];
+      // the group's first cell exists iff the group has work in this pass
+      if (s_go[k & 1] && s.cell[0] >= 0) {
         const bool fwd = k < nf;
-        // the own residuals of this warp's two rounds of (cell, variable)
-        int fc[2], r[2];
-        FinC32 fn[2];
-        double R[2];
+        const int fi = fc < CAP ? s.cell[fc] : -1, pr = fc < CAP ? s.pairs[fc] : 0;
+        const double R = fi >= 0 ? __ldcg(d.hWA + (size_t)r * d.NE + fi) : 0.0;
+        if (role == 0 && s.j[lane] >= 0) {
+          const int src = s.src[lane], ns = src >= 0 ? 1 : 32;
+          const float* np = src >= 0 ? s_res + src : &s.nb[0][lane];
+          float nb[V], c[V];
 #pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          const int x = 64 * u + 32 * h + lane;
-          fc[u] = x / V;
-          r[u] = x - fc[u] * V;
-          fn[u] = s_fin[sl][CAP * gi + min(fc[u], CAP - 1)];
-          if (fc[u] >= CAP) fn[u].i = -1;
-          R[u] = fn[u].i >= 0 ? __ldcg(d.hWA + r[u] * d.NE + fn[u].i) : 0.0;
+          for (int v = 0; v < V; ++v) nb[v] = np[v * ns];
+          flowc32_terms<NSP>(th, s, lane, nb, c);
+#pragma unroll
+          for (int v = 0; v < V; ++v) T[v][lane] = c[v];
         }
-        if (h == 0) {
-          const PairPre32<NSP> p = s_pre[sl][32 * gi + lane];
-          if (p.j >= 0) {
-            float nb[V], c[V];
-#pragma unroll
-            for (int v = 0; v < V; ++v) nb[v] = __ldcg(d.dU32 + v * d.NE + p.j);
-            terms32<NSP>(th, p, nb, c);
-            float* w = wsm + min(p.cq >> 2, CAP - 1) * V * 4 + (p.cq & 3);
-#pragma unroll
-            for (int v = 0; v < V; ++v) w[v * 4] = c[v];
-          }
-        }
-        bar_named(5 + gi, 64);
-#pragma unroll
-        for (int u = 0; u < 2; ++u) {
-          if (fn[u].i < 0) continue;
-          const float* wf = wsm + fc[u] * V * 4 + r[u] * 4;
+        const float* Tr = &T[r][pr & 255];
+        const int np = pr >> 8;
+        bar_named(5 + gi, 128);
+        if (fi >= 0) {
           float df = 0.f;
 #pragma unroll
-          for (int q = 0; q < 4; ++q)
-            if ((fn[u].mask >> q) & 1) df += wf[q];
-          const double rdd = fn[u].rdd;
-          const double uo = fwd ? (R[u] - (double)df) * rdd : R[u] - (double)df * rdd;
-          d.hWA[r[u] * d.NE + fn[u].i] = uo;
-          d.dU32[r[u] * d.NE + fn[u].i] = (float)uo;
+          for (int u = 0; u < MAXF; ++u)
+            if (u < np) df += Tr[u];
+          const double rdd = s.rdd[fc];
+          const double uo = fwd ? (R - (double)df) * rdd : R - (double)df * rdd;
+          s_res[((k % (FLOWC_BACK + 1)) * G * CAP + gi * CAP + fc) * V + r] = (float)uo;
+          d.hWA[(size_t)r * d.NE + fi] = uo;
+          d.dU32[(size_t)r * d.NE + fi] = (float)uo;
         }
-        // the scratch is written again by the next pass only after barrier 3,
-        // which follows every warp's barrier 4 below
       }
-      bar_arrive(4, T34);
+      bar_arrive(4 + 10 * (k & 1), T34);
+    }
+  } else if (warp == CW) {
+    // the starting warp: pass k is started as soon as it is prepared, before
+    // the end of pass k - 1 where that comes later
+    auto start = [&](int k) {
+      if (lane == 0) s_go[k & 1] = s_bad ? 0 : 1;
+      __syncwarp();
+      __threadfence_block();
+      bar_arrive(3 + 10 * (k & 1), T34);
+    };
+    for (int k = 0; k < n; ++k) {
+      const bool early = s_ready[k % FLOWC32_NBUF] == k + 1;
+      if (early) start(k);
+      if (k > 0) {
+        bar_named(4 + 10 * ((k - 1) & 1), T34);  // the end of pass k - 1
+        __threadfence_block();
+        if (lane == 0) s_done = k;  // passes 0 .. k - 1
+      }
+      if (!early) {
+        for (unsigned spin = 0; s_ready[k % FLOWC32_NBUF] != k + 1 && !s_bad; ++spin)
+          if (spin >= d.spin_limit) give_up();
+        start(k);
+      }
+    }
+    if (n > 0) {
+      bar_named(4 + 10 * ((n - 1) & 1), T34);
+      __threadfence_block();
+      if (lane == 0) s_done = n;
+    }
+  } else if (warp <= CW + FLOWC_PUBS) {
+    for (int k = warp - CW - 1; k < n; k += FLOWC_PUBS) {
+      const int pz = f.prec[at(k)].z;
+      if (!done(k)) break;
+      if (lane == 0) st_release(f.pflag + pz, epoch);
+    }
+  } else if (warp <= CW + FLOWC_PUBS + S) {
+    for (int k = warp - CW - 1 - FLOWC_PUBS; k < n && !s_bad; k += S) {
+      auto free = [&]() { return done(k - FLOWC32_NBUF); };
+      const int4 rec = f.prec[at(k)];
+      const int2 dep = f.pdep[at(k)];
+      int t = rec.x, e = rec.y, cnt = rec.w;
+      bool ok = true;
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        const int nc = cnt & 255, np = (cnt >> 8) & 255;
+        Slot& s = slots[(k % FLOWC32_NBUF) * G + g];
+        ok = ok && (k < nf ? flowc32_stage<NSP, true>(d, f, s, k, G, e, np, t, nc, free)
+                           : flowc32_stage<NSP, false>(d, f, s, k, G, e, np, t, nc, free));
+        t += nc;
+        e += np;
+        cnt >>= 16;
+      }
+      if (!ok) break;
+      bool set = true;
+      for (int u = lane; u < dep.y; u += 32)
+        set = set && wait_flag(f.pflag + f.deps[dep.x + u], epoch, d.err, d.spin_limit);
+      if (__any_sync(0xffffffffu, !set)) give_up();
+      __syncwarp();
+      if (!done(k - 1 - FLOWC_BACK)) break;
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        Slot& s = slots[(k % FLOWC32_NBUF) * G + g];
+        const int j = s.j[lane];
+        if (j >= 0 && s.src[lane] < 0) {
+          float y[V];
+#pragma unroll
+          for (int v = 0; v < V; ++v) y[v] = __ldcg(d.dU32 + (size_t)v * d.NE + j);
+#pragma unroll
+          for (int v = 0; v < V; ++v) s.nb[v][lane] = y[v];
+        }
+      }
+      __syncwarp();
+      __threadfence_block();
+      if (lane == 0) s_ready[k % FLOWC32_NBUF] = k + 1;
+      __syncwarp();
     }
   } else {
-    // the Newton update warps (CW + 3 ..): update warp u takes the cells of
+    // the Newton update warps: update warp u takes the cells of
     // the backward passes nf + u, nf + u + UPD, ... once finished, 32 at a
     // time, one per lane: a batch runs on from pass to pass and may end inside
     // one (off: the cells of pass k already taken)
     constexpr int UPD = FLOWC32_UPD;
-    const int u = warp - CW - 3;
+    const int u = warp - CW - 1 - FLOWC_PUBS - S;
     int* cells = s_cells[u];
     unsigned err = 0;
     for (int k = nf + u, off = 0; k < n;) {
@@ -1153,9 +1184,9 @@ __global__ void __launch_bounds__(flowc32_threads(G), 1) k_lusgs_flowc32(const D
       const int kl = k + UPD * lane;
       int cnt = 0, t0 = 0;
       if (kl < avail) {
-        const int pz = pass_of(kl);
-        cnt = f.pcount[pz];
-        t0 = f.pstart[pz];
+        const int4 rec = f.prec[at(kl)];
+        for (int g = 0, w = rec.w; g < G; ++g, w >>= 16) cnt += w & 255;
+        t0 = rec.x;
         if (lane == 0) {
           cnt -= off;
           t0 += off;
@@ -1164,15 +1195,15 @@ __global__ void __launch_bounds__(flowc32_threads(G), 1) k_lusgs_flowc32(const D
       int incl = cnt;
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
-        const int x = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += x;
+        const int y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
       }
       const int excl = incl - cnt;
       for (int c = 0; c < cnt && excl + c < 32; ++c) cells[excl + c] = t0 + c;
       const int total = __shfl_sync(0xffffffffu, incl, 31);
       const int ncell = total < 32 ? total : 32;
       __syncwarp();
-      if (lane < ncell) update_cell<NSP>(d, th64, d.swi[1][cells[lane]], err);
+      if (lane < ncell) update_cell<NSP, Num<false>>(d, th64, d.swi[1][cells[lane]], err);
       __syncwarp();
       if (total <= 32) {
         // every finished pass of this warp taken whole
@@ -1284,6 +1315,7 @@ cudaError_t mixed_lusgs_flowc(const Dev& d, const void* th32, const void* th64, 
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid);
   cfg.blockDim = dim3(flowc32_threads(G));
+  cfg.dynamicSmemBytes = G == 2 ? flowc32_dsmem<NSP, 2>() : flowc32_dsmem<NSP, 1>();
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeCooperative;
@@ -1298,8 +1330,12 @@ cudaError_t mixed_lusgs_flowc(const Dev& d, const void* th32, const void* th64, 
 template <int NSP>
 int mixed_flowc_occupancy(int G) {
   int nb = 0;
-  if (G == 2) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_lusgs_flowc32<NSP, 2>, flowc32_threads(2), 0);
-  else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_lusgs_flowc32<NSP, 1>, flowc32_threads(1), 0);
+  auto occ = [&](auto kern, int threads, int dsmem) {
+    cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, dsmem);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, threads, dsmem);
+  };
+  if (G == 2) occ(k_lusgs_flowc32<NSP, 2>, flowc32_threads(2), flowc32_dsmem<NSP, 2>());
+  else occ(k_lusgs_flowc32<NSP, 1>, flowc32_threads(1), flowc32_dsmem<NSP, 1>());
   return nb;
 }
 template <int NSP>

@@ -135,7 +135,19 @@ RCS_HD double mul(double a, double b) {
   return make(rh | ((ah ^ bh) & SIGN_BIT), (uint32_t)h);
 }
 
-RCS_HD double div(double a, double b) {
+// The reciprocal that div_by needs, from b's significand alone: 2^63 over its
+// leading 32 bits, below the true value by less than 2^-28 of it.
+RCS_HD uint32_t recip32(double b) {
+  const uint32_t bh = hi32(b), bl = lo32(b);
+  const uint32_t bn = (((bh & 0xfffffu) | 0x100000u) << 11) | (bl >> 21);  // leading 32 bits
+  const uint32_t rb = umin(rcp_bits(0x3f800000u | ((bn >> 8) & 0x7ffffeu)), 0x3f7fffffu);
+  const uint32_t V0 = (rb << 8) | SIGN_BIT;  // 2^63 / bn to 21 bits
+  const int64_t dlt = (int64_t)(((uint64_t)SIGN_BIT << 32) - (uint64_t)V0 * bn);
+  const int32_t dh = (int32_t)(dlt >> 12);
+  return V0 + (uint32_t)(smulhi(dh, (int32_t)(V0 >> 1)) >> 18) - 6u;
+}
+// a / b with V = recip32(b)
+RCS_HD double div_by(double a, double b, uint32_t V) {
   const uint32_t ah = hi32(a), al = lo32(a), bh = hi32(b), bl = lo32(b);
   const uint32_t ea = (ah & EXP_MASK) - EXP_LO, eb = (bh & EXP_MASK) - EXP_LO;
   if (umax(ea, eb) > EXP_SPAN) {
@@ -143,12 +155,6 @@ RCS_HD double div(double a, double b) {
     return a / b;
   }
   const uint32_t mah = (ah & 0xfffffu) | 0x100000u, mbh = (bh & 0xfffffu) | 0x100000u;
-  const uint32_t bn = (mbh << 11) | (bl >> 21);  // leading 32 bits
-  const uint32_t rb = umin(rcp_bits(0x3f800000u | ((bn >> 8) & 0x7ffffeu)), 0x3f7fffffu);
-  const uint32_t V0 = (rb << 8) | SIGN_BIT;  // 2^63 / bn to 21 bits
-  const int64_t dlt = (int64_t)(((uint64_t)SIGN_BIT << 32) - (uint64_t)V0 * bn);
-  const int32_t dh = (int32_t)(dlt >> 12);
-  const uint32_t V = V0 + (uint32_t)(smulhi(dh, (int32_t)(V0 >> 1)) >> 18) - 6u;  // below 2^63 / (bn + 1), by less than 2^-28
   const uint32_t an = (mah << 11) | (al >> 21);
   const uint32_t q1 = umulhi(an, V);  // 2^31 a / b, not above it
   const uint64_t ma = ((uint64_t)mah << 32) | al, mb = ((uint64_t)mbh << 32) | bl;
@@ -162,6 +168,7 @@ RCS_HD double div(double a, double b) {
   Q = (Q + 2) >> 2;
   return make(((uint32_t)(Q >> 32) + e) | ((ah ^ bh) & SIGN_BIT), (uint32_t)Q);
 }
+RCS_HD double div(double a, double b) { return div_by(a, b, recip32(b)); }
 
 RCS_HD double sqrt(double a) {
   const uint32_t ah = hi32(a), al = lo32(a);
@@ -211,6 +218,7 @@ struct SoftMul {
 // that these take, and straight-line copies (a face flux holds some 60
 // divisions and 32 exponentials) would not fit the instruction cache.
 static __device__ __noinline__ double soft_div(double a, double b) { return rcs::div(a, b); }
+static __device__ __noinline__ double soft_div_by(double a, double b, unsigned V) { return rcs::div_by(a, b, V); }
 static __device__ __noinline__ double soft_sqrt(double a) { return rcs::sqrt(a); }
 static __device__ __noinline__ double soft_exp(double x) { return rcm::exp_with<SoftMul>(x); }
 static __device__ __noinline__ double soft_log(double x) { return rcm::log_with<SoftMul>(x); }
