@@ -1604,44 +1604,66 @@ __global__ void __launch_bounds__(PERS_THREADS) k_lusgs_persistent(const Dev d, 
 // ------------------------------------------------------------ utilities ----
 // Residual norms: fixed-shape deterministic reduction (block partials then one
 // block over the partials).  out[k] = sum vol*|hWA_k|, out[V] = max WA_1.
-constexpr int NRM_BLOCKS = 304, NRM_THREADS = 256;
+constexpr int NRM_BLOCKS = 304, NRM_THREADS = 256, NRM_MAXV = 7;
 // Case blockIdx.y covers cells [coff[y], coff[y+1]) (coff null: [0, NE)); the
 // arrays have plane stride NE.  The order of the sums depends only on the
 // case's own cells, so a case gives the same norms alone and in a batch.
+// All V sums and the maximum go through one pass over the cells and one
+// tree (a tree per variable spent its time in 64 barriers: 314 us for 64 cases,
+// 20 us on 120,000 cells).
+template <int V>
 __global__ void __launch_bounds__(NRM_THREADS) k_norm_partial(const double* __restrict__ hWA,
                                                               const double* __restrict__ WA,
-                                                              const double* __restrict__ vol, int NE, int V,
+                                                              const double* __restrict__ vol, int NE,
                                                               const int* __restrict__ coff, double* part) {
-  __shared__ double sh[NRM_THREADS];
+  __shared__ double sh[V + 1][NRM_THREADS];
+  const int t = threadIdx.x;
   const int c0 = coff ? coff[blockIdx.y] : 0, n = coff ? coff[blockIdx.y + 1] - c0 : NE;
   part += (size_t)blockIdx.y * (V + 1) * NRM_BLOCKS;
   const int per = (n + NRM_BLOCKS - 1) / NRM_BLOCKS;
   const int lo = blockIdx.x * per, hi = min(n, lo + per);
-  for (int k = 0; k <= V; ++k) {
-    double a = (k == V) ? 0.0 : 0.0;
-    for (int ii = lo + threadIdx.x; ii < hi; ii += NRM_THREADS) {
-      const int i = c0 + ii;
-      a = (k == V) ? fmax2(a, WA[i]) : a + vol[i] * fabs(hWA[k * NE + i]);
+  double a[V + 1];
+#pragma unroll
+  for (int k = 0; k <= V; ++k) a[k] = 0.0;
+  for (int i = c0 + lo + t; i < c0 + hi; i += NRM_THREADS) {
+    const double v = vol[i];
+#pragma unroll
+    for (int k = 0; k < V; ++k) a[k] = a[k] + v * fabs(hWA[(size_t)k * NE + i]);
+    a[V] = fmax2(a[V], WA[i]);
+  }
+#pragma unroll
+  for (int k = 0; k <= V; ++k) sh[k][t] = a[k];
+  __syncthreads();
+  for (int w = NRM_THREADS / 2; w > 0; w >>= 1) {
+    if (t < w) {
+#pragma unroll
+      for (int k = 0; k < V; ++k) sh[k][t] = sh[k][t] + sh[k][t + w];
+      sh[V][t] = fmax2(sh[V][t], sh[V][t + w]);
     }
-    sh[threadIdx.x] = a;
-    __syncthreads();
-    for (int w = NRM_THREADS / 2; w > 0; w >>= 1) {
-      if (threadIdx.x < w) sh[threadIdx.x] = (k == V) ? fmax2(sh[threadIdx.x], sh[threadIdx.x + w])
-                                                      : sh[threadIdx.x] + sh[threadIdx.x + w];
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) part[k * NRM_BLOCKS + blockIdx.x] = sh[0];
     __syncthreads();
   }
+  if (t <= V) part[t * NRM_BLOCKS + blockIdx.x] = sh[t][0];
 }
+// Warp k of block y adds the blocks' values of variable k of case y in block
+// order (k = V: their maximum), from shared memory: the chain of 304 dependent
+// additions is what remains of 42 us with the loads and the other variables'
+// work in it.
 __global__ void k_norm_final(const double* part, int V, const double* __restrict__ total_volume, double* out) {
-  const int k = threadIdx.x;
-  if (k > V) return;
-  part += (size_t)blockIdx.x * (V + 1) * NRM_BLOCKS;
-  out += (size_t)blockIdx.x * (V + 1);
+  __shared__ double sh[NRM_MAXV + 1][NRM_BLOCKS];
+  const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  part += ((size_t)blockIdx.x * (V + 1) + k) * NRM_BLOCKS;
+  for (int b = lane; b < NRM_BLOCKS; b += 32) sh[k][b] = part[b];
+  __syncwarp();
+  if (lane) return;
   double a = 0.0;
-  for (int b = 0; b < NRM_BLOCKS; ++b) a = (k == V) ? fmax2(a, part[k * NRM_BLOCKS + b]) : a + part[k * NRM_BLOCKS + b];
-  out[k] = (k == V) ? a : a / total_volume[blockIdx.x];
+  if (k == V) {
+    for (int b = 0; b < NRM_BLOCKS; ++b) a = fmax2(a, sh[k][b]);
+  } else {
+#pragma unroll 8
+    for (int b = 0; b < NRM_BLOCKS; ++b) a = a + sh[k][b];
+    a = a / total_volume[blockIdx.x];
+  }
+  out[(size_t)blockIdx.x * (V + 1) + k] = a;
 }
 
 // Fortran (V,N) <-> device (V planes of N)
@@ -2400,10 +2422,10 @@ void q_bdf2_lusgs(rc_ctx* c) {
 // Norms of every case into norm_out ([case][V+1]), enqueued.
 void q_norms(rc_ctx* c) {
   const int nc = c->ncase;
-  k_norm_partial<<<dim3(NRM_BLOCKS, nc), NRM_THREADS, 0, c->stream>>>(c->d.hWA, c->d.WA, c->d.vol, c->NE, c->V,
-                                                                       nc > 1 ? c->case_off_dev : nullptr,
-                                                                       c->norm_part);
-  k_norm_final<<<nc, 32, 0, c->stream>>>(c->norm_part, c->V, c->case_vol_dev, c->norm_out);
+  auto partial = c->NSP == 1 ? k_norm_partial<4> : k_norm_partial<NRM_MAXV>;
+  partial<<<dim3(NRM_BLOCKS, nc), NRM_THREADS, 0, c->stream>>>(c->d.hWA, c->d.WA, c->d.vol, c->NE,
+                                                              nc > 1 ? c->case_off_dev : nullptr, c->norm_part);
+  k_norm_final<<<nc, 32 * (c->V + 1), 0, c->stream>>>(c->norm_part, c->V, c->case_vol_dev, c->norm_out);
   c->launches += 2;
 }
 // One inner iteration of BDF2_stage (Time_BDF2.f90:25-46) and the norms of
