@@ -47,61 +47,62 @@ enum : int { NB_RR = 0, NB_RRC, NB_RT, NB_RCT, NB_RCP, NB_HH, NB_EK, NB_ROU, NB_
 template <int NSP>
 __host__ __device__ constexpr int nb_ry() { return NB_H + NSP; }
 template <int NSP>
-__host__ __device__ constexpr int nb_rct() { return NB_H + NSP + (NSP - 1); }  // recip_of(Rcpcv T): 2 planes
+__host__ __device__ constexpr int nb_rct() { return NB_H + NSP + (NSP - 1); }  // recip32(Rcpcv T), as a bit pattern
 template <int NSP>
-__host__ __device__ constexpr int nbq() { return nb_rct<NSP>() + 2; }
+__host__ __device__ constexpr int nbq() { return nb_rct<NSP>() + 1; }
 
-__device__ __forceinline__ double mx(double a, double b) { return (b > a) ? b : a; }
-__device__ __forceinline__ double mn(double a, double b) { return (b < a) ? b : a; }
+// a recip32 in a slot of a double array
+__device__ __forceinline__ double v_slot(unsigned v) { return __hiloint2double(0, (int)v); }
+__device__ __forceinline__ unsigned slot_v(double x) { return (unsigned)__double2loint(x); }
 
-// ---- dgesvx steps on one row-major N x N matrix, a[r*N + c] = A(r, c)
-template <int N>
-__device__ __forceinline__ int dgeequ(const double* a, double* r, double* c, double& rowcnd, double& colcnd,
-                                      double& amax) {
-  const double smlnum = SFMIN, bignum = 1.0 / smlnum;
+// ---- dgesvx steps (T: T or Num, rc_num.cuh) on one row-major N x N matrix, a[r*N + c] = A(r, c)
+template <int N, class T>
+__device__ __forceinline__ int dgeequ(const T* a, T* r, T* c, T& rowcnd, T& colcnd,
+                                      T& amax) {
+  const T smlnum = SFMIN, bignum = 1.0 / SFMIN;
 #pragma unroll
   for (int i = 0; i < N; ++i) r[i] = 0.0;
 #pragma unroll
   for (int j = 0; j < N; ++j)
 #pragma unroll
-    for (int i = 0; i < N; ++i) r[i] = mx(r[i], fabs(a[i * N + j]));
-  double rcmin = bignum, rcmax = 0.0;
+    for (int i = 0; i < N; ++i) r[i] = fmax2(r[i], n_abs(a[i * N + j]));
+  T rcmin = bignum, rcmax = 0.0;
 #pragma unroll
-  for (int i = 0; i < N; ++i) { rcmax = mx(rcmax, r[i]); rcmin = mn(rcmin, r[i]); }
+  for (int i = 0; i < N; ++i) { rcmax = fmax2(rcmax, r[i]); rcmin = fmin2(rcmin, r[i]); }
   amax = rcmax;
-  if (rcmin == 0.0) return 1;
+  if (!nonzero(val(rcmin))) return 1;
 #pragma unroll
-  for (int i = 0; i < N; ++i) r[i] = 1.0 / mn(mx(r[i], smlnum), bignum);
-  rowcnd = mx(rcmin, smlnum) / mn(rcmax, bignum);
+  for (int i = 0; i < N; ++i) r[i] = 1.0 / fmin2(fmax2(r[i], smlnum), bignum);
+  rowcnd = fmax2(rcmin, smlnum) / fmin2(rcmax, bignum);
 #pragma unroll
   for (int j = 0; j < N; ++j) c[j] = 0.0;
 #pragma unroll
   for (int j = 0; j < N; ++j)
 #pragma unroll
-    for (int i = 0; i < N; ++i) c[j] = mx(c[j], fabs(a[i * N + j]) * r[i]);
+    for (int i = 0; i < N; ++i) c[j] = fmax2(c[j], n_abs(a[i * N + j]) * r[i]);
   rcmin = bignum; rcmax = 0.0;
 #pragma unroll
-  for (int j = 0; j < N; ++j) { rcmin = mn(rcmin, c[j]); rcmax = mx(rcmax, c[j]); }
-  if (rcmin == 0.0) return 2;
+  for (int j = 0; j < N; ++j) { rcmin = fmin2(rcmin, c[j]); rcmax = fmax2(rcmax, c[j]); }
+  if (!nonzero(val(rcmin))) return 2;
 #pragma unroll
-  for (int j = 0; j < N; ++j) c[j] = 1.0 / mn(mx(c[j], smlnum), bignum);
-  colcnd = mx(rcmin, smlnum) / mn(rcmax, bignum);
+  for (int j = 0; j < N; ++j) c[j] = 1.0 / fmin2(fmax2(c[j], smlnum), bignum);
+  colcnd = fmax2(rcmin, smlnum) / fmin2(rcmax, bignum);
   return 0;
 }
 // dlaqge; returns bit 0 = rows scaled, bit 1 = columns scaled
-template <int N>
-__device__ __forceinline__ int dlaqge(double* a, const double* r, const double* c, double rowcnd, double colcnd,
-                                      double amax) {
+template <int N, class T>
+__device__ __forceinline__ int dlaqge(T* a, const T* r, const T* c, T rowcnd, T colcnd,
+                                      T amax) {
   const double thresh = 0.1, small = SFMIN / PREC, large = 1.0 / small;
-  if (rowcnd >= thresh && amax >= small && amax <= large) {
-    if (colcnd >= thresh) return 0;
+  if (val(rowcnd) >= thresh && val(amax) >= small && val(amax) <= large) {
+    if (val(colcnd) >= thresh) return 0;
 #pragma unroll
     for (int j = 0; j < N; ++j)
 #pragma unroll
       for (int i = 0; i < N; ++i) a[i * N + j] = c[j] * a[i * N + j];
     return 2;
   }
-  if (colcnd >= thresh) {
+  if (val(colcnd) >= thresh) {
 #pragma unroll
     for (int j = 0; j < N; ++j)
 #pragma unroll
@@ -116,29 +117,29 @@ __device__ __forceinline__ int dlaqge(double* a, const double* r, const double* 
 }
 // dgetrf (partial pivoting, unit L below the diagonal); returns 0 or the
 // 1-based column of the first zero pivot
-template <int N>
-__device__ __forceinline__ int dgetrf(double* a, int* ipiv) {
+template <int N, class T>
+__device__ __forceinline__ int dgetrf(T* a, int* ipiv) {
   int info = 0;
 #pragma unroll
   for (int j = 0; j < N; ++j) {
     int jp = j;
-    double m = fabs(a[j * N + j]);
+    T m = n_abs(a[j * N + j]);
 #pragma unroll
     for (int i = j + 1; i < N; ++i)
-      if (fabs(a[i * N + j]) > m) { jp = i; m = fabs(a[i * N + j]); }
+      if (less(m, n_abs(a[i * N + j]))) { jp = i; m = n_abs(a[i * N + j]); }
     ipiv[j] = jp;
-    if (a[jp * N + j] != 0.0) {
+    if (nonzero(val(a[jp * N + j]))) {
       if (jp != j) {
 #pragma unroll
         for (int k = 0; k < N; ++k) {
-          const double t = a[j * N + k];
+          const T t = a[j * N + k];
           a[j * N + k] = a[jp * N + k];
           a[jp * N + k] = t;
         }
       }
       if (j < N - 1) {
-        if (fabs(a[j * N + j]) >= SFMIN) {
-          const double rp = 1.0 / a[j * N + j];
+        if (!less(n_abs(a[j * N + j]), T(SFMIN))) {
+          const T rp = 1.0 / a[j * N + j];
 #pragma unroll
           for (int i = j + 1; i < N; ++i) a[i * N + j] = rp * a[i * N + j];
         } else {
@@ -151,8 +152,8 @@ __device__ __forceinline__ int dgetrf(double* a, int* ipiv) {
     }
 #pragma unroll
     for (int jj = j + 1; jj < N; ++jj) {
-      if (a[j * N + jj] != 0.0) {
-        const double temp = -1.0 * a[j * N + jj];
+      if (nonzero(val(a[j * N + jj]))) {
+        const T temp = -a[j * N + jj];
 #pragma unroll
         for (int i = j + 1; i < N; ++i) a[i * N + jj] = a[i * N + jj] + a[i * N + j] * temp;
       }
@@ -160,101 +161,107 @@ __device__ __forceinline__ int dgetrf(double* a, int* ipiv) {
   }
   return info;
 }
-// the triangular solves of dgecon: kase 1 inv(L) then inv(U), kase 2 inv(U^T) then inv(L^T)
-template <int N>
-__device__ __forceinline__ void trs_kase(const double* af, int kase, double* x) {
+// x >= 0.0
+template <class T>
+__device__ __forceinline__ bool nonneg(T x) {
+  const long long b = dbits(val(x));
+  return b >= 0 ? b <= 0x7ff0000000000000LL : (b << 1) == 0;
+}
+// the triangular solves of dgecon (uv: recip32 of U's diagonal): kase 1 inv(L) then inv(U), kase 2 inv(U^T) then inv(L^T)
+template <int N, class T>
+__device__ __forceinline__ void trs_kase(const T* af, const unsigned* uv, int kase, T* x) {
   if (kase == 1) {
 #pragma unroll
     for (int j = 0; j < N; ++j)
-      if (x[j] != 0.0) {
-        const double temp = x[j];
+      if (nonzero(val(x[j]))) {
+        const T temp = x[j];
 #pragma unroll
         for (int i = j + 1; i < N; ++i) x[i] = x[i] - temp * af[i * N + j];
       }
 #pragma unroll
     for (int j = N - 1; j >= 0; --j)
-      if (x[j] != 0.0) {
-        x[j] = x[j] / af[j * N + j];
-        const double temp = x[j];
+      if (nonzero(val(x[j]))) {
+        x[j] = rcs::div_by(val(x[j]), val(af[j * N + j]), uv[j]);
+        const T temp = x[j];
 #pragma unroll
         for (int i = j - 1; i >= 0; --i) x[i] = x[i] - temp * af[i * N + j];
       }
   } else {
 #pragma unroll
     for (int j = 0; j < N; ++j) {
-      double temp = x[j];
+      T temp = x[j];
 #pragma unroll
       for (int i = 0; i < j; ++i) temp = temp - af[i * N + j] * x[i];
-      x[j] = temp / af[j * N + j];
+      x[j] = rcs::div_by(val(temp), val(af[j * N + j]), uv[j]);
     }
 #pragma unroll
     for (int j = N - 1; j >= 0; --j) {
-      double temp = x[j];
+      T temp = x[j];
 #pragma unroll
       for (int i = N - 1; i > j; --i) temp = temp - af[i * N + j] * x[i];
       x[j] = temp;
     }
   }
 }
-template <int N>
-__device__ __forceinline__ double dasum(const double* x) {
-  double t = 0.0;
+template <int N, class T>
+__device__ __forceinline__ T dasum(const T* x) {
+  T t = 0.0;
 #pragma unroll
-  for (int i = 0; i < N; ++i) t = t + fabs(x[i]);
+  for (int i = 0; i < N; ++i) t = t + n_abs(x[i]);
   return t;
 }
-template <int N>
-__device__ __forceinline__ int idamax(const double* x) {
+template <int N, class T>
+__device__ __forceinline__ int idamax(const T* x) {
   int k = 0;
-  double m = fabs(x[0]);
+  T m = n_abs(x[0]);
 #pragma unroll
   for (int i = 1; i < N; ++i)
-    if (fabs(x[i]) > m) { k = i; m = fabs(x[i]); }
+    if (less(m, n_abs(x[i]))) { k = i; m = n_abs(x[i]); }
   return k;
 }
 // dgecon('1') with dlacn2 (at most 5 iterations) unrolled
-template <int N>
-__device__ double dgecon(const double* af, double anorm) {
-  if (anorm == 0.0) return 0.0;
-  if (isnan(anorm)) return anorm;
-  double x[N], est, estold;
+template <int N, class T>
+__device__ T dgecon(const T* af, const unsigned* uv, T anorm) {
+  if (!nonzero(val(anorm))) return 0.0;
+  if (isnan(val(anorm))) return anorm;
+  T x[N], est, estold;
   int isgn[N];
 #pragma unroll
   for (int i = 0; i < N; ++i) x[i] = 1.0 / (double)N;
-  trs_kase<N>(af, 1, x);
+  trs_kase<N>(af, uv, 1, x);
   if (N == 1) {
-    est = fabs(x[0]);
+    est = n_abs(x[0]);
   } else {
     est = dasum<N>(x);
 #pragma unroll
-    for (int i = 0; i < N; ++i) { x[i] = (x[i] >= 0.0) ? 1.0 : -1.0; isgn[i] = x[i] >= 0.0 ? 1 : -1; }
-    trs_kase<N>(af, 2, x);
+    for (int i = 0; i < N; ++i) { isgn[i] = nonneg(x[i]) ? 1 : -1; x[i] = nonneg(x[i]) ? 1.0 : -1.0; }
+    trs_kase<N>(af, uv, 2, x);
     int j = idamax<N>(x), iter = 2;
     for (int guard = 0; guard < 8; ++guard) {
 #pragma unroll
       for (int i = 0; i < N; ++i) x[i] = (i == j) ? 1.0 : 0.0;
-      trs_kase<N>(af, 1, x);
+      trs_kase<N>(af, uv, 1, x);
       estold = est;
       est = dasum<N>(x);
       bool same = true;
 #pragma unroll
       for (int i = 0; i < N; ++i)
-        if ((x[i] >= 0.0 ? 1 : -1) != isgn[i]) same = false;
-      if (same || est <= estold) break;
+        if ((nonneg(x[i]) ? 1 : -1) != isgn[i]) same = false;
+      if (same || val(est) <= val(estold)) break;
 #pragma unroll
-      for (int i = 0; i < N; ++i) { x[i] = (x[i] >= 0.0) ? 1.0 : -1.0; isgn[i] = x[i] >= 0.0 ? 1 : -1; }
-      trs_kase<N>(af, 2, x);
+      for (int i = 0; i < N; ++i) { isgn[i] = nonneg(x[i]) ? 1 : -1; x[i] = nonneg(x[i]) ? 1.0 : -1.0; }
+      trs_kase<N>(af, uv, 2, x);
       const int jlast = j;
       j = idamax<N>(x);
-      double xl = 0.0;
+      T xl = 0.0;
 #pragma unroll
       for (int i = 0; i < N; ++i)
         if (i == jlast) xl = x[i];
-      double xj = 0.0;
+      T xj = 0.0;
 #pragma unroll
       for (int i = 0; i < N; ++i)
         if (i == j) xj = x[i];
-      if (xl != fabs(xj) && iter < 5) { iter = iter + 1; continue; }
+      if (val(xl) != val(n_abs(xj)) && iter < 5) { iter = iter + 1; continue; }
       break;
     }
     double altsgn = 1.0;
@@ -263,11 +270,11 @@ __device__ double dgecon(const double* af, double anorm) {
       x[i] = altsgn * (1.0 + (double)i / (double)(N - 1));
       altsgn = -altsgn;
     }
-    trs_kase<N>(af, 1, x);
-    const double temp = 2.0 * (dasum<N>(x) / (double)(3 * N));
-    if (temp > est) est = temp;
+    trs_kase<N>(af, uv, 1, x);
+    const T temp = twice_of(dasum<N>(x) / T((double)(3 * N)));
+    if (less(est, temp)) est = temp;
   }
-  if (est != 0.0) return (1.0 / est) / anorm;
+  if (nonzero(val(est))) return (1.0 / est) / anorm;
   return 0.0;
 }
 
@@ -275,11 +282,11 @@ __device__ double dgecon(const double* af, double anorm) {
 // x: this row's right-hand side (already row-scaled); returns A^-1 x for this
 // row (dgetrs('N')): the composed interchanges, then the column-oriented unit
 // lower and upper solves of dtrsm, skipping zero entries as dtrsm does.  The
-// divisions by the diagonal of U use its reciprocal pairs urh, url (div_rn:
+// divisions by the diagonal of U use its reciprocals urv (rcs::div_by:
 // the same bits as the IEEE division).
 template <int N>
 __device__ __forceinline__ double getrs_rows(double x, int src, const double* lu, const double* ukk,
-                                             const double* urh, const double* url, int r, int base) {
+                                             const unsigned* urv, int r, int base) {
   x = __shfl_sync(FULL, x, base + src);
 #pragma unroll
   for (int k = 0; k < N - 1; ++k) {
@@ -290,7 +297,7 @@ __device__ __forceinline__ double getrs_rows(double x, int src, const double* lu
   for (int k = N - 1; k >= 0; --k) {
     double xk = __shfl_sync(FULL, x, base + k);
     if (nonzero(xk)) {
-      xk = div_rn(xk, ukk[k], urh[k], url[k]);
+      xk = rcs::div_by(xk, ukk[k], urv[k]);
       if (r == k) x = xk;
       else if (r < k) x = x - xk * lu[k];
     }
@@ -316,33 +323,39 @@ __global__ void __launch_bounds__(128) k_bdf2_fixed(const Dev d, int euler) {
 }
 
 // Everything of BDF2_LU_SGS that the sweeps do not change, one thread per cell.
+// FP64 throughput bounds it: the divisions, comparisons and halvings run on the
+// integer pipes (Num).  With the sweep's divisions by shared reciprocals and
+// its staged records by word, an inner iteration on 120,000 cells takes 9.0
+// ms instead of 10.2.
 template <int NSP>
 __global__ void __launch_bounds__(128) k_bdf2_prep(const Dev d, const ThermoDev<NSP> th) {
   using namespace bdf2;
-  constexpr int V = 3 + NSP, RW = 2 * V + 4;
+  using N = Num<false>;
+  constexpr int V = 3 + NSP, RW = 2 * V + 3;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= d.NE) return;
   const int NE = d.NE;
-  const double dt = d.bpar[0], phi = d.bpar[1], vol = d.vol[i];
+  const N dt = d.bpar[0], phi = d.bpar[1], vol = d.vol[i];
   unsigned err = 0;
   // diagonal (Time_BDF2.f90:94-102) and right-hand side (:104-111)
-  double s = 0.0;
+  N s = 0.0;
   const int nf = d.nface[i];
-  for (int q = 0; q < nf; ++q) s = s + 0.5 * d.alpaF[d.cface[q * NE + i]];
-  const double ddi = s + vol * (1. / d.step[i] + (1 + phi) / dt);
+  for (int q = 0; q < nf; ++q) s = s + half_of(d.alpaF[d.cface[q * NE + i]]);
+  const N ddi = s + vol * (1. / N(d.step[i]) + (1. + phi) / dt);
+  const N wdt = (1. + phi) * vol / dt;
 #pragma unroll
   for (int k = 0; k < V; ++k)
-    d.hWA[k * NE + i] = d.hWA[k * NE + i] - (1 + phi) * vol / dt * d.WA[k * NE + i] + d.bfix[k * NE + i];
+    d.hWA[k * NE + i] = val(d.hWA[k * NE + i] - wdt * d.WA[k * NE + i] + d.bfix[k * NE + i]);
   // system matrix (:121-129)
-  double pri[V];
+  N pri[V];
 #pragma unroll
   for (int k = 0; k < V; ++k) pri[k] = d.PA[k * NE + i];
-  double a[V * V];
+  N a[V * V];
   con_to_pri_jaco<NSP>(th, pri, a, err);
 #pragma unroll
   for (int k = 0; k < V * V; ++k) a[k] = a[k] * ddi;
   if (NSP > 1) {
-    double dw[(NSP > 1 ? NSP - 1 : 1) * V];
+    N dw[(NSP > 1 ? NSP - 1 : 1) * V];
     dwdp<NSP>(th, pri, dw, err);
 #pragma unroll
     for (int j = 0; j < NSP - 1; ++j)
@@ -353,29 +366,32 @@ __global__ void __launch_bounds__(128) k_bdf2_prep(const Dev d, const ThermoDev<
   // matrix goes to the cell's record and gives its 1-norm (dlange('1')) before
   // the factorisation overwrites it in registers, so one V x V array is live
   // instead of two (the same operations as factoring a copy).
-  double rs[V], cs[V], rowcnd = 0, colcnd = 0, amax = 0;
+  N rs[V], cs[V], rowcnd = 0.0, colcnd = 0.0, amax = 0.0;
   int equ = 0;
   if (dgeequ<V>(a, rs, cs, rowcnd, colcnd, amax) == 0) equ = dlaqge<V>(a, rs, cs, rowcnd, colcnd, amax);
   double* m = d.bmat + (size_t)i * V * RW;
-  double anorm = 0.0;
+  N anorm = 0.0;
 #pragma unroll
   for (int j = 0; j < V; ++j) {
-    double sum = 0.0;
+    N sum = 0.0;
 #pragma unroll
-    for (int r = 0; r < V; ++r) sum = sum + fabs(a[r * V + j]);
-    if (anorm < sum || isnan(sum)) anorm = sum;
+    for (int r = 0; r < V; ++r) sum = sum + n_abs(a[r * V + j]);
+    if (less(anorm, sum) || isnan(val(sum))) anorm = sum;
   }
 #pragma unroll
   for (int r = 0; r < V; ++r)
 #pragma unroll
-    for (int c = 0; c < V; ++c) m[r * RW + c] = a[r * V + c];
-  double* af = a;
+    for (int c = 0; c < V; ++c) m[r * RW + c] = val(a[r * V + c]);
+  N* af = a;
   int ipiv[V];
   const int info = dgetrf<V>(af, ipiv);
+  unsigned uv[V];
+#pragma unroll
+  for (int r = 0; r < V; ++r) uv[r] = rcs::recip32(val(af[r * V + r]));
   if (info > 0) {
     err |= ERR_LINSOLVE;
   } else {
-    if (dgecon<V>(af, anorm) < EPS) err |= ERR_LINSOLVE;
+    if (val(dgecon<V>(af, uv, anorm)) < EPS) err |= ERR_LINSOLVE;
   }
   int src[V];
 #pragma unroll
@@ -389,46 +405,39 @@ __global__ void __launch_bounds__(128) k_bdf2_prep(const Dev d, const ThermoDev<
 #pragma unroll
   for (int r = 0; r < V; ++r) {
 #pragma unroll
-    for (int c = 0; c < V; ++c) m[r * RW + V + c] = af[r * V + c];
-    m[r * RW + 2 * V] = rs[r];
-    m[r * RW + 2 * V + 1] = cs[r];
-    const Recip ru = recip_of(af[r * V + r]);
-    m[r * RW + 2 * V + 2] = ru.h;
-    m[r * RW + 2 * V + 3] = ru.l;
+    for (int c = 0; c < V; ++c) m[r * RW + V + c] = val(af[r * V + c]);
+    m[r * RW + 2 * V] = val(rs[r]);
+    m[r * RW + 2 * V + 1] = val(cs[r]);
+    m[r * RW + 2 * V + 2] = v_slot(uv[r]);
     d.bperm[i * 8 + r] = src[r];
   }
   d.bperm[i * 8 + 7] = equ;
   // this cell's gas state for its neighbours' sweeps (Time_BDF2.f90:145-166)
-  double yy[NSP], entha[NSP], Cp, gama, Rcpcv;
-  double sy = 0.0;
+  N yy[NSP], entha[NSP], Cp, gama, Rcpcv;
 #pragma unroll
-  for (int k = 0; k < NSP - 1; ++k) { yy[k] = pri[4 + k]; sy = sy + yy[k]; }
-  yy[NSP - 1] = 1. - sy;
-  const double pp = pri[0], uu = pri[1], vv = pri[2], tt = pri[3];
+  for (int k = 0; k < NSP - 1; ++k) yy[k] = pri[4 + k];
+  yy[NSP - 1] = last_y<NSP>(yy);
+  const N pp = pri[0], uu = pri[1], vv = pri[2], tt = pri[3];
   gas<NSP>(th, yy, tt, Cp, gama, Rcpcv, err);
   enthalpy<NSP>(th, tt, entha, err);
-  double hh = 0.0;
-#pragma unroll
-  for (int k = 0; k < NSP; ++k) hh = hh + yy[k] * entha[k];
-  const double rct = Rcpcv * tt, rr = pp / rct, ek = 0.5 * (uu * uu + vv * vv);
+  const N hh = dot<NSP>(yy, entha);
+  const N rct = Rcpcv * tt, rr = pp / rct, ek = half_of(uu * uu + vv * vv);
   double* nb = d.bnb;
-  nb[NB_RR * NE + i] = rr;
-  nb[NB_RRC * NE + i] = rr * Rcpcv;
-  nb[NB_RT * NE + i] = rr * tt;
-  nb[NB_RCT * NE + i] = rct;
-  nb[NB_RCP * NE + i] = rr * Cp;
-  nb[NB_HH * NE + i] = hh;
-  nb[NB_EK * NE + i] = ek;
-  nb[NB_ROU * NE + i] = rr * uu;
-  nb[NB_ROV * NE + i] = rr * vv;
-  nb[NB_ROEPP * NE + i] = (rr * (hh + ek) - pp) + pp;
+  nb[NB_RR * NE + i] = val(rr);
+  nb[NB_RRC * NE + i] = val(rr * Rcpcv);
+  nb[NB_RT * NE + i] = val(rr * tt);
+  nb[NB_RCT * NE + i] = val(rct);
+  nb[NB_RCP * NE + i] = val(rr * Cp);
+  nb[NB_HH * NE + i] = val(hh);
+  nb[NB_EK * NE + i] = val(ek);
+  nb[NB_ROU * NE + i] = val(rr * uu);
+  nb[NB_ROV * NE + i] = val(rr * vv);
+  nb[NB_ROEPP * NE + i] = val((rr * (hh + ek) - pp) + pp);
 #pragma unroll
-  for (int k = 0; k < NSP; ++k) nb[(NB_H + k) * NE + i] = entha[k];
+  for (int k = 0; k < NSP; ++k) nb[(NB_H + k) * NE + i] = val(entha[k]);
 #pragma unroll
-  for (int k = 0; k < NSP - 1; ++k) nb[(nb_ry<NSP>() + k) * NE + i] = rr * yy[k];
-  const Recip rc = recip_of(rct);
-  nb[nb_rct<NSP>() * NE + i] = rc.h;
-  nb[(nb_rct<NSP>() + 1) * NE + i] = rc.l;
+  for (int k = 0; k < NSP - 1; ++k) nb[(nb_ry<NSP>() + k) * NE + i] = val(rr * yy[k]);
+  nb[nb_rct<NSP>() * NE + i] = v_slot(rcs::recip32(val(rct)));
   flag(d, err);
 }
 
@@ -439,8 +448,9 @@ template <int NSP>
 struct BSlot {
   int j;
   bool act;
-  double dx, dy, aF, uu, vv, rr, rrc, rt, rct, rcth, rctl, unormal, rou, rov, rcp, hh, ek, roepp;
+  double dx, dy, aF, uu, vv, rr, rrc, rt, rct, unormal, rou, rov, rcp, hh, ek, roepp;
   double ent[NSP], yy[NSP], ry[NSP];
+  unsigned rctv;  // recip32(rct)
 };
 template <int NSP, bool FWD>
 __device__ __forceinline__ BSlot<NSP> bslot_load(const Dev& d, int t, bool valid, int q) {
@@ -450,9 +460,9 @@ __device__ __forceinline__ BSlot<NSP> bslot_load(const Dev& d, int t, bool valid
   BSlot<NSP> b;
   b.j = valid ? d.swj[DIR][q * NE + t] : -1;
   b.act = b.j >= 0;
-  b.dx = b.dy = b.aF = b.uu = b.vv = b.rr = b.rrc = b.rt = b.rct = b.rctl = b.unormal = 0.0;
+  b.dx = b.dy = b.aF = b.uu = b.vv = b.rr = b.rrc = b.rt = b.rct = b.unormal = 0.0;
   b.rou = b.rov = b.rcp = b.hh = b.ek = b.roepp = 0.0;
-  b.rcth = 1.0;
+  b.rctv = 0;
 #pragma unroll
   for (int k = 0; k < NSP; ++k) { b.ent[k] = 0.0; b.yy[k] = 0.0; b.ry[k] = 0.0; }
   if (b.act) {
@@ -465,7 +475,7 @@ __device__ __forceinline__ BSlot<NSP> bslot_load(const Dev& d, int t, bool valid
     b.vv = d.PA[2 * NE + j];
     const double* nb = d.bnb;
     b.rr = nb[NB_RR * NE + j]; b.rrc = nb[NB_RRC * NE + j]; b.rt = nb[NB_RT * NE + j]; b.rct = nb[NB_RCT * NE + j];
-    b.rcth = nb[nb_rct<NSP>() * NE + j]; b.rctl = nb[(nb_rct<NSP>() + 1) * NE + j];
+    b.rctv = slot_v(nb[nb_rct<NSP>() * NE + j]);
     b.unormal = b.uu * b.dx + b.vv * b.dy;
     b.rou = nb[NB_ROU * NE + j];
     b.rov = nb[NB_ROV * NE + j];
@@ -483,16 +493,17 @@ __device__ __forceinline__ BSlot<NSP> bslot_load(const Dev& d, int t, bool valid
 }
 template <int NSP>
 struct BRow {
-  double arow[3 + NSP], lrow[3 + NSP], ukk[3 + NSP], urh[3 + NSP], url[3 + NSP], rsc, csc;
+  double arow[3 + NSP], lrow[3 + NSP], ukk[3 + NSP], rsc, csc;
+  unsigned urv[3 + NSP];  // recip32(ukk)
   int src, equ;
 };
 template <int NSP>
 __device__ __forceinline__ BRow<NSP> brow_load(const Dev& d, int i, bool valid, int r) {
-  constexpr int V = 3 + NSP, RW = 2 * V + 4;
+  constexpr int V = 3 + NSP, RW = 2 * V + 3;
   BRow<NSP> w;
   w.rsc = 1.0; w.csc = 1.0; w.src = 0; w.equ = 0;
 #pragma unroll
-  for (int k = 0; k < V; ++k) { w.arow[k] = 0.0; w.lrow[k] = 0.0; w.ukk[k] = 1.0; w.urh[k] = 1.0; w.url[k] = 0.0; }
+  for (int k = 0; k < V; ++k) { w.arow[k] = 0.0; w.lrow[k] = 0.0; w.ukk[k] = 1.0; w.urv[k] = 0; }
   if (valid) {
     const double* m = d.bmat + (size_t)i * V * RW;
     if (r < V) {
@@ -505,8 +516,7 @@ __device__ __forceinline__ BRow<NSP> brow_load(const Dev& d, int i, bool valid, 
 #pragma unroll
     for (int k = 0; k < V; ++k) {
       w.ukk[k] = m[k * RW + V + k];
-      w.urh[k] = m[k * RW + 2 * V + 2];
-      w.url[k] = m[k * RW + 2 * V + 3];
+      w.urv[k] = bdf2::slot_v(m[k * RW + 2 * V + 2]);
     }
     w.equ = d.bperm[i * 8 + 7];
   }
@@ -535,25 +545,25 @@ __device__ __forceinline__ void bslot_terms(const Dev& d, const ThermoDev<NSP>& 
   double s1 = 0.0;
 #pragma unroll
   for (int k = 0; k < NSP; ++k) s1 = s1 + th.R[k] * dyy[k];
-  const double drr = div_rn(dpp - b.rrc * dtt - b.rt * s1, b.rct, b.rcth, b.rctl);
+  const double drr = rcs::div_by(dpp - b.rrc * dtt - b.rt * s1, b.rct, b.rctv);
   const double dunormal = duu * b.dx + dvv * b.dy;
   const double aF = b.aF, unormal = b.unormal, rr = b.rr;
   if (lo) {
     const double dru = rr * duu + b.uu * drr;
     const double drv = rr * dvv + b.vv * drr;
-    c[0] = 0.5 * (-aF * drr + dru * b.dx + drv * b.dy);
-    c[1] = 0.5 * (-aF * dru + dru * unormal + b.rou * dunormal + dpp * b.dx);
-    c[2] = 0.5 * (-aF * drv + drv * unormal + b.rov * dunormal + dpp * b.dy);
+    c[0] = half_of(-aF * drr + dru * b.dx + drv * b.dy);
+    c[1] = half_of(-aF * dru + dru * unormal + b.rou * dunormal + dpp * b.dx);
+    c[2] = half_of(-aF * drv + drv * unormal + b.rov * dunormal + dpp * b.dy);
   } else {
     double s2 = 0.0;
 #pragma unroll
     for (int k = 0; k < NSP; ++k) s2 = s2 + b.ent[k] * dyy[k];
     const double dre = b.rcp * dtt + rr * s2 + b.hh * drr + rr * (b.uu * duu + b.vv * dvv) + b.ek * drr - dpp;
-    c[3] = 0.5 * (-aF * dre + dunormal * b.roepp + unormal * (dre + dpp));
+    c[3] = half_of(-aF * dre + dunormal * b.roepp + unormal * (dre + dpp));
 #pragma unroll
     for (int k = 0; k < NSP - 1; ++k) {
       const double dry = rr * dyy[k] + b.yy[k] * drr;
-      c[4 + k] = 0.5 * (-aF * dry + dry * unormal + b.ry[k] * dunormal);
+      c[4 + k] = half_of(-aF * dry + dry * unormal + b.ry[k] * dunormal);
     }
   }
 }
@@ -575,7 +585,7 @@ __device__ __forceinline__ long long berr_bits(double y, double wk, int r) {
   using namespace bdf2;
   const double safe1 = (V + 1) * SFMIN, safe2 = safe1 / EPS;
   long long vb = 0;
-  if (r < V) vb = dbits((dbits(wk) > dbits(safe2)) ? fabs(y) / wk : (fabs(y) + safe1) / (wk + safe1));
+  if (r < V) vb = dbits((dbits(wk) > dbits(safe2)) ? rcs::div(fabs(y), wk) : (fabs(y) + safe1) / (wk + safe1));
   vb = max(vb, (long long)__shfl_xor_sync(FULL, (unsigned long long)vb, 1));
   vb = max(vb, (long long)__shfl_xor_sync(FULL, (unsigned long long)vb, 2));
   vb = max(vb, (long long)__shfl_xor_sync(FULL, (unsigned long long)vb, 4));
@@ -625,7 +635,7 @@ __device__ __forceinline__ void bdf2_cell_step(const Dev& d, const ThermoDev<NSP
   double b = FWD ? hown - dflux : dflux;
   if (rowequ) b = rw.rsc * b;
   if (!(valid && r < V)) b = 0.0;
-  double x = getrs_rows<V>(b, rw.src, rw.lrow, rw.ukk, rw.urh, rw.url, r, base);
+  double x = getrs_rows<V>(b, rw.src, rw.lrow, rw.ukk, rw.urv, r, base);
   // dgerfs refinement: residual, componentwise backward error, correction.
   // The backward error is non-negative: its maximum and the loop tests
   // compare bit patterns; 2 berr <= lstres is berr <= lstres/2 (both exact).
@@ -636,16 +646,19 @@ __device__ __forceinline__ void bdf2_cell_step(const Dev& d, const ThermoDev<NSP
     double xs[V];
 #pragma unroll
     for (int k = 0; k < V; ++k) xs[k] = __shfl_sync(FULL, x, base + k);
-    double y = b;
+    // y = b - A x and w = |b| + |A| |x| on the same products (rounding is
+    // symmetric: (-x) a = -(x a) and |a| |x| = |x a|)
+    double y = b, wk = fabs(b);
 #pragma unroll
-    for (int k = 0; k < V; ++k) y = y + (-1.0 * xs[k]) * rw.arow[k];
-    double wk = fabs(b);
-#pragma unroll
-    for (int k = 0; k < V; ++k) wk = wk + fabs(rw.arow[k]) * fabs(xs[k]);
+    for (int k = 0; k < V; ++k) {
+      const double p = xs[k] * rw.arow[k];
+      y = y - p;
+      wk = wk + fabs(p);
+    }
     const long long vb = berr_bits<V>(y, wk, r);
     const bool cont = go && vb > dbits(EPS) && vb <= lstres_half && count <= 5;
     if (!__any_sync(FULL, cont)) break;
-    const double corr = getrs_rows<V>(y, rw.src, rw.lrow, rw.ukk, rw.urh, rw.url, r, base);
+    const double corr = getrs_rows<V>(y, rw.src, rw.lrow, rw.ukk, rw.urv, r, base);
     if (cont) {
       x = x + corr;
       lstres_half = vb - (1LL << 52);  // berr / 2: berr > eps is a normal number
@@ -707,6 +720,27 @@ struct BStage {
   double hown;
   int i, valid;
 };
+// A lane's staged record in shared memory, word w of lane l at [32 w + l]: a
+// warp moves a word without bank conflicts, and reads only the words it uses
+// (the record is about 560 bytes; as an array of records its words met in two
+// banks of the 32).
+template <class S>
+__device__ __forceinline__ void stage_put(double* sm, const S& s) {
+  static_assert(sizeof(S) % 8 == 0, "whole words");
+  double w[sizeof(S) / 8];
+  memcpy(w, &s, sizeof(S));
+#pragma unroll
+  for (int k = 0; k < (int)(sizeof(S) / 8); ++k) sm[32 * k + (threadIdx.x & 31)] = w[k];
+}
+template <class S>
+__device__ __forceinline__ S stage_get(const double* sm) {
+  double w[sizeof(S) / 8];
+#pragma unroll
+  for (int k = 0; k < (int)(sizeof(S) / 8); ++k) w[k] = sm[32 * k + (threadIdx.x & 31)];
+  S s;
+  memcpy(&s, w, sizeof(S));
+  return s;
+}
 // A pass of at most four cells runs on both compute warps split by rows
 // (bdf2_cell_step PART 1 and 2), otherwise four cells on each (PART 0).
 constexpr int BFLOW_THREADS = 160, BFLOW_NB = 96;  // all five warps; a role pair and the coordinator
@@ -718,7 +752,9 @@ __global__ void __launch_bounds__(BFLOW_THREADS, 1) k_bdf2_flow(const Dev d, con
   constexpr int V = 3 + NSP;
   static_assert(V <= 7, "one lane per row and the flags in slot 7");
   extern __shared__ __align__(16) uint8_t bflow_smem_raw[];
-  BStage<NSP>* s_st = reinterpret_cast<BStage<NSP>*>(bflow_smem_raw);  // [buffer][warp][lane]
+  auto buffer = [&](int k, int w) {  // the record of pass k for compute warp w
+    return reinterpret_cast<double*>(bflow_smem_raw) + ((k & 1) * 2 + w) * (int)(4 * sizeof(BStage<NSP>));
+  };
   __shared__ double wsm[2][4 * V * 4];
   __shared__ unsigned s_epoch;
   __shared__ volatile int s_bad, s_go[2], s_split[2];
@@ -784,7 +820,7 @@ __global__ void __launch_bounds__(BFLOW_THREADS, 1) k_bdf2_flow(const Dev d, con
       const bool valid = t < t1;
       if (w == 0 && lane == 0) s_split[k & 1] = split ? 1 : 0;
       const int i = valid ? d.swi[fwd ? 0 : 1][t] : 0;
-      BStage<NSP>& e = s_st[((k & 1) * 2 + w) * 32 + lane];
+      BStage<NSP> e;
       e.sp = fwd ? bslot_load<NSP, true>(d, t, valid, q) : bslot_load<NSP, false>(d, t, valid, q);
       e.rw = brow_load<NSP>(d, i, valid, r);
       // forward: the set-up's right-hand side, which only this cell's own
@@ -792,6 +828,7 @@ __global__ void __launch_bounds__(BFLOW_THREADS, 1) k_bdf2_flow(const Dev d, con
       e.hown = fwd && valid && r < V ? __ldcg(d.hWA + r * d.NE + i) : 0.0;
       e.i = i;
       e.valid = valid ? 1 : 0;
+      stage_put(buffer(k, w), e);
       __syncwarp();
       __threadfence_block();
       bar_arrive(5, BFLOW_NB);
@@ -805,9 +842,9 @@ __global__ void __launch_bounds__(BFLOW_THREADS, 1) k_bdf2_flow(const Dev d, con
     for (int k = 0; k < n; ++k) {
       const bool fwd = k < nf;
       bar_named(3, BFLOW_THREADS);
-      const BStage<NSP>& e = s_st[((k & 1) * 2 + warp) * 32 + lane];
-      const BSlot<NSP> sp = e.sp;
-      const BRow<NSP> rw = e.rw;
+      const BStage<NSP> e = stage_get<BStage<NSP>>(buffer(k, warp));
+      const BSlot<NSP>& sp = e.sp;
+      const BRow<NSP>& rw = e.rw;
       const int i = e.i;
       const bool valid = e.valid != 0;
       // backward: the cell's own increment, as this block's forward pass of
@@ -847,35 +884,34 @@ __global__ void __launch_bounds__(BFLOW_THREADS, 1) k_bdf2_flow(const Dev d, con
 template <int NSP>
 __global__ void __launch_bounds__(128) k_bdf2_update(const Dev d, const ThermoDev<NSP> th) {
   constexpr int V = 3 + NSP;
+  using N = Num<false>;
   pdl_wait();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= d.NE) return;
   const int NE = d.NE;
   unsigned err = 0;
-  double P[V];
+  N P[V];
 #pragma unroll
   for (int k = 0; k < V; ++k) {
     P[k] = d.PA[k * NE + i] + d.hWA[k * NE + i];
-    d.PA[k * NE + i] = P[k];
+    d.PA[k * NE + i] = val(P[k]);
   }
-  double yy[NSP], entha[NSP], Cp, gama, Rcpcv, s = 0.0;
+  N yy[NSP], entha[NSP], Cp, gama, Rcpcv;
 #pragma unroll
-  for (int k = 0; k < NSP - 1; ++k) { yy[k] = P[4 + k]; s = s + yy[k]; }
-  yy[NSP - 1] = 1.0 - s;
-  const double pp = P[0], uu = P[1], vv = P[2], tt = P[3];
+  for (int k = 0; k < NSP - 1; ++k) yy[k] = P[4 + k];
+  yy[NSP - 1] = last_y<NSP>(yy);
+  const N pp = P[0], uu = P[1], vv = P[2], tt = P[3];
   gas<NSP>(th, yy, tt, Cp, gama, Rcpcv, err);
-  const double rr = pp / (Rcpcv * tt);
+  const N rr = pp / (Rcpcv * tt);
   enthalpy<NSP>(th, tt, entha, err);
-  double hh = 0.0;
+  const N hh = dot<NSP>(yy, entha);
+  d.WA[0 * NE + i] = val(rr);
+  d.WA[1 * NE + i] = val(rr * uu);
+  d.WA[2 * NE + i] = val(rr * vv);
+  d.WA[3 * NE + i] = val(rr * (hh + half_of(uu * uu + vv * vv)) - pp);
 #pragma unroll
-  for (int k = 0; k < NSP; ++k) hh = hh + yy[k] * entha[k];
-  d.WA[0 * NE + i] = rr;
-  d.WA[1 * NE + i] = rr * uu;
-  d.WA[2 * NE + i] = rr * vv;
-  d.WA[3 * NE + i] = rr * (hh + 0.5 * (uu * uu + vv * vv)) - pp;
-#pragma unroll
-  for (int k = 0; k < NSP - 1; ++k) d.WA[(4 + k) * NE + i] = rr * yy[k];
-  if (i == 0 && isnan(rr)) err |= ERR_NAN;
+  for (int k = 0; k < NSP - 1; ++k) d.WA[(4 + k) * NE + i] = val(rr * yy[k]);
+  if (i == 0 && isnan(val(rr))) err |= ERR_NAN;
   flag(d, err);
 }
 

@@ -3673,7 +3673,7 @@ static int bdf2_setup(rc_ctx* c) {
   int st = dev_zeros(c, V * NE, &c->d.WP);
   st |= dev_zeros(c, V * NE, &c->d.WP2);
   st |= dev_zeros(c, V * NE, &c->d.bfix);
-  st |= dev_zeros(c, NE * V * (2 * V + 4), &c->d.bmat);
+  st |= dev_zeros(c, NE * V * (2 * V + 3), &c->d.bmat);
   st |= dev_zeros(c, 8 * NE, &c->d.bperm);
   st |= dev_zeros(c, (size_t)nbq * NE, &c->d.bnb);
   st |= dev_zeros(c, (size_t)2, &c->bpar_dev);
