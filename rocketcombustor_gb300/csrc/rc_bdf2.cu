@@ -351,12 +351,13 @@ __global__ void __launch_bounds__(128) k_bdf2_prep(const Dev d, const ThermoDev<
 #pragma unroll
   for (int k = 0; k < V; ++k) pri[k] = d.PA[k * NE + i];
   N a[V * V];
-  con_to_pri_jaco<NSP>(th, pri, a, err);
+  N rj, Rj;
+  con_to_pri_jaco<NSP>(th, pri, a, rj, Rj, err);
 #pragma unroll
   for (int k = 0; k < V * V; ++k) a[k] = a[k] * ddi;
   if (NSP > 1) {
     N dw[(NSP > 1 ? NSP - 1 : 1) * V];
-    dwdp<NSP>(th, pri, dw, err);
+    dwdp<NSP>(th, pri, rj, Rj, dw);
 #pragma unroll
     for (int j = 0; j < NSP - 1; ++j)
 #pragma unroll

@@ -29,17 +29,20 @@
 namespace rc {
 
 // dU/dP, row-major [V][V]; U = (rho, rho u, rho v, rho E, rho Y_1..), P = (p, u, v, T, Y_1..).
+// r and Rcpcv return the density and the gas constant, for dwdp.
 template <int NSP, class N>
-__device__ __forceinline__ void con_to_pri_jaco(const ThermoDev<NSP>& th, const N* pri, N* J, unsigned& err) {
+__device__ __forceinline__ void con_to_pri_jaco(const ThermoDev<NSP>& th, const N* pri, N* J, N& r, N& Rcpcv,
+                                                unsigned& err) {
   constexpr int V = 3 + NSP, NS1 = NSP - 1;
   const N p = pri[0], u = pri[1], v = pri[2], t = pri[3];
-  N y2[NSP], entha[NSP], dhdy[NSP], drdy[NSP], Cp, gama, Rcpcv;
-  N s = 0.0;
+  N y2[NSP], entha[NSP], dhdy[NSP], drdy[NSP], Cp, gama;
 #pragma unroll
-  for (int i = 0; i < NS1; ++i) { y2[i] = pri[4 + i]; s = s + pri[4 + i]; }
-  y2[NSP - 1] = 1. - s;
+  for (int i = 0; i < NS1; ++i) y2[i] = pri[4 + i];
+  y2[NSP - 1] = last_y<NSP>(y2);
   gas<NSP>(th, y2, t, Cp, gama, Rcpcv, err);
-  const N r = p / (Rcpcv * t);
+  const N rt = Rcpcv * t;
+  const unsigned rtv = rcs::recip32(val(rt));
+  r = div_fixed(p, rt, rtv);
   enthalpy<NSP>(th, t, entha, err);
   N h = entha[NSP - 1];
 #pragma unroll
@@ -47,9 +50,11 @@ __device__ __forceinline__ void con_to_pri_jaco(const ThermoDev<NSP>& th, const 
     h = h + pri[4 + i] * (entha[i] - entha[NSP - 1]);
     dhdy[i] = entha[i] - entha[NSP - 1];
   }
-  const N drdp = 1. / (Rcpcv * t), drdt = -p / (Rcpcv * t * t);
+  const N drdp = div_fixed(N(1.), rt, rtv), drdt = -p / (rt * t);
+  const N trr = t * Rcpcv * Rcpcv;
+  const unsigned trrv = rcs::recip32(val(trr));
 #pragma unroll
-  for (int i = 0; i < NS1; ++i) drdy[i] = -N(th.R[i] - th.R[NSP - 1]) * p / (t * Rcpcv * Rcpcv);
+  for (int i = 0; i < NS1; ++i) drdy[i] = div_fixed(-N(th.R[i] - th.R[NSP - 1]) * p, trr, trrv);
   const N ke = h + half_of(u * u + v * v);
 #pragma unroll
   for (int k = 0; k < V * V; ++k) J[k] = 0.0;
@@ -74,33 +79,28 @@ __device__ __forceinline__ void con_to_pri_jaco(const ThermoDev<NSP>& th, const 
 // d omega_i / dP, row-major [NSP-1][V].  Model 1 leaves dkfdy(3:) unset in
 // the reference (chemical_kinetics.f90:228-243); it is taken as dkfdr*drdy(3:).
 template <int NSP, class N>
-__device__ __forceinline__ void dwdp(const ThermoDev<NSP>& th, const N* pri, N* D, unsigned& err) {
+__device__ __forceinline__ void dwdp(const ThermoDev<NSP>& th, const N* pri, N rho, N Rcpcv, N* D) {
   constexpr int V = 3 + NSP, NS1 = NSP - 1;
   const N p = pri[0], T = pri[3];
-  N y[NSP], y2[NSP], drdy[NSP], dkf[V], Cp, gama, Rcpcv;
-  N s = 0.0;
+  N y[NSP], drdy[NSP], dkf[V];
 #pragma unroll
-  for (int i = 0; i < NS1; ++i) { y[i] = pri[4 + i]; y2[i] = y[i]; s = s + y[i]; }
-  y2[NSP - 1] = 1. - s;
-  gas<NSP>(th, y2, T, Cp, gama, Rcpcv, err);
-  const N rho = p / (Rcpcv * T);
-#pragma unroll
-  for (int i = 0; i < NS1; ++i) y[i] = fmin2(N(1.), fmax2(N(0.), y[i]));
+  for (int i = 0; i < NS1; ++i) y[i] = fmin2(N(1.), fmax2(N(0.), pri[4 + i]));
   if (less(y[0], N(1.0e-12))) {
 #pragma unroll
     for (int c = 0; c < V; ++c) dkf[c] = 0.;
   } else {
     N af = th.Af * n_exp(-th.E / (th.Rconstant * T));
-    const N r1 = div_fixed(y[0] * rho, N(th.mw1000[0]), th.mw1000r[0]);
-    const N dr1dr = div_fixed(y[0], N(th.mw1000[0]), th.mw1000r[0]);
-    const N dr1dy1 = div_fixed(rho, N(th.mw1000[0]), th.mw1000r[0]);
+    const N r1 = div_fixed(y[0] * rho, N(th.mw1000[0]), th.mw1000v[0]);
+    const N dr1dr = div_fixed(y[0], N(th.mw1000[0]), th.mw1000v[0]);
+    const N dr1dy1 = div_fixed(rho, N(th.mw1000[0]), th.mw1000v[0]);
     const N y1 = NS1 > 1 ? y[NS1 > 1 ? 1 : 0] : 0.0;
-    const N r2 = div_fixed(y1 * rho, N(th.mw1000[1]), th.mw1000r[1]);
-    const N dr2dr = div_fixed(y1, N(th.mw1000[1]), th.mw1000r[1]);
-    const N dr2dy2 = div_fixed(rho, N(th.mw1000[1]), th.mw1000r[1]);
+    const N r2 = div_fixed(y1 * rho, N(th.mw1000[1]), th.mw1000v[1]);
+    const N dr2dr = div_fixed(y1, N(th.mw1000[1]), th.mw1000v[1]);
+    const N dr2dy2 = div_fixed(rho, N(th.mw1000[1]), th.mw1000v[1]);
     const N drdp = rho / p, drdT = -rho / T;
+    const unsigned Rv = rcs::recip32(val(Rcpcv));
 #pragma unroll
-    for (int i = 0; i < NS1; ++i) drdy[i] = -N(th.R[i] - th.R[NSP - 1]) * rho / Rcpcv;
+    for (int i = 0; i < NS1; ++i) drdy[i] = div_fixed(-N(th.R[i] - th.R[NSP - 1]) * rho, Rcpcv, Rv);
     N dkfdr, dkfdT, dkfdy[NSP];
     if (th.model == 0) {
       const N l1 = n_log(r1), l2 = n_log(r2);
@@ -136,7 +136,7 @@ __device__ __forceinline__ void dwdp(const ThermoDev<NSP>& th, const N* pri, N* 
 // that every index is known and the system stays in registers (a loop over
 // the columns was left rolled, with the matrix in local memory).
 template <int NV, int K, class N>
-__device__ __forceinline__ bool gepp_column(N* A, N* b) {
+__device__ __forceinline__ bool gepp_column(N* A, N* b, unsigned* V) {
   int piv = K;
   N best = n_abs(A[K * NV + K]);
 #pragma unroll
@@ -155,25 +155,27 @@ __device__ __forceinline__ bool gepp_column(N* A, N* b) {
       }
   }
   const N dk = A[K * NV + K];
+  V[K] = rcs::recip32(val(dk));
 #pragma unroll
   for (int r = K + 1; r < NV; ++r) {
-    const N f = A[r * NV + K] / dk;
+    const N f = div_fixed(A[r * NV + K], dk, V[K]);
 #pragma unroll
     for (int c = K + 1; c < NV; ++c) A[r * NV + c] = A[r * NV + c] - f * A[K * NV + c];
     b[r] = b[r] - f * b[K];
   }
-  if constexpr (K + 1 < NV) return gepp_column<NV, K + 1>(A, b);
+  if constexpr (K + 1 < NV) return gepp_column<NV, K + 1>(A, b, V);
   return true;
 }
 template <int NV, class N>
 __device__ __forceinline__ bool gepp_solve(N* A, N* b) {
-  if (!gepp_column<NV, 0>(A, b)) return false;
+  unsigned V[NV];  // recip32 of the pivots
+  if (!gepp_column<NV, 0>(A, b, V)) return false;
 #pragma unroll
   for (int k = NV - 1; k >= 0; --k) {
     N s = b[k];
 #pragma unroll
     for (int c = k + 1; c < NV; ++c) s = s - A[k * NV + c] * b[c];
-    b[k] = s / A[k * NV + k];
+    b[k] = div_fixed(s, A[k * NV + k], V[k]);
   }
   return true;
 }
@@ -208,8 +210,9 @@ struct Reactor {
     N A[V * V], D[(NS1 > 0 ? NS1 : 1) * V], b[V], prod[NSP], Y[NSP], Rcpcv;
     const bool last = nacc + 1 >= maxsub || natt >= 2 * maxsub;
     if (last || less(rem, hs)) hs = rem;
-    con_to_pri_jaco<NSP>(th, P, A, err);
-    dwdp<NSP>(th, P, D, err);
+    N r;
+    con_to_pri_jaco<NSP>(th, P, A, r, Rcpcv, err);
+    dwdp<NSP>(th, P, r, Rcpcv, D);
 #pragma unroll
     for (int i = 0; i < NS1; ++i) Y[i] = P[4 + i];
     Y[NSP - 1] = last_y<NSP>(Y);

@@ -263,9 +263,12 @@ __device__ __forceinline__ void recon(const Dev& d, int c, double v0, double v1,
 // Bound by the FP64 unit (about 1,150 FP64 instructions of a warp per 32
 // faces, 77 cycles each) and, with the divisions, square roots and the
 // transport part's multiplications on them (NT), the integer pipes.  2M
-// triangles, 3.0 M faces: 15.5 -> 8.2 ms; 120,000 triangles 988 -> 552 us.
+// triangles, 3.0 M faces: 15.5 -> 7.6 ms; 120,000 triangles 988 -> 550 us.
+// Four blocks per SM (128 registers, 24 bytes spilled): with the 140 that the
+// compiler takes by itself three fit, and 120,000 triangles' 1,406 blocks are
+// 3.1 waves, 598 us.
 template <int NSP, bool VISC, class N, class NT>
-__global__ void __launch_bounds__(128) k_face_flux(const Dev d, const ThermoDev<NSP> th) {
+__global__ void __launch_bounds__(128, 4) k_face_flux(const Dev d, const ThermoDev<NSP> th) {
   constexpr int V = 3 + NSP;
   const int f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f >= d.NF) return;
@@ -420,13 +423,13 @@ __global__ void __launch_bounds__(128) k_face_flux(const Dev d, const ThermoDev<
     }
     if (NR >= 0) {
       const N dxk = d.fdxk[f], y1 = d.fysn[f], y2 = d.fysn[NF + f];
-      const Recip rk = {d.fdxkr[f], d.fdxkr[NF + f]};
+      const unsigned rk = d.fdxkv[f];
       const N dxr = d.rinv[NR], dyr = d.rinv[NE + NR];
 #pragma unroll
       for (int k = 0; k < V; ++k) {
         const N du = uR[k] - uL[k];
-        t0[k] = half_of(t0[k] + N(d.grad[(2 * k) * NE + NR]) * dxr) + div_by(y1 * du, dxk, rk);
-        t1[k] = half_of(t1[k] + N(d.grad[(2 * k + 1) * NE + NR]) * dyr) + div_by(y2 * du, dxk, rk);
+        t0[k] = half_of(t0[k] + N(d.grad[(2 * k) * NE + NR]) * dxr) + div_fixed(y1 * du, dxk, rk);
+        t1[k] = half_of(t1[k] + N(d.grad[(2 * k + 1) * NE + NR]) * dyr) + div_fixed(y2 * du, dxk, rk);
       }
     }
     N dudx = t0[1], dudy = t1[1], dvdx = t0[2], dvdy = t1[2], dtdx = t0[3], dtdy = t1[3];
@@ -2106,20 +2109,15 @@ void fill_thermo(const rc_thermo* t, const rc_config* g, ThermoDev<NSP>& th) {
   th.mw1000[0] = t->mole_weight[0] * 1000;
   th.mw1000[1] = t->mole_weight[NSP > 1 ? 1 : 0] * 1000;
   th.cfl = g->cfl;
-  // the device's recip_of, on the host (IEEE division, a correctly rounded FMA)
-  auto rp = [](double x, double* r) {
-    r[0] = 1.0 / x;
-    r[1] = std::fma(-x, r[0], 1.0) * r[0];
-  };
   for (int i = 0; i < NSP; ++i) {
-    rp(th.mw[i], th.mwr[i]);
+    th.mwv[i] = rcs::recip32(th.mw[i]);
     for (int j = 0; j < NSP; ++j) {
-      rp(th.wd[i][j], th.wdr[i][j]);
-      rp(th.dlj[i][j], th.dljr[i][j]);
+      th.wdv[i][j] = rcs::recip32(th.wd[i][j]);
+      th.dljv[i][j] = rcs::recip32(th.dlj[i][j]);
     }
   }
-  rp(th.mw1000[0], th.mw1000r[0]);
-  rp(th.mw1000[1], th.mw1000r[1]);
+  th.mw1000v[0] = rcs::recip32(th.mw1000[0]);
+  th.mw1000v[1] = rcs::recip32(th.mw1000[1]);
 }
 
 inline unsigned blocks(long n, int t) { return (unsigned)((n + t - 1) / t); }
@@ -2639,7 +2637,8 @@ int init_impl(const rc_mesh* m, const rc_thermo* t, const rc_config* g, const Ba
   // ---- faces
   std::vector<int> fNL(NF), fNR(NF);
   std::vector<double> fvec(2 * (size_t)NF), fsav(NF), fsn(2 * (size_t)NF), fss(NF), fs2(NF), fvL(2 * (size_t)NF),
-      fvR(2 * (size_t)NF), fdxk(NF), fdxkr(2 * (size_t)NF), fysn(2 * (size_t)NF);
+      fvR(2 * (size_t)NF), fdxk(NF), fysn(2 * (size_t)NF);
+  std::vector<unsigned> fdxkv(NF, 0u);
   for (int f = 1; f <= NF; ++f) {
     const int L = m->Neighbor[2 * (f - 1)], R = m->Neighbor[2 * (f - 1) + 1];
     if (m->FProperty[f - 1] == 100) return bail(RC_ERR_ARG, "periodic faces are not supported");
@@ -2666,8 +2665,7 @@ int init_impl(const rc_mesh* m, const rc_thermo* t, const rc_config* g, const Ba
       const double dlrx = C2(m->CELLXY, 1, L) - (C2(m->CELLXY, 1, R) - C2(m->SideOfs, 1, f));
       const double dlry = C2(m->CELLXY, 2, L) - (C2(m->CELLXY, 2, R) - C2(m->SideOfs, 2, f));
       fdxk[fi] = std::fabs(dlrx * fsn[fi] + dlry * fsn[NF + fi]);
-      fdxkr[fi] = 1.0 / fdxk[fi];
-      fdxkr[NF + fi] = std::fma(-fdxk[fi], fdxkr[fi], 1.0) * fdxkr[fi];
+      fdxkv[fi] = rcs::recip32(fdxk[fi]);
     }
     const double yita = 4. / 3;
     fysn[fi] = yita * fsn[fi];
@@ -2792,7 +2790,8 @@ int init_impl(const rc_mesh* m, const rc_thermo* t, const rc_config* g, const Ba
   st |= dev_upload(c, fvL, &p); d.fvL = p;
   st |= dev_upload(c, fvR, &p); d.fvR = p;
   st |= dev_upload(c, fdxk, &p); d.fdxk = p;
-  st |= dev_upload(c, fdxkr, &p); d.fdxkr = p;
+  unsigned* up;
+  st |= dev_upload(c, fdxkv, &up); d.fdxkv = up;
   st |= dev_upload(c, fysn, &p); d.fysn = p;
   st |= dev_upload(c, gtype, &i32); d.gtype = i32;
   st |= dev_upload(c, gsn, &p); d.gsn = p;

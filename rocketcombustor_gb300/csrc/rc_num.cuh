@@ -17,7 +17,10 @@ __device__ __forceinline__ double n_log(double x) { return rcm::log(x); }
 __device__ __forceinline__ double n_pow(double x, double y, double logx) {
   return rcm::pow_log<rcm::HwMul>(x, y, logx);
 }
-__device__ __forceinline__ double div_fixed(double a, double b, const double* r) { return div_rn(a, b, r); }
+// a / b with V = rcs::recip32(b) known: a divisor fixed in advance, or shared.
+// The FP64 unit has no part in it; through a pair of reciprocals in FP64 it
+// took four operations (250 cycles of a warp alone, 308 of many).
+__device__ __forceinline__ double div_fixed(double a, double b, unsigned V) { return soft_div_by(a, b, V); }
 template <bool M>
 __device__ __forceinline__ double val(Num<M> x) { return x.v; }
 template <bool M>
@@ -44,13 +47,8 @@ __device__ __forceinline__ Num<M> n_pow(Num<M> x, double y, Num<M> logx) {
 }
 template <class N>
 __device__ __forceinline__ N n_pow(N x, double y) { return n_pow(x, y, n_log(x)); }
-// a / b for a divisor fixed in advance: with the FP64 unit busy the integer
-// division (104 cycles) is cheaper than the pair's four operations (308); a
-// single warp's chain is shorter through the pair (250 against 278 cycles)
 template <bool M>
-__device__ __forceinline__ Num<M> div_fixed(Num<M> a, Num<M> b, const double* r) {
-  return M ? soft_div(a.v, b.v) : div_rn(a.v, b.v, r);
-}
+__device__ __forceinline__ Num<M> div_fixed(Num<M> a, Num<M> b, unsigned V) { return soft_div_by(a.v, b.v, V); }
 // x < 0.0
 template <class N>
 __device__ __forceinline__ bool negative(N x) { return less(val(x), 0.0); }
@@ -60,15 +58,4 @@ __device__ __forceinline__ Recip recip(N b) {
   const N h = 1.0 / b;
   return {val(h), val(N(fma(-val(b), val(h), 1.0)) * h)};
 }
-// the reciprocal pair of b for div_by, where div_by uses one
-template <class N>
-__device__ __forceinline__ Recip pair_of(N b) { return recip_of(val(b)); }
-template <>
-__device__ __forceinline__ Recip pair_of(Num<true>) { return {0.0, 0.0}; }
-template <class N>
-__device__ __forceinline__ N div_by(N a, N b, Recip r) {
-  const double p[2] = {r.h, r.l};
-  return div_fixed(a, b, p);
-}
-
 }  // namespace rc

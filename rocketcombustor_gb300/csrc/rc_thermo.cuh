@@ -43,11 +43,8 @@ struct ThermoDev {
   double prodc[NSP];             // 1000*mole_weight(ks)*(coef_r-coef_f)
   double mw1000[2];              // mole_weight(1..2)*1000
   double cfl;
-  // reciprocal pairs {RN(1/x), RN((1 - x RN(1/x)) RN(1/x))} of fixed divisors
-  double mwr[NSP][2];            // of mw
-  double wdr[NSP][NSP][2];       // of wd
-  double dljr[NSP][NSP][2];      // of dlj
-  double mw1000r[2][2];          // of mw1000
+  // rcs::recip32 of fixed divisors
+  unsigned mwv[NSP], wdv[NSP][NSP], dljv[NSP][NSP], mw1000v[2];
   int cols;                      // bit j: column j of cl or ch has a non-zero coefficient
 };
 
@@ -143,9 +140,12 @@ __device__ __forceinline__ void gas(const ThermoDev<NSP>& th, const N* Y, N tem,
   gama = c / (c - r);
 }
 
-// RN(1/3), RN(1/5) and their second parts: the pairs of rc_div.cuh
-__device__ constexpr double THIRD[2] = {0x1.5555555555555p-2, 0x1.5555555555555p-56};
-__device__ constexpr double FIFTH[2] = {0x1.999999999999ap-3, -0x1.999999999999ap-57};
+// rcs::recip32 of 3 and 5: 2^63 over their leading 32 bits, less a little
+constexpr unsigned THIRD_V = 0xaaaaaaa6u, FIFTH_V = 0xccccccc8u;
+constexpr bool below_reciprocal(unsigned v, unsigned long long b) {
+  return (1ull << 63) > v * b && (1ull << 63) - v * b < 1ull << 35;
+}
+static_assert(below_reciprocal(THIRD_V, 0xc0000000u) && below_reciprocal(FIFTH_V, 0xa0000000u), "as div_by needs");
 
 // compute_enthalpy (thermo_property.f90:114-144)
 template <int NSP, class N>
@@ -162,9 +162,9 @@ __device__ __forceinline__ void enthalpy(const ThermoDev<NSP>& th, N tem, N* ent
   if (cols & 2) poly_add(th, cols, 1, low, n_log(tem) / tem, s);
   if (cols & 4) poly_add1(th, cols, 2, low, s);
   if (cols & 8) poly_add(th, cols, 3, low, half_of(tem), s);
-  if (cols & 16) poly_add(th, cols, 4, low, div_fixed(t2, N(3.0), THIRD), s);
+  if (cols & 16) poly_add(th, cols, 4, low, div_fixed(t2, N(3.0), THIRD_V), s);
   if (cols & 32) poly_add(th, cols, 5, low, 0.25 * (tem * t2), s);
-  if (cols & 64) poly_add(th, cols, 6, low, div_fixed(t2 * t2, N(5.0), FIFTH), s);
+  if (cols & 64) poly_add(th, cols, 6, low, div_fixed(t2 * t2, N(5.0), FIFTH_V), s);
 #pragma unroll
   for (int i = 0; i < NSP; ++i) entha[i] = th.R[i] * (tem * s[i] + (low ? th.b1l[i] : th.b1h[i]));
 }
@@ -193,12 +193,12 @@ __device__ __forceinline__ N newton_T(const ThermoDev<NSP>& th, N et, const N* Y
 // diffusion_velocity.f90 form it
 template <int NSP, class N>
 __device__ __forceinline__ void mole_fractions(const ThermoDev<NSP>& th, const N* Y, N* X) {
-  N s = plus_zero(div_fixed(Y[0], N(th.mw[0]), th.mwr[0]));
+  N s = plus_zero(div_fixed(Y[0], N(th.mw[0]), th.mwv[0]));
 #pragma unroll
-  for (int i = 1; i < NSP; ++i) s = s + div_fixed(Y[i], N(th.mw[i]), th.mwr[i]);
+  for (int i = 1; i < NSP; ++i) s = s + div_fixed(Y[i], N(th.mw[i]), th.mwv[i]);
   const N ww = 1.0 / s;
 #pragma unroll
-  for (int i = 0; i < NSP; ++i) X[i] = div_fixed(ww * Y[i], N(th.mw[i]), th.mwr[i]);
+  for (int i = 0; i < NSP; ++i) X[i] = div_fixed(ww * Y[i], N(th.mw[i]), th.mwv[i]);
 }
 
 // compute_transport_property (transport_property.f90:78-125); xx: mole_fractions
@@ -213,13 +213,13 @@ __device__ __forceinline__ void transport(const ThermoDev<NSP>& th, N tem2, cons
   const int rg = low ? 0 : 1;
   const N lt = n_log(tem);
   const N t2 = tem * tem;
-  const Recip rt = pair_of(tem), rt2 = pair_of(t2);
+  const unsigned rt = rcs::recip32(t), rt2 = rcs::recip32(val(t2));
 #pragma unroll
   for (int i = 0; i < NSP; ++i) {
-    mul[i] = n_exp(th.mu[rg][0][i] * lt + div_by(N(th.mu[rg][1][i]), tem, rt) +
-                   div_by(N(th.mu[rg][2][i]), t2, rt2) + th.mu[rg][3][i]);
-    Kl[i] = n_exp(th.kk[rg][0][i] * lt + div_by(N(th.kk[rg][1][i]), tem, rt) +
-                  div_by(N(th.kk[rg][2][i]), t2, rt2) + th.kk[rg][3][i]);
+    mul[i] = n_exp(th.mu[rg][0][i] * lt + div_fixed(N(th.mu[rg][1][i]), tem, rt) +
+                   div_fixed(N(th.mu[rg][2][i]), t2, rt2) + th.mu[rg][3][i]);
+    Kl[i] = n_exp(th.kk[rg][0][i] * lt + div_fixed(N(th.kk[rg][1][i]), tem, rt) +
+                  div_fixed(N(th.kk[rg][2][i]), t2, rt2) + th.kk[rg][3][i]);
   }
 #pragma unroll
   for (int i = 0; i < NSP; ++i) { mul[i] = mul[i] * 1.0e-7; Kl[i] = Kl[i] * 1.0e-4; }
@@ -232,7 +232,7 @@ __device__ __forceinline__ void transport(const ThermoDev<NSP>& th, N tem2, cons
       // sqrt(mul(i)/mul(i)) is exactly 1
       const N sq = (i == j) ? N(1.0) : n_sqrt(mul[i] / mul[j]);
       const N q = 1.0 + sq * th.wc[i][j];
-      const N w = div_fixed(xx[j] * (q * q), N(th.wd[i][j]), th.wdr[i][j]);
+      const N w = div_fixed(xx[j] * (q * q), N(th.wd[i][j]), th.wdv[i][j]);
       phil = j ? phil + w : plus_zero(w);
     }
     phil = (0.25 * sqrt(2.0)) * phil;
@@ -258,7 +258,7 @@ __device__ __forceinline__ void diffusion(const ThermoDev<NSP>& th, N pp, N tem,
   for (int i = 0; i < NSP; ++i)
 #pragma unroll
     for (int j = i + 1; j < NSP; ++j) {
-      const N tstar = div_fixed(tem, N(th.dlj[i][j]), th.dljr[i][j]);
+      const N tstar = div_fixed(tem, N(th.dlj[i][j]), th.dljv[i][j]);
       const N om = 1.06036 * n_pow(tstar, -0.15610) + 0.19300 * n_exp(-0.47635 * tstar) +
                    1.03587 * n_exp(-1.52996 * tstar) + 1.76474 * n_exp(-3.89411 * tstar);
       const N d = num / (pp * th.dmw[i][j] * th.dcd[i][j] * om);
@@ -286,11 +286,11 @@ __device__ __forceinline__ void production(const ThermoDev<NSP>& th, N T, N rho,
   if (th.model == 0) {
     const N y1 = fmin2(N(1.0), fmax2(N(0.0), Y2[NSP > 1 ? 1 : 0]));
     kf = th.Af * n_exp(-th.E / (th.Rconstant * T));
-    kf = kf * n_pow(div_fixed(y0 * rho, N(th.mw1000[0]), th.mw1000r[0]), 0.2);
-    kf = kf * n_pow(div_fixed(y1 * rho, N(th.mw1000[1]), th.mw1000r[1]), 1.3);
+    kf = kf * n_pow(div_fixed(y0 * rho, N(th.mw1000[0]), th.mw1000v[0]), 0.2);
+    kf = kf * n_pow(div_fixed(y1 * rho, N(th.mw1000[1]), th.mw1000v[1]), 1.3);
   } else {
     kf = less(N(710.0), T) ? 1e4 : 0.0;
-    kf = kf * div_fixed(y0 * rho, N(th.mw1000[0]), th.mw1000r[0]);
+    kf = kf * div_fixed(y0 * rho, N(th.mw1000[0]), th.mw1000v[0]);
   }
 #pragma unroll
   for (int k = 0; k < NSP; ++k) prod[k] = th.prodc[k] * kf;
