@@ -278,32 +278,6 @@ __device__ T dgecon(const T* af, const unsigned* uv, T anorm) {
   return 0.0;
 }
 
-// ---- the per-row solve of one cell's system by its eight lanes
-// x: this row's right-hand side (already row-scaled); returns A^-1 x for this
-// row (dgetrs('N')): the composed interchanges, then the column-oriented unit
-// lower and upper solves of dtrsm, skipping zero entries as dtrsm does.  The
-// divisions by the diagonal of U use its reciprocals urv (rcs::div_by:
-// the same bits as the IEEE division).
-template <int N>
-__device__ __forceinline__ double getrs_rows(double x, int src, const double* lu, const double* ukk,
-                                             const unsigned* urv, int r, int base) {
-  x = __shfl_sync(FULL, x, base + src);
-#pragma unroll
-  for (int k = 0; k < N - 1; ++k) {
-    const double xk = __shfl_sync(FULL, x, base + k);
-    if (r > k && r < N && nonzero(xk)) x = x - xk * lu[k];
-  }
-#pragma unroll
-  for (int k = N - 1; k >= 0; --k) {
-    double xk = __shfl_sync(FULL, x, base + k);
-    if (nonzero(xk)) {
-      xk = rcs::div_by(xk, ukk[k], urv[k]);
-      if (r == k) x = xk;
-      else if (r < k) x = x - xk * lu[k];
-    }
-  }
-  return x;
-}
 }  // namespace bdf2
 
 // fixed = vol/dt ((1+2 phi) WP - phi WP2) (Time_BDF2.f90:88-92), or for
@@ -324,9 +298,7 @@ __global__ void __launch_bounds__(128) k_bdf2_fixed(const Dev d, int euler) {
 
 // Everything of BDF2_LU_SGS that the sweeps do not change, one thread per cell.
 // FP64 throughput bounds it: the divisions, comparisons and halvings run on the
-// integer pipes (Num).  With the sweep's divisions by shared reciprocals and
-// its staged records by word, an inner iteration on 120,000 cells takes 9.0
-// ms instead of 10.2.
+// integer pipes (Num).
 template <int NSP>
 __global__ void __launch_bounds__(128) k_bdf2_prep(const Dev d, const ThermoDev<NSP> th) {
   using namespace bdf2;
@@ -523,6 +495,75 @@ __device__ __forceinline__ BRow<NSP> brow_load(const Dev& d, int i, bool valid, 
   }
   return w;
 }
+// A lane's record in shared memory, word w of lane l at [32 w + l]: a warp
+// moves a word without bank conflicts, and reads only the words it uses (as
+// an array of records of about 560 bytes the words met in two banks of the 32).
+template <class S>
+__device__ __forceinline__ void stage_put(double* sm, const S& s) {
+  static_assert(sizeof(S) % 8 == 0, "whole words");
+  double w[sizeof(S) / 8];
+  memcpy(w, &s, sizeof(S));
+#pragma unroll
+  for (int k = 0; k < (int)(sizeof(S) / 8); ++k) sm[32 * k + (threadIdx.x & 31)] = w[k];
+}
+template <class S>
+__device__ __forceinline__ S stage_get(const double* sm) {
+  double w[sizeof(S) / 8];
+#pragma unroll
+  for (int k = 0; k < (int)(sizeof(S) / 8); ++k) w[k] = sm[32 * k + (threadIdx.x & 31)];
+  S s;
+  memcpy(&s, w, sizeof(S));
+  return s;
+}
+// This lane's row in such a record (w: its first word of this lane).
+template <int NSP>
+struct BRowRef {
+  static constexpr int V = 3 + NSP;
+  static_assert(offsetof(BRow<NSP>, lrow) == 8 * V && offsetof(BRow<NSP>, ukk) == 16 * V &&
+                    offsetof(BRow<NSP>, rsc) == 24 * V && offsetof(BRow<NSP>, urv) == 24 * V + 16 &&
+                    offsetof(BRow<NSP>, src) == 24 * V + 16 + 4 * V,
+                "words");
+  const double* w;
+  __device__ __forceinline__ double arow(int k) const { return w[32 * k]; }
+  __device__ __forceinline__ double lrow(int k) const { return w[32 * (V + k)]; }
+  __device__ __forceinline__ double ukk(int k) const { return w[32 * (2 * V + k)]; }
+  __device__ __forceinline__ double rsc() const { return w[32 * 3 * V]; }
+  __device__ __forceinline__ double csc() const { return w[32 * (3 * V + 1)]; }
+  __device__ __forceinline__ unsigned half(int h) const {  // 32-bit word h after csc
+    return reinterpret_cast<const unsigned*>(w + 32 * (3 * V + 2 + (h >> 1)))[h & 1];
+  }
+  __device__ __forceinline__ unsigned urv(int k) const { return half(k); }
+  __device__ __forceinline__ int src() const { return (int)half(V); }
+  __device__ __forceinline__ int equ() const { return (int)half(V + 1); }
+};
+// x: this row's right-hand side (already row-scaled); returns A^-1 x for this
+// row (dgetrs('N')): the composed interchanges, then the column-oriented unit
+// lower and upper solves of dtrsm, skipping zero entries as dtrsm does.  The
+// divisions by the diagonal of U use its reciprocals (rcs::div_by: the same
+// bits as the IEEE division).
+template <int NSP>
+__device__ __forceinline__ double getrs_rows(double x, const BRowRef<NSP>& rw, int r, int base) {
+  constexpr int N = 3 + NSP;
+  x = __shfl_sync(bdf2::FULL, x, base + rw.src());
+#pragma unroll
+  for (int k = 0; k < N - 1; ++k) {
+    const double lu = rw.lrow(k);
+    const double xk = __shfl_sync(bdf2::FULL, x, base + k);
+    if (r > k && r < N && nonzero(xk)) x = x - xk * lu;
+  }
+#pragma unroll
+  for (int k = N - 1; k >= 0; --k) {
+    const double lu = rw.lrow(k), u = rw.ukk(k);
+    const unsigned v = rw.urv(k);
+    double xk = __shfl_sync(bdf2::FULL, x, base + k);
+    if (nonzero(xk)) {
+      xk = rcs::div_by(xk, u, v);
+      if (r == k) x = xk;
+      else if (r < k) x = x - xk * lu;
+    }
+  }
+  return x;
+}
 // The flux difference of slot b's neighbour increment dP (Time_BDF2.f90:168-197),
 // rows 1-3 (lo) or rows 4.. (energy and species) of the slot's terms.
 // L2: the neighbour's increment read through L2 (ld.global.cg), as the
@@ -580,13 +621,18 @@ __device__ __forceinline__ void bslot_put(double* w, bool lo, int q, const doubl
   }
 }
 // the backward error of one refinement pass over a cell's rows (8 lanes):
-// max over the rows of |y| / w (or the guarded form), as a bit pattern
+// max over the rows of |y| / w (or the guarded form), as a bit pattern.  A cell
+// that is done (go false; its result is not used) and a row whose residual is
+// zero divide nothing: rcs::div leaves a zero to the hardware's division,
+// and one lane that takes it holds up the warp.
 template <int V>
-__device__ __forceinline__ long long berr_bits(double y, double wk, int r) {
+__device__ __forceinline__ long long berr_bits(double y, double wk, int r, bool go) {
   using namespace bdf2;
   const double safe1 = (V + 1) * SFMIN, safe2 = safe1 / EPS;
   long long vb = 0;
-  if (r < V) vb = dbits((dbits(wk) > dbits(safe2)) ? rcs::div(fabs(y), wk) : (fabs(y) + safe1) / (wk + safe1));
+  const bool plain = dbits(wk) > dbits(safe2);
+  if (r < V && go && (nonzero(y) || !plain || isnan(wk)))
+    vb = dbits(plain ? rcs::div(fabs(y), wk) : (fabs(y) + safe1) / (wk + safe1));
   vb = max(vb, (long long)__shfl_xor_sync(FULL, (unsigned long long)vb, 1));
   vb = max(vb, (long long)__shfl_xor_sync(FULL, (unsigned long long)vb, 2));
   vb = max(vb, (long long)__shfl_xor_sync(FULL, (unsigned long long)vb, 4));
@@ -600,75 +646,76 @@ __device__ __forceinline__ long long berr_bits(double y, double wk, int r) {
 // through w (this warp's [cell][row][slot] scratch), then the cell's system
 // (rw: row r of its factorisation) solved with one lane per row and refined
 // as dgerfs does; hown is the cell's own increment (row r), i its index.
-// PART 0: the whole step on this warp.  PART 1 and 2: two warps (warp 0 and
-// warp 1 of the block) on the same cells, PART 1 forming rows 1-3 of every
-// slot's terms, PART 2 rows 4..; they meet at named barrier 6 (64 threads),
-// after which PART 1 solves and PART 2 returns.  The terms, their places in w
-// and the sums are the same in every PART.
-template <int NSP, bool FWD, int CPW, bool L2, int PART = 0>
+// part 0: the whole step on this warp.  part 1 and 2: two warps (warp 0 and
+// warp 1 of the block) on the same cells, part 1 forming rows 1-3 of every
+// slot's terms, part 2 rows 4..; they meet at named barrier 6 (64 threads),
+// after which part 1 solves and part 2 returns.  The terms, their places in w
+// and the sums are the same in every part.
+// part and fwd are arguments, and the first solve and the corrections one
+// loop, so that every pass runs the same instructions: they have to come
+// from the instruction cache, and a pass runs each of them only a few times.
+template <int NSP, int CPW, bool L2>
 __device__ __forceinline__ void bdf2_cell_step(const Dev& d, const ThermoDev<NSP>& th, const BSlot<NSP>& sp,
-                                               const BRow<NSP>& rw, double hown, int i, bool valid, double* wsm) {
+                                               const BRowRef<NSP>& rw, bool fwd, int part, double hown, int i,
+                                               bool valid, double* wsm) {
   using namespace bdf2;
   constexpr int V = 3 + NSP;
   const int lane = threadIdx.x & 31, cell = lane >> 3, r = lane & 7, base = cell * 8;
   const int q = r & 3;
-  // PART 0: lanes 0-3 keep flux rows 1-3 of their slot, lanes 4-7 rows 4..
-  // (energy, species); PART 1 / 2: all lanes the one half, lanes 0-3 store it
-  const bool lo = PART == 0 ? r < 4 : PART == 1;
+  // part 0: lanes 0-3 keep flux rows 1-3 of their slot, lanes 4-7 rows 4..
+  // (energy, species); part 1 / 2: all lanes the one half, lanes 0-3 store it
+  const bool lo = part == 0 ? r < 4 : part == 1;
   const int NE = d.NE;
   double c[V];
   bslot_terms<NSP, L2>(d, th, sp, lo, c);
   double* w = wsm + (cell < CPW ? cell : 0) * V * 4;  // [row][slot]
-  if (cell < CPW && (PART == 0 || r < 4)) bslot_put<NSP>(w, lo, q, c);
+  if (cell < CPW && (part == 0 || r < 4)) bslot_put<NSP>(w, lo, q, c);
   __syncwarp();
-  if (PART == 2) {
+  if (part == 2) {
     bar_arrive(6, 64);
     return;
   }
-  if (PART == 1) bar_named(6, 64);
+  if (part == 1) bar_named(6, 64);
   double dflux = 0.0;
   if (r < V) {
 #pragma unroll
     for (int sl = 0; sl < 4; ++sl) dflux = dflux + w[r * 4 + sl];
   }
   // --- the cell's system, one row per lane (dgesvx after the factorisation)
-  const bool rowequ = rw.equ & 1, colequ = rw.equ & 2;
-  double b = FWD ? hown - dflux : dflux;
-  if (rowequ) b = rw.rsc * b;
+  const int equ = rw.equ();
+  const bool rowequ = equ & 1, colequ = equ & 2;
+  double b = fwd ? hown - dflux : dflux;
+  if (rowequ) b = rw.rsc() * b;
   if (!(valid && r < V)) b = 0.0;
-  double x = getrs_rows<V>(b, rw.src, rw.lrow, rw.ukk, rw.urv, r, base);
-  // dgerfs refinement: residual, componentwise backward error, correction.
-  // The backward error is non-negative: its maximum and the loop tests
-  // compare bit patterns; 2 berr <= lstres is berr <= lstres/2 (both exact).
+  // the solve, then dgerfs refinement: residual, componentwise backward error,
+  // correction.  The backward error is non-negative: its maximum and the loop
+  // tests compare bit patterns; 2 berr <= lstres is berr <= lstres/2 (both exact).
+  double x = 0.0, y = b;
   long long lstres_half = dbits(1.5);  // lstres = 3
-  int count = 1;
   bool go = valid;
-  for (int it = 0; it < 6; ++it) {
-    double xs[V];
-#pragma unroll
-    for (int k = 0; k < V; ++k) xs[k] = __shfl_sync(FULL, x, base + k);
+#pragma unroll 1
+  for (int it = 0;; ++it) {
+    const double xi = getrs_rows<NSP>(y, rw, r, base);
+    if (it == 0) x = xi;
+    else if (go) x = x + xi;
     // y = b - A x and w = |b| + |A| |x| on the same products (rounding is
     // symmetric: (-x) a = -(x a) and |a| |x| = |x a|)
-    double y = b, wk = fabs(b);
+    double wk = fabs(b);
+    y = b;
 #pragma unroll
     for (int k = 0; k < V; ++k) {
-      const double p = xs[k] * rw.arow[k];
+      const double p = __shfl_sync(FULL, x, base + k) * rw.arow(k);
       y = y - p;
       wk = wk + fabs(p);
     }
-    const long long vb = berr_bits<V>(y, wk, r);
-    const bool cont = go && vb > dbits(EPS) && vb <= lstres_half && count <= 5;
-    if (!__any_sync(FULL, cont)) break;
-    const double corr = getrs_rows<V>(y, rw.src, rw.lrow, rw.ukk, rw.urv, r, base);
-    if (cont) {
-      x = x + corr;
-      lstres_half = vb - (1LL << 52);  // berr / 2: berr > eps is a normal number
-      count = count + 1;
-    }
-    go = cont;
+    const long long vb = berr_bits<V>(y, wk, r, go);
+    // a cell that goes on has made `it` corrections
+    go = go && vb > dbits(EPS) && vb <= lstres_half && it < 5;
+    if (!__any_sync(FULL, go)) break;
+    lstres_half = vb - (1LL << 52);  // berr / 2: berr > eps is a normal number (unused once go is false)
   }
-  if (colequ) x = rw.csc * x;
-  if (valid && r < V) d.hWA[r * NE + i] = FWD ? x : hown - x;
+  if (colequ) x = rw.csc() * x;
+  if (valid && r < V) d.hWA[r * NE + i] = fwd ? x : hown - x;
 }
 
 // One level of the forward (FWD) or backward sweep, cells t0..t1-1 of the
@@ -693,7 +740,9 @@ __global__ void __launch_bounds__(32) k_bdf2_sweep(const Dev d, const ThermoDev<
   pdl_wait();
   if (!FWD && valid && r < V) hown = d.hWA[r * NE + i];
   __shared__ double wsm[CPW * V * 4];
-  bdf2_cell_step<NSP, FWD, CPW, false>(d, th, sp, rw, hown, i, valid, wsm);
+  __shared__ double s_row[32 * sizeof(BRow<NSP>) / 8];
+  stage_put(s_row, rw);  // each lane reads its own
+  bdf2_cell_step<NSP, CPW, false>(d, th, sp, BRowRef<NSP>{s_row + lane}, FWD, 0, hown, i, valid, wsm);
 }
 
 // Both BDF2 sweeps as one cooperative dataflow launch on the pass tables of
@@ -714,34 +763,22 @@ __global__ void __launch_bounds__(32) k_bdf2_sweep(const Dev d, const ThermoDev<
 // bounded wait gave up (ERR_SYNC): the compute warps then skip the pass.  The
 // last block to finish advances the epoch counter; the primitive update
 // follows as its own launch.
+struct BTail {
+  double hown;
+  int i, valid;
+};
 template <int NSP>
 struct BStage {
   BSlot<NSP> sp;
   BRow<NSP> rw;
-  double hown;
-  int i, valid;
+  BTail t;
 };
-// A lane's staged record in shared memory, word w of lane l at [32 w + l]: a
-// warp moves a word without bank conflicts, and reads only the words it uses
-// (the record is about 560 bytes; as an array of records its words met in two
-// banks of the 32).
-template <class S>
-__device__ __forceinline__ void stage_put(double* sm, const S& s) {
-  static_assert(sizeof(S) % 8 == 0, "whole words");
-  double w[sizeof(S) / 8];
-  memcpy(w, &s, sizeof(S));
-#pragma unroll
-  for (int k = 0; k < (int)(sizeof(S) / 8); ++k) sm[32 * k + (threadIdx.x & 31)] = w[k];
-}
-template <class S>
-__device__ __forceinline__ S stage_get(const double* sm) {
-  double w[sizeof(S) / 8];
-#pragma unroll
-  for (int k = 0; k < (int)(sizeof(S) / 8); ++k) w[k] = sm[32 * k + (threadIdx.x & 31)];
-  S s;
-  memcpy(&s, w, sizeof(S));
-  return s;
-}
+// A pass is one chain: per cell, of about 24,000 cycles, the record 2,500, the
+// terms with the neighbours' increments from L2 4,200, each solve 4,500, each
+// check of the backward error 3,300, of which a quarter was the hardware's
+// division for zero residuals and finished cells (berr_bits).  An inner
+// iteration on 120,000 cells: 10.2 -> 8.6 ms with that, the divisions by shared
+// reciprocals and the records by word.
 // A pass of at most four cells runs on both compute warps split by rows
 // (bdf2_cell_step PART 1 and 2), otherwise four cells on each (PART 0).
 constexpr int BFLOW_THREADS = 160, BFLOW_NB = 96;  // all five warps; a role pair and the coordinator
@@ -826,9 +863,9 @@ __global__ void __launch_bounds__(BFLOW_THREADS, 1) k_bdf2_flow(const Dev d, con
       e.rw = brow_load<NSP>(d, i, valid, r);
       // forward: the set-up's right-hand side, which only this cell's own
       // forward step changes
-      e.hown = fwd && valid && r < V ? __ldcg(d.hWA + r * d.NE + i) : 0.0;
-      e.i = i;
-      e.valid = valid ? 1 : 0;
+      e.t.hown = fwd && valid && r < V ? __ldcg(d.hWA + r * d.NE + i) : 0.0;
+      e.t.i = i;
+      e.t.valid = valid ? 1 : 0;
       stage_put(buffer(k, w), e);
       __syncwarp();
       __threadfence_block();
@@ -843,28 +880,20 @@ __global__ void __launch_bounds__(BFLOW_THREADS, 1) k_bdf2_flow(const Dev d, con
     for (int k = 0; k < n; ++k) {
       const bool fwd = k < nf;
       bar_named(3, BFLOW_THREADS);
-      const BStage<NSP> e = stage_get<BStage<NSP>>(buffer(k, warp));
-      const BSlot<NSP>& sp = e.sp;
-      const BRow<NSP>& rw = e.rw;
-      const int i = e.i;
-      const bool valid = e.valid != 0;
+      const double* rec = buffer(k, warp);
+      const BRowRef<NSP> rw = {rec + 4 * offsetof(BStage<NSP>, rw) + lane};
+      const BTail t = stage_get<BTail>(rec + 4 * offsetof(BStage<NSP>, t));
+      const int i = t.i;
+      const bool valid = t.valid != 0;
       // backward: the cell's own increment, as this block's forward pass of
       // the cell wrote it (read after the hand-over: the other warp may have
       // been finishing the forward pass that holds the same cell)
-      const double hown = fwd ? e.hown : valid && r < V ? __ldcg(d.hWA + r * d.NE + i) : 0.0;
+      const double hown = fwd ? t.hown : valid && r < V ? __ldcg(d.hWA + r * d.NE + i) : 0.0;
       if (s_go[k & 1]) {
-        if (s_split[k & 1]) {
-          if (warp == 0) {
-            if (fwd) bdf2_cell_step<NSP, true, 4, true, 1>(d, th, sp, rw, hown, i, valid, wsm[0]);
-            else bdf2_cell_step<NSP, false, 4, true, 1>(d, th, sp, rw, hown, i, valid, wsm[0]);
-          } else {
-            if (fwd) bdf2_cell_step<NSP, true, 4, true, 2>(d, th, sp, rw, hown, i, valid, wsm[0]);
-            else bdf2_cell_step<NSP, false, 4, true, 2>(d, th, sp, rw, hown, i, valid, wsm[0]);
-          }
-        } else {
-          if (fwd) bdf2_cell_step<NSP, true, 4, true>(d, th, sp, rw, hown, i, valid, wsm[warp]);
-          else bdf2_cell_step<NSP, false, 4, true>(d, th, sp, rw, hown, i, valid, wsm[warp]);
-        }
+        // both warps on the same cells, or four cells each
+        const bool split = s_split[k & 1] != 0;
+        bdf2_cell_step<NSP, 4, true>(d, th, stage_get<BSlot<NSP>>(rec + 4 * offsetof(BStage<NSP>, sp)), rw, fwd,
+                                     split ? 1 + warp : 0, hown, i, valid, split ? wsm[0] : wsm[warp]);
       }
       __syncwarp();
       bar_arrive(4, BFLOW_NB);
