@@ -22,33 +22,93 @@ using ChemNum = Num<false>;
 // as with 32).  The lanes refill when REFILL of them are idle or none is busy:
 // starting an item costs about a tenth of an attempt, for the whole warp.
 // 262,144 states at tolerance 0.005 (median 9 substeps, 90th percentile 509):
-// 276 ms with a warp taking 32 states at a time, 128 ms now.  Three blocks per
-// SM (168 registers, a few spills) against two: 133 ms; the bound is the FP64
-// unit and, when few states are left, one attempt's chain (about 60 us).
+// 276 ms with a warp taking 32 states at a time, 113 ms with the queue.
+//
+// That leaves the end of the queue: every warp then holds a few long items,
+// each attempt at the price of a full warp.  So the integration goes in rounds
+// (launches): a round gives its items, through full warps, at most park_at(round)
+// attempts in all and parks what is left of them in a list in memory, which is the
+// next round's queue.  Of unsorted items (park.cut) a round that has more than the
+// launch has lanes ends when its queue is empty: the items in the lanes are
+// parked as they are, at the end of the list, and since a list is taken from its
+// end, they go first in the next round.  The last round ends with its items.
+// Where the list is full the items stay in their lanes.  The same states: 74 ms.
 //   begin(item, r)  loads item into reactor r; false when it needs no attempt
 //   end(item, r)    stores the finished item
 constexpr int REFILL = 4;
+__host__ __device__ constexpr int park_at(int round) { return round == 0 ? 16 : 64 * round; }
+
+// list l of the parked reactors: their items and their state
+template <int NSP, class N>
+struct Parked {
+  static constexpr int V = 3 + NSP;
+  double* x;
+  int* k;
+  size_t cap;
+  __device__ __forceinline__ Parked(const ChemPark& p, int l)
+      : x(p.x + (size_t)l * CHEM_PARK_X * p.cap), k(p.k + (size_t)l * CHEM_PARK_K * p.cap), cap(p.cap) {}
+  __device__ __forceinline__ void put(size_t u, int item, const Reactor<NSP, N>& r) const {
+    static_assert(V + 4 <= CHEM_PARK_X, "room for the state");
+#pragma unroll
+    for (int v = 0; v < V; ++v) x[v * cap + u] = val(r.P[v]);
+    x[V * cap + u] = val(r.rho);
+    x[(V + 1) * cap + u] = val(r.e);
+    x[(V + 2) * cap + u] = val(r.rem);
+    x[(V + 3) * cap + u] = val(r.hs);
+    k[u] = item;
+    k[cap + u] = r.nacc;
+    k[2 * cap + u] = r.natt;
+  }
+  __device__ __forceinline__ int get(size_t u, Reactor<NSP, N>& r) const {
+#pragma unroll
+    for (int v = 0; v < V; ++v) r.P[v] = x[v * cap + u];
+    r.rho = x[V * cap + u];
+    r.e = x[(V + 1) * cap + u];
+    r.rem = x[(V + 2) * cap + u];
+    r.hs = x[(V + 3) * cap + u];
+    r.nacc = k[cap + u];
+    r.natt = k[2 * cap + u];
+    return k[u];
+  }
+};
+
+// Round 0 takes the items 0 .. n-1, a later round the list of the one before;
+// the first 32 of a warp are its own (so that few items spread over the blocks
+// in order), the others come from the round's counter.
 template <int NSP, class N, class Begin, class End>
-__device__ __forceinline__ void run_queue(const ThermoDev<NSP>& th, int n, unsigned* counter, double tol, int maxsub,
-                                          unsigned& err, Begin begin, End end) {
+__device__ __forceinline__ void run_queue(const ThermoDev<NSP>& th, int n, const ChemPark& park, int round, double tol,
+                                          int maxsub, unsigned& err, Begin begin, End end) {
   const int lane = threadIdx.x & 31;
+  const Parked<NSP, N> from(park, (round + 1) & 1), to(park, round & 1);
+  const bool final = round + 1 >= park.rounds;
+  const int limit = final ? 0x7fffffff : park_at(round);
+  if (round > 0) n = (int)min(park.count[CHEM_ROUNDS + round - 1], (unsigned)park.cap);
+  const int lanes = gridDim.x * CHEM_THREADS;
   Reactor<NSP, N> r;
   int item = -1;        // the lane's item, -1 when idle
   bool more = true;     // the queue may hold more (warp-uniform)
+  bool first = true, full = false;
   for (;;) {
     unsigned idle = __ballot_sync(0xffffffffu, item < 0);
     while (more && (__popc(idle) >= REFILL)) {
-      int base = 0;
-      if (lane == 0) base = (int)atomicAdd(counter, (unsigned)__popc(idle));
-      base = __shfl_sync(0xffffffffu, base, 0);
+      int base = blockIdx.x * CHEM_THREADS + (threadIdx.x & ~31);
+      if (!first) {
+        if (lane == 0) base = lanes + (int)atomicAdd(park.count + round, (unsigned)__popc(idle));
+        base = __shfl_sync(0xffffffffu, base, 0);
+      }
+      first = false;
       more = base + __popc(idle) < n;
       if (item < 0) {
         const int q = base + __popc(idle & ((1u << lane) - 1u));
         if (q < n) {
-          item = q;
-          if (!begin(q, r)) {
-            end(q, r);
-            item = -1;
+          if (round > 0) {
+            item = from.get(n - 1 - q, r);
+          } else {
+            item = q;
+            if (!begin(q, r)) {
+              end(q, r);
+              item = -1;
+            }
           }
         }
       }
@@ -56,9 +116,20 @@ __device__ __forceinline__ void run_queue(const ThermoDev<NSP>& th, int n, unsig
       idle = __ballot_sync(0xffffffffu, item < 0);
     }
     if (idle == 0xffffffffu) break;
-    if (item >= 0 && !r.attempt(th, tol, maxsub, err)) {
-      end(item, r);
-      item = -1;
+    // the queue is empty, in a round that had more items than lanes
+    const bool stop = park.cut && !final && n > lanes && lanes + (int)*(volatile unsigned*)(park.count + round) >= n;
+    if (item >= 0) {
+      if (!r.attempt(th, tol, maxsub, err)) {
+        end(item, r);
+        item = -1;
+      } else if (!final && (stop || r.natt >= limit) && !full) {
+        const unsigned u = atomicAdd(park.count + CHEM_ROUNDS + round, 1u);
+        full = u >= (unsigned)park.cap;
+        if (!full) {
+          to.put(u, item, r);
+          item = -1;
+        }
+      }
     }
     __syncwarp();
   }
@@ -69,12 +140,12 @@ __device__ __forceinline__ void run_queue(const ThermoDev<NSP>& th, int n, unsig
 //   src_k = vol * (rho * ((Y_k(step) - Y_k) / step)), with the reactor's rho = p / (R_mix T).
 template <int NSP, class N, class Cell>
 __device__ __forceinline__ void run_cells(const Dev& d, const ThermoDev<NSP>& th, int n, Cell cell, double tol,
-                                          int maxsub, int* nsub, unsigned* counter) {
+                                          int maxsub, int* nsub, const ChemPark& park, int round) {
   constexpr int V = 3 + NSP;
   const int NE = d.NE;
   unsigned err = 0;
   run_queue<NSP, N>(
-      th, n, counter, tol, maxsub, err,
+      th, n, park, round, tol, maxsub, err,
       [&](int q, Reactor<NSP, N>& r) {
         const int i = cell(q);
 #pragma unroll
@@ -98,8 +169,8 @@ __device__ __forceinline__ void run_cells(const Dev& d, const ThermoDev<NSP>& th
 template <int NSP, class N>
 __global__ void __launch_bounds__(CHEM_THREADS, 3) k_chem_source(const Dev d, const ThermoDev<NSP> th, double tol,
                                                               int maxsub, int* __restrict__ nsub,
-                                                              const int* __restrict__ order, unsigned* counter) {
-  run_cells<NSP, N>(d, th, d.NE, [&](int q) { return order ? order[q] : q; }, tol, maxsub, nsub, counter);
+                                                              const int* __restrict__ order, const ChemPark park, int round) {
+  run_cells<NSP, N>(d, th, d.NE, [&](int q) { return order ? order[q] : q; }, tol, maxsub, nsub, park, round);
 }
 
 // Counting sort of the cells by their previous substep count, descending
@@ -176,9 +247,10 @@ template <int NSP, class N>
 __global__ void __launch_bounds__(CHEM_THREADS, 3) k_chem_list(const Dev d, const ThermoDev<NSP> th, double tol,
                                                             int maxsub, int* __restrict__ nsub,
                                                             const int* __restrict__ list,
-                                                            const unsigned* __restrict__ nlist, unsigned* counter) {
+                                                            const unsigned* __restrict__ nlist, const ChemPark park,
+                                                            int round) {
   run_cells<NSP, N>(d, th, (int)min(*nlist, (unsigned)d.NE), [&](int q) { return list[q]; }, tol, maxsub, nsub,
-                    counter);
+                    park, round);
 }
 
 // n primitive states in SoA ([k*n + i]) integrated over dt[i].
@@ -186,12 +258,12 @@ template <int NSP, class N>
 __global__ void __launch_bounds__(CHEM_THREADS, 3) k_chem_batch(const ThermoDev<NSP> th, const double* __restrict__ Pin,
                                                              const double* __restrict__ dts, int n,
                                                              double* __restrict__ Pout, int* __restrict__ nsub,
-                                                             double tol, int maxsub, unsigned* counter,
-                                                             unsigned* errp) {
+                                                             double tol, int maxsub, const ChemPark park,
+                                                             int round, unsigned* errp) {
   constexpr int V = 3 + NSP;
   unsigned err = 0;
   run_queue<NSP, N>(
-      th, n, counter, tol, maxsub, err,
+      th, n, park, round, tol, maxsub, err,
       [&](int i, Reactor<NSP, N>& r) {
 #pragma unroll
         for (int k = 0; k < V; ++k) r.P[k] = Pin[(size_t)k * n + i];
@@ -207,20 +279,36 @@ __global__ void __launch_bounds__(CHEM_THREADS, 3) k_chem_batch(const ThermoDev<
 
 // Grid of the persistent launches: enough resident warps to fill every SM.
 template <class K>
-static int chem_grid(K kernel, int items) {
-  int dev = 0, nsm = 0, occ = 0;
+static int chem_grid(K kernel, int items, int* nsm) {
+  int dev = 0, occ = 0;
   cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  cudaDeviceGetAttribute(nsm, cudaDevAttrMultiProcessorCount, dev);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kernel, CHEM_THREADS, 0);
   const int need = (items + CHEM_THREADS - 1) / CHEM_THREADS;
-  int g = (nsm > 0 ? nsm : 1) * (occ > 0 ? occ : 1);
+  const int g = (*nsm > 0 ? *nsm : 1) * (occ > 0 ? occ : 1);
   return g < need ? g : (need > 0 ? need : 1);
+}
+// The rounds of a launch over `items`: one where there is no room to park, or
+// where one block per SM holds all items (a warp without neighbours on its
+// sub-partition has nothing to gain from full lanes).  Items that come sorted,
+// the longest of the last iteration first, need few: the last ones to start are
+// short (64 cases, a million cells, five iterations: 139.3 ms in one round, 137.5
+// in four, 140.7 in ten with the cut; unsorted states: 113, 101 and 74 ms).
+template <class K, class Launch>
+static int chem_rounds(K kernel, int items, bool sorted, ChemPark park, cudaStream_t s, Launch launch) {
+  int nsm = 0;
+  const int grid = chem_grid(kernel, items, &nsm);
+  park.rounds = park.cap == 0 || items <= nsm * CHEM_THREADS ? 1 : sorted ? 4 : CHEM_ROUNDS;
+  park.cut = !sorted;
+  cudaMemsetAsync(park.count, 0, sizeof(unsigned) * 2 * CHEM_ROUNDS, s);
+  for (int round = 0; round < park.rounds; ++round) launch(grid, park, round);
+  return park.rounds;
 }
 
 // order/hist: work arrays of NE ints and NBUCKET unsigned (order null: cell order)
 template <int NSP>
-void chem_source(const Dev& d, const void* th, double tol, int maxsub, int* nsub, int* order, unsigned* hist,
-                 unsigned* counter, cudaStream_t s) {
+int chem_source(const Dev& d, const void* th, double tol, int maxsub, int* nsub, int* order, unsigned* hist,
+                const ChemPark& park, cudaStream_t s) {
   if (order) {
     const int nb = (d.NE + NBUCKET * SORT_ITEMS - 1) / (NBUCKET * SORT_ITEMS);
     cudaMemsetAsync(hist, 0, sizeof(unsigned) * NBUCKET, s);
@@ -229,37 +317,38 @@ void chem_source(const Dev& d, const void* th, double tol, int maxsub, int* nsub
     k_chem_scatter<<<nb, NBUCKET, 0, s>>>(nsub, d.NE, hist, order);
   }
   auto k = k_chem_source<NSP, ChemNum>;
-  const int grid = chem_grid(k, d.NE);
-  cudaMemsetAsync(counter, 0, sizeof(unsigned), s);
-  k<<<grid, CHEM_THREADS, 0, s>>>(d, *static_cast<const ThermoDev<NSP>*>(th), tol, maxsub, nsub, order, counter);
+  return (order ? 3 : 0) + chem_rounds(k, d.NE, order != nullptr, park, s, [&](int grid, const ChemPark& p, int round) {
+    k<<<grid, CHEM_THREADS, 0, s>>>(d, *static_cast<const ThermoDev<NSP>*>(th), tol, maxsub, nsub, order, p, round);
+  });
 }
 
 template <int NSP>
-void chem_list(const Dev& d, const void* th, double tol, int maxsub, int* nsub, const int* list,
-               const unsigned* nlist, unsigned* counter, cudaStream_t s) {
+int chem_list(const Dev& d, const void* th, double tol, int maxsub, int* nsub, const int* list, const unsigned* nlist,
+              const ChemPark& park, cudaStream_t s) {
   auto k = k_chem_list<NSP, ChemNum>;
-  const int grid = chem_grid(k, d.NE);
-  cudaMemsetAsync(counter, 0, sizeof(unsigned), s);
-  k<<<grid, CHEM_THREADS, 0, s>>>(d, *static_cast<const ThermoDev<NSP>*>(th), tol, maxsub, nsub, list, nlist, counter);
+  return chem_rounds(k, d.NE, false, park, s, [&](int grid, const ChemPark& p, int round) {
+    k<<<grid, CHEM_THREADS, 0, s>>>(d, *static_cast<const ThermoDev<NSP>*>(th), tol, maxsub, nsub, list, nlist, p,
+                                    round);
+  });
 }
 
 template <int NSP>
-void chem_batch(const void* th, const double* P, const double* dt, int n, double* out, int* nsub, double tol,
-                int maxsub, unsigned* counter, unsigned* errp, cudaStream_t s) {
-  cudaMemsetAsync(counter, 0, sizeof(unsigned), s);
+int chem_batch(const void* th, const double* P, const double* dt, int n, double* out, int* nsub, double tol,
+               int maxsub, const ChemPark& park, unsigned* errp, cudaStream_t s) {
   auto k = k_chem_batch<NSP, ChemNum>;
-  const int grid = chem_grid(k, n);
-  k<<<grid, CHEM_THREADS, 0, s>>>(*static_cast<const ThermoDev<NSP>*>(th), P, dt, n, out, nsub, tol,
-                                                  maxsub, counter, errp);
+  return chem_rounds(k, n, false, park, s, [&](int grid, const ChemPark& p, int round) {
+    k<<<grid, CHEM_THREADS, 0, s>>>(*static_cast<const ThermoDev<NSP>*>(th), P, dt, n, out, nsub, tol, maxsub, p,
+                                    round, errp);
+  });
 }
 
-#define RC_CHEM_INST(N)                                                                                  \
-  template void chem_source<N>(const Dev&, const void*, double, int, int*, int*, unsigned*, unsigned*,   \
-                               cudaStream_t);                                                            \
-  template void chem_list<N>(const Dev&, const void*, double, int, int*, const int*, const unsigned*,      \
-                             unsigned*, cudaStream_t);                                                   \
-  template void chem_batch<N>(const void*, const double*, const double*, int, double*, int*, double, int, \
-                              unsigned*, unsigned*, cudaStream_t);
+#define RC_CHEM_INST(N)                                                                                         \
+  template int chem_source<N>(const Dev&, const void*, double, int, int*, int*, unsigned*, const ChemPark&,     \
+                              cudaStream_t);                                                                    \
+  template int chem_list<N>(const Dev&, const void*, double, int, int*, const int*, const unsigned*,            \
+                            const ChemPark&, cudaStream_t);                                                     \
+  template int chem_batch<N>(const void*, const double*, const double*, int, double*, int*, double, int,        \
+                             const ChemPark&, unsigned*, cudaStream_t);
 RC_CHEM_INST(1)
 RC_CHEM_INST(4)
 

@@ -1702,12 +1702,12 @@ template <int NSP>
 cudaError_t mixed_lusgs_flowc(const Dev&, const void*, const void*, const FlowDev&, int, int, cudaStream_t);
 template <int NSP> int mixed_flowc_occupancy(int);
 template <int NSP>
-void chem_source(const Dev&, const void*, double, int, int*, int*, unsigned*, unsigned*, cudaStream_t);
+int chem_source(const Dev&, const void*, double, int, int*, int*, unsigned*, const ChemPark&, cudaStream_t);
 template <int NSP>
-void chem_batch(const void*, const double*, const double*, int, double*, int*, double, int, unsigned*, unsigned*,
-                cudaStream_t);
+int chem_batch(const void*, const double*, const double*, int, double*, int*, double, int, const ChemPark&, unsigned*,
+               cudaStream_t);
 template <int NSP>
-void chem_list(const Dev&, const void*, double, int, int*, const int*, const unsigned*, unsigned*, cudaStream_t);
+int chem_list(const Dev&, const void*, double, int, int*, const int*, const unsigned*, const ChemPark&, cudaStream_t);
 template <int NSP> void bdf2_fixed(const Dev&, int, int, cudaStream_t);
 template <int NSP> void bdf2_prep(const Dev&, const void*, int, cudaStream_t);
 template <int NSP> void bdf2_sweep(const Dev&, const void*, bool, int, int, int, cudaStream_t);
@@ -1775,7 +1775,8 @@ struct rc_ctx {
   int* chem_nsub = nullptr;           // [NE] accepted substeps of the last integrated source
   int* chem_order = nullptr;          // [NE] cells by previous substeps, descending
   unsigned* chem_hist = nullptr;      // [256] bucket counts / cursors of that sort
-  unsigned* chem_counter = nullptr;   // work-queue counter
+  ChemPark chem_park = {};            // of the integrated source
+  ChemPark batch_park = {};           // of rc_chem_integrate, grown to its largest call
   const rc_mlp* net = nullptr;        // surrogate (RC_CHEM_SURROGATE)
   float spread_tol = 0.02f;
   int* sur_list = nullptr;            // [NE] cells handed back to the integrator
@@ -1845,6 +1846,38 @@ int dev_zeros(rc_ctx* c, size_t n, T** out) {
   RC_CU(cudaMemsetAsync(p, 0, std::max<size_t>(n, 1) * sizeof(T), c->stream));
   RC_CU(cudaStreamSynchronize(c->stream));
   *out = static_cast<T*>(p);
+  return RC_OK;
+}
+
+// Work space of the integrator's rounds for `items` states: the counters, and
+// lists for at most PARK_MAX of them (a million: 200 MB).  Lists that are too
+// short, or none where there is no memory for them, only cost speed.
+constexpr int PARK_MAX = 1 << 20;
+int park_space(rc_ctx* c, int items, ChemPark* p) {
+  if (!p->count)
+    if (int st = dev_zeros(c, (size_t)2 * CHEM_ROUNDS, &p->count)) return st;
+  int nsm = 1;
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
+  const int cap = std::min(items, PARK_MAX);
+  if (cap <= p->cap || items <= 128 * nsm) return RC_OK;  // few items run in one round
+  if (p->cap) {
+    RC_CU(cudaStreamSynchronize(c->stream));
+    for (void* q : {(void*)p->x, (void*)p->k}) {
+      c->allocs.erase(std::find(c->allocs.begin(), c->allocs.end(), q));
+      cudaFree(q);
+    }
+    p->cap = 0;
+  }
+  void *x = nullptr, *k = nullptr;
+  if (cudaMalloc(&x, sizeof(double) * 2 * CHEM_PARK_X * (size_t)cap) != cudaSuccess ||
+      cudaMalloc(&k, sizeof(int) * 2 * CHEM_PARK_K * (size_t)cap) != cudaSuccess) {
+    cudaGetLastError();
+    if (x) cudaFree(x);
+    return RC_OK;
+  }
+  c->allocs.push_back(x);
+  c->allocs.push_back(k);
+  *p = {static_cast<double*>(x), static_cast<int*>(k), p->count, cap, 1, false};
   return RC_OK;
 }
 
@@ -2275,13 +2308,11 @@ void q_chem_fork(rc_ctx* c) {
     cudaMemsetAsync(c->sur_counts, 0, 2 * sizeof(unsigned), c->stream2);
     surrogate_source(c->d, c->thermo.data(), c->net, c->spread_tol, c->sur_list, c->sur_counts, c->sur_counts + 1,
                      c->sur_mode, c->sur_dec, c->stream2);
-    chem_list<NSP>(c->d, c->thermo.data(), c->chem_tol, c->chem_maxsub, c->chem_nsub, c->sur_list, c->sur_counts,
-                   c->chem_counter, c->stream2);
-    c->launches += 2;
+    c->launches += 1 + chem_list<NSP>(c->d, c->thermo.data(), c->chem_tol, c->chem_maxsub, c->chem_nsub, c->sur_list,
+                                      c->sur_counts, c->chem_park, c->stream2);
   } else {
-    chem_source<NSP>(c->d, c->thermo.data(), c->chem_tol, c->chem_maxsub, c->chem_nsub, c->chem_order,
-                     c->chem_hist, c->chem_counter, c->stream2);
-    c->launches += 4;
+    c->launches += chem_source<NSP>(c->d, c->thermo.data(), c->chem_tol, c->chem_maxsub, c->chem_nsub, c->chem_order,
+                                    c->chem_hist, c->chem_park, c->stream2);
   }
   cudaEventRecord(c->ev_join, c->stream2);
 }
@@ -3548,11 +3579,12 @@ int rc_set_chemistry(rc_ctx* c, int mode, double tol, int max_substeps) {
     if (int st = dev_zeros(c, (size_t)c->NE, &c->chem_nsub)) return st;
     if (int st = dev_zeros(c, (size_t)c->NE, &c->chem_order)) return st;
     if (int st = dev_zeros(c, (size_t)256, &c->chem_hist)) return st;
-    if (int st = dev_zeros(c, (size_t)1, &c->chem_counter)) return st;
     RC_CU(cudaStreamCreateWithFlags(&c->stream2, cudaStreamNonBlocking));
     RC_CU(cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming));
     RC_CU(cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming));
   }
+  if (mode != RC_CHEM_EXPLICIT)
+    if (int st = park_space(c, c->NE, &c->chem_park)) return st;
   c->chem = mode;
   c->chem_tol = tol;
   c->chem_maxsub = max_substeps;
@@ -3574,11 +3606,11 @@ int rc_chem_integrate(rc_ctx* c, const double* d_P, const double* d_dt, int n, d
   if (!c || n < 0 || (n > 0 && (!d_P || !d_dt || !d_out || !d_nsub))) return RC_ERR_ARG;
   if (c->NSP < 2 || !(tol > 0.0) || max_substeps < 1) return RC_ERR_ARG;
   if (n == 0) return RC_OK;
-  if (!c->chem_counter)
-    if (int st = dev_zeros(c, (size_t)1, &c->chem_counter)) return st;
-  RC_DISPATCH(c, chem_batch, c->thermo.data(), d_P, d_dt, n, d_out, d_nsub, tol, max_substeps, c->chem_counter,
-              c->d.err, c->stream);
-  c->launches++;
+  if (int st = park_space(c, n, &c->batch_park)) return st;
+  c->launches += c->NSP == 1 ? chem_batch<1>(c->thermo.data(), d_P, d_dt, n, d_out, d_nsub, tol, max_substeps,
+                                             c->batch_park, c->d.err, c->stream)
+                             : chem_batch<4>(c->thermo.data(), d_P, d_dt, n, d_out, d_nsub, tol, max_substeps,
+                                             c->batch_park, c->d.err, c->stream);
   return check_launch(c, "rc_chem_integrate");
 }
 int rc_lusgs_stage(rc_ctx* c, int istep) {

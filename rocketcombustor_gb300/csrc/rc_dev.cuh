@@ -207,6 +207,18 @@ __device__ __forceinline__ void bar_named(int id, int count) {
 __device__ __forceinline__ void bar_arrive(int id, int count) {
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory");
 }
+// Work space of the integrator's rounds (rc_chem.cu): two lists of parked
+// reactors, [list][field][cap] each, and per round its queue counter and
+// the number it parked.
+constexpr int CHEM_ROUNDS = 10, CHEM_PARK_X = 11, CHEM_PARK_K = 3;
+struct ChemPark {
+  double* x;
+  int* k;
+  unsigned* count;  // [2 * CHEM_ROUNDS]
+  int cap;          // places in a list (0: nothing can be parked)
+  int rounds;       // of this launch
+  bool cut;         // a round ends when its queue is empty
+};
 // Tables of the dataflow LU-SGS: cells are split into per-SM blocks, a pass is
 // a run of consecutive sweep positions of one level whose cells one block owns
 // (k_lusgs_flow: at most 8 per group; k_lusgs_flowc: see below).
