@@ -430,8 +430,11 @@ __device__ __forceinline__ void cp_async_wait_all() {
 
 // BN: output columns per CTA (128 or 64; the B tile holds BN rows); grid
 // (N / BN, M / 128, split-K)
+// 8 warps: the loads and the epilogue (GELU and its stores) take most of a
+// CTA's 8 us; two warps per 32 rows of the accumulator, 8.8 -> 7.8 us.
+constexpr int GEMM_THREADS = 256;
 template <int EPI, int BN>
-__global__ void __launch_bounds__(128) k_gemm(GemmArgs g) {
+__global__ void __launch_bounds__(GEMM_THREADS) k_gemm(GemmArgs g) {
   static_assert(BN == 128 || BN == 64, "the tile widths of the epilogue and the TMEM allocation");
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = smem_raw + ((1024u - (umma::smem_u32(smem_raw) & 1023u)) & 1023u);
@@ -451,12 +454,13 @@ __global__ void __launch_bounds__(128) k_gemm(GemmArgs g) {
   __syncthreads();
   umma::tc_fence_after();
   const uint32_t tmem = *slot;
+  pdl_wait();
   uint32_t phase = 0;
   bool ok = true;
   for (int k0 = kb; k0 < kb + kper; k0 += 128) {
     // both 128 x 128 operand tiles as 16-byte asynchronous copies, all in
     // flight at once, into the swizzled layout
-    for (int q = t; q < 2048; q += 128) {
+    for (int q = t; q < 2048; q += GEMM_THREADS) {
       const int r = q >> 4, c = q & 15;
       cp_async16(sA + umma::sw128_offset(r, c * 8, 128), g.A + (size_t)(m0 + r) * g.lda + k0 + c * 8);
       if (r < BN) cp_async16(sB + umma::sw128_offset(r, c * 8, BN), g.B + (size_t)(n0 + r) * g.ldb + k0 + c * 8);
@@ -480,10 +484,11 @@ __global__ void __launch_bounds__(128) k_gemm(GemmArgs g) {
     if (!*s_ok) { ok = false; break; }
   }
   if (ok) {
-    const int m = m0 + warp * 32 + (t & 31);
-    for (int c = 0; c < BN / 32; ++c) {
+    // warps w and w + 4 read the same 32 rows, alternate blocks of 32 columns
+    const int quad = warp & 3, m = m0 + quad * 32 + (t & 31);
+    for (int c = warp >> 2; c < BN / 32; c += GEMM_THREADS / 128) {
       float v[32];
-      umma::tmem_ld32(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)(c * 32), v);
+      umma::tmem_ld32(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(c * 32), v);
       const int nc = n0 + c * 32;
       if (EPI == EPI_F32) {
         float* dst = g.C + (size_t)blockIdx.z * g.M * g.N + (size_t)m * g.N + nc;
@@ -537,16 +542,40 @@ __global__ void __launch_bounds__(128) k_gemm(GemmArgs g) {
 // layer 0 for a training batch: xn (n x 7), H0 (n x 128 FP32), A0 row / column
 // (BF16).  A block takes 32 samples (the lanes) and its 16 warps 8 outputs each;
 // warp 0 forms the samples' features.
+// With a draw the samples are batch number *it of a training set, their targets
+// go to tb: `batch` pairs drawn with replacement from the set's `set` pairs
+// (x: set x NIN, t: set x NOUT, row-major), pair index = splitmix64 (Steele,
+// Lea and Flood, "Fast splittable pseudorandom number generators", 2014) of
+// seed + (it * batch + i + 1) * golden gamma, modulo set.
+struct Draw {
+  const float* t;
+  long long set;
+  unsigned long long seed;
+  const int* it;
+  float* tb;
+};
 constexpr int L0_THREADS = 512;
-__global__ void __launch_bounds__(L0_THREADS) k_layer0(const float* __restrict__ x, Norm nr,
+template <bool DRAW>
+__global__ void __launch_bounds__(L0_THREADS) k_layer0(const float* __restrict__ x, Draw dr, Norm nr,
                                                        const float* __restrict__ P, int n, float* xn, float* H0,
                                                        __nv_bfloat16* Arow, __nv_bfloat16* Acol) {
   __shared__ float sf[32][NIN + 1];
   const int lane = threadIdx.x & 31, c8 = threadIdx.x >> 5;
   const int s = blockIdx.x * 32 + lane;
   if (c8 == 0 && s < n) {
+    long long row = s;
+    if (DRAW) {
+      unsigned long long z = dr.seed + 0x9E3779B97F4A7C15ull * ((unsigned long long)*dr.it * (unsigned long long)n +
+                                                                (unsigned long long)s + 1ull);
+      z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+      z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+      z ^= z >> 31;
+      row = (long long)(z % (unsigned long long)dr.set);
+#pragma unroll
+      for (int k = 0; k < NOUT; ++k) dr.tb[(size_t)s * NOUT + k] = dr.t[(size_t)row * NOUT + k];
+    }
     float f[NIN];
-    features(x + (size_t)s * NIN, nr, f);
+    features(x + (size_t)row * NIN, nr, f);
 #pragma unroll
     for (int i = 0; i < NIN; ++i) {
       xn[(size_t)s * NIN + i] = f[i];
@@ -584,6 +613,7 @@ __global__ void __launch_bounds__(HEAD_THREADS) k_head(const float* __restrict__
                                                        const float* __restrict__ P, int n, float* dy,
                                                        __nv_bfloat16* dHrow, __nv_bfloat16* dHcol, float* loss_part) {
   __shared__ float red[HEAD_THREADS];
+  pdl_wait();
   const int qd = threadIdx.x & 3, s = blockIdx.x * HEAD_SAMPLES + (threadIdx.x >> 2);
   const bool valid = s < n;
   const int sc_ = valid ? s : 0;
@@ -732,26 +762,76 @@ __global__ void __launch_bounds__(H) k_small_part(const float* __restrict__ xn, 
   if (o < NOUT) part[(size_t)blockIdx.x * SMALL_N + H * SMALL_PER + o] = b4;
 }
 
+// Adam's update of parameter q by gradient gq, and the BF16 copies of a hidden
+// weight: Wb[l][o][i] and WbT[l][i][o]
+struct Adam {
+  float *p, *m1, *m2;
+  float lr, b1, b2, eps, bc1, bc2;
+  const float* sched;  // lr, bc1, bc2 of this step in device memory (k_train_tail); null: the arguments
+  __nv_bfloat16 *Wb, *WbT;
+};
+__device__ __forceinline__ float adam(const Adam& ad, int q, float gq) {
+  const float lr = ad.sched ? ad.sched[0] : ad.lr, bc1 = ad.sched ? ad.sched[1] : ad.bc1,
+              bc2 = ad.sched ? ad.sched[2] : ad.bc2;
+  const float a = ad.b1 * ad.m1[q] + (1.f - ad.b1) * gq;
+  const float b = ad.b2 * ad.m2[q] + (1.f - ad.b2) * gq * gq;
+  ad.m1[q] = a;
+  ad.m2[q] = b;
+  return ad.p[q] -= lr * (a / bc1) / (sqrtf(b / bc2) + ad.eps);
+}
+// hidden weight number q of all three layers
+__device__ __forceinline__ void pack_hidden(const Adam& ad, int q, float v) {
+  const int l = q / (H * H), o = (q % (H * H)) / H, i = q % H;
+  const __nv_bfloat16 w = __float2bfloat16_rn(v);
+  ad.Wb[q] = w;
+  ad.WbT[(size_t)l * H * H + i * H + o] = w;
+}
 // The gradient vector from the partials, each summed in order: dW_1..3 over
 // the z split-K partials of the hidden weight-gradient GEMMs, the thin
-// parameters over the zs sample chunks of k_small_part.
-__global__ void k_reduce_grads(const float* __restrict__ part, int z, const float* __restrict__ spart, int zs,
-                               float* grad) {
-  const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q < 3 * H * H) {
-    const int l = q / (H * H), e = q % (H * H);
-    const float* p = part + (size_t)l * z * H * H;
+// parameters over the zs sample chunks of k_small_part.  STEP: each thread
+// goes on to Adam's update of its parameter and the packed copies.  (A training
+// step is a chain of small kernels.  It ended with six, reduction, loss, schedule,
+// Adam and two packings, and began with the draw: now the draw is in layer 0,
+// the loss and schedule run beside the backward pass, the inference kernel's weights
+// are packed after the last step.  With the programmatic launches and the GEMMs'
+// wider epilogue, 8,192 samples: 92 -> 77 us a step.)
+// Bound by the latency of the partials' loads: a block takes RED_H hidden
+// parameters, one per thread, or RED_THIN thin ones, whose up to SMALL_ZMAX
+// partials the whole block fetches to shared memory, 128 at a time.
+constexpr int RED_THREADS = 256, RED_THIN = 16, RED_TILE = 128;
+constexpr int RED_HB = 3 * H * H / RED_THREADS, RED_BLOCKS = RED_HB + (SMALL_N + RED_THIN - 1) / RED_THIN;
+static_assert(3 * H * H % RED_THREADS == 0, "whole blocks of hidden parameters");
+template <bool STEP>
+__global__ void __launch_bounds__(RED_THREADS) k_reduce_grads(const float* __restrict__ part, int z,
+                                                              const float* __restrict__ spart, int zs, float* grad,
+                                                              Adam ad) {
+  __shared__ float sp[RED_TILE][RED_THIN + 1];
+  const int t = threadIdx.x, thin = RED_BLOCKS - RED_HB;
+  if ((int)blockIdx.x >= thin) {
+    const int q = (blockIdx.x - thin) * RED_THREADS + t, l = q / (H * H), e = q % (H * H);
+    const float* p = part + (size_t)l * z * H * H + e;
     float a = 0.f;
-#pragma unroll 8
-    for (int k = 0; k < z; ++k) a += p[(size_t)k * H * H + e];
-    grad[off_w(l + 1) + e] = a;
+#pragma unroll 16
+    for (int k = 0; k < z; ++k) a += p[(size_t)k * H * H];
+    if (STEP) pack_hidden(ad, q, adam(ad, off_w(l + 1) + e, a));
+    else grad[off_w(l + 1) + e] = a;
     return;
   }
-  const int r = q - 3 * H * H;
-  if (r >= SMALL_N) return;
+  const int r0 = blockIdx.x * RED_THIN, r = r0 + t;
   float a = 0.f;
-#pragma unroll 8
-  for (int k = 0; k < zs; ++k) a += spart[(size_t)k * SMALL_N + r];
+  for (int k0 = 0; k0 < zs; k0 += RED_TILE) {
+    const int nk = min(RED_TILE, zs - k0);
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < RED_TILE * RED_THIN / RED_THREADS; ++u) {
+      const int k = (u * RED_THREADS + t) / RED_THIN, c = t % RED_THIN;
+      if (k < nk && r0 + c < SMALL_N) sp[k][c] = spart[(size_t)(k0 + k) * SMALL_N + r0 + c];
+    }
+    __syncthreads();
+    if (t < RED_THIN)
+      for (int k = 0; k < nk; ++k) a += sp[k][t];
+  }
+  if (t >= RED_THIN || r >= SMALL_N) return;
   int dst;
   if (r < H * SMALL_PER) {
     const int o = r / SMALL_PER, k = r % SMALL_PER;
@@ -760,82 +840,53 @@ __global__ void k_reduce_grads(const float* __restrict__ part, int z, const floa
   } else {
     dst = OFF_B4 + (r - H * SMALL_PER);
   }
-  grad[dst] = a;
+  if (STEP) adam(ad, dst, a);
+  else grad[dst] = a;
 }
 
 // the loss from k_head's partials: lane l sums partials l, l + 32, ... in
 // order, then a butterfly over the lanes (one warp)
-__global__ void k_loss_final(const float* part, int nb, int n, float* loss) {
-  if (blockIdx.x != 0 || threadIdx.x >= 32) return;
+__device__ __forceinline__ float loss_of(const float* part, int nb, int n) {
   float a = 0.f;
   for (int b = threadIdx.x; b < nb; b += 32) a += part[b];
 #pragma unroll
   for (int w = 16; w > 0; w >>= 1) a += __shfl_xor_sync(0xffffffffu, a, w);
-  if (threadIdx.x == 0) *loss = a / (4.f * (float)n);
+  return a / (4.f * (float)n);
+}
+__global__ void k_loss_final(const float* part, int nb, int n, float* loss) {
+  if (blockIdx.x != 0 || threadIdx.x >= 32) return;
+  const float a = loss_of(part, nb, n);
+  if (threadIdx.x == 0) *loss = a;
 }
 
-// Training batch number *it: `batch` pairs drawn with replacement from the n
-// pairs (x: n x NIN, t: n x NOUT, row-major), pair index = splitmix64 (Steele,
-// Lea and Flood, "Fast splittable pseudorandom number generators", 2014) of
-// seed + (it * batch + i + 1) * golden gamma, modulo n; gathered into xb, tb.
-__global__ void k_batch(const float* __restrict__ x, const float* __restrict__ t, long long n,
-                        unsigned long long seed, const int* it, int batch, float* xb, float* tb) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= batch) return;
-  unsigned long long z = seed + 0x9E3779B97F4A7C15ull * ((unsigned long long)*it * (unsigned long long)batch +
-                                                         (unsigned long long)i + 1ull);
-  z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
-  z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
-  z ^= z >> 31;
-  const long long j = (long long)(z % (unsigned long long)n);
-#pragma unroll
-  for (int k = 0; k < NIN; ++k) xb[(size_t)i * NIN + k] = x[(size_t)j * NIN + k];
-#pragma unroll
-  for (int k = 0; k < NOUT; ++k) tb[(size_t)i * NOUT + k] = t[(size_t)j * NOUT + k];
-}
-
-// End of training step k = *it of `steps`: the loss into hist[k] (if hist),
-// the next Adam update's learning rate (cosine decay from lr at k = 0 to
-// lr_end at k = steps - 1) and bias corrections 1 - beta^(t0 + k + 1) into
-// sched, then *it = k + 1.
+// Of training step k = *it of `steps` (one warp): the loss, also into hist[k] (if
+// hist), the Adam update's learning rate (cosine decay from lr at k = 0 to lr_end
+// at k = steps - 1) and bias corrections 1 - beta^(t0 + k + 1) into sched,
+// then *it = k + 1.
 __global__ void k_train_tail(int* it, int steps, int t0, float lr, float lr_end, float b1, float b2,
-                             const float* loss, float* hist, float* sched) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+                             const float* part, int nb, int n, float* loss, float* hist, float* sched) {
+  if (blockIdx.x != 0 || threadIdx.x >= 32) return;
+  const float a = loss_of(part, nb, n);
+  if (threadIdx.x != 0) return;
   const int k = *it;
   const double c = cos(3.141592653589793 * (double)k / (double)(steps > 1 ? steps - 1 : 1));
   sched[0] = (float)((double)lr_end + 0.5 * ((double)lr - (double)lr_end) * (1.0 + c));
   sched[1] = 1.f - powf(b1, (float)(t0 + k + 1));
   sched[2] = 1.f - powf(b2, (float)(t0 + k + 1));
-  if (hist) hist[k] = *loss;
+  *loss = a;
+  if (hist) hist[k] = a;
   *it = k + 1;
 }
 
-// sched (may be null): lr, bc1, bc2 of this step in device memory (k_train_tail)
-__global__ void k_adam(float* p, float* m1, float* m2, const float* __restrict__ g, float lr, float b1, float b2,
-                       float eps, float bc1, float bc2, const float* sched) {
+__global__ void k_adam(Adam ad, const float* __restrict__ g) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= NPARAM) return;
-  if (sched) {
-    lr = sched[0];
-    bc1 = sched[1];
-    bc2 = sched[2];
-  }
-  const float gq = g[q];
-  const float a = b1 * m1[q] + (1.f - b1) * gq;
-  const float b = b2 * m2[q] + (1.f - b2) * gq * gq;
-  m1[q] = a;
-  m2[q] = b;
-  p[q] -= lr * (a / bc1) / (sqrtf(b / bc2) + eps);
+  if (q < NPARAM) adam(ad, q, g[q]);
 }
 
-// BF16 copies of the hidden weights: Wb[l][o][i] and WbT[l][i][o]
-__global__ void k_pack(const float* __restrict__ p, __nv_bfloat16* Wb, __nv_bfloat16* WbT) {
+// BF16 copies of the hidden weights
+__global__ void k_pack(Adam ad) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= 3 * H * H) return;
-  const int l = q / (H * H), o = (q % (H * H)) / H, i = q % H;
-  const __nv_bfloat16 w = __float2bfloat16_rn(p[off_w(l + 1) + o * H + i]);
-  Wb[q] = w;
-  WbT[(size_t)l * H * H + i * H + o] = w;
+  if (q < 3 * H * H) pack_hidden(ad, q, ad.p[off_w(q / (H * H) + 1) + q % (H * H)]);
 }
 
 // F16 weights of the inference kernel, swizzled in its shared-memory order
@@ -923,12 +974,11 @@ struct rc_mlp {
   // training work buffers for up to cap samples
   int cap = 0, zsplit = 1;
   std::vector<void*> work;
-  float *xn = nullptr, *Hs[4] = {}, *dy = nullptr, *loss_part = nullptr, *loss = nullptr, *part = nullptr,
-        *grad = nullptr;
+  float *xn = nullptr, *Hs[4] = {}, *dy = nullptr, *loss_part = nullptr, *loss = nullptr, *part = nullptr;
   float* spart = nullptr;                                // k_small_part's partials
   cudaStream_t side = nullptr;                           // the weight-gradient branch
   cudaEvent_t ev_dh[4] = {}, ev_join = nullptr;          // dH_l ready / the branch done
-  float *xb = nullptr, *tb = nullptr, *sched = nullptr;  // rc_mlp_train: the batch, the step's schedule
+  float *tb = nullptr, *sched = nullptr;                 // rc_mlp_train: the batch's targets, the step's schedule
   int* it = nullptr;                                     // rc_mlp_train: the step counter
   __nv_bfloat16 *Arow[3] = {}, *Acol[3] = {}, *dHrow[4] = {}, *dHcol[4] = {};
   std::string err;
@@ -952,6 +1002,11 @@ int fused_grid(int device, int n) {
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device);
   const int ctas = ((n + 127) / 128 + mlp::FG - 1) / mlp::FG;
   return ctas < nsm ? (ctas > 0 ? ctas : 1) : nsm;
+}
+
+// the network's parameters, moments and packed copies; a schedule of zeros
+mlp::Adam adam_of(rc_mlp* m) {
+  return {m->params, m->m1, m->m2, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, nullptr, m->Wb, m->WbT};
 }
 
 template <class T>
@@ -984,7 +1039,6 @@ int ensure_work(rc_mlp* m, int n) {
   st |= alloc_work(m, N * mlp::NOUT, &m->dy);
   st |= alloc_work(m, (N + mlp::HEAD_SAMPLES - 1) / mlp::HEAD_SAMPLES, &m->loss_part);
   st |= alloc_work(m, (size_t)1, &m->loss);
-  st |= alloc_work(m, N * mlp::NIN, &m->xb);
   st |= alloc_work(m, N * mlp::NOUT, &m->tb);
   st |= alloc_work(m, (size_t)4, &m->sched);
   st |= alloc_work(m, (size_t)1, &m->it);
@@ -1034,7 +1088,7 @@ int rc_mlp_create(int device, rc_mlp** out) {
   if (cudaSetDevice(device) != cudaSuccess) return bail(RC_ERR_CUDA);
   const size_t P = mlp::NPARAM;
   if (cudaMalloc(&m->params, P * sizeof(float)) != cudaSuccess || cudaMalloc(&m->m1, P * sizeof(float)) != cudaSuccess ||
-      cudaMalloc(&m->m2, P * sizeof(float)) != cudaSuccess || cudaMalloc(&m->grad, P * sizeof(float)) != cudaSuccess ||
+      cudaMalloc(&m->m2, P * sizeof(float)) != cudaSuccess ||
       cudaMalloc(&m->Wb, 3 * mlp::H * mlp::H * sizeof(__nv_bfloat16)) != cudaSuccess ||
       cudaMalloc(&m->WbT, 3 * mlp::H * mlp::H * sizeof(__nv_bfloat16)) != cudaSuccess ||
       cudaMalloc(&m->Wh, mlp::WH_BYTES) != cudaSuccess || cudaMalloc(&m->derr, sizeof(unsigned)) != cudaSuccess)
@@ -1072,7 +1126,7 @@ int rc_mlp_create(int device, rc_mlp** out) {
 int rc_mlp_destroy(rc_mlp* m) {
   if (!m) return RC_OK;
   for (void* p : m->work) cudaFree(p);
-  cudaFree(m->params); cudaFree(m->m1); cudaFree(m->m2); cudaFree(m->grad);
+  cudaFree(m->params); cudaFree(m->m1); cudaFree(m->m2);
   cudaFree(m->Wb); cudaFree(m->WbT); cudaFree(m->Wh); cudaFree(m->derr);
   for (cudaEvent_t e : m->ev_dh)
     if (e) cudaEventDestroy(e);
@@ -1090,7 +1144,7 @@ int rc_mlp_set_params(rc_mlp* m, const float* params) {
   MLP_CU(cudaMemset(m->m1, 0, sizeof(float) * mlp::NPARAM));
   MLP_CU(cudaMemset(m->m2, 0, sizeof(float) * mlp::NPARAM));
   m->step = 0;
-  mlp::k_pack<<<(3 * mlp::H * mlp::H + 255) / 256, 256>>>(m->params, m->Wb, m->WbT);
+  mlp::k_pack<<<(3 * mlp::H * mlp::H + 255) / 256, 256>>>(adam_of(m));
   mlp::k_pack16<<<(mlp::PACK16_N + 255) / 256, 256>>>(m->params, m->Wh);
   MLP_CU(cudaGetLastError());
   MLP_CU(cudaDeviceSynchronize());
@@ -1129,10 +1183,38 @@ int rc_mlp_forward(rc_mlp* m, const float* d_x, int n, float* d_y, void* stream)
 }  // extern "C"
 
 namespace {
-// the kernels of one loss-and-gradient evaluation on n samples (work buffers
-// sized for n), enqueued on s without synchronising
-int enqueue_gradient(rc_mlp* m, const float* d_x, const float* d_t, int n, float* d_grad, cudaStream_t s) {
+// What ends a gradient evaluation: its reduction to `grad` and the loss, or, in
+// a training step (steps > 0), the loss, the schedule and Adam's update.
+struct GradEnd {
+  float* grad;
+  mlp::Adam ad;
+  int steps;
+  float lr, lr_end;
+  float* hist;
+};
+// The kernels of one loss-and-gradient evaluation on n samples (work buffers
+// sized for n), enqueued on s without synchronising; with `draw` the samples
+// are drawn from its set.  The kernels of the chain layer 0 .. dH0 are launched
+// programmatically: a launch is prepared before its predecessor ends.  (A
+// trigger at the start of each kernel, which lets the next one's blocks take
+// their shared memory and wait there, costs more than it gives: 94 us a step
+// against 80 without it and 84 with plain launches.)
+int enqueue_gradient(rc_mlp* m, const float* d_x, const float* d_t, const mlp::Draw* draw, int n, const GradEnd& end,
+                     cudaStream_t s) {
   using namespace mlp;
+  auto pdl = [&](auto kernel, dim3 grid, unsigned block, size_t smem, auto... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+  };
   // split-K of the weight gradients: about 2 chunks of 128 samples per CTA
   // (at most ZSPLIT_MAX splits), an exact divisor of the n / 128 chunks (each
   // split a whole number of chunks)
@@ -1141,7 +1223,12 @@ int enqueue_gradient(rc_mlp* m, const float* d_x, const float* d_t, int n, float
   // sample chunks of the thin parameters' gradients: 64 samples or more, at
   // most SMALL_ZMAX chunks (n is a multiple of 128, so every chunk is whole tiles)
   const int chunk = 64 * ((n + 64 * SMALL_ZMAX - 1) / (64 * SMALL_ZMAX)), zs = (n + chunk - 1) / chunk;
-  k_layer0<<<(n + 31) / 32, L0_THREADS, 0, s>>>(d_x, m->norm, m->params, n, m->xn, m->Hs[0], m->Arow[0], m->Acol[0]);
+  if (draw)
+    k_layer0<true><<<(n + 31) / 32, L0_THREADS, 0, s>>>(d_x, *draw, m->norm, m->params, n, m->xn, m->Hs[0], m->Arow[0],
+                                                        m->Acol[0]);
+  else
+    k_layer0<false><<<(n + 31) / 32, L0_THREADS, 0, s>>>(d_x, Draw{}, m->norm, m->params, n, m->xn, m->Hs[0],
+                                                         m->Arow[0], m->Acol[0]);
   // hidden layers 1..3 forward: H_l = A_{l-1} W_l^T + b_l
   for (int l = 1; l <= 3; ++l) {
     GemmArgs g{};
@@ -1153,10 +1240,11 @@ int enqueue_gradient(rc_mlp* m, const float* d_x, const float* d_t, int n, float
     g.Orow = l < 3 ? m->Arow[l] : m->dHrow[3];   // A3 row is not needed (the head recomputes it)
     g.Ocol = l < 3 ? m->Acol[l] : m->dHcol[3];   // scratch for l = 3, overwritten by the head
     g.err = m->derr;
-    k_gemm<EPI_FWD, 64><<<dim3(H / 64, n / 128, 1), 128, GEMM_SMEM, s>>>(g);
+    MLP_CU(pdl(k_gemm<EPI_FWD, 64>, dim3(H / 64, n / 128, 1), GEMM_THREADS, GEMM_SMEM, g));
   }
-  k_head<<<(n + HEAD_SAMPLES - 1) / HEAD_SAMPLES, HEAD_THREADS, 0, s>>>(m->Hs[3], d_t, m->params, n, m->dy,
-                                                                         m->dHrow[3], m->dHcol[3], m->loss_part);
+  const int nb = (n + HEAD_SAMPLES - 1) / HEAD_SAMPLES;
+  MLP_CU(pdl(k_head, dim3(nb), HEAD_THREADS, 0, (const float*)m->Hs[3], d_t, (const float*)m->params, n, m->dy,
+             m->dHrow[3], m->dHcol[3], m->loss_part));
   // backward data: dH_{l-1} = (dH_l W_l) * gelu'(H_{l-1}) on s; each weight
   // gradient dW_l = dH_l^T A_{l-1} (split-K partials) on the side stream as
   // soon as dH_l is ready, then the thin parameters' partials; s joins the
@@ -1168,7 +1256,7 @@ int enqueue_gradient(rc_mlp* m, const float* d_x, const float* d_t, int n, float
     g.M = H; g.N = H; g.K = n;
     g.C = m->part + (size_t)(l - 1) * z * H * H;
     g.err = m->derr;
-    k_gemm<EPI_F32, 128><<<dim3(1, 1, z), 128, GEMM_SMEM, m->side>>>(g);
+    k_gemm<EPI_F32, 128><<<dim3(1, 1, z), GEMM_THREADS, GEMM_SMEM, m->side>>>(g);
   };
   MLP_CU(cudaEventRecord(m->ev_dh[3], s));
   MLP_CU(cudaStreamWaitEvent(m->side, m->ev_dh[3], 0));
@@ -1182,7 +1270,7 @@ int enqueue_gradient(rc_mlp* m, const float* d_x, const float* d_t, int n, float
     g.Orow = m->dHrow[l - 1];
     g.Ocol = m->dHcol[l - 1];
     g.err = m->derr;
-    k_gemm<EPI_BWD, 64><<<dim3(H / 64, n / 128, 1), 128, GEMM_SMEM, s>>>(g);
+    MLP_CU(pdl(k_gemm<EPI_BWD, 64>, dim3(H / 64, n / 128, 1), GEMM_THREADS, GEMM_SMEM, g));
     MLP_CU(cudaEventRecord(m->ev_dh[l - 1], s));
     MLP_CU(cudaStreamWaitEvent(m->side, m->ev_dh[l - 1], 0));
     if (l > 1) wgrad(l - 1);
@@ -1190,9 +1278,15 @@ int enqueue_gradient(rc_mlp* m, const float* d_x, const float* d_t, int n, float
   k_small_part<<<zs, H, SMALL_SMEM, m->side>>>(m->xn, m->dHrow[0], m->dHrow[1], m->dHrow[2], m->dHrow[3], m->Hs[3],
                                               m->dy, n, chunk, m->spart);
   MLP_CU(cudaEventRecord(m->ev_join, m->side));
+  // beside the side stream's last kernels
+  if (end.steps > 0)
+    k_train_tail<<<1, 32, 0, s>>>(m->it, end.steps, m->step, end.lr, end.lr_end, end.ad.b1, end.ad.b2, m->loss_part, nb,
+                                  n, m->loss, end.hist, m->sched);
+  else
+    k_loss_final<<<1, 32, 0, s>>>(m->loss_part, nb, n, m->loss);
   MLP_CU(cudaStreamWaitEvent(s, m->ev_join, 0));
-  k_reduce_grads<<<(3 * H * H + SMALL_N + 255) / 256, 256, 0, s>>>(m->part, z, m->spart, zs, d_grad);
-  k_loss_final<<<1, 32, 0, s>>>(m->loss_part, (n + HEAD_SAMPLES - 1) / HEAD_SAMPLES, n, m->loss);
+  const auto reduce = end.steps > 0 ? k_reduce_grads<true> : k_reduce_grads<false>;
+  reduce<<<RED_BLOCKS, RED_THREADS, 0, s>>>(m->part, z, m->spart, zs, end.grad, end.ad);
   MLP_CU(cudaGetLastError());
   return RC_OK;
 }
@@ -1205,7 +1299,7 @@ int rc_mlp_gradient(rc_mlp* m, const float* d_x, const float* d_t, int n, float*
   if (!m || !d_x || !d_t || !d_grad || n <= 0 || n % 128) return RC_ERR_ARG;
   if (int st = ensure_work(m, n)) return st;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (int st = enqueue_gradient(m, d_x, d_t, n, d_grad, s)) return st;
+  if (int st = enqueue_gradient(m, d_x, d_t, nullptr, n, GradEnd{d_grad}, s)) return st;
   if (loss) {
     MLP_CU(cudaMemcpyAsync(loss, m->loss, sizeof(float), cudaMemcpyDeviceToHost, s));
     unsigned e = 0;
@@ -1224,15 +1318,16 @@ int rc_mlp_adam(rc_mlp* m, const float* d_grad, float lr, float beta1, float bet
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   m->step += 1;
   const float bc1 = 1.f - std::pow(beta1, (float)m->step), bc2 = 1.f - std::pow(beta2, (float)m->step);
-  mlp::k_adam<<<(mlp::NPARAM + 255) / 256, 256, 0, s>>>(m->params, m->m1, m->m2, d_grad, lr, beta1, beta2, eps, bc1,
-                                                       bc2, nullptr);
-  mlp::k_pack<<<(3 * mlp::H * mlp::H + 255) / 256, 256, 0, s>>>(m->params, m->Wb, m->WbT);
+  mlp::Adam ad = adam_of(m);
+  ad.lr = lr; ad.b1 = beta1; ad.b2 = beta2; ad.eps = eps; ad.bc1 = bc1; ad.bc2 = bc2;
+  mlp::k_adam<<<(mlp::NPARAM + 255) / 256, 256, 0, s>>>(ad, d_grad);
+  mlp::k_pack<<<(3 * mlp::H * mlp::H + 255) / 256, 256, 0, s>>>(ad);
   mlp::k_pack16<<<(mlp::PACK16_N + 255) / 256, 256, 0, s>>>(m->params, m->Wh);
   MLP_CU(cudaGetLastError());
   return RC_OK;
 }
 
-// Adam on `steps` batches drawn on the device (k_batch), the learning rate
+// Adam on `steps` batches drawn on the device (k_layer0), the learning rate
 // and bias corrections formed on the device (k_train_tail): one step (draw,
 // loss and gradient, Adam, the packed weights) is captured once as a CUDA
 // graph on a private stream and launched `steps` times on the caller's.
@@ -1253,18 +1348,20 @@ int rc_mlp_train(rc_mlp* m, const float* d_x, const float* d_t, long long n, int
   int st = RC_OK;
   cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
   if (e == cudaSuccess) {
-    k_batch<<<(batch + 127) / 128, 128, 0, cs>>>(d_x, d_t, n, seed, m->it, batch, m->xb, m->tb);
-    st = enqueue_gradient(m, m->xb, m->tb, batch, m->grad, cs);
-    k_train_tail<<<1, 32, 0, cs>>>(m->it, steps, m->step, lr, lr_end, beta1, beta2, m->loss, d_loss, m->sched);
-    k_adam<<<(NPARAM + 255) / 256, 256, 0, cs>>>(m->params, m->m1, m->m2, m->grad, lr, beta1, beta2, eps, 1.f, 1.f,
-                                                m->sched);
-    k_pack<<<(3 * H * H + 255) / 256, 256, 0, cs>>>(m->params, m->Wb, m->WbT);
-    k_pack16<<<(PACK16_N + 255) / 256, 256, 0, cs>>>(m->params, m->Wh);
+    const Draw draw{d_t, n, seed, m->it, m->tb};
+    GradEnd end{nullptr, adam_of(m), steps, lr, lr_end, d_loss};
+    end.ad.b1 = beta1; end.ad.b2 = beta2; end.ad.eps = eps;
+    end.ad.sched = m->sched;
+    st = enqueue_gradient(m, d_x, m->tb, &draw, batch, end, cs);
     const cudaError_t e2 = cudaStreamEndCapture(cs, &g);
     e = e2 != cudaSuccess ? e2 : cudaGetLastError();
   }
   if (e == cudaSuccess && st == RC_OK) e = cudaGraphInstantiate(&ge, g, 0);
   for (int k = 0; e == cudaSuccess && st == RC_OK && k < steps; ++k) e = cudaGraphLaunch(ge, s);
+  if (e == cudaSuccess && st == RC_OK) {
+    k_pack16<<<(PACK16_N + 255) / 256, 256, 0, s>>>(m->params, m->Wh);
+    e = cudaGetLastError();
+  }
   unsigned derr = 0;
   if (e == cudaSuccess && st == RC_OK) e = cudaMemcpyAsync(&derr, m->derr, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess && st == RC_OK) e = cudaStreamSynchronize(s);
