@@ -2437,18 +2437,33 @@ void q_stage(rc_ctx* c) {
     q_sweeps<NSP>(c, 1);
     return;
   }
-  mixed_ts_face<NSP>(c->d, c->thermo32.data(), c->visc, c->stream);
-  c->launches++;
-  if (c->mode == RC_PREC_MIXED) {
-    mixed_cell<NSP>(c->d, c->thermo32.data(), TH<NSP>(c), 1, c->limit, c->comb && c->chem == RC_CHEM_EXPLICIT,
-                    c->visc, c->stream);
+  auto cell32 = [&](int do_step, cudaStream_t s) {
+    mixed_cell<NSP>(c->d, c->thermo32.data(), TH<NSP>(c), do_step, c->limit, c->comb && c->chem == RC_CHEM_EXPLICIT,
+                    c->visc, s);
     c->launches++;
+  };
+  const bool beside = c->mode == RC_PREC_MIXED && !(c->comb && c->chem != RC_CHEM_EXPLICIT);
+  if (beside) {  // as in q_step_recon
+    cudaEventRecord(c->ts_fork, c->stream);
+    cudaStreamWaitEvent(c->ts_stream, c->ts_fork, 0);
+    cell32(0, c->stream);
+    mixed_ts_face<NSP>(c->d, c->thermo32.data(), c->visc, c->ts_stream);
+    c->launches++;
+    cell32(2, c->ts_stream);
+    cudaEventRecord(c->ts_join, c->ts_stream);
   } else {
-    q_cell<NSP>(c, 1, 1, c->stream);
-    mixed_pack<NSP>(c->d, c->stream);
+    mixed_ts_face<NSP>(c->d, c->thermo32.data(), c->visc, c->stream);
     c->launches++;
+    if (c->mode == RC_PREC_MIXED) {
+      cell32(1, c->stream);
+    } else {
+      q_cell<NSP>(c, 1, 1, c->stream);
+      mixed_pack<NSP>(c->d, c->stream);
+      c->launches++;
+    }
   }
   q_flux_mode<NSP>(c);
+  if (beside) q_step_join(c);
   q_sweeps32<NSP>(c);
 }
 

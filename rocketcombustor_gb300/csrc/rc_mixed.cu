@@ -63,6 +63,7 @@ __global__ void __launch_bounds__(128) k_ts_face32(const Dev d, const ThermoDev3
 }
 
 // --------------------------------------------------------- cell kernel -----
+// do_step 0: the reconstruction, 1: with the step and the diagonal, 2: these alone
 template <int NSP>
 __global__ void __launch_bounds__(128) k_cell32(const Dev d, const ThermoDev32<NSP> th, const ThermoDev<NSP> th64,
                                                 int do_step, int limit, int comb, int visc) {
@@ -85,6 +86,7 @@ __global__ void __launch_bounds__(128) k_cell32(const Dev d, const ThermoDev32<N
     d.step[i] = st;
     d.dd[i] = dsum + vol / st;
   }
+  if (do_step == 2) return;
   double P64[V];
   float P[V], Y[NSP];
 #pragma unroll
