@@ -46,8 +46,6 @@ __device__ __forceinline__ double div_rn(double a, double b, double yh, double y
   const int hi = (__double2hiint(q) & 0x7fffffff) | ((__double2hiint(a) ^ __double2hiint(b)) & (int)0x80000000);
   return __hiloint2double(hi, __double2loint(q));
 }
-// a / b for a divisor fixed in advance, its reciprocal pair given as r[0], r[1]
-__device__ __forceinline__ double div_rn(double a, double b, const double* r) { return div_rn(a, b, r[0], r[1]); }
 
 // x != 0.0 without an FP64 compare (NaN counts as non-zero, -0 as zero)
 __device__ __forceinline__ bool nonzero(double x) { return (__double_as_longlong(x) << 1) != 0; }

@@ -6,10 +6,10 @@
 // same code the CPU oracle runs, so the results are bit-identical.  Constants
 // that depend on species data only (pair terms of the Wilke and Chapman-Enskog
 // sums) are evaluated once on the host with the reference's expressions and
-// passed in ThermoDev, with reciprocal pairs of the fixed divisors; divisions
-// by those, and the transport fits' divisions by T and T^2, use the correctly
-// rounded division of rc_div.cuh (the IEEE quotient bit for bit, four FP64
-// operations instead of a division sequence).
+// passed in ThermoDev, with 32-bit reciprocals of the fixed divisors; divisions
+// by those, and the transport fits' divisions by T and T^2, take the integer
+// division of rc_soft.cuh with its reciprocal at hand (the IEEE quotient bit for
+// bit, no FP64 operation).
 #pragma once
 #include <cstdint>
 
