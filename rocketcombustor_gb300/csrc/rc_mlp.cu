@@ -13,10 +13,11 @@
 //   k_mlp_fwd16<Io>   inference, persistent over tiles of 128 samples: all
 //                     weights stay in shared memory, activations never leave
 //                     the SM (inputs and outputs through Io);
-//   k_gemm<EPI, BN>   training GEMMs, one 128 x BN output tile per CTA, K in
-//                     chunks of 128, optional split-K: forward layers (bias +
-//                     GELU epilogue), backward data (x GELU' epilogue) and
-//                     weight gradients (FP32 partials);
+//   k_chain<FWD>      training, the three hidden layers of a tile of 128 samples,
+//                     forward (bias + GELU epilogue) or backward (x GELU'
+//                     epilogue), one CTA per tile;
+//   k_wgrad           the hidden weight gradients, K in chunks of 128, split-K
+//                     (FP32 partials);
 //   k_layer0, k_head, k_small_part, k_reduce_grads, k_adam, k_pack, k_pack16: the thin
 //                     layers, the loss, the small reductions, Adam and the
 //                     BF16 / F16 weight copies.
@@ -404,21 +405,6 @@ struct IoSolver {
 };
 
 // -------------------------------------------------------- training kernels --
-struct GemmArgs {
-  const __nv_bfloat16* A; int lda;   // M x K, K contiguous
-  const __nv_bfloat16* B; int ldb;   // N x K, K contiguous
-  int M, N, K;                       // multiples of 128; K split evenly over gridDim.z
-  const float* bias;                 // EPI_FWD [N]
-  const float* Hin;                  // EPI_BWD pre-activation [M][N]
-  float* Hout;                       // EPI_FWD pre-activation [M][N]
-  __nv_bfloat16* Orow;               // [M][N]
-  __nv_bfloat16* Ocol;               // [N][M]
-  float* C;                          // EPI_F32 [gridDim.z][M][N]
-  unsigned* err;
-};
-enum { EPI_FWD = 0, EPI_BWD = 1, EPI_F32 = 2 };
-constexpr int GS_BAR = 2 * TILE_BYTES, GS_SLOT = GS_BAR + 8, GS_OK = GS_SLOT + 4, GEMM_SMEM = GS_OK + 4 + 1024;
-
 // 16-byte copy global -> shared (cp.async, L2 only); cp_async_wait_all: this
 // thread's copies are complete
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
@@ -428,14 +414,142 @@ __device__ __forceinline__ void cp_async_wait_all() {
   asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
 }
 
-// BN: output columns per CTA (128 or 64; the B tile holds BN rows); grid
-// (N / BN, M / 128, split-K)
-// 8 warps: the loads and the epilogue (GELU and its stores) take most of a
-// CTA's 8 us; two warps per 32 rows of the accumulator, 8.8 -> 7.8 us.
+// The three hidden layers of a training step over one tile of 128 samples,
+// forward (H_l = A_{l-1} W_l^T + b_l, A_l = GELU(H_l)) or backward
+// (dH_{l-1} = (dH_l W_l) GELU'(H_{l-1})): a tile's layers depend on each other
+// only, so its activations stay in shared memory and the three weight tiles are
+// copied in at the start.  A launch per layer, two CTAs a tile, took 7.8-8.2 us
+// each, most of it launch, loads and stores: a step of 8,192 samples 77 -> 69 us,
+// with the weight gradients in one launch.  16 warps: warp w finishes rows
+// 32 (w % 4) .., columns 32 (w / 4) ...
+struct ChainArgs {
+  const __nv_bfloat16* A;      // [M][H] of the first layer
+  const __nv_bfloat16* W[3];   // [H][H], K contiguous, in the order of the chain
+  const float* bias[3];        // forward
+  const float* Hin[3];         // backward: pre-activations [M][H]
+  float* Hout[3];              // forward: pre-activations [M][H]
+  __nv_bfloat16* Orow[3];      // results [M][H] (null: not needed in memory)
+  __nv_bfloat16* Ocol[3];      // results [H][M] (null: not needed)
+  int M;                       // a multiple of 128
+  unsigned* err;
+};
+constexpr int CHAIN_THREADS = 512;
+constexpr int CS_BAR = 4 * TILE_BYTES, CS_SLOT = CS_BAR + 8, CS_OK = CS_SLOT + 4, CHAIN_SMEM = CS_OK + 4 + 1024;
+static_assert(H == 128, "one tile per layer");
+template <bool FWD>
+__global__ void __launch_bounds__(CHAIN_THREADS) k_chain(ChainArgs g) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* base = smem_raw + ((1024u - (umma::smem_u32(smem_raw) & 1023u)) & 1023u);
+  const uint32_t sA = umma::smem_u32(base);
+  uint64_t* bar = reinterpret_cast<uint64_t*>(base + CS_BAR);
+  uint32_t* slot = reinterpret_cast<uint32_t*>(base + CS_SLOT);
+  int* s_ok = reinterpret_cast<int*>(base + CS_OK);
+  const int t = threadIdx.x, warp = t >> 5, m0 = blockIdx.x * 128;
+  const int row = (warp & 3) * 32 + (t & 31), col = (warp >> 2) * 32, m = m0 + row;
+  if (t == 0) umma::mbar_init(bar, 1);
+  if (warp == 0) {
+    umma::tmem_alloc(slot, 128);
+    umma::tmem_relinquish();
+  }
+  // the weights are older than the chain's first launch
+  for (int l = 0; l < 3; ++l)
+    for (int q = t; q < 2048; q += CHAIN_THREADS) {
+      const int r = q >> 4, c = q & 15;
+      cp_async16(sA + (uint32_t)((1 + l) * TILE_BYTES) + umma::sw128_offset(r, c * 8, 128), g.W[l] + r * H + c * 8);
+    }
+  umma::tc_fence_before();
+  __syncthreads();
+  umma::tc_fence_after();
+  const uint32_t tmem = *slot;
+  pdl_wait();
+  for (int q = t; q < 2048; q += CHAIN_THREADS) {
+    const int r = q >> 4, c = q & 15;
+    cp_async16(sA + umma::sw128_offset(r, c * 8, 128), g.A + (size_t)(m0 + r) * H + c * 8);
+  }
+  cp_async_wait_all();
+  uint32_t phase = 0;
+  bool ok = true;
+#pragma unroll 1
+  for (int l = 0; l < 3; ++l) {
+    umma::fence_async_smem();
+    umma::tc_fence_before();
+    __syncthreads();
+    if (t == 0) {
+      umma::tc_fence_after();
+      const uint32_t sB = sA + (uint32_t)((1 + l) * TILE_BYTES);
+#pragma unroll
+      for (int kk = 0; kk < 8; ++kk)
+        umma::mma_bf16(tmem, umma::sdesc_k(sA, 128, kk), umma::sdesc_k(sB, 128, kk), umma::idesc_bf16(128, 128),
+                       kk > 0 ? 1u : 0u);
+      umma::mma_commit(bar);
+      *s_ok = umma::mbar_wait(bar, phase) ? 1 : 0;
+    }
+    // the epilogue's other operand arrives beside the MMAs
+    float4 h[8];
+    const float4* hs = FWD ? reinterpret_cast<const float4*>(g.bias[l] + col)
+                           : reinterpret_cast<const float4*>(g.Hin[l] + (size_t)m * H + col);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) h[j] = hs[j];
+    __syncthreads();
+    phase ^= 1u;
+    umma::tc_fence_after();
+    if (!*s_ok) { ok = false; break; }
+    float v[32], o[32];
+    umma::tmem_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)col, v);
+    if (FWD) {
+      float4* hd = reinterpret_cast<float4*>(g.Hout[l] + (size_t)m * H + col);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float4 x = make_float4(v[4 * j] + h[j].x, v[4 * j + 1] + h[j].y, v[4 * j + 2] + h[j].z,
+                                     v[4 * j + 3] + h[j].w);
+        hd[j] = x;
+        o[4 * j] = gelu(x.x);
+        o[4 * j + 1] = gelu(x.y);
+        o[4 * j + 2] = gelu(x.z);
+        o[4 * j + 3] = gelu(x.w);
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        o[4 * j] = v[4 * j] * gelu_d(h[j].x);
+        o[4 * j + 1] = v[4 * j + 1] * gelu_d(h[j].y);
+        o[4 * j + 2] = v[4 * j + 2] * gelu_d(h[j].z);
+        o[4 * j + 3] = v[4 * j + 3] * gelu_d(h[j].w);
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint4 x = pack8(o + 8 * j);
+      // the MMAs have read the tile: it takes the next layer's operand
+      if (l < 2) *reinterpret_cast<uint4*>(base + umma::sw128_offset(row, col + 8 * j, 128)) = x;
+      if (g.Orow[l]) reinterpret_cast<uint4*>(g.Orow[l] + (size_t)m * H + col)[j] = x;
+    }
+    if (g.Ocol[l])
+#pragma unroll
+      for (int j = 0; j < 32; ++j) g.Ocol[l][(size_t)(col + j) * g.M + m] = __float2bfloat16_rn(o[j]);
+  }
+  if (!ok && t == 0) atomicOr(g.err, ERR_SYNC);
+  umma::tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    umma::tc_fence_after();
+    umma::tmem_dealloc(tmem, 128);
+  }
+}
+
+// The weight gradients dW_l = dH_l^T A_{l-1} of the three hidden layers
+// (blockIdx.x: l - 1): FP32 partials [3][z][H][H], blockIdx.z sums its n / z
+// samples in chunks of 128.  8 warps: the loads and the stores take most of a
+// CTA's 8 us; two warps per 32 rows of the accumulator.
+struct WgradArgs {
+  const __nv_bfloat16 *A[3], *B[3];  // [H][n]
+  float* C;
+  int n;
+  unsigned* err;
+};
+constexpr int GS_BAR = 2 * TILE_BYTES, GS_SLOT = GS_BAR + 8, GS_OK = GS_SLOT + 4, GEMM_SMEM = GS_OK + 4 + 1024;
 constexpr int GEMM_THREADS = 256;
-template <int EPI, int BN>
-__global__ void __launch_bounds__(GEMM_THREADS) k_gemm(GemmArgs g) {
-  static_assert(BN == 128 || BN == 64, "the tile widths of the epilogue and the TMEM allocation");
+__global__ void __launch_bounds__(GEMM_THREADS) k_wgrad(WgradArgs g) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* base = smem_raw + ((1024u - (umma::smem_u32(smem_raw) & 1023u)) & 1023u);
   const uint32_t sA = umma::smem_u32(base), sB = sA + TILE_BYTES;
@@ -443,18 +557,17 @@ __global__ void __launch_bounds__(GEMM_THREADS) k_gemm(GemmArgs g) {
   uint32_t* slot = reinterpret_cast<uint32_t*>(base + GS_SLOT);
   int* s_ok = reinterpret_cast<int*>(base + GS_OK);
   const int t = threadIdx.x, warp = t >> 5;
-  const int m0 = blockIdx.y * 128, n0 = blockIdx.x * BN;
-  const int kper = g.K / gridDim.z, kb = blockIdx.z * kper;
+  const __nv_bfloat16 *A = g.A[blockIdx.x], *B = g.B[blockIdx.x];
+  const int kper = g.n / gridDim.z, kb = blockIdx.z * kper;
   if (t == 0) umma::mbar_init(bar, 1);
   if (warp == 0) {
-    umma::tmem_alloc(slot, BN);
+    umma::tmem_alloc(slot, 128);
     umma::tmem_relinquish();
   }
   umma::tc_fence_before();
   __syncthreads();
   umma::tc_fence_after();
   const uint32_t tmem = *slot;
-  pdl_wait();
   uint32_t phase = 0;
   bool ok = true;
   for (int k0 = kb; k0 < kb + kper; k0 += 128) {
@@ -462,8 +575,8 @@ __global__ void __launch_bounds__(GEMM_THREADS) k_gemm(GemmArgs g) {
     // flight at once, into the swizzled layout
     for (int q = t; q < 2048; q += GEMM_THREADS) {
       const int r = q >> 4, c = q & 15;
-      cp_async16(sA + umma::sw128_offset(r, c * 8, 128), g.A + (size_t)(m0 + r) * g.lda + k0 + c * 8);
-      if (r < BN) cp_async16(sB + umma::sw128_offset(r, c * 8, BN), g.B + (size_t)(n0 + r) * g.ldb + k0 + c * 8);
+      cp_async16(sA + umma::sw128_offset(r, c * 8, 128), A + (size_t)r * g.n + k0 + c * 8);
+      cp_async16(sB + umma::sw128_offset(r, c * 8, 128), B + (size_t)r * g.n + k0 + c * 8);
     }
     cp_async_wait_all();
     umma::fence_async_smem();
@@ -473,7 +586,7 @@ __global__ void __launch_bounds__(GEMM_THREADS) k_gemm(GemmArgs g) {
       umma::tc_fence_after();
 #pragma unroll
       for (int kk = 0; kk < 8; ++kk)
-        umma::mma_bf16(tmem, umma::sdesc_k(sA, 128, kk), umma::sdesc_k(sB, BN, kk), umma::idesc_bf16(128, BN),
+        umma::mma_bf16(tmem, umma::sdesc_k(sA, 128, kk), umma::sdesc_k(sB, 128, kk), umma::idesc_bf16(128, 128),
                        (k0 > kb || kk > 0) ? 1u : 0u);
       umma::mma_commit(bar);
       *s_ok = umma::mbar_wait(bar, phase) ? 1 : 0;
@@ -484,49 +597,14 @@ __global__ void __launch_bounds__(GEMM_THREADS) k_gemm(GemmArgs g) {
     if (!*s_ok) { ok = false; break; }
   }
   if (ok) {
-    // warps w and w + 4 read the same 32 rows, alternate blocks of 32 columns
-    const int quad = warp & 3, m = m0 + quad * 32 + (t & 31);
-    for (int c = warp >> 2; c < BN / 32; c += GEMM_THREADS / 128) {
+    const int quad = warp & 3, m = quad * 32 + (t & 31);
+    float* C = g.C + ((size_t)blockIdx.x * gridDim.z + blockIdx.z) * H * H + (size_t)m * H;
+    for (int c = warp >> 2; c < H / 32; c += GEMM_THREADS / 128) {
       float v[32];
       umma::tmem_ld32(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(c * 32), v);
-      const int nc = n0 + c * 32;
-      if (EPI == EPI_F32) {
-        float* dst = g.C + (size_t)blockIdx.z * g.M * g.N + (size_t)m * g.N + nc;
 #pragma unroll
-        for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(dst + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
-      } else {
-        float o[32];
-        if (EPI == EPI_FWD) {
-          float4* hd = reinterpret_cast<float4*>(g.Hout + (size_t)m * g.N + nc);
-          const float4* bz = reinterpret_cast<const float4*>(g.bias + nc);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const float4 b4 = bz[j];
-            const float4 h = make_float4(v[4 * j] + b4.x, v[4 * j + 1] + b4.y, v[4 * j + 2] + b4.z,
-                                         v[4 * j + 3] + b4.w);
-            hd[j] = h;
-            o[4 * j] = gelu(h.x);
-            o[4 * j + 1] = gelu(h.y);
-            o[4 * j + 2] = gelu(h.z);
-            o[4 * j + 3] = gelu(h.w);
-          }
-        } else {
-          const float4* hs = reinterpret_cast<const float4*>(g.Hin + (size_t)m * g.N + nc);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            const float4 h = hs[j];
-            o[4 * j] = v[4 * j] * gelu_d(h.x);
-            o[4 * j + 1] = v[4 * j + 1] * gelu_d(h.y);
-            o[4 * j + 2] = v[4 * j + 2] * gelu_d(h.z);
-            o[4 * j + 3] = v[4 * j + 3] * gelu_d(h.w);
-          }
-        }
-        uint4* rd = reinterpret_cast<uint4*>(g.Orow + (size_t)m * g.N + nc);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) rd[j] = pack8(o + 8 * j);
-#pragma unroll
-        for (int j = 0; j < 32; ++j) g.Ocol[(size_t)(nc + j) * g.M + m] = __float2bfloat16_rn(o[j]);
-      }
+      for (int j = 0; j < 32; j += 4)
+        *reinterpret_cast<float4*>(C + c * 32 + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
     }
   } else if (t == 0) {
     atomicOr(g.err, ERR_SYNC);
@@ -535,7 +613,7 @@ __global__ void __launch_bounds__(GEMM_THREADS) k_gemm(GemmArgs g) {
   __syncthreads();
   if (warp == 0) {
     umma::tc_fence_after();
-    umma::tmem_dealloc(tmem, BN);
+    umma::tmem_dealloc(tmem, 128);
   }
 }
 
@@ -793,8 +871,8 @@ __device__ __forceinline__ void pack_hidden(const Adam& ad, int q, float v) {
 // step is a chain of small kernels.  It ended with six, reduction, loss, schedule,
 // Adam and two packings, and began with the draw: now the draw is in layer 0,
 // the loss and schedule run beside the backward pass, the inference kernel's weights
-// are packed after the last step.  With the programmatic launches and the GEMMs'
-// wider epilogue, 8,192 samples: 92 -> 77 us a step.)
+// are packed after the last step.  With the programmatic launches,
+// 8,192 samples: 92 -> 77 us a step.)
 // Bound by the latency of the partials' loads: a block takes RED_H hidden
 // parameters, one per thread, or RED_THIN thin ones, whose up to SMALL_ZMAX
 // partials the whole block fetches to shared memory, 128 at a time.
@@ -976,11 +1054,11 @@ struct rc_mlp {
   std::vector<void*> work;
   float *xn = nullptr, *Hs[4] = {}, *dy = nullptr, *loss_part = nullptr, *loss = nullptr, *part = nullptr;
   float* spart = nullptr;                                // k_small_part's partials
-  cudaStream_t side = nullptr;                           // the weight-gradient branch
-  cudaEvent_t ev_dh[4] = {}, ev_join = nullptr;          // dH_l ready / the branch done
+  cudaStream_t side = nullptr;                           // the branch of the loss and the thin parameters
+  cudaEvent_t ev_head = nullptr, ev_dh = nullptr, ev_join = nullptr;  // the head, dH_0 .. / the branch done
   float *tb = nullptr, *sched = nullptr;                 // rc_mlp_train: the batch's targets, the step's schedule
   int* it = nullptr;                                     // rc_mlp_train: the step counter
-  __nv_bfloat16 *Arow[3] = {}, *Acol[3] = {}, *dHrow[4] = {}, *dHcol[4] = {};
+  __nv_bfloat16 *Arow = nullptr, *Acol[3] = {}, *dHrow[4] = {}, *dHcol[4] = {};  // dHcol[0] is not needed
   std::string err;
 };
 
@@ -1029,13 +1107,11 @@ int ensure_work(rc_mlp* m, int n) {
   st |= alloc_work(m, N * mlp::NIN, &m->xn);
   for (int l = 0; l < 4; ++l) st |= alloc_work(m, N * Hh, &m->Hs[l]);
   for (int l = 0; l < 3; ++l) {
-    st |= alloc_work(m, N * Hh, &m->Arow[l]);
     st |= alloc_work(m, N * Hh, &m->Acol[l]);
+    st |= alloc_work(m, N * Hh, &m->dHcol[l + 1]);
   }
-  for (int l = 0; l < 4; ++l) {
-    st |= alloc_work(m, N * Hh, &m->dHrow[l]);
-    st |= alloc_work(m, N * Hh, &m->dHcol[l]);
-  }
+  st |= alloc_work(m, N * Hh, &m->Arow);
+  for (int l = 0; l < 4; ++l) st |= alloc_work(m, N * Hh, &m->dHrow[l]);
   st |= alloc_work(m, N * mlp::NOUT, &m->dy);
   st |= alloc_work(m, (N + mlp::HEAD_SAMPLES - 1) / mlp::HEAD_SAMPLES, &m->loss_part);
   st |= alloc_work(m, (size_t)1, &m->loss);
@@ -1099,9 +1175,8 @@ int rc_mlp_create(int device, rc_mlp** out) {
   cudaMemset(m->m2, 0, P * sizeof(float));
   cudaMemset(m->derr, 0, sizeof(unsigned));
   if (cudaStreamCreateWithFlags(&m->side, cudaStreamNonBlocking) != cudaSuccess) return bail(RC_ERR_CUDA);
-  for (auto& e : m->ev_dh)
-    if (cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess) return bail(RC_ERR_CUDA);
-  if (cudaEventCreateWithFlags(&m->ev_join, cudaEventDisableTiming) != cudaSuccess) return bail(RC_ERR_CUDA);
+  for (cudaEvent_t* e : {&m->ev_head, &m->ev_dh, &m->ev_join})
+    if (cudaEventCreateWithFlags(e, cudaEventDisableTiming) != cudaSuccess) return bail(RC_ERR_CUDA);
   // the fills run on the legacy stream; the network's kernels may run on
   // non-blocking streams, which are not ordered after it
   if (cudaDeviceSynchronize() != cudaSuccess) return bail(RC_ERR_CUDA);
@@ -1110,12 +1185,11 @@ int rc_mlp_create(int device, rc_mlp** out) {
   for (int i = 0; i < 6; ++i) m->norm.dom[i] = dom[i];
   if (cudaFuncSetAttribute(mlp::k_mlp_fwd16<mlp::IoRaw>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            mlp::F2_SMEM) != cudaSuccess ||
-      cudaFuncSetAttribute(mlp::k_gemm<mlp::EPI_FWD, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, mlp::GEMM_SMEM) !=
+      cudaFuncSetAttribute(mlp::k_chain<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, mlp::CHAIN_SMEM) !=
           cudaSuccess ||
-      cudaFuncSetAttribute(mlp::k_gemm<mlp::EPI_BWD, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, mlp::GEMM_SMEM) !=
+      cudaFuncSetAttribute(mlp::k_chain<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, mlp::CHAIN_SMEM) !=
           cudaSuccess ||
-      cudaFuncSetAttribute(mlp::k_gemm<mlp::EPI_F32, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, mlp::GEMM_SMEM) !=
-          cudaSuccess ||
+      cudaFuncSetAttribute(mlp::k_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, mlp::GEMM_SMEM) != cudaSuccess ||
       cudaFuncSetAttribute(mlp::k_small_part, cudaFuncAttributeMaxDynamicSharedMemorySize, mlp::SMALL_SMEM) !=
           cudaSuccess)
     return bail(RC_ERR_CUDA);
@@ -1128,9 +1202,8 @@ int rc_mlp_destroy(rc_mlp* m) {
   for (void* p : m->work) cudaFree(p);
   cudaFree(m->params); cudaFree(m->m1); cudaFree(m->m2);
   cudaFree(m->Wb); cudaFree(m->WbT); cudaFree(m->Wh); cudaFree(m->derr);
-  for (cudaEvent_t e : m->ev_dh)
+  for (cudaEvent_t e : {m->ev_head, m->ev_dh, m->ev_join})
     if (e) cudaEventDestroy(e);
-  if (m->ev_join) cudaEventDestroy(m->ev_join);
   if (m->side) cudaStreamDestroy(m->side);
   delete m;
   return RC_OK;
@@ -1197,8 +1270,8 @@ struct GradEnd {
 // are drawn from its set.  The kernels of the chain layer 0 .. dH0 are launched
 // programmatically: a launch is prepared before its predecessor ends.  (A
 // trigger at the start of each kernel, which lets the next one's blocks take
-// their shared memory and wait there, costs more than it gives: 94 us a step
-// against 80 without it and 84 with plain launches.)
+// their shared memory and wait there, costs more than it gives: with a launch per
+// layer 94 us a step against 80 without it and 84 with plain launches.)
 int enqueue_gradient(rc_mlp* m, const float* d_x, const float* d_t, const mlp::Draw* draw, int n, const GradEnd& end,
                      cudaStream_t s) {
   using namespace mlp;
@@ -1224,66 +1297,47 @@ int enqueue_gradient(rc_mlp* m, const float* d_x, const float* d_t, const mlp::D
   // most SMALL_ZMAX chunks (n is a multiple of 128, so every chunk is whole tiles)
   const int chunk = 64 * ((n + 64 * SMALL_ZMAX - 1) / (64 * SMALL_ZMAX)), zs = (n + chunk - 1) / chunk;
   if (draw)
-    k_layer0<true><<<(n + 31) / 32, L0_THREADS, 0, s>>>(d_x, *draw, m->norm, m->params, n, m->xn, m->Hs[0], m->Arow[0],
+    k_layer0<true><<<(n + 31) / 32, L0_THREADS, 0, s>>>(d_x, *draw, m->norm, m->params, n, m->xn, m->Hs[0], m->Arow,
                                                         m->Acol[0]);
   else
     k_layer0<false><<<(n + 31) / 32, L0_THREADS, 0, s>>>(d_x, Draw{}, m->norm, m->params, n, m->xn, m->Hs[0],
-                                                         m->Arow[0], m->Acol[0]);
-  // hidden layers 1..3 forward: H_l = A_{l-1} W_l^T + b_l
-  for (int l = 1; l <= 3; ++l) {
-    GemmArgs g{};
-    g.A = m->Arow[l - 1]; g.lda = H;
-    g.B = m->Wb + (size_t)(l - 1) * H * H; g.ldb = H;
-    g.M = n; g.N = H; g.K = H;
-    g.bias = m->params + off_b(l);
-    g.Hout = m->Hs[l];
-    g.Orow = l < 3 ? m->Arow[l] : m->dHrow[3];   // A3 row is not needed (the head recomputes it)
-    g.Ocol = l < 3 ? m->Acol[l] : m->dHcol[3];   // scratch for l = 3, overwritten by the head
-    g.err = m->derr;
-    MLP_CU(pdl(k_gemm<EPI_FWD, 64>, dim3(H / 64, n / 128, 1), GEMM_THREADS, GEMM_SMEM, g));
+                                                         m->Arow, m->Acol[0]);
+  ChainArgs fw{}, bw{};
+  fw.A = m->Arow;
+  bw.A = m->dHrow[3];
+  for (int k = 0; k < 3; ++k) {  // forward layer k + 1, backward layer 3 - k
+    fw.W[k] = m->Wb + (size_t)k * H * H;
+    fw.bias[k] = m->params + off_b(k + 1);
+    fw.Hout[k] = m->Hs[k + 1];
+    fw.Ocol[k] = k < 2 ? m->Acol[k + 1] : nullptr;  // A3: the head recomputes it
+    bw.W[k] = m->WbT + (size_t)(2 - k) * H * H;
+    bw.Hin[k] = m->Hs[2 - k];
+    bw.Orow[k] = m->dHrow[2 - k];
+    bw.Ocol[k] = k < 2 ? m->dHcol[2 - k] : nullptr;
   }
+  fw.M = bw.M = n;
+  fw.err = bw.err = m->derr;
+  MLP_CU(pdl(k_chain<true>, dim3(n / 128), CHAIN_THREADS, CHAIN_SMEM, fw));
   const int nb = (n + HEAD_SAMPLES - 1) / HEAD_SAMPLES;
   MLP_CU(pdl(k_head, dim3(nb), HEAD_THREADS, 0, (const float*)m->Hs[3], d_t, (const float*)m->params, n, m->dy,
              m->dHrow[3], m->dHcol[3], m->loss_part));
-  // backward data: dH_{l-1} = (dH_l W_l) * gelu'(H_{l-1}) on s; each weight
-  // gradient dW_l = dH_l^T A_{l-1} (split-K partials) on the side stream as
-  // soon as dH_l is ready, then the thin parameters' partials; s joins the
-  // side stream before the reduction
-  auto wgrad = [&](int l) {
-    GemmArgs g{};
-    g.A = m->dHcol[l]; g.lda = n;
-    g.B = m->Acol[l - 1]; g.ldb = n;
-    g.M = H; g.N = H; g.K = n;
-    g.C = m->part + (size_t)(l - 1) * z * H * H;
-    g.err = m->derr;
-    k_gemm<EPI_F32, 128><<<dim3(1, 1, z), GEMM_THREADS, GEMM_SMEM, m->side>>>(g);
-  };
-  MLP_CU(cudaEventRecord(m->ev_dh[3], s));
-  MLP_CU(cudaStreamWaitEvent(m->side, m->ev_dh[3], 0));
-  wgrad(3);
-  for (int l = 3; l >= 1; --l) {
-    GemmArgs g{};
-    g.A = m->dHrow[l]; g.lda = H;
-    g.B = m->WbT + (size_t)(l - 1) * H * H; g.ldb = H;
-    g.M = n; g.N = H; g.K = H;
-    g.Hin = m->Hs[l - 1];
-    g.Orow = m->dHrow[l - 1];
-    g.Ocol = m->dHcol[l - 1];
-    g.err = m->derr;
-    MLP_CU(pdl(k_gemm<EPI_BWD, 64>, dim3(H / 64, n / 128, 1), GEMM_THREADS, GEMM_SMEM, g));
-    MLP_CU(cudaEventRecord(m->ev_dh[l - 1], s));
-    MLP_CU(cudaStreamWaitEvent(m->side, m->ev_dh[l - 1], 0));
-    if (l > 1) wgrad(l - 1);
-  }
+  // the loss and the schedule on the side stream beside the backward chain,
+  // then the thin parameters' partials there beside the weight gradients
+  MLP_CU(cudaEventRecord(m->ev_head, s));
+  MLP_CU(cudaStreamWaitEvent(m->side, m->ev_head, 0));
+  if (end.steps > 0)
+    k_train_tail<<<1, 32, 0, m->side>>>(m->it, end.steps, m->step, end.lr, end.lr_end, end.ad.b1, end.ad.b2,
+                                        m->loss_part, nb, n, m->loss, end.hist, m->sched);
+  else
+    k_loss_final<<<1, 32, 0, m->side>>>(m->loss_part, nb, n, m->loss);
+  MLP_CU(pdl(k_chain<false>, dim3(n / 128), CHAIN_THREADS, CHAIN_SMEM, bw));
+  MLP_CU(cudaEventRecord(m->ev_dh, s));
+  MLP_CU(cudaStreamWaitEvent(m->side, m->ev_dh, 0));
   k_small_part<<<zs, H, SMALL_SMEM, m->side>>>(m->xn, m->dHrow[0], m->dHrow[1], m->dHrow[2], m->dHrow[3], m->Hs[3],
                                               m->dy, n, chunk, m->spart);
   MLP_CU(cudaEventRecord(m->ev_join, m->side));
-  // beside the side stream's last kernels
-  if (end.steps > 0)
-    k_train_tail<<<1, 32, 0, s>>>(m->it, end.steps, m->step, end.lr, end.lr_end, end.ad.b1, end.ad.b2, m->loss_part, nb,
-                                  n, m->loss, end.hist, m->sched);
-  else
-    k_loss_final<<<1, 32, 0, s>>>(m->loss_part, nb, n, m->loss);
+  WgradArgs wg{{m->dHcol[1], m->dHcol[2], m->dHcol[3]}, {m->Acol[0], m->Acol[1], m->Acol[2]}, m->part, n, m->derr};
+  k_wgrad<<<dim3(3, 1, z), GEMM_THREADS, GEMM_SMEM, s>>>(wg);
   MLP_CU(cudaStreamWaitEvent(s, m->ev_join, 0));
   const auto reduce = end.steps > 0 ? k_reduce_grads<true> : k_reduce_grads<false>;
   reduce<<<RED_BLOCKS, RED_THREADS, 0, s>>>(m->part, z, m->spart, zs, end.grad, end.ad);
