@@ -419,8 +419,9 @@ __device__ __forceinline__ void cp_async_wait_all() {
 // (dH_{l-1} = (dH_l W_l) GELU'(H_{l-1})): a tile's layers depend on each other
 // only, so its activations stay in shared memory and the three weight tiles are
 // copied in at the start.  A launch per layer, two CTAs a tile, took 7.8-8.2 us
-// each, most of it launch, loads and stores: a step of 8,192 samples 77 -> 69 us,
-// with the weight gradients in one launch.  16 warps: warp w finishes rows
+// each, most of it launch, loads and stores: a step of 8,192 samples 77 -> 61 us,
+// with the weight gradients in one launch (69 with a row of 16-byte accesses per
+// thread to the pre-activations and results).  16 warps: warp w finishes rows
 // 32 (w % 4) .., columns 32 (w / 4) ...
 struct ChainArgs {
   const __nv_bfloat16* A;      // [M][H] of the first layer
@@ -428,13 +429,17 @@ struct ChainArgs {
   const float* bias[3];        // forward
   const float* Hin[3];         // backward: pre-activations [M][H]
   float* Hout[3];              // forward: pre-activations [M][H]
-  __nv_bfloat16* Orow[3];      // results [M][H] (null: not needed in memory)
+  __nv_bfloat16* Orow[3];      // backward: results [M][H]
   __nv_bfloat16* Ocol[3];      // results [H][M] (null: not needed)
   int M;                       // a multiple of 128
   unsigned* err;
 };
 constexpr int CHAIN_THREADS = 512;
-constexpr int CS_BAR = 4 * TILE_BYTES, CS_SLOT = CS_BAR + 8, CS_OK = CS_SLOT + 4, CHAIN_SMEM = CS_OK + 4 + 1024;
+// per warp a 32 x 32 block of pre-activations, rows padded to 36 floats: a thread
+// has a row, but memory takes eight lanes per row (32 rows in one access are
+// 32 lines)
+constexpr int CHAIN_PAD = 36, CS_STAGE = 4 * TILE_BYTES;
+constexpr int CS_BAR = CS_STAGE + CHAIN_THREADS * CHAIN_PAD * 4, CS_SLOT = CS_BAR + 8, CS_OK = CS_SLOT + 4, CHAIN_SMEM = CS_OK + 4 + 1024;
 static_assert(H == 128, "one tile per layer");
 template <bool FWD>
 __global__ void __launch_bounds__(CHAIN_THREADS) k_chain(ChainArgs g) {
@@ -445,7 +450,10 @@ __global__ void __launch_bounds__(CHAIN_THREADS) k_chain(ChainArgs g) {
   uint32_t* slot = reinterpret_cast<uint32_t*>(base + CS_SLOT);
   int* s_ok = reinterpret_cast<int*>(base + CS_OK);
   const int t = threadIdx.x, warp = t >> 5, m0 = blockIdx.x * 128;
-  const int row = (warp & 3) * 32 + (t & 31), col = (warp >> 2) * 32, m = m0 + row;
+  const int lane = t & 31, row0 = (warp & 3) * 32, row = row0 + lane, col = (warp >> 2) * 32, m = m0 + row;
+  float* stage = reinterpret_cast<float*>(base + CS_STAGE) + warp * 32 * CHAIN_PAD;
+  // this lane's 16 bytes of access j to a block of rows: row r8 + 4 j, floats c4 ..
+  const int r8 = lane >> 3, c4 = 4 * (lane & 7);
   if (t == 0) umma::mbar_init(bar, 1);
   if (warp == 0) {
     umma::tmem_alloc(slot, 128);
@@ -467,6 +475,15 @@ __global__ void __launch_bounds__(CHAIN_THREADS) k_chain(ChainArgs g) {
     cp_async16(sA + umma::sw128_offset(r, c * 8, 128), g.A + (size_t)(m0 + r) * H + c * 8);
   }
   cp_async_wait_all();
+  // the result in the tile to memory, rows of 256 bytes
+  auto result = [&](__nv_bfloat16* out) {
+#pragma unroll
+    for (int q = t; q < 2048; q += CHAIN_THREADS) {
+      const int r = q >> 4, c = q & 15;
+      *reinterpret_cast<uint4*>(out + (size_t)(m0 + r) * H + c * 8) =
+          *reinterpret_cast<const uint4*>(base + umma::sw128_offset(r, c * 8, 128));
+    }
+  };
   uint32_t phase = 0;
   bool ok = true;
 #pragma unroll 1
@@ -484,12 +501,17 @@ __global__ void __launch_bounds__(CHAIN_THREADS) k_chain(ChainArgs g) {
       umma::mma_commit(bar);
       *s_ok = umma::mbar_wait(bar, phase) ? 1 : 0;
     }
-    // the epilogue's other operand arrives beside the MMAs
+    // beside the MMAs: the epilogue's other operand, and the result before to memory
     float4 h[8];
-    const float4* hs = FWD ? reinterpret_cast<const float4*>(g.bias[l] + col)
-                           : reinterpret_cast<const float4*>(g.Hin[l] + (size_t)m * H + col);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) h[j] = hs[j];
+    for (int j = 0; j < 8; ++j)
+      h[j] = *reinterpret_cast<const float4*>(FWD ? g.bias[l] + col + 4 * j
+                                                  : g.Hin[l] + (size_t)(m0 + row0 + r8 + 4 * j) * H + col + c4);
+    if (!FWD) {
+      if (l > 0) result(g.Orow[l - 1]);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) *reinterpret_cast<float4*>(stage + (r8 + 4 * j) * CHAIN_PAD + c4) = h[j];
+    }
     __syncthreads();
     phase ^= 1u;
     umma::tc_fence_after();
@@ -497,33 +519,36 @@ __global__ void __launch_bounds__(CHAIN_THREADS) k_chain(ChainArgs g) {
     float v[32], o[32];
     umma::tmem_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)col, v);
     if (FWD) {
-      float4* hd = reinterpret_cast<float4*>(g.Hout[l] + (size_t)m * H + col);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const float4 x = make_float4(v[4 * j] + h[j].x, v[4 * j + 1] + h[j].y, v[4 * j + 2] + h[j].z,
                                      v[4 * j + 3] + h[j].w);
-        hd[j] = x;
+        *reinterpret_cast<float4*>(stage + lane * CHAIN_PAD + 4 * j) = x;
         o[4 * j] = gelu(x.x);
         o[4 * j + 1] = gelu(x.y);
         o[4 * j + 2] = gelu(x.z);
         o[4 * j + 3] = gelu(x.w);
       }
+      __syncwarp();
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        *reinterpret_cast<float4*>(g.Hout[l] + (size_t)(m0 + row0 + r8 + 4 * j) * H + col + c4) =
+            *reinterpret_cast<const float4*>(stage + (r8 + 4 * j) * CHAIN_PAD + c4);
     } else {
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        o[4 * j] = v[4 * j] * gelu_d(h[j].x);
-        o[4 * j + 1] = v[4 * j + 1] * gelu_d(h[j].y);
-        o[4 * j + 2] = v[4 * j + 2] * gelu_d(h[j].z);
-        o[4 * j + 3] = v[4 * j + 3] * gelu_d(h[j].w);
+        const float4 x = *reinterpret_cast<const float4*>(stage + lane * CHAIN_PAD + 4 * j);
+        o[4 * j] = v[4 * j] * gelu_d(x.x);
+        o[4 * j + 1] = v[4 * j + 1] * gelu_d(x.y);
+        o[4 * j + 2] = v[4 * j + 2] * gelu_d(x.z);
+        o[4 * j + 3] = v[4 * j + 3] * gelu_d(x.w);
       }
     }
+    // the MMAs have read the tile: it takes the result, the next layer's operand
+    if (!FWD || l < 2)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const uint4 x = pack8(o + 8 * j);
-      // the MMAs have read the tile: it takes the next layer's operand
-      if (l < 2) *reinterpret_cast<uint4*>(base + umma::sw128_offset(row, col + 8 * j, 128)) = x;
-      if (g.Orow[l]) reinterpret_cast<uint4*>(g.Orow[l] + (size_t)m * H + col)[j] = x;
-    }
+      for (int j = 0; j < 4; ++j)
+        *reinterpret_cast<uint4*>(base + umma::sw128_offset(row, col + 8 * j, 128)) = pack8(o + 8 * j);
     if (g.Ocol[l])
 #pragma unroll
       for (int j = 0; j < 32; ++j) g.Ocol[l][(size_t)(col + j) * g.M + m] = __float2bfloat16_rn(o[j]);
@@ -531,6 +556,7 @@ __global__ void __launch_bounds__(CHAIN_THREADS) k_chain(ChainArgs g) {
   if (!ok && t == 0) atomicOr(g.err, ERR_SYNC);
   umma::tc_fence_before();
   __syncthreads();
+  if (!FWD && ok) result(g.Orow[2]);
   if (warp == 0) {
     umma::tc_fence_after();
     umma::tmem_dealloc(tmem, 128);
