@@ -664,9 +664,12 @@ __global__ void __launch_bounds__(L0_THREADS) k_layer0(const float* __restrict__
                                                        const float* __restrict__ P, int n, float* xn, float* H0,
                                                        __nv_bfloat16* Arow, __nv_bfloat16* Acol) {
   __shared__ float sf[32][NIN + 1];
+  // the block's H0 and A0, rows padded: a thread has a row's 8 columns, memory takes whole rows
+  __shared__ __align__(16) float sh[32][H + 4];
+  __shared__ __align__(16) __nv_bfloat16 sa[32][H + 8];
   const int lane = threadIdx.x & 31, c8 = threadIdx.x >> 5;
   const int s = blockIdx.x * 32 + lane;
-  if (c8 == 0 && s < n) {
+  if (c8 == 0) {  // n is a multiple of 128: whole blocks
     long long row = s;
     if (DRAW) {
       unsigned long long z = dr.seed + 0x9E3779B97F4A7C15ull * ((unsigned long long)*dr.it * (unsigned long long)n +
@@ -687,7 +690,6 @@ __global__ void __launch_bounds__(L0_THREADS) k_layer0(const float* __restrict__
     }
   }
   __syncthreads();
-  if (s >= n) return;
   float f[NIN];
 #pragma unroll
   for (int i = 0; i < NIN; ++i) f[i] = sf[lane][i];
@@ -701,10 +703,20 @@ __global__ void __launch_bounds__(L0_THREADS) k_layer0(const float* __restrict__
     a[e] = gelu(h[e]);
     Acol[(size_t)o * n + s] = __float2bfloat16_rn(a[e]);
   }
-  float4* hd = reinterpret_cast<float4*>(H0 + (size_t)s * H + c8 * 8);
+  float4* hd = reinterpret_cast<float4*>(&sh[lane][c8 * 8]);
   hd[0] = make_float4(h[0], h[1], h[2], h[3]);
   hd[1] = make_float4(h[4], h[5], h[6], h[7]);
-  reinterpret_cast<uint4*>(Arow + (size_t)s * H)[c8] = pack8(a);
+  *reinterpret_cast<uint4*>(&sa[lane][c8 * 8]) = pack8(a);
+  __syncthreads();
+  const size_t s0 = (size_t)blockIdx.x * 32;
+#pragma unroll
+  for (int u = 0; u < 32 * H / 4 / L0_THREADS; ++u) {
+    const int q = u * L0_THREADS + threadIdx.x, r = q / (H / 4), c = q % (H / 4);
+    reinterpret_cast<float4*>(H0 + (s0 + r) * H)[c] = *reinterpret_cast<const float4*>(&sh[r][4 * c]);
+  }
+  static_assert(32 * H / 8 == L0_THREADS, "one 16-byte piece of A0 per thread");
+  const int r = threadIdx.x / (H / 8), c = threadIdx.x % (H / 8);
+  reinterpret_cast<uint4*>(Arow + (s0 + r) * H)[c] = *reinterpret_cast<const uint4*>(&sa[r][8 * c]);
 }
 
 // output layer, loss and its gradient down to dH3: y = W4 gelu(H3) + b4,
@@ -717,14 +729,25 @@ __global__ void __launch_bounds__(HEAD_THREADS) k_head(const float* __restrict__
                                                        const float* __restrict__ P, int n, float* dy,
                                                        __nv_bfloat16* dHrow, __nv_bfloat16* dHcol, float* loss_part) {
   __shared__ float red[HEAD_THREADS];
+  // the block's H3 (rows of four quarters of 36 floats) and dH3 (rows of 136):
+  // a thread has a quarter of a row, memory takes whole rows and columns
+  constexpr int QP = 36, RP = 4 * QP, DP = H + 8;
+  __shared__ __align__(16) float sh[HEAD_SAMPLES * RP];
+  __shared__ __align__(16) __nv_bfloat16 sd[HEAD_SAMPLES * DP];
   pdl_wait();
-  const int qd = threadIdx.x & 3, s = blockIdx.x * HEAD_SAMPLES + (threadIdx.x >> 2);
-  const bool valid = s < n;
-  const int sc_ = valid ? s : 0;
+  const int t = threadIdx.x, qd = t & 3, sl = t >> 2, s0 = blockIdx.x * HEAD_SAMPLES, s = s0 + sl;
+  // n is a multiple of 128: whole blocks
+#pragma unroll
+  for (int u = 0; u < HEAD_SAMPLES * H / 4 / HEAD_THREADS; ++u) {
+    const int q = u * HEAD_THREADS + t, r = q / (H / 4), c = q % (H / 4);
+    *reinterpret_cast<float4*>(sh + r * RP + (c >> 3) * QP + (c & 7) * 4) =
+        reinterpret_cast<const float4*>(H3 + (size_t)(s0 + r) * H)[c];
+  }
+  __syncthreads();
   float h[32];
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
-    const float4 v = reinterpret_cast<const float4*>(H3 + (size_t)sc_ * H + qd * 32)[j];
+    const float4 v = *reinterpret_cast<const float4*>(sh + sl * RP + qd * QP + 4 * j);
     h[4 * j] = v.x;
     h[4 * j + 1] = v.y;
     h[4 * j + 2] = v.z;
@@ -749,26 +772,35 @@ __global__ void __launch_bounds__(HEAD_THREADS) k_head(const float* __restrict__
   const float sc = 2.f / (4.f * (float)n);
 #pragma unroll
   for (int m = 0; m < NOUT; ++m) {
-    const float e = valid ? y[m] + P[OFF_B4 + m] - tgt[(size_t)s * NOUT + m] : 0.f;
+    const float e = y[m] + P[OFF_B4 + m] - tgt[(size_t)s * NOUT + m];
     l2 = fmaf(e, e, l2);
     g[m] = sc * e;
-    if (valid && qd == 0) dy[(size_t)s * NOUT + m] = g[m];
+    if (qd == 0) dy[(size_t)s * NOUT + m] = g[m];
   }
-  if (valid) {
 #pragma unroll
-    for (int c8 = 0; c8 < 4; ++c8) {
-      float o[8];
+  for (int c8 = 0; c8 < 4; ++c8) {
+    float o[8];
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const int i = qd * 32 + c8 * 8 + e;
-        float da = 0.f;
+    for (int e = 0; e < 8; ++e) {
+      const int i = qd * 32 + c8 * 8 + e;
+      float da = 0.f;
 #pragma unroll
-        for (int m = 0; m < NOUT; ++m) da = fmaf(P[OFF_W4 + m * H + i], g[m], da);
-        o[e] = da * gelu_d(h[c8 * 8 + e]);
-        dHcol[(size_t)i * n + s] = __float2bfloat16_rn(o[e]);
-      }
-      reinterpret_cast<uint4*>(dHrow + (size_t)s * H + qd * 32)[c8] = pack8(o);
+      for (int m = 0; m < NOUT; ++m) da = fmaf(P[OFF_W4 + m * H + i], g[m], da);
+      o[e] = da * gelu_d(h[c8 * 8 + e]);
     }
+    *reinterpret_cast<uint4*>(sd + sl * DP + qd * 32 + c8 * 8) = pack8(o);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < HEAD_SAMPLES * H / 8 / HEAD_THREADS; ++u) {
+    const int q = u * HEAD_THREADS + t, r = q / (H / 8), c = q % (H / 8);
+    reinterpret_cast<uint4*>(dHrow + (size_t)(s0 + r) * H)[c] = *reinterpret_cast<const uint4*>(sd + r * DP + 8 * c);
+  }
+  static_assert(HEAD_SAMPLES == 32 && HEAD_THREADS == H, "a warp has 32 columns of 32 samples");
+#pragma unroll 8
+  for (int i = 0; i < 32; ++i) {
+    const int o = (t & ~31) + i;
+    dHcol[(size_t)o * n + s0 + (t & 31)] = sd[(t & 31) * DP + o];
   }
   red[threadIdx.x] = qd == 0 ? l2 : 0.f;
   __syncthreads();
