@@ -1365,7 +1365,7 @@ __device__ __forceinline__ void flowc_step(const Dev& d, const ThermoDev<NSP>& t
 //    and from the block's passes up to k - 1 - FLOWC_BACK (nb); those of the
 //    block's last FLOWC_BACK passes it reads from shared memory, where their
 //    finishing lanes put them.  s_ready[slot] = k + 1 marks pass k prepared;
-//  - the starting warp: arrives on pass k's start barrier (3 or 13, by k's
+//  - the starting warp (rc_flowc.cuh): arrives on pass k's start barrier (3 or 13, by k's
 //    parity) once the pass is prepared, which the compute warps reach when they
 //    are done with pass k - 1, and marks passes done (s_done) at their end
 //    barriers (4 or 14);
@@ -1409,20 +1409,7 @@ __global__ void __launch_bounds__(flowc_threads(G), 1) k_lusgs_flowc(const Dev d
   const int nf = f.boff[0][b + 1] - f0, n = nf + (f.boff[1][b + 1] - b0);
   // the block's k-th pass in the tables
   auto at = [&](int k) { return k < nf ? f0 + k : f.nfwd + b0 + k - nf; };
-  auto give_up = [&]() {
-    if (lane == 0) {
-      s_bad = 1;
-      atomicOr(d.err, ERR_SYNC);
-    }
-    __syncwarp();
-  };
-  // wait until passes 0 .. k are done; false after a give-up
-  auto done = [&](int k) {
-    for (unsigned spin = 0; s_done <= k && !s_bad; ++spin)
-      if (spin >= d.spin_limit) give_up();
-    __threadfence_block();
-    return !s_bad;
-  };
+  FlowWarp<FlowLane> w = {{{lane, d.err}, &s_bad, d.spin_limit}, &s_done, s_ready, s_go, FLOWC_NBUF};
   if (warp < CW) {
     const int gi = G > 1 ? warp >> 3 : 0, role = warp & 7;
     for (int k = 0; k < n; ++k) {
@@ -1437,42 +1424,16 @@ __global__ void __launch_bounds__(flowc_threads(G), 1) k_lusgs_flowc(const Dev d
       bar_arrive(4 + 10 * (k & 1), T34);
     }
   } else if (warp == CW) {
-    // the starting warp: pass k is started as soon as it is prepared, before
-    // the end of pass k - 1 where that comes later
-    auto start = [&](int k) {
-      if (lane == 0) s_go[k & 1] = s_bad ? 0 : 1;
-      __syncwarp();
-      __threadfence_block();
-      bar_arrive(3 + 10 * (k & 1), T34);
-    };
-    for (int k = 0; k < n; ++k) {
-      const bool early = s_ready[k % FLOWC_NBUF] == k + 1;
-      if (early) start(k);
-      if (k > 0) {
-        bar_named(4 + 10 * ((k - 1) & 1), T34);  // the end of pass k - 1
-        __threadfence_block();
-        if (lane == 0) s_done = k;  // passes 0 .. k - 1
-      }
-      if (!early) {
-        for (unsigned spin = 0; s_ready[k % FLOWC_NBUF] != k + 1 && !s_bad; ++spin)
-          if (spin >= d.spin_limit) give_up();
-        start(k);
-      }
-    }
-    if (n > 0) {
-      bar_named(4 + 10 * ((n - 1) & 1), T34);
-      __threadfence_block();
-      if (lane == 0) s_done = n;
-    }
+    w.start_passes(n, T34);
   } else if (warp <= CW + FLOWC_PUBS) {
     for (int k = warp - CW - 1; k < n; k += FLOWC_PUBS) {
       const int pz = f.prec[at(k)].z;
-      if (!done(k)) break;
+      if (!w.passes_done(k)) break;
       if (lane == 0) st_release(f.pflag + pz, epoch);
     }
   } else {
-    for (int k = warp - CW - 1 - FLOWC_PUBS; k < n && !s_bad; k += S) {
-      auto free = [&]() { return done(k - FLOWC_NBUF); };
+    for (int k = warp - CW - 1 - FLOWC_PUBS; k < n; k += S) {
+      auto free = [&]() { return w.passes_done(k - FLOWC_NBUF); };
       const int4 rec = f.prec[at(k)];
       const int2 dep = f.pdep[at(k)];
       int t = rec.x, e = rec.y, cnt = rec.w;
@@ -1491,9 +1452,8 @@ __global__ void __launch_bounds__(flowc_threads(G), 1) k_lusgs_flowc(const Dev d
       bool set = true;
       for (int u = lane; u < dep.y; u += 32)
         set = set && wait_flag(f.pflag + f.deps[dep.x + u], epoch, d.err, d.spin_limit);
-      if (__any_sync(0xffffffffu, !set)) give_up();
-      __syncwarp();
-      if (!done(k - 1 - FLOWC_BACK)) break;
+      if (__any_sync(0xffffffffu, !set)) w.give_up();
+      if (!w.passes_done(k - 1 - FLOWC_BACK)) break;
 #pragma unroll
       for (int g = 0; g < G; ++g) {
         Slot& s = slots[(k % FLOWC_NBUF) * G + g];
@@ -1506,10 +1466,7 @@ __global__ void __launch_bounds__(flowc_threads(G), 1) k_lusgs_flowc(const Dev d
           for (int v = 0; v < V; ++v) s.nb[v][lane] = x[v];
         }
       }
-      __syncwarp();
-      __threadfence_block();
-      if (lane == 0) s_ready[k % FLOWC_NBUF] = k + 1;
-      __syncwarp();
+      w.set_ready(k);
     }
   }
   __syncthreads();

@@ -3,6 +3,7 @@
 #include <cstdint>
 #include <utility>
 
+#include "rc_flowc.cuh"
 #include "rc_thermo.cuh"
 
 namespace rc {
@@ -207,6 +208,20 @@ __device__ __forceinline__ void bar_named(int id, int count) {
 __device__ __forceinline__ void bar_arrive(int id, int count) {
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory");
 }
+// A lane of the dataflow launches' waits (rc_flowc.cuh).
+struct FlowLane {
+  int lane;
+  unsigned* err;
+  __device__ __forceinline__ int load(const volatile int* p) const { return *p; }
+  __device__ __forceinline__ void store(volatile int* p, int v) const { *p = v; }
+  __device__ __forceinline__ int lane0(int x) const { return __shfl_sync(0xffffffffu, x, 0); }
+  __device__ __forceinline__ void sync() const { __syncwarp(); }
+  __device__ __forceinline__ void fence() const { __threadfence_block(); }
+  __device__ __forceinline__ void arrive(int id, int n) const { bar_arrive(id, n); }
+  __device__ __forceinline__ void meet(int id, int n) const { bar_named(id, n); }
+  __device__ __forceinline__ void latch() const { atomicOr(err, ERR_SYNC); }
+  __device__ __forceinline__ void nap() const { __nanosleep(256); }
+};
 // Work space of the integrator's rounds (rc_chem.cu): two lists of parked
 // reactors, [list][field][cap] each, and per round its queue counter and
 // the number it parked.

@@ -758,19 +758,11 @@ __global__ void __launch_bounds__(FLOW32_THREADS, 1) k_lusgs_flow32(const Dev d,
   const int f0 = f.boff[0][b], b0 = f.boff[1][b];
   const int nf = f.boff[0][b + 1] - f0, n = nf + (f.boff[1][b + 1] - b0);
   auto pass_of = [&](int k) { return k < nf ? f.blist[0][f0 + k] : f.blist[1][b0 + k - nf]; };
-  auto give_up = [&]() {
-    if (lane == 0) {
-      s_bad = 1;
-      atomicOr(d.err, ERR_SYNC);
-    }
-    __syncwarp();
-  };
+  WarpWait<FlowLane> w = {{lane, d.err}, &s_bad, d.spin_limit};
   if (warp == 1) {
-    for (int k = 0; k < n && !s_bad; ++k) {
+    for (int k = 0; k < n; ++k) {
       // pass k reuses the buffer of pass k - NBUF once warp 0 has taken it
-      for (unsigned spin = 0; s_consumed < k - FLOW32_NBUF + 1 && !s_bad; ++spin)
-        if (spin >= d.spin_limit) give_up();
-      if (s_bad) break;
+      if (!w.until(&s_consumed, k - FLOW32_NBUF + 1)) break;
       const int pz = pass_of(k), t0 = f.pstart[pz], t1 = t0 + f.pcount[pz];
       if (k < nf) s_pre[k % FLOW32_NBUF][lane] = sweep_load32<NSP, true>(d, t0 + (lane >> 2), t1, lane & 3);
       else s_pre[k % FLOW32_NBUF][lane] = sweep_load32<NSP, false>(d, t0 + (lane >> 2), t1, lane & 3);
@@ -780,21 +772,17 @@ __global__ void __launch_bounds__(FLOW32_THREADS, 1) k_lusgs_flow32(const Dev d,
       __syncwarp();
     }
   } else if (warp == 2) {
-    auto staged = [&](int k) {  // wait (bounded) until pass k is staged
-      for (unsigned spin = 0; s_staged <= k && !s_bad; ++spin)
-        if (spin >= d.spin_limit) give_up();
-      __threadfence_block();
-    };
+    auto staged = [&](int k) { w.until(&s_staged, k + 1); };  // wait (bounded) until pass k is staged
     auto poll = [&](int k) {
-      if (s_bad) return;
+      if (w.see(s_bad)) return;
       const int pz = pass_of(k), d0 = f.doff[pz], nd = f.doff[pz + 1] - d0;
       bool ok = true;
       for (int u = lane; u < nd; u += 32) ok = ok && wait_flag(f.pflag + f.deps[d0 + u], epoch, d.err, d.spin_limit);
-      if (__any_sync(0xffffffffu, !ok)) give_up();
+      if (__any_sync(0xffffffffu, !ok)) w.give_up();
     };
     auto ready = [&](int k) -> bool {
-      if (s_bad) return true;
-      if (s_staged <= k) return false;
+      const int s = w.see(s_bad ? 2 : s_staged > k ? 1 : 0);
+      if (s != 1) return s == 2;
       const int pz = pass_of(k), d0 = f.doff[pz], nd = f.doff[pz + 1] - d0;
       bool ok = true;
       for (int u = lane; u < nd; u += 32) ok = ok && ld_acquire(f.pflag + f.deps[d0 + u]) >= epoch;
@@ -824,7 +812,7 @@ __global__ void __launch_bounds__(FLOW32_THREADS, 1) k_lusgs_flow32(const Dev d,
       // after a give-up warp 2 still hands every pass over (the barrier
       // counts must match) but warp 1 has stopped staging: the buffer may
       // hold no pass at all, so nothing of it is read
-      if (s_bad) {
+      if (w.see(s_bad)) {
         bar_arrive(4, 64);
         continue;
       }
@@ -847,13 +835,8 @@ __global__ void __launch_bounds__(FLOW32_THREADS, 1) k_lusgs_flow32(const Dev d,
       // bounded wait for pass k; the polls are spaced out, as these warps
       // wait through the whole forward sweep and must not take issue slots
       // from warp 2 on their sub-partition
-      for (unsigned spin = 0; s_done <= k && !s_bad; ++spin) {
-        if (spin >= d.spin_limit) give_up();
-        __nanosleep(256);
-      }
-      if (s_bad) break;
-      __threadfence_block();
-      const int avail = s_done;
+      if (!w.until(&s_done, k + 1, true)) break;
+      const int avail = w.see(s_done);
       // lane l looks at this warp's pass k + 2l; the finished ones whose
       // cells fit in 32 lanes (a prefix of the lanes: at least pass k) are
       // taken, their sweep positions listed in order in cells[]
@@ -1039,20 +1022,7 @@ __global__ void __launch_bounds__(flowc32_threads(G), 1) k_lusgs_flowc32(const D
   const int nf = f.boff[0][b + 1] - f0, n = nf + (f.boff[1][b + 1] - b0);
   // the block's k-th pass in the tables
   auto at = [&](int k) { return k < nf ? f0 + k : f.nfwd + b0 + k - nf; };
-  auto give_up = [&]() {
-    if (lane == 0) {
-      s_bad = 1;
-      atomicOr(d.err, ERR_SYNC);
-    }
-    __syncwarp();
-  };
-  // wait until passes 0 .. k are done; false after a give-up
-  auto done = [&](int k) {
-    for (unsigned spin = 0; s_done <= k && !s_bad; ++spin)
-      if (spin >= d.spin_limit) give_up();
-    __threadfence_block();
-    return !s_bad;
-  };
+  FlowWarp<FlowLane> w = {{{lane, d.err}, &s_bad, d.spin_limit}, &s_done, s_ready, s_go, FLOWC32_NBUF};
   if (warp < CW) {
     const int gi = G > 1 ? warp >> 2 : 0, role = warp & 3, x = role * 32 + lane, fc = x / V, r = x - fc * V;
     float(*T)[32] = s_T[gi];
@@ -1092,42 +1062,16 @@ __global__ void __launch_bounds__(flowc32_threads(G), 1) k_lusgs_flowc32(const D
       bar_arrive(4 + 10 * (k & 1), T34);
     }
   } else if (warp == CW) {
-    // the starting warp: pass k is started as soon as it is prepared, before
-    // the end of pass k - 1 where that comes later
-    auto start = [&](int k) {
-      if (lane == 0) s_go[k & 1] = s_bad ? 0 : 1;
-      __syncwarp();
-      __threadfence_block();
-      bar_arrive(3 + 10 * (k & 1), T34);
-    };
-    for (int k = 0; k < n; ++k) {
-      const bool early = s_ready[k % FLOWC32_NBUF] == k + 1;
-      if (early) start(k);
-      if (k > 0) {
-        bar_named(4 + 10 * ((k - 1) & 1), T34);  // the end of pass k - 1
-        __threadfence_block();
-        if (lane == 0) s_done = k;  // passes 0 .. k - 1
-      }
-      if (!early) {
-        for (unsigned spin = 0; s_ready[k % FLOWC32_NBUF] != k + 1 && !s_bad; ++spin)
-          if (spin >= d.spin_limit) give_up();
-        start(k);
-      }
-    }
-    if (n > 0) {
-      bar_named(4 + 10 * ((n - 1) & 1), T34);
-      __threadfence_block();
-      if (lane == 0) s_done = n;
-    }
+    w.start_passes(n, T34);
   } else if (warp <= CW + FLOWC_PUBS) {
     for (int k = warp - CW - 1; k < n; k += FLOWC_PUBS) {
       const int pz = f.prec[at(k)].z;
-      if (!done(k)) break;
+      if (!w.passes_done(k)) break;
       if (lane == 0) st_release(f.pflag + pz, epoch);
     }
   } else if (warp <= CW + FLOWC_PUBS + S) {
-    for (int k = warp - CW - 1 - FLOWC_PUBS; k < n && !s_bad; k += S) {
-      auto free = [&]() { return done(k - FLOWC32_NBUF); };
+    for (int k = warp - CW - 1 - FLOWC_PUBS; k < n; k += S) {
+      auto free = [&]() { return w.passes_done(k - FLOWC32_NBUF); };
       const int4 rec = f.prec[at(k)];
       const int2 dep = f.pdep[at(k)];
       int t = rec.x, e = rec.y, cnt = rec.w;
@@ -1146,9 +1090,8 @@ __global__ void __launch_bounds__(flowc32_threads(G), 1) k_lusgs_flowc32(const D
       bool set = true;
       for (int u = lane; u < dep.y; u += 32)
         set = set && wait_flag(f.pflag + f.deps[dep.x + u], epoch, d.err, d.spin_limit);
-      if (__any_sync(0xffffffffu, !set)) give_up();
-      __syncwarp();
-      if (!done(k - 1 - FLOWC_BACK)) break;
+      if (__any_sync(0xffffffffu, !set)) w.give_up();
+      if (!w.passes_done(k - 1 - FLOWC_BACK)) break;
 #pragma unroll
       for (int g = 0; g < G; ++g) {
         Slot& s = slots[(k % FLOWC32_NBUF) * G + g];
@@ -1161,10 +1104,7 @@ __global__ void __launch_bounds__(flowc32_threads(G), 1) k_lusgs_flowc32(const D
           for (int v = 0; v < V; ++v) s.nb[v][lane] = y[v];
         }
       }
-      __syncwarp();
-      __threadfence_block();
-      if (lane == 0) s_ready[k % FLOWC32_NBUF] = k + 1;
-      __syncwarp();
+      w.set_ready(k);
     }
   } else {
     // the Newton update warps: update warp u takes the cells of
@@ -1176,18 +1116,13 @@ __global__ void __launch_bounds__(flowc32_threads(G), 1) k_lusgs_flowc32(const D
     int* cells = s_cells[u];
     unsigned err = 0;
     for (int k = nf + u, off = 0; k < n;) {
-      for (unsigned spin = 0; s_done <= k && !s_bad; ++spin) {
-        if (spin >= d.spin_limit) give_up();
-        __nanosleep(256);
-      }
-      if (s_bad) break;
-      __threadfence_block();
-      const int avail = s_done;
+      if (!w.until(&s_done, k + 1, true)) break;
+      const int avail = w.see(s_done);
       const int kl = k + UPD * lane;
       int cnt = 0, t0 = 0;
       if (kl < avail) {
         const int4 rec = f.prec[at(kl)];
-        for (int g = 0, w = rec.w; g < G; ++g, w >>= 16) cnt += w & 255;
+        for (int g = 0, x = rec.w; g < G; ++g, x >>= 16) cnt += x & 255;
         t0 = rec.x;
         if (lane == 0) {
           cnt -= off;
