@@ -180,13 +180,13 @@ int rc_lusgs_stage(rc_ctx* ctx, int istep); /* lu_sgs_stage   Time_LUSGS_steady.
  * No counterpart in the reference (it has a single FP64 path). */
 int rc_set_precision(rc_ctx* ctx, int precision);
 
-/* Polls after which a level wait of the persistent LU-SGS kernels gives up
- * (default 2^24): the kernel then latches RC_ERR_SYNC and returns, leaving the
- * context usable.  A small limit forces the timeout path (fault tests).  The
- * Newton-update warps of the mixed forms' dataflow launch wait through the
- * whole forward sweep with polls at least 256 ns apart and count them against
- * the same limit, so a limit set by hand must cover the forward sweep's
- * duration divided by 256 ns (the default covers over 4 s). */
+/* The bound on every wait inside the LU-SGS and BDF2 launches, in units of at
+ * least 256 ns (default 2^24, over 4 s): a wait that lasts longer gives up, the
+ * kernel latches RC_ERR_SYNC and returns, leaving the context usable.  A small limit
+ * forces the timeout path (fault tests).  In the dataflow launches some warps wait
+ * through a whole sweep, so a limit set by hand must cover the launch's duration
+ * divided by 256 ns, in every schedule and precision.  A unit is a fixed number of
+ * polls, by what is polled; the argument's name is from a unit of one poll. */
 int rc_set_wait_limit(rc_ctx* ctx, unsigned polls);
 /* Clear the latched stop conditions (after the caller has dealt with them). */
 int rc_clear_error(rc_ctx* ctx);

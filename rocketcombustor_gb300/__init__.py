@@ -384,7 +384,7 @@ class Solver:
         self._check(load().rc_set_chemistry(self._h, int(mode), float(tol), int(max_substeps)))
 
     def set_wait_limit(self, polls: int):
-        """Polls before a level wait of the persistent LU-SGS gives up (RC_ERR_SYNC)."""
+        """Units of 256 ns before a wait inside the sweeps' launches gives up (RC_ERR_SYNC)."""
         self._check(load().rc_set_wait_limit(self._h, int(polls)))
 
     def clear_error(self):

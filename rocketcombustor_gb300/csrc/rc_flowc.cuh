@@ -15,7 +15,13 @@
 //   void fence()                     orders shared memory for the block
 //   void arrive(int id, int n), void meet(int id, int n)   named barriers
 //   void latch()                     records that a wait gave up
-//   void nap()                       about 256 ns
+//   void nap()                       256 ns at least
+//
+// Waits are bounded, `limit` units of 256 ns (530 cycles at 2.07 GHz) each or a
+// little more, whatever is polled; some warps wait through a whole sweep.  The
+// units are counted in polls: 16 of a word in shared memory (59 cycles each), two
+// of a flag in memory (280 to 340), one with a nap in between (1,060).  (Read from
+// the clock instead, they cost 4 to 8 % of a mixed iteration on 120,000 cells.)
 #pragma once
 
 #ifdef __CUDACC__
@@ -26,11 +32,16 @@
 
 namespace rc {
 
+// polls of a word in shared memory, and of a flag in memory, in a unit of a limit
+constexpr unsigned WORD_POLLS = 16, FLAG_POLLS = 2;
+// n polls for each of `limit` units, at most 2^32 - 1 in all (two minutes)
+RCF_HD unsigned polls_of(unsigned limit, unsigned n) { return limit < 0xffffffffu / n ? n * limit : 0xffffffffu; }
+
 template <class L>
 struct WarpWait {
   L l;
   volatile int* bad;  // a wait of the block gave up
-  unsigned limit;     // polls
+  unsigned limit;     // units
   // lane 0's x
   RCF_HD int see(int x) { return l.lane0(x); }
   RCF_HD void give_up() {
@@ -42,13 +53,14 @@ struct WarpWait {
   }
   // Waits until *p >= v; false after a give-up of this wait or of any other.
   RCF_HD bool until(const volatile int* p, int v, bool spaced = false) {
+    const unsigned most = polls_of(limit, spaced ? 1u : WORD_POLLS);
     for (unsigned spin = 0;; ++spin) {
       const int s = see((l.load(p) >= v ? 1 : 0) | (l.load(bad) ? 2 : 0));
       if (s) {
         l.fence();
         return s == 1;
       }
-      if (spin >= limit) {
+      if (spin >= most) {
         give_up();
         return false;
       }

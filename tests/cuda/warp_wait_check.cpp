@@ -90,10 +90,14 @@ struct Lane {
     return *word(p);
   }
   void store(volatile int* p, int v) const { *word(p) = v; }
+  mutable long polls = 0;
 #ifdef PER_LANE
   int lane0(int x) const { return x; }
 #else
-  int lane0(int x) const { return B->m.come(lane, 1, x); }
+  int lane0(int x) const {
+    ++polls;
+    return B->m.come(lane, 1, x);
+  }
 #endif
   void sync() const { B->m.come(lane, 2, 0); }
   void fence() const {}
@@ -118,7 +122,7 @@ std::atomic<int> Lane::seen{0};
 
 static volatile int* raw(std::atomic<int>& a) { return reinterpret_cast<volatile int*>(&a); }
 static rc::FlowWarp<Lane> warp_of(int lane, unsigned limit) {
-  return {{{lane}, raw(B->bad), limit}, raw(B->done), raw(B->ready[0]), raw(B->go[0]), Block::NBUF};
+  return {{Lane{lane}, raw(B->bad), limit}, raw(B->done), raw(B->ready[0]), raw(B->go[0]), Block::NBUF};
 }
 static void lanes(const std::function<void(int)>& f) {
   std::vector<std::thread> t;
@@ -194,17 +198,21 @@ static void give_up_beside(int n) {
   }
 }
 
-// A wait that runs out: false in every lane, one report.
+// A wait that runs out: false in every lane, one report, and not before its
+// `limit` units of 256 ns (530 cycles) for polls of a load and a shuffle, 40
+// cycles at least.
 static void runs_out() {
   Block b;
   B = &b;
   failed = false;
   moving = false;
-  std::atomic<int> yes{0};
+  std::atomic<int> yes{0}, early{0};
   lanes([&](int l) {
-    if (warp_of(l, 3).passes_done(0)) ++yes;
+    auto w = warp_of(l, 50);
+    if (w.passes_done(0)) ++yes;
+    if (w.l.polls * 40 < 50 * 530) ++early;
   });
-  if (!failed && (yes != 0 || b.latched != 1 || b.bad != 1)) ++errors;
+  if (!failed && (yes != 0 || early != 0 || b.latched != 1 || b.bad != 1)) ++errors;
 }
 
 int main() {
