@@ -234,7 +234,11 @@ int rc_chem_substeps(rc_ctx* ctx, int* nsub);
 /* Integrate n primitive states over their own dt with the same integrator:
  * d_P and d_out are DEVICE arrays in SoA layout (component k of state i at
  * [k*n + i], NVar components), d_dt and d_nsub device arrays of n.  Runs on the
- * context's stream; stop conditions latch like the other calls. */
+ * context's stream; stop conditions latch like the other calls.  Work space, up to
+ * 200 MB, grows with the largest call and is kept until rc_finalize.  A call may
+ * be captured into a CUDA graph, of any n, after a first call outside a capture
+ * (of any n >= 1; of the captured call's n for full speed), and replayed beside
+ * later calls on the same stream. */
 int rc_chem_integrate(rc_ctx* ctx, const double* d_P, const double* d_dt, int n, double* d_out, int* d_nsub,
                       double tol, int max_substeps);
 

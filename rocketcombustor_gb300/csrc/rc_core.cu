@@ -1810,7 +1810,11 @@ int dev_zeros(rc_ctx* c, size_t n, T** out) {
 
 // Work space of the integrator's rounds for `items` states: the counters, and
 // lists for at most PARK_MAX of them (a million: 200 MB).  Lists that are too
-// short, or none where there is no memory for them, only cost speed.
+// short, or none where there is no memory for them, only cost speed; so a call
+// that is being captured takes the lists that are there, and allocates nothing.
+// A captured call holds the addresses of its lists: those that a larger call
+// outgrows stay until rc_finalize.  Lists at least double, so all of them together
+// are at most twice the largest.
 constexpr int PARK_MAX = 1 << 20;
 int park_space(rc_ctx* c, int items, ChemPark* p) {
   if (!p->count)
@@ -1819,24 +1823,22 @@ int park_space(rc_ctx* c, int items, ChemPark* p) {
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
   const int cap = std::min(items, PARK_MAX);
   if (cap <= p->cap || items <= 128 * nsm) return RC_OK;  // few items run in one round
-  if (p->cap) {
-    RC_CU(cudaStreamSynchronize(c->stream));
-    for (void* q : {(void*)p->x, (void*)p->k}) {
-      c->allocs.erase(std::find(c->allocs.begin(), c->allocs.end(), q));
-      cudaFree(q);
-    }
-    p->cap = 0;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(c->stream, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return RC_OK;
   }
+  const int size = std::min(PARK_MAX, std::max(cap, 2 * p->cap));
   void *x = nullptr, *k = nullptr;
-  if (cudaMalloc(&x, sizeof(double) * 2 * CHEM_PARK_X * (size_t)cap) != cudaSuccess ||
-      cudaMalloc(&k, sizeof(int) * 2 * CHEM_PARK_K * (size_t)cap) != cudaSuccess) {
+  if (cudaMalloc(&x, sizeof(double) * 2 * CHEM_PARK_X * (size_t)size) != cudaSuccess ||
+      cudaMalloc(&k, sizeof(int) * 2 * CHEM_PARK_K * (size_t)size) != cudaSuccess) {
     cudaGetLastError();
     if (x) cudaFree(x);
     return RC_OK;
   }
   c->allocs.push_back(x);
   c->allocs.push_back(k);
-  *p = {static_cast<double*>(x), static_cast<int*>(k), p->count, cap, 1, false};
+  *p = {static_cast<double*>(x), static_cast<int*>(k), p->count, size, 1, false};
   return RC_OK;
 }
 
