@@ -80,10 +80,10 @@ __device__ __forceinline__ void run_queue(const ThermoDev<NSP>& th, int n, const
                                           int maxsub, unsigned& err, Begin begin, End end) {
   const int lane = threadIdx.x & 31;
   const Parked<NSP, N> from(park, (round + 1) & 1), to(park, round & 1);
-  const bool final = round + 1 >= park.rounds;
-  const int limit = final ? 0x7fffffff : park_at(round);
   if (round > 0) n = (int)min(park.count[CHEM_ROUNDS + round - 1], (unsigned)park.cap);
   const int lanes = gridDim.x * CHEM_THREADS;
+  const bool final = round + 1 >= park.rounds || (park.listed && n <= lanes);
+  const int limit = final ? 0x7fffffff : park_at(round);
   Reactor<NSP, N> r;
   int item = -1;        // the lane's item, -1 when idle
   bool more = true;     // the queue may hold more (warp-uniform)
@@ -293,13 +293,21 @@ static int chem_grid(K kernel, int items, int* nsm) {
 // sub-partition has nothing to gain from full lanes).  Items that come sorted,
 // the longest of the last iteration first, need few: the last ones to start are
 // short (64 cases, a million cells, five iterations: 139.3 ms in one round, 137.5
-// in four, 140.7 in ten with the cut; unsorted states: 113, 101 and 74 ms).
+// in four, 140.7 in ten with the cut; unsorted states: 113, 101 and 74 ms).  How
+// many items a list on the device holds is known there only, and often there are
+// none: it goes in three rounds, and a round that has no more items than the
+// launch has lanes ends with them (an iteration with the surrogate and all cells
+// in the list, one / two / three / ten rounds, ms: 30,000 cells 11.30 / 11.52 / 11.32 /
+// 11.75; 120,000 15.19 / 15.42 / 15.22 / 15.57; 600,000 51.98 / 50.07 / 49.20 / 49.25).
+enum ChemItems { CHEM_UNSORTED, CHEM_SORTED, CHEM_LISTED };
 template <class K, class Launch>
-static int chem_rounds(K kernel, int items, bool sorted, ChemPark park, cudaStream_t s, Launch launch) {
+static int chem_rounds(K kernel, int items, ChemItems kind, ChemPark park, cudaStream_t s, Launch launch) {
   int nsm = 0;
   const int grid = chem_grid(kernel, items, &nsm);
-  park.rounds = park.cap == 0 || items <= nsm * CHEM_THREADS ? 1 : sorted ? 4 : CHEM_ROUNDS;
-  park.cut = !sorted;
+  park.rounds = kind == CHEM_SORTED ? 4 : kind == CHEM_LISTED ? 3 : CHEM_ROUNDS;
+  if (park.cap == 0 || items <= nsm * CHEM_THREADS) park.rounds = 1;
+  park.cut = kind != CHEM_SORTED;
+  park.listed = kind == CHEM_LISTED;
   cudaMemsetAsync(park.count, 0, sizeof(unsigned) * 2 * CHEM_ROUNDS, s);
   for (int round = 0; round < park.rounds; ++round) launch(grid, park, round);
   return park.rounds;
@@ -317,16 +325,17 @@ int chem_source(const Dev& d, const void* th, double tol, int maxsub, int* nsub,
     k_chem_scatter<<<nb, NBUCKET, 0, s>>>(nsub, d.NE, hist, order);
   }
   auto k = k_chem_source<NSP, ChemNum>;
-  return (order ? 3 : 0) + chem_rounds(k, d.NE, order != nullptr, park, s, [&](int grid, const ChemPark& p, int round) {
+  auto launch = [&](int grid, const ChemPark& p, int round) {
     k<<<grid, CHEM_THREADS, 0, s>>>(d, *static_cast<const ThermoDev<NSP>*>(th), tol, maxsub, nsub, order, p, round);
-  });
+  };
+  return (order ? 3 : 0) + chem_rounds(k, d.NE, order ? CHEM_SORTED : CHEM_UNSORTED, park, s, launch);
 }
 
 template <int NSP>
 int chem_list(const Dev& d, const void* th, double tol, int maxsub, int* nsub, const int* list, const unsigned* nlist,
               const ChemPark& park, cudaStream_t s) {
   auto k = k_chem_list<NSP, ChemNum>;
-  return chem_rounds(k, d.NE, false, park, s, [&](int grid, const ChemPark& p, int round) {
+  return chem_rounds(k, d.NE, CHEM_LISTED, park, s, [&](int grid, const ChemPark& p, int round) {
     k<<<grid, CHEM_THREADS, 0, s>>>(d, *static_cast<const ThermoDev<NSP>*>(th), tol, maxsub, nsub, list, nlist, p,
                                     round);
   });
@@ -336,7 +345,7 @@ template <int NSP>
 int chem_batch(const void* th, const double* P, const double* dt, int n, double* out, int* nsub, double tol,
                int maxsub, const ChemPark& park, unsigned* errp, cudaStream_t s) {
   auto k = k_chem_batch<NSP, ChemNum>;
-  return chem_rounds(k, n, false, park, s, [&](int grid, const ChemPark& p, int round) {
+  return chem_rounds(k, n, CHEM_UNSORTED, park, s, [&](int grid, const ChemPark& p, int round) {
     k<<<grid, CHEM_THREADS, 0, s>>>(*static_cast<const ThermoDev<NSP>*>(th), P, dt, n, out, nsub, tol, maxsub, p,
                                     round, errp);
   });
