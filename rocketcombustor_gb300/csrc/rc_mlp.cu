@@ -1180,31 +1180,47 @@ int alloc_work(rc_mlp* m, size_t count, T** out) {
 
 // split-K slices of the hidden weight-gradient GEMMs, at most
 constexpr int ZSPLIT_MAX = 64;
-int ensure_work(rc_mlp* m, int n) {
-  if (n <= m->cap) return RC_OK;
+void drop_work(rc_mlp* m) {
   for (void* p : m->work) cudaFree(p);
   m->work.clear();
+  m->cap = 0;
+}
+int alloc_all(rc_mlp* m, int n) {
   const size_t N = (size_t)n, Hh = mlp::H;
-  int st = 0;
-  st |= alloc_work(m, N * mlp::NIN, &m->xn);
-  for (int l = 0; l < 4; ++l) st |= alloc_work(m, N * Hh, &m->Hs[l]);
+  int st = RC_OK;
+  auto get = [&](size_t count, auto** out) {
+    if (!st) st = alloc_work(m, count, out);
+  };
+  get(N * mlp::NIN, &m->xn);
+  for (int l = 0; l < 4; ++l) get(N * Hh, &m->Hs[l]);
   for (int l = 0; l < 3; ++l) {
-    st |= alloc_work(m, N * Hh, &m->Acol[l]);
-    st |= alloc_work(m, N * Hh, &m->dHcol[l + 1]);
+    get(N * Hh, &m->Acol[l]);
+    get(N * Hh, &m->dHcol[l + 1]);
   }
-  st |= alloc_work(m, N * Hh, &m->Arow);
-  for (int l = 0; l < 4; ++l) st |= alloc_work(m, N * Hh, &m->dHrow[l]);
-  st |= alloc_work(m, N * mlp::NOUT, &m->dy);
-  st |= alloc_work(m, (N + mlp::HEAD_SAMPLES - 1) / mlp::HEAD_SAMPLES, &m->loss_part);
-  st |= alloc_work(m, (size_t)1, &m->loss);
-  st |= alloc_work(m, N * mlp::NOUT, &m->tb);
-  st |= alloc_work(m, (size_t)4, &m->sched);
-  st |= alloc_work(m, (size_t)1, &m->it);
-  // split-K partials of the weight gradients, for up to n / 1024 splits
+  get(N * Hh, &m->Arow);
+  for (int l = 0; l < 4; ++l) get(N * Hh, &m->dHrow[l]);
+  get(N * mlp::NOUT, &m->dy);
+  get((N + mlp::HEAD_SAMPLES - 1) / mlp::HEAD_SAMPLES, &m->loss_part);
+  get((size_t)1, &m->loss);
+  get(N * mlp::NOUT, &m->tb);
+  get((size_t)4, &m->sched);
+  get((size_t)1, &m->it);
+  // split-K partials of the weight gradients, for up to n / 256 splits
   m->zsplit = std::max(1, std::min(ZSPLIT_MAX, n / 256));
-  st |= alloc_work(m, (size_t)3 * m->zsplit * Hh * Hh, &m->part);
-  st |= alloc_work(m, (size_t)mlp::SMALL_ZMAX * mlp::SMALL_N, &m->spart);
-  if (st) return st;
+  get((size_t)3 * m->zsplit * Hh * Hh, &m->part);
+  get((size_t)mlp::SMALL_ZMAX * mlp::SMALL_N, &m->spart);
+  return st;
+}
+// Work buffers for n samples.  Where there is no memory for them nothing is left,
+// neither buffers nor an error, and the next call allocates its own.
+int ensure_work(rc_mlp* m, int n) {
+  if (n <= m->cap) return RC_OK;
+  drop_work(m);
+  if (int st = alloc_all(m, n)) {
+    drop_work(m);
+    cudaGetLastError();
+    return st;
+  }
   m->cap = n;
   return RC_OK;
 }
