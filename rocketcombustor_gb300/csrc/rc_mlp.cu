@@ -1509,10 +1509,15 @@ int rc_mlp_train(rc_mlp* m, const float* d_x, const float* d_t, long long n, int
     e = e2 != cudaSuccess ? e2 : cudaGetLastError();
   }
   if (e == cudaSuccess && st == RC_OK) e = cudaGraphInstantiate(&ge, g, 0);
-  for (int k = 0; e == cudaSuccess && st == RC_OK && k < steps; ++k) e = cudaGraphLaunch(ge, s);
-  if (e == cudaSuccess && st == RC_OK) {
+  int launched = 0;
+  while (e == cudaSuccess && st == RC_OK && launched < steps)
+    if ((e = cudaGraphLaunch(ge, s)) == cudaSuccess) ++launched;
+  // the inference kernel's weights follow the steps that were launched, also if
+  // a later launch failed
+  if (launched) {
     k_pack16<<<(PACK16_N + 255) / 256, 256, 0, s>>>(m->params, m->Wh);
-    e = cudaGetLastError();
+    const cudaError_t e2 = cudaGetLastError();
+    if (e == cudaSuccess) e = e2;
   }
   unsigned derr = 0;
   if (e == cudaSuccess && st == RC_OK) e = cudaMemcpyAsync(&derr, m->derr, sizeof(unsigned), cudaMemcpyDeviceToHost, s);
