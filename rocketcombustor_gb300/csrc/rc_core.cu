@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(128) k_cell(const Dev d, const ThermoDev<NSP> 
     d.step[i] = val(st);
     const N ddv = dsum + N(vol) / st;
     d.dd[i] = val(ddv);
-    const Recip rd = recip(ddv);
+    const Recip rd = recip_of(ddv);
     d.rcp[4 * NE + i] = rd.h;
     d.rcp[5 * NE + i] = rd.l;
   }
@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(128) k_cell(const Dev d, const ThermoDev<NSP> 
   d.cst[0 * NE + i] = val(rr);
   d.cst[1 * NE + i] = val(gama);
   {
-    const Recip a = recip(rr), b = recip(gama - 1.0);
+    const Recip a = recip_of(rr), b = recip_of(gama - 1.0);
     d.rcp[0 * NE + i] = a.h; d.rcp[1 * NE + i] = a.l; d.rcp[2 * NE + i] = b.h; d.rcp[3 * NE + i] = b.l;
   }
   d.cst[2 * NE + i] = val(rr * (hh + half_of(P[1] * P[1] + P[2] * P[2])) - P[0]);

@@ -32,10 +32,11 @@ __device__ __forceinline__ bool div_rn_safe(double a, double b) {
 struct Recip {
   double h, l;
 };
-__device__ __forceinline__ Recip recip_of(double b) {
-  const double h = 1.0 / b;
-  const double e = fma(-b, h, 1.0);
-  return {h, e * h};
+__device__ __forceinline__ double val(double x) { return x; }
+template <class N>  // double or Num (rc_num.cuh)
+__device__ __forceinline__ Recip recip_of(N b) {
+  const N h = 1.0 / b;
+  return {val(h), val(N(fma(-val(b), val(h), 1.0)) * h)};
 }
 // a / b, given recip_of(b) = {yh, yl} (b finite and non-zero)
 __device__ __forceinline__ double div_rn(double a, double b, double yh, double yl) {

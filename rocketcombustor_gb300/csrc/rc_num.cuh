@@ -9,9 +9,7 @@
 namespace rc {
 
 // The operations that double and Num spell differently.
-__device__ __forceinline__ double val(double x) { return x; }
 __device__ __forceinline__ double n_abs(double x) { return fabs(x); }
-__device__ __forceinline__ double n_sqrt(double x) { return sqrt(x); }
 __device__ __forceinline__ double n_exp(double x) { return rcm::exp(x); }
 __device__ __forceinline__ double n_log(double x) { return rcm::log(x); }
 __device__ __forceinline__ double n_pow(double x, double y, double logx) {
@@ -52,10 +50,4 @@ __device__ __forceinline__ Num<M> div_fixed(Num<M> a, Num<M> b, unsigned V) { re
 // x < 0.0
 template <class N>
 __device__ __forceinline__ bool negative(N x) { return less(val(x), 0.0); }
-// the reciprocal pair of b, to be stored
-template <class N>
-__device__ __forceinline__ Recip recip(N b) {
-  const N h = 1.0 / b;
-  return {val(h), val(N(fma(-val(b), val(h), 1.0)) * h)};
-}
 }  // namespace rc
