@@ -33,6 +33,10 @@ using ChemNum = Num<false>;
 // parked as they are, at the end of the list, and since a list is taken from its
 // end, they go first in the next round.  The last round ends with its items.
 // Where the list is full the items stay in their lanes.  The same states: 74 ms.
+// One / two / four / ten rounds, ms: tolerance 0.05, 65,536 states 7.7 / 6.1 / 6.2 /
+// 6.2, 262,144 17.2 / 13.8 / 13.7 / 13.7; 0.005, 30,000 34.5 / 27.9 / 27.9 / 28.0,
+// 131,072 57.8 / 55.2 / 55.2 / 50.8.  The kernels spill 434-462 bytes at the 168
+// registers that three blocks per SM leave a thread.
 //   begin(item, r)  loads item into reactor r; false when it needs no attempt
 //   end(item, r)    stores the finished item
 constexpr int REFILL = 4;
@@ -75,14 +79,15 @@ struct Parked {
 // Round 0 takes the items 0 .. n-1, a later round the list of the one before;
 // the first 32 of a warp are its own (so that few items spread over the blocks
 // in order), the others come from the round's counter.
-template <int NSP, class N, class Begin, class End>
+// LISTED: a round with at most one item per lane is the last.
+template <int NSP, class N, bool LISTED, class Begin, class End>
 __device__ __forceinline__ void run_queue(const ThermoDev<NSP>& th, int n, const ChemPark& park, int round, double tol,
                                           int maxsub, unsigned& err, Begin begin, End end) {
   const int lane = threadIdx.x & 31;
   const Parked<NSP, N> from(park, (round + 1) & 1), to(park, round & 1);
   if (round > 0) n = (int)min(park.count[CHEM_ROUNDS + round - 1], (unsigned)park.cap);
   const int lanes = gridDim.x * CHEM_THREADS;
-  const bool final = round + 1 >= park.rounds || (park.listed && n <= lanes);
+  const bool final = round + 1 >= park.rounds || (LISTED && n <= lanes);
   const int limit = final ? 0x7fffffff : park_at(round);
   Reactor<NSP, N> r;
   int item = -1;        // the lane's item, -1 when idle
@@ -138,13 +143,13 @@ __device__ __forceinline__ void run_queue(const ThermoDev<NSP>& th, int n, const
 // Integrated source of cell i (sourceterm.f90:43-51 with omega replaced by
 // the mean rate over the cell's pseudo time step):
 //   src_k = vol * (rho * ((Y_k(step) - Y_k) / step)), with the reactor's rho = p / (R_mix T).
-template <int NSP, class N, class Cell>
+template <int NSP, class N, bool LISTED, class Cell>
 __device__ __forceinline__ void run_cells(const Dev& d, const ThermoDev<NSP>& th, int n, Cell cell, double tol,
                                           int maxsub, int* nsub, const ChemPark& park, int round) {
   constexpr int V = 3 + NSP;
   const int NE = d.NE;
   unsigned err = 0;
-  run_queue<NSP, N>(
+  run_queue<NSP, N, LISTED>(
       th, n, park, round, tol, maxsub, err,
       [&](int q, Reactor<NSP, N>& r) {
         const int i = cell(q);
@@ -170,7 +175,7 @@ template <int NSP, class N>
 __global__ void __launch_bounds__(CHEM_THREADS, 3) k_chem_source(const Dev d, const ThermoDev<NSP> th, double tol,
                                                               int maxsub, int* __restrict__ nsub,
                                                               const int* __restrict__ order, const ChemPark park, int round) {
-  run_cells<NSP, N>(d, th, d.NE, [&](int q) { return order ? order[q] : q; }, tol, maxsub, nsub, park, round);
+  run_cells<NSP, N, false>(d, th, d.NE, [&](int q) { return order ? order[q] : q; }, tol, maxsub, nsub, park, round);
 }
 
 // Counting sort of the cells by their previous substep count, descending
@@ -249,7 +254,7 @@ __global__ void __launch_bounds__(CHEM_THREADS, 3) k_chem_list(const Dev d, cons
                                                             const int* __restrict__ list,
                                                             const unsigned* __restrict__ nlist, const ChemPark park,
                                                             int round) {
-  run_cells<NSP, N>(d, th, (int)min(*nlist, (unsigned)d.NE), [&](int q) { return list[q]; }, tol, maxsub, nsub,
+  run_cells<NSP, N, true>(d, th, (int)min(*nlist, (unsigned)d.NE), [&](int q) { return list[q]; }, tol, maxsub, nsub,
                     park, round);
 }
 
@@ -262,7 +267,7 @@ __global__ void __launch_bounds__(CHEM_THREADS, 3) k_chem_batch(const ThermoDev<
                                                              int round, unsigned* errp) {
   constexpr int V = 3 + NSP;
   unsigned err = 0;
-  run_queue<NSP, N>(
+  run_queue<NSP, N, false>(
       th, n, park, round, tol, maxsub, err,
       [&](int i, Reactor<NSP, N>& r) {
 #pragma unroll
@@ -307,7 +312,6 @@ static int chem_rounds(K kernel, int items, ChemItems kind, ChemPark park, cudaS
   park.rounds = kind == CHEM_SORTED ? 4 : kind == CHEM_LISTED ? 3 : CHEM_ROUNDS;
   if (park.cap == 0 || items <= nsm * CHEM_THREADS) park.rounds = 1;
   park.cut = kind != CHEM_SORTED;
-  park.listed = kind == CHEM_LISTED;
   cudaMemsetAsync(park.count, 0, sizeof(unsigned) * 2 * CHEM_ROUNDS, s);
   for (int round = 0; round < park.rounds; ++round) launch(grid, park, round);
   return park.rounds;

@@ -1839,7 +1839,7 @@ int park_space(rc_ctx* c, int items, ChemPark* p) {
   }
   c->allocs.push_back(x);
   c->allocs.push_back(k);
-  *p = {static_cast<double*>(x), static_cast<int*>(k), p->count, size, 1, false, false};
+  *p = {static_cast<double*>(x), static_cast<int*>(k), p->count, size, 1, false};
   return RC_OK;
 }
 

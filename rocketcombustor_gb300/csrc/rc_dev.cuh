@@ -233,7 +233,6 @@ struct ChemPark {
   int cap;          // places in a list (0: nothing can be parked)
   int rounds;       // of this launch
   bool cut;         // a round ends when its queue is empty
-  bool listed;      // a round with at most one item per lane is the last
 };
 // Tables of the dataflow LU-SGS: cells are split into per-SM blocks, a pass is
 // a run of consecutive sweep positions of one level whose cells one block owns
