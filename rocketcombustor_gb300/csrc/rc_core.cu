@@ -1410,7 +1410,7 @@ __global__ void __launch_bounds__(flowc_threads(G), 1) k_lusgs_flowc(const Dev d
   const int nf = f.boff[0][b + 1] - f0, n = nf + (f.boff[1][b + 1] - b0);
   // the block's k-th pass in the tables
   auto at = [&](int k) { return k < nf ? f0 + k : f.nfwd + b0 + k - nf; };
-  FlowWarp<FlowLane> w = {{{lane, d.err}, &s_bad, d.spin_limit}, &s_done, s_ready, s_go, FLOWC_NBUF};
+  FlowWarp<FlowLane<false>> w = {{{lane, d.err}, &s_bad, d.spin_limit}, &s_done, s_ready, s_go, FLOWC_NBUF};
   if (warp < CW) {
     const int gi = G > 1 ? warp >> 3 : 0, role = warp & 7;
     for (int k = 0; k < n; ++k) {

@@ -209,7 +209,9 @@ __device__ __forceinline__ void bar_arrive(int id, int count) {
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(count) : "memory");
 }
 // A lane of the dataflow launches' waits (rc_flowc.cuh).
+template <bool COLD>
 struct FlowLane {
+  static constexpr bool cold = COLD;
   int lane;
   unsigned* err;
   __device__ __forceinline__ int load(const volatile int* p) const { return *p; }

@@ -10,6 +10,11 @@
 // L is one lane and its primitives (FlowLane in rc_dev.cuh; the tests run the
 // same code on processor threads):
 //   int lane                         its number
+//   static constexpr bool cold       give_up is a call.  The mixed launches run the
+//                                    Newton update's code beside the passes' and
+//                                    want the waits short (120,000 cells, ten
+//                                    iterations 9.67 -> 9.55 ms), the FP64 ones do
+//                                    not (20,000 cells 5.38, as a call 5.40)
 //   int load(const volatile int*), void store(volatile int*, int)
 //   int lane0(int x)                 lane 0's x; void sync(): the warp meets
 //   void fence()                     orders shared memory for the block
@@ -26,8 +31,10 @@
 
 #ifdef __CUDACC__
 #define RCF_HD __device__ __forceinline__
+#define RCF_COLD __device__ __noinline__
 #else
 #define RCF_HD inline
+#define RCF_COLD inline
 #endif
 
 namespace rc {
@@ -45,6 +52,11 @@ struct WarpWait {
   // lane 0's x
   RCF_HD int see(int x) { return l.lane0(x); }
   RCF_HD void give_up() {
+    if (L::cold) give_up_cold();
+    else give_up_here();
+  }
+  RCF_COLD void give_up_cold() { give_up_here(); }
+  RCF_HD void give_up_here() {
     if (l.lane == 0) {
       l.store(bad, 1);
       l.latch();

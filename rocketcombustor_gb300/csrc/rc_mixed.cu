@@ -758,7 +758,7 @@ __global__ void __launch_bounds__(FLOW32_THREADS, 1) k_lusgs_flow32(const Dev d,
   const int f0 = f.boff[0][b], b0 = f.boff[1][b];
   const int nf = f.boff[0][b + 1] - f0, n = nf + (f.boff[1][b + 1] - b0);
   auto pass_of = [&](int k) { return k < nf ? f.blist[0][f0 + k] : f.blist[1][b0 + k - nf]; };
-  WarpWait<FlowLane> w = {{lane, d.err}, &s_bad, d.spin_limit};
+  WarpWait<FlowLane<true>> w = {{lane, d.err}, &s_bad, d.spin_limit};
   if (warp == 1) {
     for (int k = 0; k < n; ++k) {
       // pass k reuses the buffer of pass k - NBUF once warp 0 has taken it
@@ -1022,7 +1022,7 @@ __global__ void __launch_bounds__(flowc32_threads(G), 1) k_lusgs_flowc32(const D
   const int nf = f.boff[0][b + 1] - f0, n = nf + (f.boff[1][b + 1] - b0);
   // the block's k-th pass in the tables
   auto at = [&](int k) { return k < nf ? f0 + k : f.nfwd + b0 + k - nf; };
-  FlowWarp<FlowLane> w = {{{lane, d.err}, &s_bad, d.spin_limit}, &s_done, s_ready, s_go, FLOWC32_NBUF};
+  FlowWarp<FlowLane<true>> w = {{{lane, d.err}, &s_bad, d.spin_limit}, &s_done, s_ready, s_go, FLOWC32_NBUF};
   if (warp < CW) {
     const int gi = G > 1 ? warp >> 2 : 0, role = warp & 3, x = role * 32 + lane, fc = x / V, r = x - fc * V;
     float(*T)[32] = s_T[gi];

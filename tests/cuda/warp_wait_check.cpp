@@ -75,6 +75,7 @@ static Block* B;
 static std::atomic<bool> moving{false};  // the words are about to move
 
 struct Lane {
+  static constexpr bool cold = false;
   int lane;
   static std::atomic<int>* word(const volatile int* p) {
     return reinterpret_cast<std::atomic<int>*>(const_cast<int*>(p));
