@@ -177,6 +177,9 @@ int rc_lusgs_stage(rc_ctx* ctx, int istep); /* lu_sgs_stage   Time_LUSGS_steady.
 /* Switch the precision of the following calls: RC_PREC_FP64 on any context,
  * RC_PREC_MIXED / RC_PREC_MIXED_DC on contexts created with a mixed mode.  A
  * driver switches MIXED -> MIXED_DC when the FP32 residual stops decreasing.
+ * The LU-SGS schedule and its blocks stay those that rc_init chose for its
+ * precision or rc_autotune for the present one: the results do not depend on them,
+ * the speed does.
  * No counterpart in the reference (it has a single FP64 path). */
 int rc_set_precision(rc_ctx* ctx, int precision);
 

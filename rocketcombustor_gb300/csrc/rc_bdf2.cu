@@ -773,14 +773,14 @@ struct BStage {
   BRow<NSP> rw;
   BTail t;
 };
-// A pass is one chain: per cell, of about 24,000 cycles, the record 2,500, the
-// terms with the neighbours' increments from L2 4,200, each solve 4,500, each
-// check of the backward error 3,300, of which a quarter was the hardware's
-// division for zero residuals and finished cells (berr_bits).  An inner
+// A pass is one chain: per cell, of about 22,000 cycles, the record 2,500, the
+// terms with the neighbours' increments from L2 4,200, the solve 6,600, a check of
+// the backward error 2,700 (3,300 with the hardware's division for zero residuals
+// and finished cells, see berr_bits), the correction's solve 4,500.  An inner
 // iteration on 120,000 cells: 10.2 -> 8.6 ms with that, the divisions by shared
 // reciprocals and the records by word.
 // A pass of at most four cells runs on both compute warps split by rows
-// (bdf2_cell_step PART 1 and 2), otherwise four cells on each (PART 0).
+// (bdf2_cell_step, part 1 and 2), otherwise four cells on each (part 0).
 constexpr int BFLOW_THREADS = 160, BFLOW_NB = 96;  // all five warps; a role pair and the coordinator
 template <int NSP>
 constexpr int bflow_smem() { return (int)(2 * 2 * 32 * sizeof(BStage<NSP>)); }

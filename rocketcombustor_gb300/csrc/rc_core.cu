@@ -2043,15 +2043,21 @@ inline long flowc_length(int NE, int G, const SweepOrder& so, const std::vector<
   }
   return sum;
 }
-// Blocks of the compact plan of one group per pass: the fewest, in steps of
-// 15 % from one per SM, that lengthen no level's passes.  A pass costs the same
-// for one cell as for a full group, and every block boundary that the sweep
-// crosses costs a publication, a poll and a fetch through L2 (about 3,000
-// cycles), so small meshes run on few SMs: 720 cells 0.74 -> 0.54 ms per FP64
-// iteration, 0.42 -> 0.23 mixed (152 -> 6 blocks); 120,000 cells 2.49 -> 2.33 FP64
-// (36 blocks; 28, with two passes in some levels, 3.18).  In the mixed forms at
-// most about 6.5 cells of a level per block: their blocks also run the Newton
-// update (120,000 cells: 152 blocks 1.10, 64 1.00, 36 1.08 ms).
+// Blocks of the compact plan of one group per pass: of the numbers tried, one per
+// SM and 15 % fewer each time until two have been too few, the smallest whose
+// flowc_length is not above that of one block per SM (a sum over the levels: one
+// may grow where another shrinks).  A pass costs the same for one cell as for a full
+// group, and every block boundary that the sweep crosses costs a publication, a poll
+// and a fetch through L2 (about 3,000 cycles), so small meshes run on few SMs.  In
+// the mixed forms at most about 6.5 cells of a level per block: their blocks also
+// run the Newton update.  Us per iteration, nozzles in the reference's cell order,
+// chosen blocks / one per SM / best of eleven numbers tried: 1,440 cells FP64 318 (4
+// blocks) / 364 / 318, mixed 155 (6) / 181 / 155; 20,000 876 (13) / 1,064 / 876 and
+// 426 (21) / 599 / 426; 42,000 1,137 (21) / 1,276 / 1,137 and 545 (36) / 658 / 545;
+// 120,000 2,229 (35) / 2,394 / 2,229 and 925 (62) / 1,054 / 925; 300,000 3,975 (57)
+// / 4,258 / 3,975 and 1,517 (103) / 1,711 / 1,493; 600,000 6,550 (93) / 6,746 / 6,550
+// and 2,283 (152) / 2,285 / 2,259.  Fewer blocks than a level's passes need cost a third
+// more (120,000 cells on 26 blocks: 3,069 and 1,311).
 template <class NF>
 int flowc_blocks(int NE, int nsm, bool mixed, const NF& nface, const std::vector<int>& cother, const SweepOrder& so,
                  int cap) {
@@ -3018,9 +3024,13 @@ int init_impl(const rc_mesh* m, const rc_thermo* t, const rc_config* g, const Ba
     // / 2.55 / 3.57 (four warps), mixed 1.00 / 1.12 / 1.44; 64 cases (32 cells)
     // FP64 31.0 / 30.6 / 32.4; 120,000 cells in random order (11 levels, 72
     // cells) FP64 1.50 / 1.41 / 1.33, mixed 0.52 / 0.51 / 0.34; 12,000 cells in 10
-    // levels mixed 0.17 / 0.17 / 0.12, FP64 0.33 / 0.33 / 0.34.  Where the
-    // dataflow launch cannot run: the four-warp per-level sweeps for FP64, the
-    // per-level sweeps for the mixed forms.
+    // levels mixed 0.17 / 0.17 / 0.12, FP64 0.33 / 0.33 / 0.34; mixed, us, random order:
+    // 800 cells in 7 levels 96 / 95 / 78, 4,000 in 9 120 / 114 / 84, 300,000 in 13 1,021 /
+    // 1,013 / 605; in the reference's order 128 cells in 13 levels 91 / 117 / 90, 288 in
+    // 19 105 / 124 / 109, 1,152 in 37 150 / 175 / 170.  Where the dataflow launch cannot
+    // run: the four-warp per-level sweeps for FP64, the per-level sweeps for the mixed
+    // forms.  Blocks and schedule are chosen for the precision given to rc_init and stay
+    // after rc_set_precision (the same results).
     const double per_sm = (double)NE / (std::max<size_t>(c->fwd_off.size(), 2) - 1) / std::max(nsm, 1);
     const double group = flowc_cells(c->V);
     const bool few = g->precision != RC_PREC_FP64 && c->fwd_off.size() - 1 <= 16;

@@ -11,7 +11,11 @@
 // 278, 608 / 302: only division and square root gain there.  An addition done
 // this way takes 102 cycles and stays on the FP64 unit.
 //
-// Methods: significands as 53-bit integers.  Multiplication: the 106-bit
+// Methods (software floating point on integers as in J.-M. Muller et al., Handbook
+// of Floating-Point Arithmetic, Birkhaeuser 2010, chapter 10; quotient digits
+// from a truncated reciprocal and a correction, N. Moeller and T. Granlund,
+// "Improved division by invariant integers", IEEE Trans. Computers 60(2), 2011):
+// significands as 53-bit integers.  Multiplication: the 106-bit
 // product from four 32 x 32 products, normalised and rounded on the bits
 // below.  Division: digit by digit with a 32-bit reciprocal (hardware FP32
 // reciprocal and one Newton step in integers, kept below the true value), two
