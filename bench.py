@@ -59,8 +59,8 @@ def algo_bytes_per_cell(V: int, nf_ne: float, viscous: bool, combustion: bool) -
 # dram__bytes_write.sum and sm__inst_executed_pipe_fp64.sum over the
 # subroutine's launches, divided by the cells: profiles/c4_500k_fp64_counters.md).
 # Both grow with the cells.
-NCU_DRAM_PER_CELL = {"timestep": 197.8, "reconstruction": 331.5, "flux_sourceterm": 653.6,
-                     "lu_sgs_steady": 586.2}
+NCU_DRAM_PER_CELL = {"timestep": 197.5, "reconstruction": 331.7, "flux_sourceterm": 653.4,
+                     "lu_sgs_steady": 583.3}
 NCU_FP64_INST_PER_CELL = {"timestep": 11.72, "reconstruction": 16.02, "flux_sourceterm": 56.48,
                           "lu_sgs_steady": 31.00}
 NCU_TRAFFIC_SOURCE = ("ncu capture of one FP64 iteration of the same physics at 500,000 cells (compact dataflow "
