@@ -20,12 +20,18 @@
 
 using Clock = std::chrono::steady_clock;
 struct Mismatch {};
+// how long lanes wait for one another: with PER_LANE some never come
+#ifdef PER_LANE
+constexpr std::chrono::seconds PATIENCE(3);
+#else
+constexpr std::chrono::seconds PATIENCE(60);
+#endif
 static std::atomic<bool> failed{false};
 static long mismatches = 0, errors = 0;
 
-// until f(), at most five seconds; false then
+// until f(), at most PATIENCE; false then
 static bool soon(const std::function<bool()>& f) {
-  const auto end = Clock::now() + std::chrono::seconds(5);
+  const auto end = Clock::now() + PATIENCE;
   while (!f()) {
     if (failed || Clock::now() > end) return false;
     std::this_thread::yield();
@@ -51,7 +57,7 @@ struct Meeting {
       ++round;
     }
     if (failed || round != r) cv.notify_all();
-    if (!cv.wait_for(lock, std::chrono::seconds(5), [&] { return failed || round != r; })) {
+    if (!cv.wait_for(lock, PATIENCE, [&] { return failed || round != r; })) {
       failed = true;
       cv.notify_all();
     }
